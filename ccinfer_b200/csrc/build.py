@@ -68,6 +68,7 @@ GROUPS = {
         "scalar_memory.cu",
         "memory_chunks.cu",
         "delta_rule.cu",
+        "chunk_recurrence.cu",
         "delta_head.cu",
         "linear_attention.cu",
         "ssm.cu",

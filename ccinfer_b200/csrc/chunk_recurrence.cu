@@ -1,0 +1,625 @@
+// The gated recurrences of csrc/delta_rule.cu over portions of prompts, in chunks of 64 tokens on tensor cores:
+//
+//   S <- diag(g_t) S;  u_t = beta_t (v_t - S^T k_t);  S <- S + k_t u_t^T;  o_t = S^T q_t        (delta rule)
+//   S <- diag(g_t) S + k_t v_t^T;                     o_t = S^T q_t                              (without: u = v)
+//
+// with one decay per key channel or one per head.  With c_t the sum of log g over the chunk up to t (per channel), S0
+// the memory before the chunk and x . y over key channels,
+//
+//   M_ts = (k_t e^{c_t - c_s}) . k_s,   P_ts = (q_t e^{c_t - c_s}) . k_s
+//   (I + strictly_lower(diag(beta) M)) [W | U] = diag(beta) [K e^c | V]
+//   u = U - W S0;   o = (Q e^c) S0 + lower(P) u;   S = e^{c_64} S0 + (K e^{c_64 - c})^T u
+//
+// so only the last line walks the chunks in order; everything before it is independent of the memory.  Two kernels:
+//
+//   chunk_prepare  a block per (chunk, head): the sums of logarithms, M and P, the triangular solve (a thread a column,
+//                  its 64 values in registers, float multiply-adds), and the scaled rows of q and k
+//   chunk_walk     a block per (request, head, 32 value columns), eight warps: the memory in float registers, four
+//                  products a chunk on mma.sync; a warp takes 16 rows x 16 columns of u and o and 16 key channels of S
+//
+// Exponents of decays are never positive: within a run of 16 tokens every pair's decay is taken per channel as it is, and
+// between runs both factors refer to a place between them.  Logarithms are summed within a run and runs are added up, so
+// that a difference never cancels more than a run's sum.  What the model computes in 32 bits stays so to about 2^-17:
+// logarithms, sums, exponentials, the solve and the memory are float, and every operand of a product (rows, scores,
+// memory) goes in as TWO bfloat16, its rounding and what the rounding left, in three products.  A decay below 2^-115
+// counts as that: it keeps nothing that a float can tell from zero.
+//
+// Bound by: the walk by the chain of its products (one block an SM), the preparation by what it issues.  Measured on B200,
+// 2,048 tokens of one request, 32 heads of 128 x 128: see launch_walk.
+#include "common.cuh"
+#include "mma_common.cuh"
+#include <type_traits>
+
+using namespace ccb;
+
+namespace {
+
+constexpr int kChunk = 64;
+constexpr int kThreads = 256;
+constexpr int kRun = 16;           // tokens of a run
+constexpr float kLeastLog2 = -115.f;
+
+struct ChunkRows {
+  const float *q, *k, *v, *g, *beta;   // q, k [T, G, DK]; v [T, H, dv]; g [T, H, DK], or [T, H] with one decay a head
+  __nv_bfloat16 *qs, *ks, *w;          // [T, H, 2, DK]: a row's bfloat16 values, then what their rounding left
+  float* u;                            // [T, H, dv]
+  __nv_bfloat16* p;                    // [T, H, 2, 64]
+  float* keep;                         // [T / 64 + entries, H, DK]: e^{c_64} of a chunk
+  float *state, *out;                  // [slots, H, dv, DK], [T, H, dv]
+  const int *cu_q, *state_slot;
+  int entry0, G, H, dv, n_slots;
+};
+
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// bfloat16 pair of (x, y) and of what their rounding left
+__device__ __forceinline__ void split2(float x, float y, uint32_t& hi, uint32_t& lo) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+  const float2 f = __bfloat1622float2(h);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  lo = pack_bf16(x - f.x, y - f.y);
+}
+
+// c += a b with both operands as two bfloat16
+__device__ __forceinline__ void mma3(float* c, const uint32_t* ah, const uint32_t* al, uint32_t bh0, uint32_t bh1, uint32_t bl0,
+                                     uint32_t bl1) {
+  mma_bf16_16816(c, al, bh0, bh1);
+  mma_bf16_16816(c, ah, bl0, bl1);
+  mma_bf16_16816(c, ah, bh0, bh1);
+}
+
+// rows of DK floats: the eight-float groups of neighbouring rows sit in different banks
+template <int DK> __device__ __forceinline__ int at(int row, int col) { return row * DK + (col ^ ((row & 3) << 3)); }
+
+constexpr int kPitchL = kChunk;
+
+template <int DK, bool DELTA, bool HEAD> struct PrepShape {
+  static constexpr int kC = HEAD ? kChunk : kChunk * DK;   // sums of logarithms
+  static constexpr int kFloats = 2 * kChunk * DK + kC + (DELTA ? kChunk * kPitchL : 0) + kChunk;   // (two blocks an SM)
+  static constexpr int kBytes = kFloats * 4 + 16;
+};
+
+// 32 values a lane, one for each lane: the sum of value i over all lanes ends in lane i
+__device__ __forceinline__ float transpose_sum(float (&v)[32], int lane) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < o; ++i) {
+      const float mine = up ? v[i + o] : v[i], other = up ? v[i] : v[i + o];
+      v[i] = mine + __shfl_xor_sync(0xffffffffu, other, o);
+    }
+  }
+  return v[0];
+}
+
+template <int DK, bool DELTA, bool HEAD>
+__global__ void __launch_bounds__(kThreads, 2)
+chunk_prepare_kernel(const ChunkRows a) {
+  ccb::pdl_begin();
+  using Sh = PrepShape<DK, DELTA, HEAD>;
+  extern __shared__ __align__(16) float smem[];
+  float* q_s = smem;                         // [64][DK]
+  float* k_s = q_s + kChunk * DK;
+  float* c_s = k_s + kChunk * DK;            // [64][DK] or [64]: log2 of the decay since the token's run began
+  float* l_s = c_s + Sh::kC;                 // [64][64]: diag(beta) M below the diagonal
+  float* b_s = l_s + (DELTA ? kChunk * kPitchL : 0);
+  int* next_row = reinterpret_cast<int*>(b_s + kChunk);
+
+  const int e = a.entry0 + blockIdx.z, h = blockIdx.y, chunk = blockIdx.x;
+  const int first = a.cu_q[e], n = a.cu_q[e + 1] - first;
+  const int slot = a.state_slot[e];
+  if (slot < 0 || slot >= a.n_slots || chunk * kChunk >= n) return;
+  const int r0 = first + chunk * kChunk, cnt = min(kChunk, n - chunk * kChunk);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int kvh = h / (a.H / a.G);
+
+  for (int i = tid; i < kChunk * DK / 4; i += kThreads) {
+    const int t = i / (DK / 4), c = 4 * (i % (DK / 4));
+    float4 q = make_float4(0.f, 0.f, 0.f, 0.f), k = q;
+    if (t < cnt) {
+      const size_t row = ((size_t)(r0 + t) * a.G + kvh) * DK + c;
+      q = *reinterpret_cast<const float4*>(a.q + row);
+      k = *reinterpret_cast<const float4*>(a.k + row);
+    }
+    *reinterpret_cast<float4*>(q_s + at<DK>(t, c)) = q;
+    *reinterpret_cast<float4*>(k_s + at<DK>(t, c)) = k;
+  }
+  if (tid < kChunk) b_s[tid] = DELTA && tid < cnt ? a.beta[(size_t)(r0 + tid) * a.H + h] : 0.f;
+  if (tid == 0) *next_row = 0;
+  auto log_decay = [](float g) {
+    const float x = log2f(g);
+    return x < kLeastLog2 ? kLeastLog2 : x;
+  };
+  if constexpr (HEAD) {
+    if (warp == 0) {   // two tokens a lane, eight lanes a run
+      float x[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int t = 2 * lane + i;
+        x[i] = t < cnt ? log_decay(a.g[(size_t)(r0 + t) * a.H + h]) : 0.f;
+      }
+      float before = x[0] + x[1];
+#pragma unroll
+      for (int o = 1; o < kRun / 2; o <<= 1) {
+        const float y = __shfl_up_sync(0xffffffffu, before, o, kRun / 2);
+        if ((lane & (kRun / 2 - 1)) >= o) before += y;
+      }
+      before = __shfl_up_sync(0xffffffffu, before, 1, kRun / 2);
+      if ((lane & (kRun / 2 - 1)) == 0) before = 0.f;
+      c_s[2 * lane] = before + x[0];
+      c_s[2 * lane + 1] = before + x[0] + x[1];
+    }
+  } else {   // a thread a channel and some runs
+    constexpr int PT = kChunk * DK / kThreads;
+    static_assert(PT % kRun == 0, "whole runs");
+    const int d = tid % DK, part = tid / DK;
+    float x[PT];
+#pragma unroll
+    for (int i = 0; i < PT; ++i) {
+      const int t = part * PT + i;
+      x[i] = t < cnt ? a.g[((size_t)(r0 + t) * a.H + h) * DK + d] : 1.f;
+    }
+    float sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < PT; ++i) {
+      sum = (i % kRun == 0 ? 0.f : sum) + log_decay(x[i]);
+      c_s[at<DK>(part * PT + i, d)] = sum;
+    }
+  }
+  __syncthreads();
+  auto in_run = [&](int t, int d) { return HEAD ? c_s[t] : c_s[at<DK>(t, d)]; };
+  // the decay of whole runs lo .. hi - 1
+  auto over_runs = [&](int lo, int hi, int d) {
+    float sum = 0.f;
+#pragma unroll
+    for (int m = 0; m < kChunk / kRun; ++m)
+      if (m >= lo && m < hi) sum += in_run(m * kRun + kRun - 1, d);
+    return sum;
+  };
+  const size_t p_row = (size_t)a.H * 2 * kChunk;   // elements from a token's scores to the next one's
+  __nv_bfloat16* p_out = a.p + ((size_t)r0 * a.H + h) * 2 * kChunk;
+
+  // ---- blocks of 16 x 16 pairs: rows of run i, columns of run j (j < i; with one decay a head also j = i)
+  const int gid = lane >> 2, tig = lane & 3;
+  constexpr int kPairs = HEAD ? 10 : 6;
+  for (int unit = warp; unit < kPairs; unit += kThreads / 32) {
+    int i = HEAD ? 0 : 1, j = unit;
+    while (j >= (HEAD ? i + 1 : i)) { j -= HEAD ? i + 1 : i; ++i; }
+    if (i * kRun >= cnt) continue;
+    const int edge = (j + 1) * kRun - 1;   // the place that both factors refer to: the end of run j
+    float sq[2][4], sk[2][4];
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+      for (int y = 0; y < 4; ++y) sq[x][y] = sk[x][y] = 0.f;
+#pragma unroll 2
+    for (int ks = 0; ks < DK / 16; ++ks) {
+      uint32_t qh[4], ql[4], kh[4], kl[4], bh[2][2], bl[2][2];
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int col = ks * 16 + 2 * tig + 8 * half;
+        float2 ce = make_float2(0.f, 0.f), mid = ce;   // of run j, and of the runs between j and i
+        if (!HEAD) {
+          ce = *reinterpret_cast<const float2*>(c_s + at<DK>(edge, col));
+          for (int m = j + 1; m < i; ++m) {
+            const float2 c = *reinterpret_cast<const float2*>(c_s + at<DK>(m * kRun + kRun - 1, col));
+            mid.x += c.x;
+            mid.y += c.y;
+          }
+        }
+#pragma unroll
+        for (int up = 0; up < 2; ++up) {
+          const int t = i * kRun + gid + 8 * up;
+          float2 q = *reinterpret_cast<const float2*>(q_s + at<DK>(t, col));
+          float2 k = make_float2(0.f, 0.f);
+          if (DELTA) k = *reinterpret_cast<const float2*>(k_s + at<DK>(t, col));
+          if (!HEAD) {
+            const float2 c = *reinterpret_cast<const float2*>(c_s + at<DK>(t, col));
+            const float fx = ex2(c.x + mid.x), fy = ex2(c.y + mid.y);
+            q.x *= fx; q.y *= fy;
+            k.x *= fx; k.y *= fy;
+          }
+          split2(q.x, q.y, qh[2 * half + up], ql[2 * half + up]);
+          if (DELTA) split2(k.x, k.y, kh[2 * half + up], kl[2 * half + up]);
+        }
+#pragma unroll
+        for (int nb = 0; nb < 2; ++nb) {
+          const int s = j * kRun + nb * 8 + gid;
+          float2 k = *reinterpret_cast<const float2*>(k_s + at<DK>(s, col));
+          if (!HEAD) {
+            const float2 c = *reinterpret_cast<const float2*>(c_s + at<DK>(s, col));
+            k.x *= ex2(ce.x - c.x);
+            k.y *= ex2(ce.y - c.y);
+          }
+          split2(k.x, k.y, bh[nb][half], bl[nb][half]);
+        }
+      }
+#pragma unroll
+      for (int nb = 0; nb < 2; ++nb) {
+        mma3(sq[nb], qh, ql, bh[nb][0], bh[nb][1], bl[nb][0], bl[nb][1]);
+        if (DELTA) mma3(sk[nb], kh, kl, bh[nb][0], bh[nb][1], bl[nb][0], bl[nb][1]);
+      }
+    }
+#pragma unroll
+    for (int nb = 0; nb < 2; ++nb)
+#pragma unroll
+      for (int up = 0; up < 2; ++up) {
+        const int t = i * kRun + gid + 8 * up, s = j * kRun + nb * 8 + 2 * tig;
+        float f0 = 1.f, f1 = 1.f;
+        if (HEAD) {
+          f0 = s <= t ? ex2(i == j ? c_s[t] - c_s[s] : c_s[t] + (over_runs(j + 1, i, 0) + (c_s[edge] - c_s[s]))) : 0.f;
+          f1 = s + 1 <= t ? ex2(i == j ? c_s[t] - c_s[s + 1] : c_s[t] + (over_runs(j + 1, i, 0) + (c_s[edge] - c_s[s + 1]))) : 0.f;
+        }
+        if (t < cnt) {
+          uint32_t hi, lo;
+          split2(sq[nb][2 * up] * f0, sq[nb][2 * up + 1] * f1, hi, lo);
+          *reinterpret_cast<uint32_t*>(p_out + t * p_row + s) = hi;
+          *reinterpret_cast<uint32_t*>(p_out + t * p_row + kChunk + s) = lo;
+        }
+        if (DELTA) {
+          const float b = b_s[t];
+          l_s[t * kPitchL + s] = !HEAD || s < t ? sk[nb][2 * up] * f0 * b : 0.f;
+          l_s[t * kPitchL + s + 1] = !HEAD || s + 1 < t ? sk[nb][2 * up + 1] * f1 * b : 0.f;
+        }
+      }
+  }
+  // ---- pairs within a run, a decay for every pair and channel: a warp a row, its lanes the channels.  Rows with many
+  // pairs first, to whoever is free.
+  if constexpr (!HEAD) {
+    constexpr int CL = DK / 32;   // channels a lane
+    for (;;) {
+      int item = 0;
+      if (lane == 0) item = atomicAdd(next_row, 1);
+      item = __shfl_sync(0xffffffffu, item, 0);
+      if (item >= kChunk) break;
+      const int run = item & 3, lt = kRun - 1 - (item >> 2), t = run * kRun + lt;
+      if (t >= cnt) continue;
+      float q[CL], k[CL], c[CL], v[32];
+#pragma unroll
+      for (int x = 0; x < CL; ++x) {
+        q[x] = q_s[at<DK>(t, lane + 32 * x)];
+        k[x] = k_s[at<DK>(t, lane + 32 * x)];
+        c[x] = c_s[at<DK>(t, lane + 32 * x)];
+      }
+#pragma unroll
+      for (int s = 0; s < kRun; ++s) {
+        v[s] = v[kRun + s] = 0.f;
+        if (s > lt) continue;
+        const int row = run * kRun + s;
+#pragma unroll
+        for (int x = 0; x < CL; ++x) {
+          const float ke = k_s[at<DK>(row, lane + 32 * x)] * ex2(c[x] - c_s[at<DK>(row, lane + 32 * x)]);
+          v[s] = fmaf(q[x], ke, v[s]);
+          if (DELTA) v[kRun + s] = fmaf(k[x], ke, v[kRun + s]);
+        }
+      }
+      const float sum = transpose_sum(v, lane);
+      const int s = lane & 15;
+      if (lane < kRun) {
+        const float x = s <= lt ? sum : 0.f;
+        const __nv_bfloat16 hi = __float2bfloat16_rn(x);
+        p_out[t * p_row + run * kRun + s] = hi;
+        p_out[t * p_row + kChunk + run * kRun + s] = __float2bfloat16_rn(x - __bfloat162float(hi));
+      } else if (DELTA) {
+        l_s[t * kPitchL + run * kRun + s] = s < lt ? sum * b_s[t] : 0.f;
+      }
+    }
+  }
+  // ---- the rows that meet the memory: q e^c, k e^{c_64 - c}, and e^{c_64}
+  for (int i = tid; i < kChunk * DK / 2; i += kThreads) {
+    const int t = i / (DK / 2), d = 2 * (i % (DK / 2)), run = t / kRun;
+    if (t >= cnt) break;
+    const float2 q = *reinterpret_cast<const float2*>(q_s + at<DK>(t, d)), k = *reinterpret_cast<const float2*>(k_s + at<DK>(t, d));
+    float fq[2], fk[2];
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+      const float c = in_run(t, d + x);
+      fq[x] = ex2(over_runs(0, run, d + x) + c);
+      fk[x] = ex2(over_runs(run + 1, kChunk / kRun, d + x) + (in_run(run * kRun + kRun - 1, d + x) - c));   // (rows past the end decay nothing)
+    }
+    const size_t row = ((size_t)(r0 + t) * a.H + h) * 2 * DK;
+    uint32_t hi, lo;
+    split2(q.x * fq[0], q.y * fq[1], hi, lo);
+    *reinterpret_cast<uint32_t*>(a.qs + row + d) = hi;
+    *reinterpret_cast<uint32_t*>(a.qs + row + DK + d) = lo;
+    split2(k.x * fk[0], k.y * fk[1], hi, lo);
+    *reinterpret_cast<uint32_t*>(a.ks + row + d) = hi;
+    *reinterpret_cast<uint32_t*>(a.ks + row + DK + d) = lo;
+  }
+  const int place = (first >> 6) + e + chunk;   // (distinct: an entry's last chunk comes before the next entry's first)
+  for (int d = tid; d < DK; d += kThreads) a.keep[((size_t)place * a.H + h) * DK + d] = ex2(over_runs(0, kChunk / kRun, d));
+
+  // ---- the triangular solve: a thread a column of [K e^c | V]
+  if constexpr (DELTA) {
+    __syncthreads();
+    for (int col = tid; col < DK + a.dv; col += kThreads) {
+      const bool is_w = col < DK;
+      float x[kChunk];
+#pragma unroll
+      for (int t = 0; t < kChunk; ++t) {
+        float y = 0.f;
+        if (t < cnt)
+          y = is_w ? k_s[at<DK>(t, col)] * ex2(over_runs(0, t / kRun, col) + in_run(t, col)) : a.v[((size_t)(r0 + t) * a.H + h) * a.dv + col - DK];
+        x[t] = y * b_s[t];
+      }
+#pragma unroll
+      for (int t = 1; t < kChunk; ++t) {
+        float y[4] = {x[t], 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int s = 0; s < t; s += 4) {
+          const float4 l = *reinterpret_cast<const float4*>(l_s + t * kPitchL + s);   // (zero from the diagonal on)
+          y[0] = fmaf(-l.x, x[s], y[0]);
+          if (s + 1 < t) y[1] = fmaf(-l.y, x[s + 1], y[1]);
+          if (s + 2 < t) y[2] = fmaf(-l.z, x[s + 2], y[2]);
+          if (s + 3 < t) y[3] = fmaf(-l.w, x[s + 3], y[3]);
+        }
+        x[t] = (y[0] + y[1]) + (y[2] + y[3]);
+      }
+#pragma unroll
+      for (int t = 0; t < kChunk; ++t) {
+        if (t >= cnt) continue;
+        if (is_w) {
+          const __nv_bfloat16 hi = __float2bfloat16_rn(x[t]);
+          const size_t row = ((size_t)(r0 + t) * a.H + h) * 2 * DK + col;
+          a.w[row] = hi;
+          a.w[row + DK] = __float2bfloat16_rn(x[t] - __bfloat162float(hi));
+        } else {
+          a.u[((size_t)(r0 + t) * a.H + h) * a.dv + col - DK] = x[t];
+        }
+      }
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+constexpr int kCols = 32;          // value columns a block
+constexpr int kPitch = kCols + 8;  // elements: eight rows of an ldmatrix fall into different banks
+
+template <int DK, bool DELTA> struct WalkShape {
+  static constexpr int kTile = 2 * kChunk * DK;                 // elements of the two halves of 64 rows
+  static constexpr int kElements = (DELTA ? 3 : 2) * kTile + 2 * kChunk * kChunk + 2 * DK * kPitch + 2 * kChunk * kPitch;
+  static constexpr int kBytes = kElements * 2;
+};
+
+template <int DK, bool DELTA>
+__global__ void __launch_bounds__(kThreads)
+chunk_walk_kernel(const ChunkRows a) {
+  ccb::pdl_begin();
+  using Sh = WalkShape<DK, DELTA>;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __nv_bfloat16* q_s = reinterpret_cast<__nv_bfloat16*>(smem_raw);   // [2][64][DK], swizzled
+  __nv_bfloat16* k_s = q_s + Sh::kTile;
+  __nv_bfloat16* w_s = k_s + Sh::kTile;
+  __nv_bfloat16* p_s = w_s + (DELTA ? Sh::kTile : 0);                // [2][64][64], swizzled
+  __nv_bfloat16* s_hi = p_s + 2 * kChunk * kChunk;                   // [DK][kPitch]
+  __nv_bfloat16* s_lo = s_hi + DK * kPitch;
+  __nv_bfloat16* u_hi = s_lo + DK * kPitch;                          // [64][kPitch]
+  __nv_bfloat16* u_lo = u_hi + kChunk * kPitch;
+
+  const int e = a.entry0 + blockIdx.z, h = blockIdx.y, col0 = blockIdx.x * kCols;
+  const int slot = a.state_slot[e];
+  const int r0 = a.cu_q[e], n = a.cu_q[e + 1] - r0;
+  if (slot < 0 || slot >= a.n_slots || n <= 0) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int gid = lane >> 2, tig = lane & 3;
+  const int wr = warp & 3, wc = warp >> 2;   // 16 rows of the chunk, 16 columns of the slice
+
+  // 64 rows of two halves of `COLS` elements each, a row (r0 + t, h), into two swizzled tiles
+  auto issue = [&](__nv_bfloat16* dst, const __nv_bfloat16* src, int chunk, auto cols) {
+    constexpr int COLS = decltype(cols)::value;
+    const int t0 = chunk * kChunk;
+#pragma unroll
+    for (int i = 0; i < 2 * kChunk * (COLS / 8) / kThreads; ++i) {
+      const int idx = tid + kThreads * i;
+      const int row = idx / (COLS / 4), c = idx % (COLS / 4), half = c / (COLS / 8), c8 = c % (COLS / 8);
+      const bool ok = t0 + row < n;
+      cp_async16(smem_u32(dst + half * kChunk * COLS + swz<COLS>(row, c8)),
+                 src + ((size_t)(r0 + t0 + (ok ? row : 0)) * a.H + h) * 2 * COLS + c * 8, ok);
+    }
+  };
+  using Dk = std::integral_constant<int, DK>;
+  using P64 = std::integral_constant<int, kChunk>;
+  auto issue_read = [&](int chunk) {    // what meets the memory
+    issue(q_s, a.qs, chunk, Dk{});
+    if (DELTA) issue(w_s, a.w, chunk, Dk{});
+    cp_async_commit();
+  };
+  auto issue_write = [&](int chunk) {   // what meets u
+    issue(p_s, a.p, chunk, P64{});
+    issue(k_s, a.ks, chunk, Dk{});
+    cp_async_commit();
+  };
+  issue_read(0);
+
+  // S: key channels 16 warp .. + 15 (with 64 channels only the first four warps have some), all columns of the slice
+  constexpr int SW = DK / 16;   // warps with channels
+  float S[4][4];
+  float* sp = a.state + ((size_t)slot * a.H + h) * (size_t)a.dv * DK;
+  auto store_s = [&]() {
+#pragma unroll
+    for (int nb = 0; nb < 4; ++nb)
+#pragma unroll
+      for (int up = 0; up < 2; ++up) {
+        const int row = warp * 16 + gid + 8 * up, c = nb * 8 + 2 * tig;
+        uint32_t hi, lo;
+        split2(S[nb][2 * up], S[nb][2 * up + 1], hi, lo);
+        *reinterpret_cast<uint32_t*>(s_hi + row * kPitch + c) = hi;
+        *reinterpret_cast<uint32_t*>(s_lo + row * kPitch + c) = lo;
+      }
+  };
+  if (warp < SW) {
+#pragma unroll
+    for (int nb = 0; nb < 4; ++nb)
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+        S[nb][x] = sp[(size_t)(col0 + nb * 8 + 2 * tig + (x & 1)) * DK + warp * 16 + gid + 8 * (x >> 1)];
+    store_s();
+  }
+  const int arow = (lane & 7) + 8 * ((lane >> 3) & 1), achunk = lane >> 4;   // A operand, row-major
+  const int trow = arow, tcol = 8 * (lane >> 4);                             // B operand whose k runs over rows
+
+  const int chunks = (n + kChunk - 1) / kChunk;
+  for (int ch = 0; ch < chunks; ++ch) {
+    const int left = n - ch * kChunk;
+    // this thread's places of u and o: rows wr * 16 + gid (+ 8), columns wc * 16 + 2 tig (+ 1, + 8, + 9)
+    float u[2][4], o[2][4];
+    const float* src = DELTA ? a.u : a.v;
+#pragma unroll
+    for (int up = 0; up < 2; ++up) {
+      const int t = wr * 16 + gid + 8 * up;
+      const float* row = src + ((size_t)(r0 + ch * kChunk + t) * a.H + h) * a.dv + col0 + wc * 16 + 2 * tig;
+#pragma unroll
+      for (int nb = 0; nb < 2; ++nb) {
+        const float2 x = t < left ? *reinterpret_cast<const float2*>(row + nb * 8) : make_float2(0.f, 0.f);
+        u[nb][2 * up] = x.x;
+        u[nb][2 * up + 1] = x.y;
+        o[nb][2 * up] = o[nb][2 * up + 1] = 0.f;
+      }
+    }
+    float keep[2] = {0.f, 0.f};
+    if (warp < SW) {
+      const float* kp = a.keep + ((size_t)((r0 >> 6) + e + ch) * a.H + h) * DK + warp * 16 + gid;
+      keep[0] = kp[0];
+      keep[1] = kp[8];
+    }
+    cp_async_wait<0>();
+    __syncthreads();   // q and w of this chunk and the memory before it are there; p and k of the last one are done with
+    issue_write(ch);
+
+    float d[2][4];   // W S0
+#pragma unroll
+    for (int nb = 0; nb < 2; ++nb) d[nb][0] = d[nb][1] = d[nb][2] = d[nb][3] = 0.f;
+#pragma unroll 2
+    for (int ks = 0; ks < DK / 16; ++ks) {
+      uint32_t bh[4], bl[4], xh[4], xl[4];
+      ldmatrix_x4_trans(bh[0], bh[1], bh[2], bh[3], smem_u32(s_hi + (ks * 16 + trow) * kPitch + wc * 16 + tcol));
+      ldmatrix_x4_trans(bl[0], bl[1], bl[2], bl[3], smem_u32(s_lo + (ks * 16 + trow) * kPitch + wc * 16 + tcol));
+      const int pos = swz<DK>(wr * 16 + arow, 2 * ks + achunk);
+      if (DELTA) {
+        ldmatrix_x4(xh[0], xh[1], xh[2], xh[3], smem_u32(w_s + pos));
+        ldmatrix_x4(xl[0], xl[1], xl[2], xl[3], smem_u32(w_s + kChunk * DK + pos));
+        mma3(d[0], xh, xl, bh[0], bh[1], bl[0], bl[1]);
+        mma3(d[1], xh, xl, bh[2], bh[3], bl[2], bl[3]);
+      }
+      ldmatrix_x4(xh[0], xh[1], xh[2], xh[3], smem_u32(q_s + pos));
+      ldmatrix_x4(xl[0], xl[1], xl[2], xl[3], smem_u32(q_s + kChunk * DK + pos));
+      mma3(o[0], xh, xl, bh[0], bh[1], bl[0], bl[1]);
+      mma3(o[1], xh, xl, bh[2], bh[3], bl[2], bl[3]);
+    }
+#pragma unroll
+    for (int nb = 0; nb < 2; ++nb)
+#pragma unroll
+      for (int up = 0; up < 2; ++up) {
+        uint32_t hi, lo;
+        split2(u[nb][2 * up] - d[nb][2 * up], u[nb][2 * up + 1] - d[nb][2 * up + 1], hi, lo);
+        const int pos = (wr * 16 + gid + 8 * up) * kPitch + wc * 16 + nb * 8 + 2 * tig;
+        *reinterpret_cast<uint32_t*>(u_hi + pos) = hi;
+        *reinterpret_cast<uint32_t*>(u_lo + pos) = lo;
+      }
+    cp_async_wait<0>();
+    __syncthreads();   // u, p and k are there; q, w and the memory's halves have been read
+    if (ch + 1 < chunks) issue_read(ch + 1);
+
+#pragma unroll
+    for (int ks = 0; ks < kChunk / 16; ++ks) {   // o += P u: the keys of the runs up to the rows' own
+      if (ks > wr) continue;
+      uint32_t bh[4], bl[4], xh[4], xl[4];
+      ldmatrix_x4_trans(bh[0], bh[1], bh[2], bh[3], smem_u32(u_hi + (ks * 16 + trow) * kPitch + wc * 16 + tcol));
+      ldmatrix_x4_trans(bl[0], bl[1], bl[2], bl[3], smem_u32(u_lo + (ks * 16 + trow) * kPitch + wc * 16 + tcol));
+      const int pos = swz<kChunk>(wr * 16 + arow, 2 * ks + achunk);
+      ldmatrix_x4(xh[0], xh[1], xh[2], xh[3], smem_u32(p_s + pos));
+      ldmatrix_x4(xl[0], xl[1], xl[2], xl[3], smem_u32(p_s + kChunk * kChunk + pos));
+      mma3(o[0], xh, xl, bh[0], bh[1], bl[0], bl[1]);
+      mma3(o[1], xh, xl, bh[2], bh[3], bl[2], bl[3]);
+    }
+    if (warp < SW) {   // S = e^{c_64} S + K^T u
+#pragma unroll
+      for (int nb = 0; nb < 4; ++nb)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) S[nb][x] *= keep[x >> 1];
+#pragma unroll
+      for (int ks = 0; ks < kChunk / 16; ++ks) {
+        uint32_t xh[4], xl[4];   // keys as the A operand, transposed: rows are key channels, k are tokens
+        const int pos = swz<DK>(ks * 16 + (lane & 7) + 8 * (lane >> 4), warp * 2 + ((lane >> 3) & 1));
+        ldmatrix_x4_trans(xh[0], xh[1], xh[2], xh[3], smem_u32(k_s + pos));
+        ldmatrix_x4_trans(xl[0], xl[1], xl[2], xl[3], smem_u32(k_s + kChunk * DK + pos));
+#pragma unroll
+        for (int np = 0; np < 2; ++np) {
+          uint32_t bh[4], bl[4];
+          ldmatrix_x4_trans(bh[0], bh[1], bh[2], bh[3], smem_u32(u_hi + (ks * 16 + trow) * kPitch + np * 16 + tcol));
+          ldmatrix_x4_trans(bl[0], bl[1], bl[2], bl[3], smem_u32(u_lo + (ks * 16 + trow) * kPitch + np * 16 + tcol));
+          mma3(S[2 * np], xh, xl, bh[0], bh[1], bl[0], bl[1]);
+          mma3(S[2 * np + 1], xh, xl, bh[2], bh[3], bl[2], bl[3]);
+        }
+      }
+      if (ch + 1 < chunks) store_s();
+    }
+#pragma unroll
+    for (int up = 0; up < 2; ++up) {
+      const int t = wr * 16 + gid + 8 * up;
+      if (t >= left) continue;
+      float* row = a.out + ((size_t)(r0 + ch * kChunk + t) * a.H + h) * a.dv + col0 + wc * 16 + 2 * tig;
+#pragma unroll
+      for (int nb = 0; nb < 2; ++nb) *reinterpret_cast<float2*>(row + nb * 8) = make_float2(o[nb][2 * up], o[nb][2 * up + 1]);
+    }
+  }
+  if (warp < SW) {
+#pragma unroll
+    for (int nb = 0; nb < 4; ++nb)
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+        sp[(size_t)(col0 + nb * 8 + 2 * tig + (x & 1)) * DK + warp * 16 + gid + 8 * (x >> 1)] = S[nb][x];
+  }
+}
+
+template <int DK, bool DELTA, bool HEAD>
+int launch_chunked(const ChunkRows& a, int n_entries, int max_tokens, cudaStream_t stream) {
+  auto prepare = chunk_prepare_kernel<DK, DELTA, HEAD>;
+  auto walk = chunk_walk_kernel<DK, DELTA>;
+  constexpr int prep_bytes = PrepShape<DK, DELTA, HEAD>::kBytes, walk_bytes = WalkShape<DK, DELTA>::kBytes;
+  static_assert(walk_bytes <= 227 * 1024 && prep_bytes <= 227 * 1024, "shared memory of a block");
+  cudaError_t err = cudaFuncSetAttribute(prepare, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_bytes);
+  if (err == cudaSuccess) err = cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, walk_bytes);
+  if (err != cudaSuccess) return (int)err;
+  ccb_launch(prepare, dim3((max_tokens + kChunk - 1) / kChunk, a.H, n_entries), kThreads, prep_bytes, stream, a);
+  err = cudaGetLastError();
+  if (err != cudaSuccess) return (int)err;
+  ccb_launch(walk, dim3(a.dv / kCols, a.H, n_entries), kThreads, walk_bytes, stream, a);
+  return ccb_launch_status();
+}
+
+}  // namespace
+
+// Entries entry0 .. entry0 + n_entries - 1, the longest of max_tokens tokens.  Key sizes 64 and 128, value sizes that are
+// multiples of 32 (others: CCB_REFUSE_SIZE).  q, k float [T, G, dk], v float [T, H, dv], g float [T, H, dk] (head_decay 0)
+// or [T, H], beta float [T, H] (null: no delta rule).  Workspace: qs, ks and (delta rule) w [T, H, 2, dk] and p
+// [T, H, 2, 64] bfloat16, u float [T, H, dv] (delta rule), keep float [T / 64 + entries, H, dk].  qs, ks, w and u may be
+// the memory of q, k (where G = H), g (one decay per channel) and v: a block writes a row after it has read it, and
+// nobody else reads it.
+CCB_API int ccb_chunk_recurrence(const float* q, const float* k, const float* v, const float* g, const float* beta, void* qs,
+                                 void* ks, void* w, float* u, void* p, float* keep, float* state, float* out,
+                                 const int* cu_q, const int* state_slot, int entry0, int n_entries, int max_tokens, int G, int H,
+                                 int dk, int dv, int n_slots, int head_decay, cudaStream_t stream) {
+  if (n_entries <= 0) return 0;
+  if (G <= 0 || H <= 0 || H % G || (dk != 64 && dk != 128) || dv <= 0 || dv % kCols || entry0 < 0 || max_tokens <= 0 ||
+      H > 65535 || n_entries > 65535)
+    return CCB_REFUSE_SIZE;
+  if (beta != nullptr && (w == nullptr || u == nullptr)) return CCB_REFUSE_ARG;
+  const auto bits = [](const void* x) { return reinterpret_cast<uintptr_t>(x); };
+  if ((bits(q) | bits(k) | bits(v) | bits(g) | bits(qs) | bits(ks) | bits(w) | bits(u) | bits(p) | bits(out)) & 15)
+    return CCB_REFUSE_ARG;
+  if (G != H && (qs == (const void*)q || ks == (const void*)k)) return CCB_REFUSE_ARG;
+  const ChunkRows a{q, k, v, g, beta, (__nv_bfloat16*)qs, (__nv_bfloat16*)ks, (__nv_bfloat16*)w, u, (__nv_bfloat16*)p, keep,
+                    state, out, cu_q, state_slot, entry0, G, H, dv, n_slots};
+#define CCB_CHUNK(DK, DELTA)                                                                \
+  (head_decay ? launch_chunked<DK, DELTA, true>(a, n_entries, max_tokens, stream) \
+              : launch_chunked<DK, DELTA, false>(a, n_entries, max_tokens, stream))
+  if (dk == 128) return beta != nullptr ? CCB_CHUNK(128, true) : CCB_CHUNK(128, false);
+  return beta != nullptr ? CCB_CHUNK(64, true) : CCB_CHUNK(64, false);
+#undef CCB_CHUNK
+}

@@ -72,6 +72,13 @@ class Runtime:
         self.merge_counters = torch.zeros(8192, dtype=torch.int32, device=self.device)  # attention split counters
         self._sink_turn = 0
 
+    def chunk_scratch(self, key: str, per: str, shape, dtype: torch.dtype) -> torch.Tensor:
+        """A workspace of ``kernels.chunk_recurrence``: a row for each of a step's tokens or of its chunks of 64.  Layers of
+        other sizes have buffers of their own (only portions use them: they must not grow once graphs hold addresses)."""
+        n = self.max_tokens if per == "tokens" else self.max_tokens // 64 + self.max_entries
+        name = ":".join([key] + [str(d) for d in shape])
+        return self.scratch.get(name, (n,) + tuple(shape), dtype)
+
     @staticmethod
     def rows(x):
         """x as a plain tensor (rows that a norm left short of their factor are finished, and a pair's or the experts' sum

@@ -203,6 +203,7 @@ _SIGNATURES = {
                        + [c_void_p] * 4 + [c_int] + [c_void_p] * 4 + [c_float, c_float, c_int, c_void_p]
                        + [c_int] * 7 + [c_float, c_float, c_int, c_int, c_void_p],
     "ccb_memory_chunks": [c_void_p] * 4 + [c_int, c_void_p, c_int] + [c_void_p] * 6 + [c_int] * 7 + [c_float, c_void_p],
+    "ccb_chunk_recurrence": [c_void_p] * 15 + [c_int] * 9 + [c_void_p],
     "ccb_memory_output": [c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int,
                           c_float, c_int, c_void_p],
     "ccb_relu_squared": [c_void_p, c_void_p, c_longlong, c_int, c_void_p],
@@ -636,6 +637,43 @@ def delta_recurrence(qn, kn, vv, gg, bb, state, out, cu_q, state_slot, n_entries
     assert state.dtype == torch.float32 and state.shape[1:] == (H, dv, dk) and out.dtype == torch.float32
     _check(lib().ccb_delta_recurrence(_p(qn), _p(kn), _p(vv), _p(gg), _p(bb), _p(state), _p(out), _p(cu_q),
                                       _p(state_slot), n_entries, G, H, dk, dv, _stream()), "delta_recurrence")
+
+
+# Tokens of a step's longest portion from which the recurrences run in chunks.  The token-by-token kernel costs half a
+# microsecond a token whatever runs beside it, a chunk of 64 tokens (however few of them are there) 4 us of its walk
+# after some 10 us of preparation.
+CHUNK_RECURRENCE_MIN_TOKENS = 32
+
+
+def chunk_recurrence_fits(dtype, dk: int, dv: int, max_tokens: int) -> bool:
+    """Whether portions of prompts, the longest of max_tokens tokens, run as chunks on tensor cores: the 16-bit path (in
+    the 32-bit path every operand stays a float) with the sizes the kernel takes."""
+    return dtype == torch.bfloat16 and dk in (64, 128) and dv % 32 == 0 and max_tokens >= CHUNK_RECURRENCE_MIN_TOKENS
+
+
+def chunk_recurrence(scratch, qn, kn, vv, gg, bb, state, out, cu_q, state_slot, entry0: int, n_entries: int,
+                     max_tokens: int, G: int, H: int, dk: int, dv: int) -> None:
+    """``delta_recurrence`` / ``delta_head_recurrence`` (gg [T, H]) / with bb None ``gated_linear_recurrence`` for the
+    entries entry0 .. entry0 + n_entries - 1 in chunks on tensor cores.  The rows are consumed: what the chunks leave
+    between the two kernels goes into the memory of qn, kn, vv and gg where sizes allow.  ``scratch(key, tokens_or_chunks,
+    shape, dtype)``: a workspace of shape [tokens or chunks, *shape]."""
+    _cuda(qn, kn, vv, gg, bb, state, out, cu_q, state_slot)
+    assert all(t.dtype == torch.float32 for t in (qn, kn, vv, gg, state, out)) and state.shape[1:] == (H, dv, dk)
+    T, head = vv.shape[0], gg.dim() == 2
+    assert qn.shape == kn.shape == (T, G, dk) and vv.shape == out.shape == (T, H, dv)
+    assert tuple(gg.shape) == ((T, H) if head else (T, H, dk)) and (bb is None or bb.shape == (T, H))
+    bf = torch.bfloat16
+    qs = qn if G == H else scratch("chunk_q", "tokens", (H, 2, dk), bf)
+    ks = kn if G == H else scratch("chunk_k", "tokens", (H, 2, dk), bf)
+    w = None if bb is None else (scratch("chunk_w", "tokens", (H, 2, dk), bf) if head else gg)
+    p = scratch("chunk_p", "tokens", (H, 2, 64), bf)
+    keep = scratch("chunk_keep", "chunks", (H, dk), torch.float32)
+    assert all(t is None or t.shape[0] >= T for t in (qs, ks, w, p)) and keep.shape[0] >= T // 64 + entry0 + n_entries
+    _check(lib().ccb_chunk_recurrence(_p(qn), _p(kn), _p(vv), _p(gg), _p(bb), _p(qs), _p(ks), _p(w),
+                                      _p(vv if bb is not None else None), _p(p), _p(keep), _p(state), _p(out), _p(cu_q),
+                                      _p(state_slot), int(entry0), int(n_entries), int(max_tokens), G, H, dk, dv,
+                                      state.shape[0], 1 if head else 0, _stream()), "chunk_recurrence")
+    counters.own += 1   # two kernels
 
 
 class HeadDelta:

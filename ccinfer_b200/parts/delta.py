@@ -140,7 +140,12 @@ class ChannelGatedDelta(Mixer):
         kernels.conv_state_update(proj, offsets, conv, self.taps, step.cu_q, step.state_slot, step.n_entries,
                                   G, H, dk, dv)
         o = rt.scratch.get("delta_o", (rt.max_tokens, H, dv), f32)[:T]
-        kernels.delta_recurrence(qn, kn, vv, gg, bb, S, o, step.cu_q, step.state_slot, step.n_entries, G, H, dk, dv)
+        # (a step lists its single tokens first: they, and short portions, go token by token)
+        n1 = step.n_single if kernels.chunk_recurrence_fits(rt.dtype, dk, dv, step.max_q_len) else step.n_entries
+        kernels.delta_recurrence(qn, kn, vv, gg, bb, S, o, step.cu_q, step.state_slot, n1, G, H, dk, dv)
+        if step.n_entries > n1:
+            kernels.chunk_recurrence(rt.chunk_scratch, qn, kn, vv, gg, bb, S, o, step.cu_q, step.state_slot, n1,
+                                     step.n_entries - n1, step.max_q_len, G, H, dk, dv)
         y = rt.scratch.get("delta_y", (rt.max_tokens, self.v_width), rt.dtype)[:T]
         kernels.gated_head_rmsnorm(y, o, ag[:, self.oga:], self.norm_w, H, dv, self.eps)
         out = rt.scratch.get(self.out_key, (rt.max_tokens, self.hidden), rt.dtype)[:T]
@@ -236,7 +241,11 @@ class HeadGatedDelta(Mixer):
             kernels.delta_head_prepare(self.rule, proj, ring, step.positions, step.entry_of_token, step.cu_q,
                                        step.state_slot, qn, kn, vv, gg, bb, n1, T - n1)
             kernels.conv_ring_write(self.rule, proj, ring, step.positions, step.cu_q, step.state_slot, n1, many)
-            kernels.delta_head_recurrence(qn, kn, vv, gg, bb, S, o, step.cu_q, step.state_slot, n1, many, G, H, dk, dv)
+            if kernels.chunk_recurrence_fits(rt.dtype, dk, dv, step.max_q_len):
+                kernels.chunk_recurrence(rt.chunk_scratch, qn, kn, vv, gg, bb, S, o, step.cu_q, step.state_slot, n1, many,
+                                         step.max_q_len, G, H, dk, dv)
+            else:
+                kernels.delta_head_recurrence(qn, kn, vv, gg, bb, S, o, step.cu_q, step.state_slot, n1, many, G, H, dk, dv)
             kernels.gated_head_rmsnorm(y[n1:], o[n1:], proj[n1:, self.og:self.og + self.v_width], self.norm_w, H, dv,
                                        self.eps, silu_gate=True)
         out = rt.scratch.get(self.out_key, (rt.max_tokens, self.hidden), rt.dtype)[:T]

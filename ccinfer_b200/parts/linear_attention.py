@@ -92,7 +92,12 @@ class GatedLinearAttention(Mixer):
         kernels.gla_prepare(proj, (self.oq, self.ok, self.ov), a, self.a2_bias, qn, kn, vv, gg, H, dk, dv,
                             dk ** -0.5, self.tau)
         o = rt.scratch.get("delta_o", (rt.max_tokens, H, dv), f32)[:T]
-        kernels.gated_linear_recurrence(qn, kn, vv, gg, state, o, step.cu_q, step.state_slot, step.n_entries, H, dk, dv)
+        # (a step lists its single tokens first: they, and short portions, go token by token)
+        n1 = step.n_single if kernels.chunk_recurrence_fits(rt.dtype, dk, dv, step.max_q_len) else step.n_entries
+        kernels.gated_linear_recurrence(qn, kn, vv, gg, state, o, step.cu_q, step.state_slot, n1, H, dk, dv)
+        if step.n_entries > n1:
+            kernels.chunk_recurrence(rt.chunk_scratch, qn, kn, vv, gg, None, state, o, step.cu_q, step.state_slot, n1,
+                                     step.n_entries - n1, step.max_q_len, H, H, dk, dv)
         y = rt.scratch.get("delta_y", (rt.max_tokens, H * dv), rt.dtype)[:T]
         kernels.gated_head_rmsnorm(y, o, proj[:, self.og:], self.norm_w, H, dv, self.eps, silu_gate=True)
         out = rt.scratch.get(self.out_key, (rt.max_tokens, self.hidden), rt.dtype)[:T]

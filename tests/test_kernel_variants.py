@@ -48,3 +48,67 @@ def test_float_product_of_every_shape_is_one_order_of_sums(M, N, K, pad, batch):
         c1 = torch.full((n, N), float("nan"), device="cuda")
         k.gemm_f32(c1, a[0, M - n:], w[0])
         assert torch.equal(c1, c[0, M - n:])
+
+
+def _recurrence64(q, k, v, g, beta, S):
+    """Token by token in float64: q, k [n, H, dk], v [n, H, dv], g [n, H, dk or 1], beta [n, H] or None, S [H, dv, dk]."""
+    out = torch.empty_like(v)
+    for t in range(q.shape[0]):
+        S = S * g[t][:, None, :]
+        u = v[t] if beta is None else beta[t][:, None] * (v[t] - (S * k[t][:, None, :]).sum(-1))
+        S = S + u[:, :, None] * k[t][:, None, :]
+        out[t] = (S * q[t][:, None, :]).sum(-1)
+    return out, S
+
+
+# decays: of every size down to zero; near one; strong ones beside weak ones (runs of tokens far below float's range)
+@pytest.mark.parametrize("decay", ["any", "slow", "strong"])
+@pytest.mark.parametrize("rule", ["delta", "head delta", "linear", "head linear"])
+@pytest.mark.parametrize("H,G,dk,dv", [(2, 2, 128, 128), (4, 2, 128, 32), (2, 1, 64, 96), (3, 3, 64, 64)])
+def test_recurrence_in_chunks(H, G, dk, dv, rule, decay):
+    """Portions of one token up to several chunks against the recurrence in float64.  An operand as two bfloat16 is right
+    to 2^-17, a product of two to 2^-16 of its factors' norms; an output has passed four of them in a row: 2^-14 of the
+    largest."""
+    delta, head = "delta" in rule, "head" in rule
+    g = _gen(dk + dv + len(rule) + len(decay))
+    lens = [1, 2, 15, 16, 17, 63, 64, 65, 130, 200]
+    n_slots, first = len(lens) + 2, 2   # the first two entries of the step are somebody else's
+    T = sum(lens)
+
+    def rnd(*shape):
+        return torch.randn(shape, generator=g, device="cuda")
+
+    q, k = (torch.nn.functional.normalize(rnd(T, G, dk), dim=-1) for _ in range(2))
+    v = rnd(T, H, dv)
+    shape = (T, H) if head else (T, H, dk)
+    u = torch.rand(shape, generator=g, device="cuda")
+    a = {"any": u, "slow": 1 - 0.02 * u, "strong": torch.where(u < 0.1, torch.zeros_like(u), torch.where(u < 0.3, 1e-30 * u, 0.9 + 0.1 * u))}[decay]
+    beta = torch.rand((T, H), generator=g, device="cuda") if delta else None
+    state = rnd(n_slots, H, dv, dk)
+    slots = torch.randperm(n_slots, generator=torch.Generator().manual_seed(3)).tolist()
+    cu = [0] + torch.tensor(lens).cumsum(0).tolist()
+    want, after = torch.zeros(T, H, dv, dtype=torch.float64, device="cuda"), state.double()
+    for e, slot in enumerate(slots[:len(lens)]):
+        if e < first:
+            continue
+        s = slice(cu[e], cu[e + 1])
+        rep = H // G
+        want[s], after[slot] = _recurrence64(
+            q[s].double().repeat_interleave(rep, 1), k[s].double().repeat_interleave(rep, 1), v[s].double(),
+            (a[s, :, None] if head else a[s]).double(), beta[s].double() if delta else None, state[slot].double())
+    out = torch.zeros(T, H, dv, device="cuda")
+    bufs = {}
+
+    def scratch(key, per, shape, dtype):
+        n = T if per == "tokens" else T // 64 + len(lens)
+        bufs[key] = torch.full((n,) + tuple(shape), float("nan"), dtype=dtype, device="cuda")
+        return bufs[key]
+
+    def dev(x):
+        return torch.tensor(x, dtype=torch.int32, device="cuda")
+
+    _k().chunk_recurrence(scratch, q.clone(), k.clone(), v.clone(), a.clone(), beta, state, out, dev(cu), dev(slots[:len(lens)]),
+                          first, len(lens) - first, max(lens), G, H, dk, dv)
+    assert torch.isfinite(out).all() and torch.isfinite(state).all()
+    assert (out.double() - want).abs().max() <= 2.0 ** -14 * want.abs().max()
+    assert (state.double() - after).abs().max() <= 2.0 ** -14 * after.abs().max()

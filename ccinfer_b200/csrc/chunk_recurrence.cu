@@ -12,13 +12,15 @@
 //
 // so only the last line walks the chunks in order; everything before it is independent of the memory.  Two kernels:
 //
-//   chunk_prepare  a block per (chunk, head): the sums of logarithms, M and P, the triangular solve (a thread a column,
-//                  its 64 values in registers, float multiply-adds), and the scaled rows of q and k
+//   chunk_prepare  a block per (chunk, head): the sums of logarithms, M and P, the scaled rows of q and k, and the
+//                  triangular solve: the four 16 x 16 blocks on the diagonal are inverted in float, the rest are products
+//                  of a warp's 32 columns, transposed, so that one block's result is the next one's operand as it is
 //   chunk_walk     a block per (request, head, 32 value columns), eight warps: the memory in float registers, four
 //                  products a chunk on mma.sync; a warp takes 16 rows x 16 columns of u and o and 16 key channels of S
 //
-// Exponents of decays are never positive: within a run of 16 tokens every pair's decay is taken per channel as it is, and
-// between runs both factors refer to a place between them.  Logarithms are summed within a run and runs are added up, so
+// Exponents of decays are never positive between runs of 16 tokens, where both factors refer to a place between them.
+// Within a run they refer to its eighth token where every channel stays within 2^-55 of it, which slow and ordinary
+// decays do; else every pair's decay is taken per channel as it is, one exponential each.  Logarithms are summed within a run and runs are added up, so
 // that a difference never cancels more than a run's sum.  What the model computes in 32 bits stays so to about 2^-17:
 // logarithms, sums, exponentials, the solve and the memory are float, and every operand of a product (rows, scores,
 // memory) goes in as TWO bfloat16, its rounding and what the rounding left, in three products.  A decay below 2^-115
@@ -38,6 +40,7 @@ constexpr int kChunk = 64;
 constexpr int kThreads = 256;
 constexpr int kRun = 16;           // tokens of a run
 constexpr float kLeastLog2 = -115.f;
+constexpr float kSteepLog2 = 55.f;   // (2^110 times 128 products stays in a float, also in places that nobody sees)
 
 struct ChunkRows {
   const float *q, *k, *v, *g, *beta;   // q, k [T, G, DK]; v [T, H, dv]; g [T, H, DK], or [T, H] with one decay a head
@@ -76,11 +79,12 @@ __device__ __forceinline__ void mma3(float* c, const uint32_t* ah, const uint32_
 template <int DK> __device__ __forceinline__ int at(int row, int col) { return row * DK + (col ^ ((row & 3) << 3)); }
 
 constexpr int kPitchL = kChunk;
+__device__ __forceinline__ int lat(int t, int s) { return t * kPitchL + (s ^ ((t & 3) << 3)); }   // place (t, s) of l_s
 
 template <int DK, bool DELTA, bool HEAD> struct PrepShape {
   static constexpr int kC = HEAD ? kChunk : kChunk * DK;   // sums of logarithms
   static constexpr int kFloats = 2 * kChunk * DK + kC + (DELTA ? kChunk * kPitchL : 0) + kChunk;   // (two blocks an SM)
-  static constexpr int kBytes = kFloats * 4 + 16;
+  static constexpr int kBytes = kFloats * 4 + 16;   // (two blocks an SM)
 };
 
 // 32 values a lane, one for each lane: the sum of value i over all lanes ends in lane i
@@ -108,7 +112,8 @@ chunk_prepare_kernel(const ChunkRows a) {
   float* c_s = k_s + kChunk * DK;            // [64][DK] or [64]: log2 of the decay since the token's run began
   float* l_s = c_s + Sh::kC;                 // [64][64]: diag(beta) M below the diagonal
   float* b_s = l_s + (DELTA ? kChunk * kPitchL : 0);
-  int* next_row = reinterpret_cast<int*>(b_s + kChunk);
+  int* next_item = reinterpret_cast<int*>(b_s + kChunk);
+  int* steep = next_item + 1;                // a bit for each run that takes every pair's decay by itself
 
   const int e = a.entry0 + blockIdx.z, h = blockIdx.y, chunk = blockIdx.x;
   const int first = a.cu_q[e], n = a.cu_q[e + 1] - first;
@@ -130,7 +135,8 @@ chunk_prepare_kernel(const ChunkRows a) {
     *reinterpret_cast<float4*>(k_s + at<DK>(t, c)) = k;
   }
   if (tid < kChunk) b_s[tid] = DELTA && tid < cnt ? a.beta[(size_t)(r0 + tid) * a.H + h] : 0.f;
-  if (tid == 0) *next_row = 0;
+  if (tid == 0) *next_item = *steep = 0;
+  __syncthreads();
   auto log_decay = [](float g) {
     const float x = log2f(g);
     return x < kLeastLog2 ? kLeastLog2 : x;
@@ -164,12 +170,21 @@ chunk_prepare_kernel(const ChunkRows a) {
       const int t = part * PT + i;
       x[i] = t < cnt ? a.g[((size_t)(r0 + t) * a.H + h) * DK + d] : 1.f;
     }
-    float sum = 0.f;
+    int mine = 0;
 #pragma unroll
-    for (int i = 0; i < PT; ++i) {
-      sum = (i % kRun == 0 ? 0.f : sum) + log_decay(x[i]);
-      c_s[at<DK>(part * PT + i, d)] = sum;
+    for (int m = 0; m < PT / kRun; ++m) {
+      float sum = 0.f, first_sum = 0.f, mid = 0.f;
+#pragma unroll
+      for (int i = 0; i < kRun; ++i) {
+        sum += log_decay(x[m * kRun + i]);
+        c_s[at<DK>(part * PT + m * kRun + i, d)] = sum;
+        if (i == 0) first_sum = sum;
+        if (i == kRun / 2 - 1) mid = sum;
+      }
+      if (!(first_sum - mid <= kSteepLog2 && mid - sum <= kSteepLog2)) mine |= 1 << (part * (PT / kRun) + m);
     }
+    mine = __reduce_or_sync(0xffffffffu, mine);
+    if (mine != 0 && lane == 0) atomicOr(steep, mine);
   }
   __syncthreads();
   auto in_run = [&](int t, int d) { return HEAD ? c_s[t] : c_s[at<DK>(t, d)]; };
@@ -184,14 +199,22 @@ chunk_prepare_kernel(const ChunkRows a) {
   const size_t p_row = (size_t)a.H * 2 * kChunk;   // elements from a token's scores to the next one's
   __nv_bfloat16* p_out = a.p + ((size_t)r0 * a.H + h) * 2 * kChunk;
 
-  // ---- blocks of 16 x 16 pairs: rows of run i, columns of run j (j < i; with one decay a head also j = i)
+  // ---- blocks of 16 x 16 pairs, a warp each, to whoever is free: rows of run i, columns of run j
   const int gid = lane >> 2, tig = lane & 3;
-  constexpr int kPairs = HEAD ? 10 : 6;
-  for (int unit = warp; unit < kPairs; unit += kThreads / 32) {
-    int i = HEAD ? 0 : 1, j = unit;
-    while (j >= (HEAD ? i + 1 : i)) { j -= HEAD ? i + 1 : i; ++i; }
-    if (i * kRun >= cnt) continue;
-    const int edge = (j + 1) * kRun - 1;   // the place that both factors refer to: the end of run j
+  const int steep_runs = HEAD ? 0 : *steep;
+  auto take = [&]() {
+    int item = 0;
+    if (lane == 0) item = atomicAdd(next_item, 1);
+    return __shfl_sync(0xffffffffu, item, 0);
+  };
+  constexpr int kPairs = 10;
+  int item = take();
+  for (; item < kPairs; item = take()) {
+    int i = 0, j = item;
+    while (j > i) j -= ++i;
+    if (i * kRun >= cnt || (i == j && (steep_runs >> i & 1))) continue;
+    // the place that both factors refer to: the end of run j, or the middle of a run
+    const int edge = (j + 1) * kRun - 1 - (i == j ? kRun / 2 : 0);
     float sq[2][4], sk[2][4];
 #pragma unroll
     for (int x = 0; x < 2; ++x)
@@ -220,6 +243,7 @@ chunk_prepare_kernel(const ChunkRows a) {
           if (DELTA) k = *reinterpret_cast<const float2*>(k_s + at<DK>(t, col));
           if (!HEAD) {
             const float2 c = *reinterpret_cast<const float2*>(c_s + at<DK>(t, col));
+            if (i == j) mid = make_float2(-ce.x, -ce.y);
             const float fx = ex2(c.x + mid.x), fy = ex2(c.y + mid.y);
             q.x *= fx; q.y *= fy;
             k.x *= fx; k.y *= fy;
@@ -250,35 +274,34 @@ chunk_prepare_kernel(const ChunkRows a) {
 #pragma unroll
       for (int up = 0; up < 2; ++up) {
         const int t = i * kRun + gid + 8 * up, s = j * kRun + nb * 8 + 2 * tig;
-        float f0 = 1.f, f1 = 1.f;
+        float f[2] = {1.f, 1.f};
         if (HEAD) {
-          f0 = s <= t ? ex2(i == j ? c_s[t] - c_s[s] : c_s[t] + (over_runs(j + 1, i, 0) + (c_s[edge] - c_s[s]))) : 0.f;
-          f1 = s + 1 <= t ? ex2(i == j ? c_s[t] - c_s[s + 1] : c_s[t] + (over_runs(j + 1, i, 0) + (c_s[edge] - c_s[s + 1]))) : 0.f;
+          const int end = (j + 1) * kRun - 1;
+#pragma unroll
+          for (int x = 0; x < 2; ++x)
+            f[x] = ex2(i == j ? fminf(c_s[t] - c_s[s + x], 0.f) : c_s[t] + (over_runs(j + 1, i, 0) + (c_s[end] - c_s[s + x])));
         }
+        const float p0 = s <= t ? sq[nb][2 * up] * f[0] : 0.f, p1 = s + 1 <= t ? sq[nb][2 * up + 1] * f[1] : 0.f;
         if (t < cnt) {
           uint32_t hi, lo;
-          split2(sq[nb][2 * up] * f0, sq[nb][2 * up + 1] * f1, hi, lo);
+          split2(p0, p1, hi, lo);
           *reinterpret_cast<uint32_t*>(p_out + t * p_row + s) = hi;
           *reinterpret_cast<uint32_t*>(p_out + t * p_row + kChunk + s) = lo;
         }
         if (DELTA) {
           const float b = b_s[t];
-          l_s[t * kPitchL + s] = !HEAD || s < t ? sk[nb][2 * up] * f0 * b : 0.f;
-          l_s[t * kPitchL + s + 1] = !HEAD || s + 1 < t ? sk[nb][2 * up + 1] * f1 * b : 0.f;
+          l_s[lat(t, s)] = s < t ? sk[nb][2 * up] * f[0] * b : 0.f;
+          l_s[lat(t, s + 1)] = s + 1 < t ? sk[nb][2 * up + 1] * f[1] * b : 0.f;
         }
       }
   }
   // ---- pairs within a run, a decay for every pair and channel: a warp a row, its lanes the channels.  Rows with many
-  // pairs first, to whoever is free.
-  if constexpr (!HEAD) {
+  // pairs first.
+  if (!HEAD && steep_runs) {
     constexpr int CL = DK / 32;   // channels a lane
-    for (;;) {
-      int item = 0;
-      if (lane == 0) item = atomicAdd(next_row, 1);
-      item = __shfl_sync(0xffffffffu, item, 0);
-      if (item >= kChunk) break;
-      const int run = item & 3, lt = kRun - 1 - (item >> 2), t = run * kRun + lt;
-      if (t >= cnt) continue;
+    for (; item < kPairs + kChunk; item = take()) {
+      const int run = (item - kPairs) & 3, lt = kRun - 1 - ((item - kPairs) >> 2), t = run * kRun + lt;
+      if (t >= cnt || !(steep_runs >> run & 1)) continue;
       float q[CL], k[CL], c[CL], v[32];
 #pragma unroll
       for (int x = 0; x < CL; ++x) {
@@ -306,71 +329,136 @@ chunk_prepare_kernel(const ChunkRows a) {
         p_out[t * p_row + run * kRun + s] = hi;
         p_out[t * p_row + kChunk + run * kRun + s] = __float2bfloat16_rn(x - __bfloat162float(hi));
       } else if (DELTA) {
-        l_s[t * kPitchL + run * kRun + s] = s < lt ? sum * b_s[t] : 0.f;
+        l_s[lat(t, run * kRun + s)] = s < lt ? sum * b_s[t] : 0.f;
       }
     }
   }
   // ---- the rows that meet the memory: q e^c, k e^{c_64 - c}, and e^{c_64}
-  for (int i = tid; i < kChunk * DK / 2; i += kThreads) {
-    const int t = i / (DK / 2), d = 2 * (i % (DK / 2)), run = t / kRun;
-    if (t >= cnt) break;
-    const float2 q = *reinterpret_cast<const float2*>(q_s + at<DK>(t, d)), k = *reinterpret_cast<const float2*>(k_s + at<DK>(t, d));
-    float fq[2], fk[2];
-#pragma unroll
-    for (int x = 0; x < 2; ++x) {
-      const float c = in_run(t, d + x);
-      fq[x] = ex2(over_runs(0, run, d + x) + c);
-      fk[x] = ex2(over_runs(run + 1, kChunk / kRun, d + x) + (in_run(run * kRun + kRun - 1, d + x) - c));   // (rows past the end decay nothing)
+  {   // a thread two channels of some rows of a run
+    constexpr int PARTS = kThreads / (DK / 2), ROWS = kChunk / PARTS;
+    const int d = 2 * (tid % (DK / 2)), t0 = (tid / (DK / 2)) * ROWS, run = t0 / kRun;
+    const float before[2] = {over_runs(0, run, d), over_runs(0, run, d + 1)};
+    const float after[2] = {over_runs(run + 1, kChunk / kRun, d), over_runs(run + 1, kChunk / kRun, d + 1)};
+    const float end[2] = {in_run(run * kRun + kRun - 1, d), in_run(run * kRun + kRun - 1, d + 1)};   // (rows past the end decay nothing)
+#pragma unroll 4
+    for (int t = t0; t < min(t0 + ROWS, cnt); ++t) {
+      const float2 q = *reinterpret_cast<const float2*>(q_s + at<DK>(t, d)), k = *reinterpret_cast<const float2*>(k_s + at<DK>(t, d));
+      const float c0 = in_run(t, d), c1 = in_run(t, d + 1);
+      const size_t row = ((size_t)(r0 + t) * a.H + h) * 2 * DK + d;
+      uint32_t hi, lo;
+      split2(q.x * ex2(before[0] + c0), q.y * ex2(before[1] + c1), hi, lo);
+      *reinterpret_cast<uint32_t*>(a.qs + row) = hi;
+      *reinterpret_cast<uint32_t*>(a.qs + row + DK) = lo;
+      split2(k.x * ex2(after[0] + (end[0] - c0)), k.y * ex2(after[1] + (end[1] - c1)), hi, lo);
+      *reinterpret_cast<uint32_t*>(a.ks + row) = hi;
+      *reinterpret_cast<uint32_t*>(a.ks + row + DK) = lo;
     }
-    const size_t row = ((size_t)(r0 + t) * a.H + h) * 2 * DK;
-    uint32_t hi, lo;
-    split2(q.x * fq[0], q.y * fq[1], hi, lo);
-    *reinterpret_cast<uint32_t*>(a.qs + row + d) = hi;
-    *reinterpret_cast<uint32_t*>(a.qs + row + DK + d) = lo;
-    split2(k.x * fk[0], k.y * fk[1], hi, lo);
-    *reinterpret_cast<uint32_t*>(a.ks + row + d) = hi;
-    *reinterpret_cast<uint32_t*>(a.ks + row + DK + d) = lo;
   }
   const int place = (first >> 6) + e + chunk;   // (distinct: an entry's last chunk comes before the next entry's first)
   for (int d = tid; d < DK; d += kThreads) a.keep[((size_t)place * a.H + h) * DK + d] = ex2(over_runs(0, kChunk / kRun, d));
 
-  // ---- the triangular solve: a thread a column of [K e^c | V]
+  // ---- the triangular solve for X = [W | U]: with L the strictly lower blocks, X_i = (I + L_ii)^-1 (B_i - sum L_ij X_j)
   if constexpr (DELTA) {
     __syncthreads();
-    for (int col = tid; col < DK + a.dv; col += kThreads) {
-      const bool is_w = col < DK;
-      float x[kChunk];
+    if (tid < kChunk) {   // a thread a column of an inverse, which takes its block's place
+      const int run = tid / kRun, c = tid % kRun;
+      float y[kRun];
 #pragma unroll
-      for (int t = 0; t < kChunk; ++t) {
-        float y = 0.f;
-        if (t < cnt)
-          y = is_w ? k_s[at<DK>(t, col)] * ex2(over_runs(0, t / kRun, col) + in_run(t, col)) : a.v[((size_t)(r0 + t) * a.H + h) * a.dv + col - DK];
-        x[t] = y * b_s[t];
-      }
+      for (int t = 0; t < kRun; ++t) {
+        float x = t == c ? 1.f : 0.f;
+        if (run * kRun + t < cnt) {
 #pragma unroll
-      for (int t = 1; t < kChunk; ++t) {
-        float y[4] = {x[t], 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int s = 0; s < t; s += 4) {
-          const float4 l = *reinterpret_cast<const float4*>(l_s + t * kPitchL + s);   // (zero from the diagonal on)
-          y[0] = fmaf(-l.x, x[s], y[0]);
-          if (s + 1 < t) y[1] = fmaf(-l.y, x[s + 1], y[1]);
-          if (s + 2 < t) y[2] = fmaf(-l.z, x[s + 2], y[2]);
-          if (s + 3 < t) y[3] = fmaf(-l.w, x[s + 3], y[3]);
+          for (int s = 0; s < t; ++s) x = fmaf(-l_s[lat(run * kRun + t, run * kRun + s)], y[s], x);
         }
-        x[t] = (y[0] + y[1]) + (y[2] + y[3]);
+        y[t] = x;
       }
+      __syncwarp();
 #pragma unroll
-      for (int t = 0; t < kChunk; ++t) {
-        if (t >= cnt) continue;
-        if (is_w) {
-          const __nv_bfloat16 hi = __float2bfloat16_rn(x[t]);
-          const size_t row = ((size_t)(r0 + t) * a.H + h) * 2 * DK + col;
-          a.w[row] = hi;
-          a.w[row + DK] = __float2bfloat16_rn(x[t] - __bfloat162float(hi));
-        } else {
-          a.u[((size_t)(r0 + t) * a.H + h) * a.dv + col - DK] = x[t];
+      for (int t = 0; t < kRun; ++t) l_s[lat(run * kRun + t, run * kRun + c)] = y[t];
+    }
+    __syncthreads();
+    const int runs = (cnt + kRun - 1) / kRun;
+    // A warp 16 columns at a time: the transposed block [columns, tokens] is an accumulator, and split in two an A operand
+    for (int c0 = 16 * warp; c0 < DK + a.dv; c0 += 16 * (kThreads / 32)) {
+      const bool is_w = c0 < DK;
+      uint32_t xh[3][4], xl[3][4];   // X_j of the runs before
+      float before[2] = {0.f, 0.f};
+#pragma unroll
+      for (int i = 0; i < kChunk / kRun; ++i) {
+        if (i >= runs) break;
+        float x[2][4];   // [8 tokens][place]
+#pragma unroll
+          for (int up = 0; up < 2; ++up) {
+            const int col = c0 + gid + 8 * up;
+#pragma unroll
+            for (int nb = 0; nb < 2; ++nb)
+#pragma unroll
+              for (int y = 0; y < 2; ++y) {
+                const int t = i * kRun + nb * 8 + 2 * tig + y;
+                float b = 0.f;
+                if (t < cnt)
+                  b = is_w ? k_s[at<DK>(t, col)] * ex2(before[up] + in_run(t, col))
+                           : a.v[((size_t)(r0 + t) * a.H + h) * a.dv + col - DK];
+                x[nb][2 * up + y] = b * b_s[t];
+              }
+            if (is_w) before[up] += in_run(i * kRun + kRun - 1, col);
+          }
+#pragma unroll
+        for (int j = 0; j < i; ++j) {
+#pragma unroll
+          for (int nb = 0; nb < 2; ++nb) {
+            uint32_t bh[2], bl[2];
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+              const int t = i * kRun + nb * 8 + gid;
+              const float2 l = *reinterpret_cast<const float2*>(l_s + lat(t, j * kRun + 8 * half + 2 * tig));
+              split2(t < cnt ? -l.x : 0.f, t < cnt ? -l.y : 0.f, bh[half], bl[half]);
+            }
+            mma3(x[nb], xh[j], xl[j], bh[0], bh[1], bl[0], bl[1]);
+          }
         }
+        uint32_t ah[4], al[4];
+#pragma unroll
+          for (int nb = 0; nb < 2; ++nb)
+#pragma unroll
+            for (int up = 0; up < 2; ++up) {
+              split2(x[nb][2 * up], x[nb][2 * up + 1], ah[2 * nb + up], al[2 * nb + up]);
+              x[nb][2 * up] = x[nb][2 * up + 1] = 0.f;
+            }
+#pragma unroll
+        for (int nb = 0; nb < 2; ++nb) {
+          uint32_t bh[2], bl[2];
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            const float2 l = *reinterpret_cast<const float2*>(l_s + lat(i * kRun + nb * 8 + gid, i * kRun + 8 * half + 2 * tig));
+            split2(l.x, l.y, bh[half], bl[half]);
+          }
+          mma3(x[nb], ah, al, bh[0], bh[1], bl[0], bl[1]);
+        }
+#pragma unroll
+          for (int nb = 0; nb < 2; ++nb)
+#pragma unroll
+            for (int up = 0; up < 2; ++up) {
+              uint32_t hi, lo;
+              split2(x[nb][2 * up], x[nb][2 * up + 1], hi, lo);
+              if (i < 3) {
+                xh[i < 3 ? i : 0][2 * nb + up] = hi;
+                xl[i < 3 ? i : 0][2 * nb + up] = lo;
+              }
+              const int col = c0 + gid + 8 * up;
+#pragma unroll
+              for (int y = 0; y < 2; ++y) {
+                const int t = i * kRun + nb * 8 + 2 * tig + y;
+                if (t >= cnt) continue;
+                if (is_w) {
+                  unsigned short* w = reinterpret_cast<unsigned short*>(a.w) + ((size_t)(r0 + t) * a.H + h) * 2 * DK + col;
+                  w[0] = (unsigned short)(hi >> (16 * y));
+                  w[DK] = (unsigned short)(lo >> (16 * y));
+                } else {
+                  a.u[((size_t)(r0 + t) * a.H + h) * a.dv + col - DK] = x[nb][2 * up + y];
+                }
+              }
+            }
       }
     }
   }

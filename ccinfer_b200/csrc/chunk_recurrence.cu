@@ -26,8 +26,9 @@
 // memory) goes in as TWO bfloat16, its rounding and what the rounding left, in three products.  A decay below 2^-115
 // counts as that: it keeps nothing that a float can tell from zero.
 //
-// Bound by: the walk by the chain of its products (one block an SM), the preparation by what it issues.  Measured on B200,
-// 2,048 tokens of one request, 32 heads of 128 x 128: see launch_walk.
+// Bound by: the walk by the chain of its products (one block of eight warps an SM, an instruction on 0.31 of the cycles),
+// the preparation by what it issues (0.42).  Measured on B200, 2,048 tokens of one request, 32 heads of 128 x 128 with a
+// decay per channel and the delta rule: 189 + 103 us; token by token 959 us.
 #include "common.cuh"
 #include "mma_common.cuh"
 #include <type_traits>

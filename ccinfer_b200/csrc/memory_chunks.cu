@@ -18,6 +18,11 @@
 // for the read-out and DK / 4 key channels of S for the update.  With a column of ones after the values (a running sum
 // of the keys: n . q is one more column of o) the first slice takes it as one more block of eight columns.
 // The next chunk's rows arrive through cp.async while this one is computed; two barriers a chunk.
+//
+// A state space layer's recurrence is the same with values that are floats (they enter as two bfloat16 as well, one barrier
+// a chunk more) and with groups of heads that share queries and keys.  2,048 tokens of two requests, 128 heads of 64 x 128:
+// 1,034 us token by token, 459 us in chunks (one block of four warps an SM: the two halves of queries and keys fill its
+// shared memory).
 #include "common.cuh"
 #include "mma_common.cuh"
 #include <math_constants.h>
@@ -31,7 +36,9 @@ constexpr int kThreads = 128;
 
 struct ChunkArgs {
   const __nv_bfloat16 *q, *q_lo, *k, *k_lo, *v;
+  const float* v32;           // float values in v's place
   int ldqk, ldv;              // row strides (q and k in one; q_lo, k_lo as q and k)
+  int group;                  // neighbouring heads that share queries and keys
   const float* log_a;         // [tokens, H]
   const float* log_b;         // [tokens, H] or null: zero
   float* state;               // [slots, H, dvo, DK]
@@ -49,7 +56,7 @@ __device__ __forceinline__ void split2(float x, float y, uint32_t& hi, uint32_t&
   lo = pack_bf16(x - f.x, y - f.y);
 }
 
-template <int DK, int NB, bool SPLIT, bool ONES>
+template <int DK, int NB, bool SPLIT, bool ONES, bool V32>
 __global__ void __launch_bounds__(kThreads)
 memory_chunks_kernel(const ChunkArgs a) {
   ccb::pdl_begin();
@@ -61,12 +68,13 @@ memory_chunks_kernel(const ChunkArgs a) {
   constexpr int QK = SPLIT ? 4 : 2;            // tiles of a stage: q, k (, their second halves)
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __nv_bfloat16* tiles = reinterpret_cast<__nv_bfloat16*>(smem_raw);   // [2][QK][64][DK], swizzled
-  __nv_bfloat16* v_s = tiles + 2 * QK * TILE;                          // [2][64][VP]
+  __nv_bfloat16* v_s = tiles + 2 * QK * TILE;                          // [2][64][VP] (V32: the values' two halves)
   __nv_bfloat16* s_hi = v_s + 2 * VT;                                  // [DK][VP]
   __nv_bfloat16* s_lo = s_hi + DK * VP;
   __nv_bfloat16* w_hi = s_lo + DK * VP;                                // [64][VP]
   __nv_bfloat16* w_lo = w_hi + VT;
   float* gates = reinterpret_cast<float*>(w_lo + VT);                  // [2][4][64]: c_t, exp(c_t), log b - c, weights
+  float* v32_s = gates + 2 * 4 * kChunk;                               // V32: [2][64][BN]
 
   const int e = a.entry0 + blockIdx.z, h = blockIdx.y, slice = blockIdx.x;
   const int slot = a.state_slot[e];
@@ -74,6 +82,7 @@ memory_chunks_kernel(const ChunkArgs a) {
   if (slot < 0 || slot >= a.max_slots || n <= 0) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gid = lane >> 2, tig = lane & 3;
+  const int kvh = h / a.group;
   const int col0 = slice * BN;
   const bool ones = ONES && slice == 0;
   const int nt = NB + (ones ? 1 : 0);
@@ -90,8 +99,20 @@ memory_chunks_kernel(const ChunkArgs a) {
         const int row = idx / (DK / 8), c = idx % (DK / 8);
         const bool ok = t0 + row < n;
         cp_async16(smem_u32(dst + x * TILE + swz<DK>(row, c)),
-                   src[x] + (size_t)(r0 + t0 + (ok ? row : 0)) * a.ldqk + h * DK + c * 8, ok);
+                   src[x] + (size_t)(r0 + t0 + (ok ? row : 0)) * a.ldqk + kvh * DK + c * 8, ok);
       }
+    if constexpr (V32) {
+#pragma unroll
+      for (int i = 0; i < kChunk * 2 * NB / kThreads; ++i) {
+        const int idx = tid + kThreads * i;
+        const int row = idx / (2 * NB), c = idx % (2 * NB);
+        const bool ok = t0 + row < n;
+        cp_async16(smem_u32(v32_s + (st * kChunk + row) * BN + c * 4),
+                   a.v32 + (size_t)(r0 + t0 + (ok ? row : 0)) * a.ldv + h * a.dv + col0 + c * 4, ok);
+      }
+      cp_async_commit();
+      return;
+    }
 #pragma unroll
     for (int i = 0; i < (kChunk * NB + kThreads - 1) / kThreads; ++i) {
       const int idx = tid + kThreads * i;
@@ -141,8 +162,9 @@ memory_chunks_kernel(const ChunkArgs a) {
     load_gates(1);
   }
   // the column of ones beside the values (and zeros after it): the same in both stages, for good
-  for (int i = tid; i < 2 * kChunk * 8; i += kThreads)
-    v_s[(i >> 3) * VP + BN + (i & 7)] = __float2bfloat16_rn((i & 7) == 0 && ones ? 1.f : 0.f);
+  if constexpr (!V32)   // (V32 has no such column)
+    for (int i = tid; i < 2 * kChunk * 8; i += kThreads)
+      v_s[(i >> 3) * VP + BN + (i & 7)] = __float2bfloat16_rn((i & 7) == 0 && ones ? 1.f : 0.f);
   for (int i = tid; i < kChunk * 8; i += kThreads) {
     w_hi[(i >> 3) * VP + BN + (i & 7)] = __float2bfloat16_rn(0.f);
     w_lo[(i >> 3) * VP + BN + (i & 7)] = __float2bfloat16_rn(0.f);
@@ -199,12 +221,26 @@ memory_chunks_kernel(const ChunkArgs a) {
       load_gates(ch + 2);
     }
     const __nv_bfloat16 *qt = tiles + st * QK * TILE, *kt = qt + TILE, *ql = qt + 2 * TILE, *kl = qt + 3 * TILE;
-    const __nv_bfloat16* vt = v_s + st * VT;
+    const __nv_bfloat16* vt = v_s + (V32 ? 0 : st * VT);
     const float *gc = gates + st * 4 * kChunk, *ga = gc + kChunk, *gb = ga + kChunk, *gw = gb + kChunk;
 
     {   // the values times their weights in the chunk's contribution to S
       const int row = tid >> 1, part = (tid & 1) * (BN / 2);
       const float w = gw[row];
+      if constexpr (V32) {
+        const float* v32 = v32_s + (st * kChunk + row) * BN + part;
+#pragma unroll
+        for (int c = 0; c < BN / 2; c += 2) {
+          const float2 f = *reinterpret_cast<const float2*>(v32 + c);
+          uint32_t hi, lo;
+          split2(f.x, f.y, hi, lo);
+          *reinterpret_cast<uint32_t*>(v_s + row * VP + part + c) = hi;
+          *reinterpret_cast<uint32_t*>(v_s + VT + row * VP + part + c) = lo;
+          split2(f.x * w, f.y * w, hi, lo);
+          *reinterpret_cast<uint32_t*>(w_hi + row * VP + part + c) = hi;
+          *reinterpret_cast<uint32_t*>(w_lo + row * VP + part + c) = lo;
+        }
+      } else {
 #pragma unroll
       for (int c = 0; c < BN / 2; c += 2) {
         const __nv_bfloat162 x = *reinterpret_cast<const __nv_bfloat162*>(vt + row * VP + part + c);
@@ -213,6 +249,7 @@ memory_chunks_kernel(const ChunkArgs a) {
         split2(f.x * w, f.y * w, hi, lo);
         *reinterpret_cast<uint32_t*>(w_hi + row * VP + part + c) = hi;
         *reinterpret_cast<uint32_t*>(w_lo + row * VP + part + c) = lo;
+      }
       }
       if (ones && (tid & 1) == 0) {
         const __nv_bfloat16 hi = __float2bfloat16_rn(w);
@@ -266,6 +303,7 @@ memory_chunks_kernel(const ChunkArgs a) {
         }
       }
     }
+    if (V32) __syncthreads();   // the values' halves are complete
     const int t_lo = warp * 16 + gid, t_hi = t_lo + 8;
     const float a_lo = ga[t_lo] * a.q_mult, a_hi = ga[t_hi] * a.q_mult;
     const float c_lo = gc[t_lo], c_hi = gc[t_hi];
@@ -301,6 +339,11 @@ memory_chunks_kernel(const ChunkArgs a) {
         if (!single) {
           mma_bf16_16816(acc[nb + 1 < NT ? nb + 1 : nb], ph, b[2], b[3]);
           mma_bf16_16816(acc[nb + 1 < NT ? nb + 1 : nb], pl, b[2], b[3]);
+        }
+        if constexpr (V32) {
+          load_b(vt + VT, np * 16, nb, single, b);
+          mma_bf16_16816(acc[nb], ph, b[0], b[1]);
+          if (!single) mma_bf16_16816(acc[nb + 1 < NT ? nb + 1 : nb], ph, b[2], b[3]);
         }
       }
     }
@@ -372,20 +415,20 @@ memory_chunks_kernel(const ChunkArgs a) {
       }
 }
 
-template <int DK, int NB, bool SPLIT, bool ONES>
+template <int DK, int NB, bool SPLIT, bool ONES, bool V32 = false>
 int launch_chunks(const ChunkArgs& a, int n_entries, cudaStream_t stream) {
   constexpr int VP = 8 * NB + 8;
   constexpr size_t smem = (size_t)(2 * (SPLIT ? 4 : 2) * kChunk * DK + 2 * kChunk * VP + 2 * DK * VP + 2 * kChunk * VP) * 2 +
-                          2 * 4 * kChunk * sizeof(float);
+                          2 * 4 * kChunk * sizeof(float) + (V32 ? (size_t)2 * kChunk * 8 * NB * sizeof(float) : 0);
   static_assert(smem <= 227 * 1024, "shared memory of a block");
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(memory_chunks_kernel<DK, NB, SPLIT, ONES>,
+    cudaError_t e = cudaFuncSetAttribute(memory_chunks_kernel<DK, NB, SPLIT, ONES, V32>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  ccb_launch(memory_chunks_kernel<DK, NB, SPLIT, ONES>, dim3(a.dv / (8 * NB), a.H, n_entries), dim3(kThreads), smem, stream,
+  ccb_launch(memory_chunks_kernel<DK, NB, SPLIT, ONES, V32>, dim3(a.dv / (8 * NB), a.H, n_entries), dim3(kThreads), smem, stream,
              a);
   return ccb_launch_status();
 }
@@ -415,10 +458,28 @@ CCB_API int ccb_memory_chunks(const void* q, const void* q_lo, const void* k, co
   if ((bits(q) | bits(q_lo) | bits(k) | bits(k_lo) | bits(v)) & 15) return CCB_REFUSE_ARG;
   const __nv_bfloat16 *qp = (const __nv_bfloat16*)q, *qlp = (const __nv_bfloat16*)q_lo, *kp = (const __nv_bfloat16*)k,
                       *klp = (const __nv_bfloat16*)k_lo, *vp = (const __nv_bfloat16*)v;
-  const ChunkArgs a{qp, qlp, kp, klp, vp, ldqk, ldv, log_a, log_b, state, out, cu_q, state_slot, entry0, H, dv, dvo,
+  const ChunkArgs a{qp, qlp, kp, klp, vp, nullptr, ldqk, ldv, 1, log_a, log_b, state, out, cu_q, state_slot, entry0, H, dv, dvo,
                     max_slots, q_mult};
   // slices of 32 columns where they give enough blocks, else of 16
   const bool wide = dv % 32 == 0 && (long long)(dv / 32) * H * n_entries >= 96;
   if (dk == 128) return wide ? pick_chunks<128, 4>(a, n_entries, stream) : pick_chunks<128, 2>(a, n_entries, stream);
   return wide ? pick_chunks<64, 4>(a, n_entries, stream) : pick_chunks<64, 2>(a, n_entries, stream);
+}
+
+// The same for a state space layer: values float [tokens, H, P] (their rows ldv apart), queries and keys of G groups of N
+// coordinates [tokens, ldqk] as two bfloat16 each; N 64 or 128, P a multiple of 16.
+CCB_API int ccb_ssm_chunks(const void* q, const void* q_lo, const void* k, const void* k_lo, int ldqk, const float* v, int ldv,
+                           const float* log_a, const float* log_b, float* state, float* out, const int* cu_q,
+                           const int* state_slot, int entry0, int n_entries, int G, int H, int N, int P, int max_slots,
+                           cudaStream_t stream) {
+  if (n_entries <= 0) return 0;
+  if (G <= 0 || H <= 0 || H % G || (N != 64 && N != 128) || P <= 0 || P % 16 || ldqk % 8 || ldv % 4) return CCB_REFUSE_SIZE;
+  if (q_lo == nullptr || k_lo == nullptr || log_a == nullptr) return CCB_REFUSE_ARG;
+  const auto bits = [](const void* p) { return reinterpret_cast<uintptr_t>(p); };
+  if ((bits(q) | bits(q_lo) | bits(k) | bits(k_lo) | bits(v)) & 15) return CCB_REFUSE_ARG;
+  const ChunkArgs a{(const __nv_bfloat16*)q, (const __nv_bfloat16*)q_lo, (const __nv_bfloat16*)k, (const __nv_bfloat16*)k_lo,
+                    nullptr, v, ldqk, ldv, H / G, log_a, log_b, state, out, cu_q, state_slot, entry0, H, P, P, max_slots, 1.f};
+  const bool wide = P % 32 == 0 && (long long)(P / 32) * H * n_entries >= 96;
+  if (N == 128) return wide ? launch_chunks<128, 4, true, false, true>(a, n_entries, stream) : launch_chunks<128, 2, true, false, true>(a, n_entries, stream);
+  return wide ? launch_chunks<64, 4, true, false, true>(a, n_entries, stream) : launch_chunks<64, 2, true, false, true>(a, n_entries, stream);
 }

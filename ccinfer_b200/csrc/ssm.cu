@@ -20,12 +20,23 @@
 //                      the only one that reads that channel's state, so a decode step needs no second kernel
 //   ssm_gate_norm      a block per (token, slice): (o + D x) silu(z), its root mean square, the weight
 //
+// Portions of prompts in the 16-bit path go through ccb_ssm_chunks (memory_chunks.cu) instead of the recurrence: for their
+// rows ssm_prepare leaves B and C as two bfloat16 each and the logarithms of dt and a.
+//
 // Everything after the projection is float; the projection's rows and the convolution state are of the storage type.
 #include "common.cuh"
 
 using namespace ccb;
 
 namespace {
+
+// Where the rows from row `from` on go in place of bs, cs, dts and as: B and C as their bfloat16 values and what the
+// rounding left, the logarithms of dt and of the decay.
+struct SsmChunkRows {
+  int from;
+  __nv_bfloat16 *b_hi, *b_lo, *c_hi, *c_lo;
+  float *log_a, *log_dt;
+};
 
 __device__ __forceinline__ float sigmoid_acc(float x) { return 1.f / (1.f + expf(-x)); }
 __device__ __forceinline__ float softplus_acc(float x) { return x > 20.f ? x : log1pf(expf(x)); }
@@ -110,7 +121,7 @@ __global__ void ssm_prepare_vec_kernel(const T* __restrict__ proj, int ld, int o
                                        const int* __restrict__ cu_q, const int* __restrict__ state_slot,
                                        float* __restrict__ xs, float* __restrict__ bs, float* __restrict__ cs,
                                        float* __restrict__ dts, float* __restrict__ as, int rows, int H, int P, int G,
-                                       int N, T* state_rw, int shift_single) {   // (state_rw is conv_state: no __restrict__ on either)
+                                       int N, T* state_rw, int shift_single, const SsmChunkRows chunk) {   // (state_rw is conv_state: no __restrict__ on either)
   ccb::pdl_begin();
   const int inner = H * P, gn = G * N;
   const int C = inner + 2 * gn;
@@ -125,7 +136,13 @@ __global__ void ssm_prepare_vec_kernel(const T* __restrict__ proj, int ld, int o
       float dt = 0.f, a = 1.f;
       if (e >= 0) {
         dt = softplus_acc(to_f32(proj[(size_t)t * ld + odt + h]) + dt_bias[h]);
-        a = expf(-expf(A_log[h]) * dt);
+        const float log_a = -expf(A_log[h]) * dt;
+        if (t >= chunk.from) {
+          chunk.log_a[(size_t)t * H + h] = log_a;
+          chunk.log_dt[(size_t)t * H + h] = logf(dt);
+          continue;
+        }
+        a = expf(log_a);
       }
       dts[(size_t)t * H + h] = dt;
       as[(size_t)t * H + h] = a;
@@ -156,6 +173,21 @@ __global__ void ssm_prepare_vec_kernel(const T* __restrict__ proj, int ld, int o
           for (int x = 0; x < 4; ++x) st[(size_t)k * C + x] = st[(size_t)(k + 1) * C + x];
         for (int x = 0; x < 4; ++x) st[(size_t)(taps - 2) * C + x] = proj[(size_t)t * ld + ox + c + x];
       }
+    }
+    if (c >= inner && t >= chunk.from) {
+      const bool is_b = c < inner + gn;
+      const size_t at = (size_t)t * gn + (c - inner - (is_b ? 0 : gn));
+      const __nv_bfloat162 h0 = __floats2bfloat162_rn(v.x, v.y), h1 = __floats2bfloat162_rn(v.z, v.w);
+      const float2 f0 = __bfloat1622float2(h0), f1 = __bfloat1622float2(h1);
+      const __nv_bfloat162 l0 = __floats2bfloat162_rn(v.x - f0.x, v.y - f0.y), l1 = __floats2bfloat162_rn(v.z - f1.x, v.w - f1.y);
+      uint2 hi, lo;
+      hi.x = *reinterpret_cast<const uint32_t*>(&h0);
+      hi.y = *reinterpret_cast<const uint32_t*>(&h1);
+      lo.x = *reinterpret_cast<const uint32_t*>(&l0);
+      lo.y = *reinterpret_cast<const uint32_t*>(&l1);
+      *reinterpret_cast<uint2*>((is_b ? chunk.b_hi : chunk.c_hi) + at) = hi;
+      *reinterpret_cast<uint2*>((is_b ? chunk.b_lo : chunk.c_lo) + at) = lo;
+      continue;
     }
     float* dst = c < inner ? xs + (size_t)t * inner + c
                            : (c < inner + gn ? bs + (size_t)t * gn + (c - inner) : cs + (size_t)t * gn + (c - inner - gn));
@@ -226,6 +258,7 @@ CCB_API int ccb_ssm_prepare(const void* proj, int ld, int ox, int odt, const flo
                             int taps, const void* conv_state, const float* A_log, const float* dt_bias,
                             const int* entry_of_token, const int* cu_q, const int* state_slot, float* xs, float* bs,
                             float* cs, float* dts, float* as, int rows, int H, int P, int G, int N, int shift_single,
+                            int chunk_from, void* b_hi, void* b_lo, void* c_hi, void* c_lo, float* log_a, float* log_dt,
                             int dtype, cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (H <= 0 || P <= 0 || G <= 0 || N <= 0 || H % G || taps < 1 || taps > 64) return CCB_REFUSE_SIZE;
@@ -237,6 +270,13 @@ CCB_API int ccb_ssm_prepare(const void* proj, int ld, int ox, int odt, const flo
                      reinterpret_cast<uintptr_t>(conv_w) | reinterpret_cast<uintptr_t>(conv_b) |
                      reinterpret_cast<uintptr_t>(xs) | reinterpret_cast<uintptr_t>(bs) |
                      reinterpret_cast<uintptr_t>(cs)) & 15) == 0;
+  // (rows for chunks: the caller asks for them with the sizes and addresses that the vector kernel takes)
+  const SsmChunkRows chunk{chunk_from < 0 ? rows : chunk_from, (__nv_bfloat16*)b_hi, (__nv_bfloat16*)b_lo, (__nv_bfloat16*)c_hi,
+                           (__nv_bfloat16*)c_lo, log_a, log_dt};
+  if (chunk_from >= 0 && (!vec || !b_hi || !b_lo || !c_hi || !c_lo || !log_a || !log_dt ||
+                          ((reinterpret_cast<uintptr_t>(b_hi) | reinterpret_cast<uintptr_t>(b_lo) |
+                            reinterpret_cast<uintptr_t>(c_hi) | reinterpret_cast<uintptr_t>(c_lo)) & 7)))
+    return CCB_REFUSE_ARG;
   if (vec && (dtype == CCB_F32 || dtype == CCB_BF16)) {
     const size_t total4 = (size_t)rows * ((inner_ + 2 * gn_) / 4 + H);
     const size_t want4 = (total4 + threads - 1) / threads;
@@ -244,11 +284,11 @@ CCB_API int ccb_ssm_prepare(const void* proj, int ld, int ox, int odt, const flo
     if (dtype == CCB_F32)
       ccb_launch(ssm_prepare_vec_kernel<float>, blocks4, threads, 0, stream, (const float*)proj, ld, ox, odt, conv_w,
                  conv_b, taps, (const float*)conv_state, A_log, dt_bias, entry_of_token, cu_q, state_slot, xs, bs, cs,
-                 dts, as, rows, H, P, G, N, (float*)conv_state, shift_single);
+                 dts, as, rows, H, P, G, N, (float*)conv_state, shift_single, chunk);
     else
       ccb_launch(ssm_prepare_vec_kernel<__nv_bfloat16>, blocks4, threads, 0, stream, (const __nv_bfloat16*)proj, ld, ox,
                  odt, conv_w, conv_b, taps, (const __nv_bfloat16*)conv_state, A_log, dt_bias, entry_of_token, cu_q,
-                 state_slot, xs, bs, cs, dts, as, rows, H, P, G, N, (__nv_bfloat16*)conv_state, shift_single);
+                 state_slot, xs, bs, cs, dts, as, rows, H, P, G, N, (__nv_bfloat16*)conv_state, shift_single, chunk);
     return ccb_launch_status();
   }
   const size_t total = (size_t)rows * (H * P + 2 * G * N + H);

@@ -177,7 +177,8 @@ _SIGNATURES = {
     "ccb_init_random": [c_void_p, c_longlong, c_int, ctypes.c_ulonglong, ctypes.c_ulonglong, c_float, c_int, c_void_p],
     "ccb_ssm_prepare": [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                         c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-                        c_int, c_int, c_int, c_void_p],
+                        c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p],
+    "ccb_ssm_chunks": [c_void_p] * 4 + [c_int, c_void_p, c_int] + [c_void_p] * 6 + [c_int] * 7 + [c_void_p],
     "ccb_conv_state_shift": [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                              c_void_p],
     "ccb_gemm_fewrows_relu2_bf16": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
@@ -1366,13 +1367,16 @@ def scaled_sum(out, a, b, sa: float, sb: float) -> None:
 
 
 def ssm_prepare(proj, ox: int, odt: int, conv_w, conv_b, taps: int, conv_state, A_log, dt_bias, entry_of_token, cu_q,
-                state_slot, xs, bs, cs, dts, decay, H: int, P: int, G: int, N: int, shift_single: bool = False) -> None:
+                state_slot, xs, bs, cs, dts, decay, H: int, P: int, G: int, N: int, shift_single: bool = False,
+                chunk=None) -> None:
     """The inputs of a selective state space recurrence from the input projection's rows ``proj`` [T, >=]: the
     channels x | B | C (from column ``ox``) pass the convolution ``conv_w`` [taps, channels] (+ ``conv_b``) and silu,
     rows before the step's first one coming from ``conv_state`` [slots, taps - 1, channels]; dt = softplus(proj[:,
     odt + h] + dt_bias[h]), decay = exp(-exp(A_log[h]) dt).  Outputs float: xs [T, H, P], bs and cs [T, G, N], dts
     and decay [T, H].  ``shift_single``: a request that brings one token has its convolution state moved on here
-    (then ``conv_state_shift`` is for the others only)."""
+    (then ``conv_state_shift`` is for the others only).  ``chunk`` = (first row, b_hi, b_lo, c_hi, c_lo, log_a, log_dt):
+    from that row on B and C go to bfloat16 [T, G, N], their values and what the rounding left, and dt and decay as
+    their logarithms, float [T, H] (``ssm_chunks`` takes them)."""
     _cuda(conv_w, conv_b, conv_state, A_log, dt_bias, entry_of_token, cu_q, state_slot, xs, bs, cs, dts, decay)
     T = xs.shape[0]
     C = H * P + 2 * G * N
@@ -1382,7 +1386,32 @@ def ssm_prepare(proj, ox: int, odt: int, conv_w, conv_b, taps: int, conv_state, 
     _check(lib().ccb_ssm_prepare(_p(proj), proj.stride(0), int(ox), int(odt), _p(conv_w), _p(conv_b), int(taps),
                                  _p(conv_state), _p(A_log), _p(dt_bias), _p(entry_of_token), _p(cu_q), _p(state_slot),
                                  _p(xs), _p(bs), _p(cs), _p(dts), _p(decay), T, H, P, G, N, 1 if shift_single else 0,
+                                 *((-1,) + (0,) * 6 if chunk is None else (int(chunk[0]),) + tuple(_p(t) for t in chunk[1:])),
                                  _dt(proj), _stream()), "ssm_prepare")
+
+
+# (as CHUNK_RECURRENCE_MIN_TOKENS: a chunk costs what some tokens of the recurrence cost)
+SSM_CHUNKS_MIN_TOKENS = 32
+
+
+def ssm_chunks_fits(dtype, N: int, P: int, max_tokens: int) -> bool:
+    """Whether portions of prompts, the longest of max_tokens tokens, run as chunks on tensor cores: the 16-bit path with
+    the sizes the kernel takes."""
+    return dtype == torch.bfloat16 and N in (64, 128) and P % 16 == 0 and max_tokens >= SSM_CHUNKS_MIN_TOKENS
+
+
+def ssm_chunks(chunk, xs, state, out, cu_q, state_slot, entry0: int, n_entries: int, G: int, H: int, N: int, P: int) -> None:
+    """``ssm_recurrence`` for the entries entry0 .. entry0 + n_entries - 1 in chunks of 64 tokens on tensor cores, from what
+    ``ssm_prepare`` left in ``chunk``."""
+    _, b_hi, b_lo, c_hi, c_lo, log_a, log_dt = chunk
+    _cuda(b_hi, b_lo, c_hi, c_lo, log_a, log_dt, xs, state, out, cu_q, state_slot)
+    T = xs.shape[0]
+    assert all(t.dtype == torch.bfloat16 and t.shape == (T, G, N) for t in (b_hi, b_lo, c_hi, c_lo))
+    assert log_a.shape == log_dt.shape == (T, H) and state.shape[1:] == (H, P, N) and out.shape == xs.shape == (T, H, P)
+    assert all(t.dtype == torch.float32 for t in (log_a, log_dt, xs, state, out))
+    _check(lib().ccb_ssm_chunks(_p(c_hi), _p(c_lo), _p(b_hi), _p(b_lo), G * N, _p(xs), H * P, _p(log_a), _p(log_dt), _p(state),
+                                _p(out), _p(cu_q), _p(state_slot), int(entry0), int(n_entries), G, H, N, P, state.shape[0],
+                                _stream()), "ssm_chunks")
 
 
 def conv_state_shift(rows, taps: int, state, cu_q, state_slot, n_entries: int, entry0: int = 0) -> None:

@@ -89,15 +89,25 @@ class SelectiveStateSpace(Mixer):
         dts = rt.scratch.get("ssm_dt", (rt.max_tokens, H), f32)[:T]
         decay = rt.scratch.get("ssm_a", (rt.max_tokens, H), f32)[:T]
         S, conv = state["S"], state["conv"]
+        # portions of prompts go in chunks on tensor cores (a step lists its single tokens first: they, and short portions,
+        # go token by token).  The chunks' rows take the places of those that the recurrence would read.
+        n1 = step.n_single if kernels.ssm_chunks_fits(rt.dtype, N, P, step.max_q_len) else step.n_entries
+        chunk = None
+        if step.n_entries > n1:
+            halves = [rt.scratch.get(f"ssm_chunk{i}:{G * N}", (rt.max_tokens, G, N), rt.dtype)[:T] for i in range(4)]
+            logs = [rt.scratch.get(f"ssm_log{i}:{H}", (rt.max_tokens, H), f32)[:T] for i in range(2)]
+            chunk = (n1, *halves, *logs)   # (single tokens: one row each)
         ox, odt = self.inner, self.inner + self.conv_width
         kernels.ssm_prepare(proj, ox, odt, self.conv_w, self.conv_b, self.taps, conv, self.A_log, self.dt_bias,
                             step.entry_of_token, step.cu_q, step.state_slot, xs, bs, cs, dts, decay, H, P, G, N,
-                            shift_single=True)
+                            shift_single=True, chunk=chunk)
         # (requests that bring one token, which a step lists first, were moved on by the kernel above)
         kernels.conv_state_shift(proj[:, ox:ox + self.conv_width], self.taps, conv, step.cu_q, step.state_slot,
                                  step.n_entries - step.n_single, entry0=step.n_single)
         o = rt.scratch.get("ssm_o", (rt.max_tokens, H, P), f32)[:T]
-        kernels.ssm_recurrence(cs, bs, xs, decay, dts, S, o, step.cu_q, step.state_slot, step.n_entries, G, H, N, P)
+        kernels.ssm_recurrence(cs, bs, xs, decay, dts, S, o, step.cu_q, step.state_slot, n1, G, H, N, P)
+        if chunk is not None:
+            kernels.ssm_chunks(chunk, xs, S, o, step.cu_q, step.state_slot, n1, step.n_entries - n1, G, H, N, P)
         y = rt.scratch.get("ssm_y", (rt.max_tokens, self.inner), rt.dtype)[:T]
         kernels.ssm_gate_norm(y, o, xs, proj, 0, self.skip, self.norm_w, H, P, self.parts, self.eps)
         out = rt.scratch.get(self.out_key, (rt.max_tokens, self.hidden), rt.dtype)[:T]

@@ -112,3 +112,50 @@ def test_recurrence_in_chunks(H, G, dk, dv, rule, decay):
     assert torch.isfinite(out).all() and torch.isfinite(state).all()
     assert (out.double() - want).abs().max() <= 2.0 ** -14 * want.abs().max()
     assert (state.double() - after).abs().max() <= 2.0 ** -14 * after.abs().max()
+
+
+@pytest.mark.parametrize("H,G,N,P", [(4, 2, 128, 64), (2, 1, 128, 16), (3, 3, 64, 48), (4, 1, 64, 32)])
+def test_state_space_recurrence_in_chunks(H, G, N, P):
+    """Portions of a prompt beside single tokens, from the projection's rows: the chunks' rows and the recurrence in float64.
+    An operand as two bfloat16 is right to 2^-17; sums of logarithms over 64 tokens that cancel to 2^-18 of 64 steps."""
+    k, g = _k(), _gen(H + G + N + P)
+    lens = [1, 1, 2, 63, 64, 65, 150]
+    T, taps, C = sum(lens), 4, H * P + 2 * G * N
+
+    def rnd(*shape):
+        return torch.randn(shape, generator=g, device="cuda")
+
+    def dev(x):
+        return torch.tensor(x, dtype=torch.int32, device="cuda")
+
+    width = -(-(C + H) // 8) * 8
+    proj = rnd(T, width).to(torch.bfloat16)
+    conv_w, conv_b, dt_bias = 0.5 * rnd(taps, C), rnd(C), rnd(H) - 2
+    A_log = torch.log(1 + 15 * torch.rand(H, generator=g, device="cuda"))
+    conv = torch.zeros(len(lens), taps - 1, C, dtype=torch.bfloat16, device="cuda")
+    state = rnd(len(lens), H, P, N)
+    first, slots = state.double(), dev(list(range(len(lens)))[::-1])
+    cu = dev([0] + torch.tensor(lens).cumsum(0).tolist())
+    entry = dev([e for e, n in enumerate(lens) for _ in range(n)])
+    xs, bs, cs = (torch.full(s, float("nan"), device="cuda") for s in ((T, H, P), (T, G, N), (T, G, N)))
+    dts, decay, log_a, log_dt = (torch.full((T, H), float("nan"), device="cuda") for _ in range(4))
+    halves = [torch.full((T, G, N), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(4)]
+    out = torch.full((T, H, P), float("nan"), device="cuda")
+    chunk = (2, *halves, log_a, log_dt)
+    k.ssm_prepare(proj, 0, C, conv_w, conv_b, taps, conv, A_log, dt_bias, entry, cu, slots, xs, bs, cs, dts, decay, H, P, G, N,
+                  chunk=chunk)
+    k.ssm_recurrence(cs, bs, xs, decay, dts, state, out, cu, slots, 2, G, H, N, P)
+    k.ssm_chunks(chunk, xs, state, out, cu, slots, 2, len(lens) - 2, G, H, N, P)
+    for e, n in enumerate(lens):
+        r0 = int(cu[e])
+        x = proj[r0:r0 + n, :C].double()
+        pad = torch.cat([x.new_zeros(taps - 1, C), x])
+        y = torch.nn.functional.silu(sum(pad[j:j + n] * conv_w[j].double() for j in range(taps)) + conv_b.double())
+        v, b, c = y[:, :H * P].view(n, H, P), y[:, H * P:H * P + G * N].view(n, G, N), y[:, H * P + G * N:].view(n, G, N)
+        dt = torch.nn.functional.softplus(proj[r0:r0 + n, C:C + H].double() + dt_bias.double())
+        a = torch.exp(-torch.exp(A_log.double()) * dt)
+        rep, slot = H // G, len(lens) - 1 - e
+        want, after = _recurrence64(c.repeat_interleave(rep, 1), b.repeat_interleave(rep, 1), v * dt[..., None], a[..., None],
+                                    None, first[slot])
+        assert (out[r0:r0 + n].double() - want).abs().max() <= 2.0 ** -14 * want.abs().max()
+        assert (state[slot].double() - after).abs().max() <= 2.0 ** -14 * after.abs().max()

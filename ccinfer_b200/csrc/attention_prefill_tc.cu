@@ -31,6 +31,7 @@
 #include "common.cuh"
 #include "tc_common.cuh"
 #include "tma_host.h"
+#include "dense_rows.cuh"
 #include <math_constants.h>
 
 using namespace ccb;
@@ -78,32 +79,49 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
-// HD = 64 * NH
-template <int NH>
+// Keys and values that lie side by side in rows instead of pages (latent attention's, made from its cached rows for one
+// step): a request's rows are those from `dense_first_key` of its first new token on, rounded up to whole tiles, requests
+// one after another.  A key is NK - 1 blocks of 64 columns of its own head's and one block that all heads share, from
+// another matrix.
+// Measured on B200, 2,048 tokens of 32 heads after 1,500 others, window 1,024, latent size 512: rows, queries, the product and
+// this 4.6 + 9.6 + 62 + 80 us in place of 1,517 us over the latent rows themselves (mma.sync, bound by shared memory) and of
+// two products per head (41 us).
+struct DenseKeys {
+  int head0;        // the first block's head: queries and results are those of heads head0 + blockIdx.x
+  int head_cols;    // columns of a head in the rows of keys and values
+  int value_col;    // where its values begin there
+  int shared_col;   // where the shared block begins in the other matrix
+  int value_dim;    // coordinates of a result
+};
+
+// Keys of 64 NK, values of 64 NV coordinates.
+template <int NK, int NV, bool DENSE>
 __global__ void __launch_bounds__(kTcThreads, 1)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                            const __grid_constant__ CUtensorMap tmV, __nv_bfloat16* __restrict__ out,
+                            const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmShared,
+                            const DenseKeys dense, __nv_bfloat16* __restrict__ out,
                             const int* __restrict__ cu_q, const int* __restrict__ pos0,
                             const int* __restrict__ block_table, int bt_stride, int entry0, int nq, int nkv,
                             int page_size, int page_shift, int num_pages, int window, float scale_log2,
                             AttnExtra ex, int* status) {
-  constexpr int HD = 64 * NH;
-  constexpr int HALF_BYTES = 128 * 128;            // 128 rows x 128 bytes: one 64-column half of a tile
-  constexpr int TILE_BYTES = NH * HALF_BYTES;      // Q, K or V tile
+  constexpr int HD = 64 * NK, VD = 64 * NV;
+  constexpr int HALF_BYTES = 128 * 128;            // 128 rows x 128 bytes: one block of 64 columns of a tile
+  constexpr int TILE_BYTES = NK * HALF_BYTES;      // Q or K tile
+  constexpr int V_BYTES = NV * HALF_BYTES;         // V tile
   constexpr int TMEM_COLS = 512;                   // S: two buffers of 128 columns, O: HD columns, P: two of 64
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* sQ = smem;
   uint8_t* sK = sQ + TILE_BYTES;                   // [stages]
   uint8_t* sV = sK + kKvStages * TILE_BYTES;       // [stages]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sV + kKvStages * TILE_BYTES);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sV + kKvStages * V_BYTES);
   // barriers: q_full, k_full[3], v_full[3], k_empty[3], v_empty[3], s_full[2], p_ready, pv_done[2]
   const uint32_t b_q = s32(bars), b_kf = s32(bars + 1), b_vf = s32(bars + 4), b_ke = s32(bars + 7),
                  b_ve = s32(bars + 10), b_sf = s32(bars + 13), b_pr = s32(bars + 15), b_pv = s32(bars + 16);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
 
   const int b = entry0 + blockIdx.z;
-  const int h = blockIdx.x;
+  const int h = DENSE ? dense.head0 + (int)blockIdx.x : (int)blockIdx.x;
   const int row_begin = cu_q[b], n_new = cu_q[b + 1] - row_begin;
   const int n_qtiles = (n_new + kTQ - 1) / kTQ;
   // Blocks start in the order of their linear index, x fastest: with the heads in x, every head's longest
@@ -112,7 +130,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
   const int qt = n_qtiles - 1 - (int)blockIdx.y;
   if (qt < 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kvh = h / (nq / nkv);
+  const int kvh = DENSE ? 0 : h / (nq / nkv);
   const int p0 = pos0[b];
   const int q_first = qt * kTQ;
   const int rows_here = min(kTQ, n_new - q_first);
@@ -157,7 +175,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
     if (warp == 0 && lane == 0) {
       mbar_expect_tx(b_q, TILE_BYTES);
 #pragma unroll
-      for (int hf = 0; hf < NH; ++hf)
+      for (int hf = 0; hf < NK; ++hf)
         tma_load_2d(s32(sQ + hf * HALF_BYTES), &tmQ, h * HD + hf * 64, row_begin + q_first, b_q);
     }
     const int pages_per_tile = kTK >> page_shift;
@@ -184,6 +202,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
     // its own instruction, and one warp issuing them all was what set the pace of the whole block.  A key
     // stage is free as soon as ITS product Q K^T has run, long before the same tile's P V.
     const bool keys = warp == 0;
+    const uint32_t tile_bytes = keys ? TILE_BYTES : V_BYTES;
+    const int row0 = DENSE ? dense_base(cu_q, pos0, entry0, b, window, lane) - dense_first_key(p0, window) : 0;
     const uint32_t b_full = keys ? b_kf : b_vf, b_empty = keys ? b_ke : b_ve;
     uint8_t* stage0 = keys ? sK : sV;
     const CUtensorMap* tm = keys ? &tmK : &tmV;
@@ -192,15 +212,22 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
       int ok = 1;
       if (lane == 0) {
         ok = mbar_wait(b_empty + 8 * s, ph ^ 1) ? 1 : 0;
-        if (ok) mbar_expect_tx(b_full + 8 * s, TILE_BYTES);
+        if (ok) mbar_expect_tx(b_full + 8 * s, tile_bytes);
         else set_status(status, CCB_ST_WAIT_TIMEOUT);
       }
       ok = __shfl_sync(0xffffffffu, ok, 0);
       if (!ok) break;
-      if (lane < pages_per_tile) {
+      if constexpr (DENSE) {
+        const int grow = row0 + (first_tile + i) * kTK, hd0 = (int)blockIdx.x * dense.head_cols;
+        if (lane < (keys ? NK : NV)) {
+          const bool shared = keys && lane == NK - 1;
+          tma_load_2d(s32(stage0 + s * tile_bytes + lane * HALF_BYTES), shared ? &tmShared : tm,
+                      shared ? dense.shared_col : hd0 + (keys ? 0 : dense.value_col) + lane * 64, grow, b_full + 8 * s);
+        }
+      } else if (lane < pages_per_tile) {
         const int grow = page_row(i);
 #pragma unroll
-        for (int hf = 0; hf < NH; ++hf)
+        for (int hf = 0; hf < NK; ++hf)
           tma_load_2d(s32(stage0 + s * TILE_BYTES + hf * HALF_BYTES) + off, tm, hf * 64, grow, b_full + 8 * s);
       }
       __syncwarp();
@@ -209,7 +236,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
     if (lane == 0) {  // ---- MMA issuer ----
       // S = Q K^T: M 128, N 128, both K-major.  O += P V: M 128, N HD, A K-major, B (V) MN-major (bit 16).
       constexpr uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-      constexpr uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(HD >> 3) << 17) |
+      constexpr uint32_t idesc_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((uint32_t)(VD >> 3) << 17) |
                                    ((uint32_t)(128 >> 4) << 24);
       // S of tile t goes to buffer t & 1: the product of the NEXT tile is issued before this tile's P V, so it
       // runs while the softmax warps work on this tile, and their next S is ready when they come back.
@@ -245,7 +272,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
           // P is the A operand in tensor memory (lane = query row, a column = two consecutive keys: 16 keys
           // = 8 columns).  V: 16 keys further = 16 rows of 128 bytes; 64 head columns further = the next half;
           // 8 keys = 1024 bytes
-          const uint64_t db = smem_desc_mn(s32(sV + s * TILE_BYTES) + ks * 2048, HALF_BYTES, 1024);
+          const uint64_t db = smem_desc_mn(s32(sV + s * V_BYTES) + ks * 2048, HALF_BYTES, 1024);
           tc_mma_ts(tmem_o, tmem_p + (i & 1) * 64 + ks * 8, db, idesc_o, (i > 0 || ks > 0) ? 1u : 0u);
         }
         tc_commit(b_ve + 8 * s);  // the value stage may be refilled
@@ -307,7 +334,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
           if (!alive) break;
           tc_fence_after();
 #pragma unroll 1
-          for (int c0 = 0; c0 < HD; c0 += 32) {
+          for (int c0 = 0; c0 < VD; c0 += 32) {
             uint32_t o[32];
             tc_ld32(tmem_o + lane_addr + c0, o);
             tc_wait_ld();
@@ -357,15 +384,17 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
         inv = f / (l * f + ex2(sk - m2));
       }
       if (row < rows_here) inv *= attn_gate<__nv_bfloat16>(ex, row_begin + q_first + row, h);
-      __nv_bfloat16* orow = out + ((size_t)(row_begin + q_first + row) * nq + h) * HD;
+      const int od = DENSE ? dense.value_dim : VD;
+      __nv_bfloat16* orow = out + ((size_t)(row_begin + q_first + row) * nq + h) * od;
 #pragma unroll 1
-      for (int c0 = 0; c0 < HD; c0 += 32) {
+      for (int c0 = 0; c0 < VD; c0 += 32) {
         uint32_t v[32];
         tc_ld32(tmem_o + lane_addr + c0, v);
         tc_wait_ld();
         if (row < rows_here) {
 #pragma unroll
           for (int e = 0; e < 32; e += 8) {
+            if (DENSE && c0 + e >= od) break;
             uint32_t p4[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
@@ -741,14 +770,29 @@ int launch(const void* q, const void* k_cache, const void* v_cache, void* out, c
   const size_t smem = (size_t)(1 + 2 * kKvStages) * NH * 128 * 128 + 20 * 8 + 1024;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel<NH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(attention_prefill_tc_kernel<NH, NH, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
   dim3 grid(nq, (max_new + kTQ - 1) / kTQ, n_entries);
-  ccb_launch(attention_prefill_tc_kernel<NH>, grid, kTcThreads, smem, stream, tmQ, tmK, tmV, (__nv_bfloat16*)out, cu_q,
-             pos0, block_table, bt_stride, entry0, nq, nkv, page_size, page_shift, num_pages, window,
+  ccb_launch(attention_prefill_tc_kernel<NH, NH, false>, grid, kTcThreads, smem, stream, tmQ, tmK, tmV, tmK, DenseKeys{},
+             (__nv_bfloat16*)out, cu_q, pos0, block_table, bt_stride, entry0, nq, nkv, page_size, page_shift, num_pages, window,
+             scale * 1.4426950408889634f, ex, status);
+  return ccb_launch_status();
+}
+
+template <int NK, int NV>
+int launch_dense(const CUtensorMap& tmQ, const CUtensorMap& tmKV, const CUtensorMap& tmShared, const DenseKeys& dense, void* out,
+                 const int* cu_q, const int* pos0, int entry0, int n_entries, int max_new, int heads, int nq, int window,
+                 float scale, AttnExtra ex, int* status, cudaStream_t stream) {
+  constexpr size_t smem = (size_t)((1 + kKvStages) * NK + kKvStages * NV) * 128 * 128 + 20 * 8 + 1024;
+  static_assert(smem <= 227 * 1024, "shared memory of a block");
+  auto kernel = attention_prefill_tc_kernel<NK, NV, true>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return (int)e;
+  ccb_launch(kernel, dim3(heads, (max_new + kTQ - 1) / kTQ, n_entries), kTcThreads, smem, stream, tmQ, tmKV, tmKV, tmShared,
+             dense, (__nv_bfloat16*)out, cu_q, pos0, (const int*)nullptr, 0, entry0, nq, 1, 1, 0, 1, window,
              scale * 1.4426950408889634f, ex, status);
   return ccb_launch_status();
 }
@@ -785,4 +829,38 @@ CCB_API int ccb_attention_prefill_tc(const void* q, const void* k_cache, const v
 CCB_API int ccb_attention_prefill_tc_single_head(int on) {
   g_ccb_prefill_single_head = on ? 1 : 0;
   return 0;
+}
+
+// Attention over keys and values that lie side by side in rows (see DenseKeys): q [n_tokens, nq, 64 (nd + 1)], kv [rows,
+// heads * 64 (nd + nv)] (a head's nd blocks of key columns, then its nv of value columns) of the heads head0 .. head0 +
+// heads - 1, shared [rows, ld_shared] with the last key block in the columns from shared_col on (columns past shared_cols
+// count as zeros); out [n_tokens, nq, value_dim].  A query at position p sees p - window + 1 .. p.
+CCB_API int ccb_attention_prefill_dense(const void* q, const void* kv, const void* shared, void* out, const int* cu_q,
+                                        const int* pos0, int entry0, int n_entries, int max_new, int n_tokens, int rows,
+                                        int head0, int heads, int nq, int nd, int nv, int ld_shared, int shared_col,
+                                        int shared_cols, int value_dim, int window, float scale, const float* sink,
+                                        const void* gate, int gate_stride, int* status, cudaStream_t stream) {
+  if (n_entries <= 0 || max_new <= 0) return 0;
+  if (gate != nullptr && gate_stride < nq) return CCB_REFUSE_ARG;
+  if (nq <= 0 || heads <= 0 || head0 < 0 || head0 + heads > nq || rows <= 0 || rows % kTK != 0 || n_entries > 65535 ||
+      shared_col % 8 != 0 || ld_shared % 8 != 0 || shared_cols > ld_shared || value_dim <= 0 || value_dim % 8 != 0 ||
+      value_dim > 64 * nv || window <= 0 ||
+      ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(kv) | reinterpret_cast<uintptr_t>(shared) |
+        reinterpret_cast<uintptr_t>(out)) & 15) != 0)
+    return CCB_REFUSE_SIZE;
+  const DenseKeys dense{head0, 64 * (nd + nv), 64 * nd, shared_col, value_dim};
+  const AttnExtra ex{0, sink, gate, gate_stride, 0};
+  const unsigned long long qc = (unsigned long long)nq * 64 * (nd + 1), kc = (unsigned long long)heads * 64 * (nd + nv);
+  CUtensorMap tmQ, tmKV, tmShared;
+  if (!ccb_tensor_map_2d(q, n_tokens, qc, qc, 64, 128, &tmQ) || !ccb_tensor_map_2d(kv, rows, kc, kc, 64, 128, &tmKV) ||
+      !ccb_tensor_map_2d(shared, rows, shared_cols, ld_shared, 64, 128, &tmShared))
+    return CCB_REFUSE_ARG;
+#define CCB_DENSE(NK, NV) \
+  launch_dense<NK, NV>(tmQ, tmKV, tmShared, dense, out, cu_q, pos0, entry0, n_entries, max_new, heads, nq, window, scale, ex, status, stream)
+  if (nd == 1 && nv == 1) return CCB_DENSE(2, 1);
+  if (nd == 1 && nv == 2) return CCB_DENSE(2, 2);
+  if (nd == 2 && nv == 1) return CCB_DENSE(3, 1);
+  if (nd == 2 && nv == 2) return CCB_DENSE(3, 2);
+#undef CCB_DENSE
+  return CCB_REFUSE_SIZE;
 }

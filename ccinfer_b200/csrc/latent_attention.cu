@@ -18,9 +18,15 @@
 //                     a time are staged in shared memory as floats; a warp owns one (query, head): a lane
 //                     takes a key for the scores, then a slice of the coordinates for the weighted sum
 //
+//   latent_rows        (portions of prompts in the 16-bit path) the cached rows that a step's portions see, side by side:
+//                      a product then makes every head's keys and values from them and attention runs over those, which
+//                      takes d + r + vdim instead of 2 R + r products a pair and head (attention_prefill_tc.cu)
+//   latent_query_rows  the queries for that, rotated, in blocks of 64 columns
+//
 // Scores, weights, sums and the rotation are float whatever the storage type.
 #include "common.cuh"
 #include "mma_common.cuh"
+#include "dense_rows.cuh"
 #include <math_constants.h>
 
 using namespace ccb;
@@ -125,6 +131,79 @@ __global__ void __launch_bounds__(kPrepThreads) latent_prepare_kernel(const Late
       const int h = i / r, k = i - h * r;
       a.qa[((size_t)t * a.H + h) * (R + r) + R + k] = rotated(qrow + (size_t)h * (a.d + r) + a.d, k);
     }
+  }
+}
+
+// A warp a row of dst [rows, W]: the row of a key that some new token of the request sees, or zeros.  W a multiple of 8.
+constexpr int kRowWarps = 8;
+__global__ void __launch_bounds__(kRowWarps * 32)
+latent_rows_kernel(__nv_bfloat16* __restrict__ dst, int rows, const __nv_bfloat16* __restrict__ cache, int W,
+                   const int* __restrict__ cu_q, const int* __restrict__ pos0, const int* __restrict__ block_table, int bt_stride,
+                   int entry0, int page_size, int num_pages, int window, int* status) {
+  ccb::pdl_begin();
+  const int e = entry0 + blockIdx.y, lane = threadIdx.x & 31;
+  const int i = blockIdx.x * kRowWarps + (threadIdx.x >> 5);
+  if (i >= dense_rows(cu_q, pos0, e, window)) return;
+  const int row = dense_base(cu_q, pos0, entry0, e, window, lane) + i;
+  if (row >= rows) {   // (the caller's bound does not hold)
+    if (lane == 0) set_status(status, CCB_ST_BAD_ROW);
+    return;
+  }
+  const int p0 = pos0[e], j = dense_first_key(p0, window) + i;
+  const uint4* src = nullptr;
+  if (j >= p0 - window + 1 && j < p0 + cu_q[e + 1] - cu_q[e]) {
+    const int lp = j / page_size, page = lp < bt_stride ? block_table[(size_t)e * bt_stride + lp] : -1;
+    if (page >= 0 && page < num_pages) src = reinterpret_cast<const uint4*>(cache + ((size_t)page * page_size + (j - lp * page_size)) * W);
+    else if (lane == 0) set_status(status, CCB_ST_BAD_PAGE);
+  }
+  uint4* out = reinterpret_cast<uint4*>(dst + (size_t)row * W);
+  for (int c = lane; c < W / 8; c += 32) out[c] = src ? src[c] : make_uint4(0u, 0u, 0u, 0u);
+}
+
+// A block a token, eight coordinates a thread at a time: dst [T, H, 64 nd + 64] = a head's d unrotated coordinates, zeros
+// up to 64 nd, its r rotated ones (as latent_prepare turns them), zeros.  d, r and rot_dims / 2 multiples of 8.
+__global__ void __launch_bounds__(kPrepThreads)
+latent_query_rows_kernel(__nv_bfloat16* __restrict__ dst, const __nv_bfloat16* __restrict__ q, int ldq,
+                         const float* __restrict__ inv_freq, int rot_dims, float amp, const int* __restrict__ positions, int H,
+                         int d, int r, int nd) {
+  ccb::pdl_begin();
+  extern __shared__ float2 turn[];
+  const int t = blockIdx.x, half = rot_dims >> 1;
+  const float pos = (float)positions[t];
+  for (int i = threadIdx.x; i < half; i += kPrepThreads) {
+    float sn, cs;
+    sincosf(pos * inv_freq[i], &sn, &cs);
+    turn[i] = make_float2(cs * amp, sn * amp);
+  }
+  __syncthreads();
+  const int width = 64 * nd + 64, pieces = width / 8;
+  const __nv_bfloat16* qrow = q + (size_t)t * ldq;
+  __nv_bfloat16* drow = dst + (size_t)t * H * width;
+  for (int i = threadIdx.x; i < H * pieces; i += kPrepThreads) {
+    const int h = i / pieces, c = 8 * (i - h * pieces);
+    const __nv_bfloat16* x = qrow + (size_t)h * (d + r);
+    const int k = c - 64 * nd;   // place among the rotated ones
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (c < d) {
+      v = *reinterpret_cast<const uint4*>(x + c);
+    } else if (k >= 0 && k < r) {
+      v = *reinterpret_cast<const uint4*>(x + d + k);
+      if (k < rot_dims) {
+        const int j = k < half ? k : k - half;
+        const uint4 w = *reinterpret_cast<const uint4*>(x + d + (k < half ? k + half : k - half));
+        uint32_t* vp = reinterpret_cast<uint32_t*>(&v);
+        const uint32_t* wp = reinterpret_cast<const uint32_t*>(&w);
+        const float sign = k < half ? -1.f : 1.f;
+#pragma unroll
+        for (int y = 0; y < 4; ++y) {
+          const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(vp + y));
+          const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(wp + y));
+          const float2 c0 = turn[j + 2 * y], c1 = turn[j + 2 * y + 1];
+          vp[y] = pack_bf16(a.x * c0.x + sign * b.x * c0.y, a.y * c1.x + sign * b.y * c1.y);
+        }
+      }
+    }
+    *reinterpret_cast<uint4*>(drow + (size_t)h * width + c) = v;
   }
 }
 
@@ -622,6 +701,33 @@ CCB_API int ccb_latent_prepare(const void* proj, int ld, int oc, const void* q, 
   else if (dtype == CCB_BF16) CCB_PREP(__nv_bfloat16);
   else return CCB_REFUSE_DTYPE;
 #undef CCB_PREP
+  return ccb_launch_status();
+}
+
+// dst bfloat16 [rows, W]: the cached rows that the portions of entries entry0 .. see, laid out as dense_rows.cuh says;
+// max_rows: of one request at most.
+CCB_API int ccb_latent_rows(void* dst, int rows, int max_rows, const void* cache, int W, const int* cu_q, const int* pos0,
+                            const int* block_table, int bt_stride, int entry0, int n_entries, int page_size, int num_pages,
+                            int window, int* status, cudaStream_t stream) {
+  if (n_entries <= 0 || max_rows <= 0) return 0;
+  if (W <= 0 || W % 8 || page_size <= 0 || window <= 0 || n_entries > 65535 ||
+      ((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(cache)) & 15))
+    return CCB_REFUSE_SIZE;
+  ccb_launch(latent_rows_kernel, dim3((max_rows + kRowWarps - 1) / kRowWarps, n_entries), kRowWarps * 32, 0, stream,
+             (__nv_bfloat16*)dst, rows, (const __nv_bfloat16*)cache, W, cu_q, pos0, block_table, bt_stride, entry0, page_size,
+             num_pages, window, status);
+  return ccb_launch_status();
+}
+
+// dst bfloat16 [T, H, 64 nd + 64] from q [T, ldq] with H heads of [d | r] (see latent_query_rows_kernel).
+CCB_API int ccb_latent_query_rows(void* dst, const void* q, int ldq, const float* inv_freq, int rot_dims, float amp,
+                                  const int* positions, int T, int H, int d, int r, int nd, cudaStream_t stream) {
+  if (T <= 0) return 0;
+  if (H <= 0 || nd < 1 || d < 0 || d > 64 * nd || r < 0 || r > 64 || d % 8 || r % 8 || rot_dims % 16 || rot_dims > r || ldq % 8 ||
+      (rot_dims > 0 && inv_freq == nullptr) || ((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(q)) & 15))
+    return CCB_REFUSE_SIZE;
+  ccb_launch(latent_query_rows_kernel, dim3(T), kPrepThreads, (size_t)(rot_dims / 2) * sizeof(float2), stream,
+             (__nv_bfloat16*)dst, (const __nv_bfloat16*)q, ldq, inv_freq, rot_dims, amp, positions, H, d, r, nd);
   return ccb_launch_status();
 }
 

@@ -205,6 +205,10 @@ _SIGNATURES = {
                        + [c_int] * 7 + [c_float, c_float, c_int, c_int, c_void_p],
     "ccb_memory_chunks": [c_void_p] * 4 + [c_int, c_void_p, c_int] + [c_void_p] * 6 + [c_int] * 7 + [c_float, c_void_p],
     "ccb_chunk_recurrence": [c_void_p] * 15 + [c_int] * 9 + [c_void_p],
+    "ccb_latent_rows": [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p] + [c_int] * 6
+                       + [c_void_p, c_void_p],
+    "ccb_latent_query_rows": [c_void_p, c_void_p, c_int, c_void_p, c_int, c_float, c_void_p] + [c_int] * 5 + [c_void_p],
+    "ccb_attention_prefill_dense": [c_void_p] * 6 + [c_int] * 15 + [c_float, c_void_p, c_void_p, c_int, c_void_p, c_void_p],
     "ccb_memory_output": [c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int,
                           c_float, c_int, c_void_p],
     "ccb_relu_squared": [c_void_p, c_void_p, c_longlong, c_int, c_void_p],
@@ -837,6 +841,65 @@ def latent_attention(qa, cache, sink, gate, out, cu_q, pos0, entry_of_token, blo
 def latent_attention_mma_fits(dtype, R: int, r: int) -> bool:
     """Whether the tensor-core form of latent attention takes these sizes."""
     return dtype == torch.bfloat16 and R % 16 == 0 and r % 16 == 0 and 0 < R <= 512
+
+
+# Tokens of a step's longest portion from which the heads' keys and values are made from the cached rows for the step.  Per
+# cached row and head that costs (64 nd + 64 nv) R products once, and saves 2 R + r - 64 (nd + nv + 1) a query; with the
+# rates of the two attention kernels (0.18 against 0.6 PFLOP/s) and of the product some twenty queries pay for a row.
+LATENT_DENSE_MIN_TOKENS = 32
+LATENT_DENSE_ELEMENTS = 96 << 20   # of the made keys and values at most: heads go in groups where all would be more
+LATENT_DENSE_ROWS = 1 << 16        # cached rows at most
+
+
+def latent_dense_fits(dtype, d: int, r: int, rot_dims: int, dv: int, R: int) -> bool:
+    """Whether portions of prompts may run over keys and values made for the step (``attention_prefill_dense``)."""
+    return (dtype == torch.bfloat16 and 0 < d <= 128 and 0 < r <= 64 and 0 < dv <= 128
+            and d % 8 == r % 8 == dv % 8 == rot_dims % 16 == R % 8 == 0)
+
+
+def latent_dense_rows(pos0: int, n: int, window: int) -> int:
+    """Rows of a request with ``pos0`` cached and ``n`` new tokens (see ``csrc/dense_rows.cuh``)."""
+    return -(-(pos0 + n) // 128) * 128 - max(0, pos0 - window + 1) // 128 * 128
+
+
+def latent_rows(dst, max_rows: int, cache, cu_q, pos0, block_table, entry0: int, n_entries: int, window: int,
+                status=None) -> None:
+    """dst [rows, W]: the rows of ``cache`` [pages, page_size, W] that the portions of entries entry0 .. see, side by side;
+    ``max_rows``: of one request at most."""
+    _cuda(dst, cache, cu_q, pos0, block_table, status)
+    assert dst.dtype == cache.dtype == torch.bfloat16 and dst.shape[1] == cache.shape[2]
+    _check(lib().ccb_latent_rows(_p(dst), dst.shape[0], int(max_rows), _p(cache), cache.shape[2], _p(cu_q), _p(pos0),
+                                 _p(block_table), block_table.stride(0), int(entry0), int(n_entries), cache.shape[1],
+                                 cache.shape[0], int(window), _p(status), _stream()), "latent_rows")
+
+
+def latent_query_rows(dst, q, inv_freq, rot_dims: int, amp: float, positions, d: int, r: int) -> None:
+    """dst [T, H, 64 nd + 64]: the d unrotated coordinates of every head of q [T, >= H (d + r)] (zeros after them), then the
+    r rotated ones (zeros after them)."""
+    _cuda(dst, inv_freq, positions)
+    T, H, width = dst.shape
+    assert dst.dtype == q.dtype == torch.bfloat16 and q.stride(1) == 1 and q.shape[0] == T and width % 64 == 0
+    _check(lib().ccb_latent_query_rows(_p(dst), _p(q), q.stride(0), _p(inv_freq), int(rot_dims), float(amp), _p(positions), T,
+                                       H, int(d), int(r), width // 64 - 1, _stream()), "latent_query_rows")
+
+
+def attention_prefill_dense(q, kv, shared, shared_col: int, out, cu_q, pos0, entry0: int, n_entries: int, max_q: int,
+                            head0: int, heads: int, nv: int, window: int, scale: float, sink=None, gate=None,
+                            status=None) -> None:
+    """Attention of the portions of entries entry0 .. over rows as ``latent_rows`` lays them out: ``q`` [T, H, 64 nd + 64],
+    ``kv`` [rows, heads * 64 (nd + nv)] the keys' first nd blocks of 64 columns and the values of heads head0 .., their last
+    key block in ``shared`` [rows, W] from ``shared_col`` on; ``out`` [T, H, vdim]."""
+    _cuda(q, kv, shared, out, cu_q, pos0, sink, status)
+    T, H, width = q.shape
+    nd = width // 64 - 1
+    assert all(t.dtype == torch.bfloat16 for t in (q, kv, shared, out)) and out.shape[:2] == (T, H)
+    assert kv.shape[1] == heads * 64 * (nd + nv) and shared.shape[0] == kv.shape[0]
+    assert gate is None or (gate.dtype == torch.bfloat16 and gate.stride(1) == 1)
+    _check(lib().ccb_attention_prefill_dense(
+        _p(q), _p(kv), _p(shared), _p(out), _p(cu_q), _p(pos0), int(entry0), int(n_entries), int(max_q), T, kv.shape[0],
+        int(head0), int(heads), H, nd, int(nv), shared.stride(0), int(shared_col), shared.shape[1], out.shape[2], int(window),
+        float(scale), _p(sink), _p(gate), gate.stride(0) if gate is not None else 0, _p(status), _stream()),
+        "attention_prefill_dense")
 
 
 LATENT_MMA_KEYS = 32       # keys a block of the tensor-core form takes at a time

@@ -20,8 +20,10 @@ slow pairs turn slower and cosine and sine carry a factor, as ``position.RotaryH
 
 What a token leaves in the cache is the row [c | kr] alone.  Attention runs over those rows: the unrotated part
 of a query is carried into the latent space first, (Wuk_h^T q_h) . c = q_h . (Wuk_h c), and the weighted sum of c
-comes back out through Wuv_h afterwards (two products per head, batched over the heads).  q (or c_q), the latent row
-and the gate are ONE merged product of x.
+comes back out through Wuv_h afterwards (two products per head, batched over the heads).  Portions of prompts, where many
+queries see a row, take the equation the other way round in bfloat16: ONE product makes every head's Wuk_h c and Wuv_h c from
+the rows that the step sees, and attention runs over those (``_dense``).  q (or c_q), the latent row and the gate are ONE
+merged product of x.
 """
 from __future__ import annotations
 
@@ -38,7 +40,7 @@ def _pad8(n: int) -> int:
 
 
 class LatentAttention(Mixer):
-    kernel_groups = ("latent",)
+    kernel_groups = ("latent", "attention")
     def __init__(self, hidden: int, heads: int, dim: int, rot_dim: int, value_dim: int, rank: int, window: int,
                  scale: float, rot_base: float, rot_dims: int, norm_eps: float, names: dict,
                  interleaved: bool = False, own_kv: bool = True, q_rank: int = None, ramp_scaling: dict = None):
@@ -129,6 +131,14 @@ class LatentAttention(Mixer):
         # per head: [rank, dim] so that (q_h Wuk_h) is a product with the weights' usual layout [out, in]
         self.w_uk_t = fetch(n["uk"]).view(H, self.d, self.R).transpose(1, 2).contiguous()
         self.w_uv = fetch(n["uv"]).view(H, self.dv, self.R).contiguous()
+        # the same two for ``_dense``, a head's blocks of 64 rows of Wuk and then of Wuv, zeros where it has fewer
+        self.w_kv = None
+        if kernels.latent_dense_fits(rt.dtype, self.d, self.r, self.rot_dims, self.dv, self.R):
+            self.nd, self.nv = -(-self.d // 64), -(-self.dv // 64)
+            w_kv = torch.zeros((H, 64 * (self.nd + self.nv), self.R), dtype=rt.dtype, device=rt.device)
+            w_kv[:, :self.d] = fetch(n["uk"]).view(H, self.d, self.R)
+            w_kv[:, 64 * self.nd:64 * self.nd + self.dv] = self.w_uv
+            self.w_kv = w_kv.view(-1, self.R)
         self.w_o = fetch(n["o"])
         self.inv_freq, self.amp = None, 1.0
         if self.rot_dims:
@@ -139,6 +149,44 @@ class LatentAttention(Mixer):
             amp = rot.amplitude()
             self.amp = 1.0 if amp is None else float(amp[0])
 
+    def _dense_rows(self, step):
+        """(rows in all, rows of a request at most) that the step's portions see, or None where they do not run over made keys
+        and values: no portion is long enough, or the rows are too many.  From the host's arrays where the step has them,
+        else a bound."""
+        n1, many = step.n_single, step.n_entries - step.n_single
+        if self.w_kv is None or many == 0 or step.max_q_len < kernels.LATENT_DENSE_MIN_TOKENS:
+            return None
+        if step.host is not None:
+            spans = [kernels.latent_dense_rows(int(p), int(c) - int(p), self.kernel_window)
+                     for p, c in zip(step.host.pos0[n1:step.n_entries], step.host.ctx_after[n1:step.n_entries])]
+            rows, most = sum(spans), max(spans)
+        else:
+            most = -(-min(step.max_ctx, step.max_q_len + self.kernel_window + 126) // 128) * 128
+            rows = many * most
+        return (rows, most) if rows <= kernels.LATENT_DENSE_ROWS else None
+
+    def _dense(self, q, rows, span, gate, o, step, g):
+        """Attention of the step's portions over keys and values of every head, made from the cached rows they see."""
+        rt, H, R, W = self.rt, self.H, self.R, self.R + self.r
+        T, n1, many = q.shape[0], step.n_single, step.n_entries - step.n_single
+        n, most = span
+        cap = 1 << (n - 1).bit_length()   # (buffers of the next power of two: no graph holds their addresses)
+        seen = rt.scratch.get(f"latent_seen:{cap}:{W}", (cap, W), rt.dtype)[:n]
+        kernels.latent_rows(seen, most, rows, step.cu_q, step.pos0, g.block_table, n1, many, self.kernel_window,
+                            status=rt.status)
+        qr = rt.scratch.get(f"latent_query:{H}:{self.nd}", (rt.max_tokens, H, 64 * self.nd + 64), rt.dtype)[:T]
+        kernels.latent_query_rows(qr, q, self.inv_freq, self.rot_dims, self.amp, step.positions, self.d, self.r)
+        cols = 64 * (self.nd + self.nv)
+        heads = max(1, min(H, kernels.LATENT_DENSE_ELEMENTS // (cap * cols)))
+        kv = rt.scratch.get(f"latent_kv:{cap}:{heads * cols}", (cap * heads * cols,), rt.dtype)
+        for h0 in range(0, H, heads):
+            hn = min(heads, H - h0)
+            part = kv[:n * hn * cols].view(n, hn * cols)
+            rt.linear(part, seen[:, :R], self.w_kv[h0 * cols:(h0 + hn) * cols])
+            kernels.attention_prefill_dense(qr, part, seen, R, o, step.cu_q, step.pos0, n1, many, step.max_q_len, h0, hn,
+                                            self.nv, self.kernel_window, self.scale, sink=self.sink, gate=gate,
+                                            status=rt.status)
+
     def forward(self, x, step, cache, state):
         rt = self.rt
         x = rt.rows(x)
@@ -147,30 +195,38 @@ class LatentAttention(Mixer):
         g = cache.group
         proj = rt.scratch.get("latent_proj", (rt.max_tokens, self.in_width), rt.dtype)[:T]
         rt.linear(proj, x, self.w_in)
-        qa = rt.scratch.get("latent_q", (rt.max_tokens, H, R + r), torch.float32)[:T]
         rows = cache.tensors["latent"]
+        span = self._dense_rows(step)
+        Ta = T if span is None else step.n_single   # rows whose queries are carried into the latent space
+        qa = rt.scratch.get("latent_q", (rt.max_tokens, H, R + r), torch.float32)[:Ta]
         prepare = (self.oc, self.norm_w, self.inv_freq, self.rot_dims, step.positions, g.slot_map if cache.own else None,
                    rows, H, d, r, R, self.eps)
         if self.q_rank is None:
             q = proj[:, self.oq:self.oq + self.q_width]
-            kernels.latent_prepare(proj, *prepare, q=q, qa=qa, amp=self.amp, status=rt.status)
+            own = {"q": q, "qa": qa} if Ta == T else {}
+            if cache.own or own:
+                kernels.latent_prepare(proj, *prepare, **own, amp=self.amp, status=rt.status)
         else:
             cq = rt.scratch.get("latent_cq", (rt.max_tokens, self.w_uq.shape[1]), rt.dtype)[:T]
             kernels.latent_prepare(proj, *prepare, amp=self.amp, low=(self.oq, self.q_rank, self.cq_norm_w, cq),
                                    status=rt.status)
             q = rt.scratch.get("latent_uq", (rt.max_tokens, self.w_uq.shape[0]), rt.dtype)[:T]
             rt.linear(q, cq, self.w_uq)
-            kernels.latent_prepare(q, *prepare[:5], None, None, *prepare[7:], q=q, qa=qa, amp=self.amp, status=rt.status)
-            q = q[:, :self.q_width]
-        if d > 0:
-            qu = q.view(T, H, d + r)[:, :, :d]
+            q, own = q[:, :self.q_width], {}
+        if Ta > 0 and not own:
+            kernels.latent_prepare(q[:Ta], *prepare[:5], None, None, *prepare[7:], q=q[:Ta], qa=qa, amp=self.amp,
+                                   status=rt.status)
+        if Ta > 0 and d > 0:
+            qu = q[:Ta].view(Ta, H, d + r)[:, :, :d]
             rt.linear_batched(qa[:, :, :R].permute(1, 0, 2), qu.permute(1, 0, 2), self.w_uk_t)
-        else:
+        elif Ta > 0:
             qa[:, :, :R].zero_()
-        ol = rt.scratch.get("latent_o", (rt.max_tokens, H, R), rt.dtype)[:T]
+        ol = rt.scratch.get("latent_o", (rt.max_tokens, H, R), rt.dtype)[:Ta]
         gate = proj[:, self.og:self.og + H] if self.has_gate else None
         args = (qa, rows, self.sink, gate, ol, step.cu_q, step.pos0, step.entry_of_token, g.block_table)
         n1, many = step.n_single, step.n_entries - step.n_single
+        if span is not None:
+            many = 0   # (``_dense`` takes them)
         if kernels.latent_attention_mma_fits(rt.dtype, R, r):
             # tensor cores: the heads are the rows of the products.  The step's single tokens come first; their
             # key ranges are cut into pieces so that a few rows still fill the machine
@@ -194,6 +250,9 @@ class LatentAttention(Mixer):
                 kernels.latent_attention(*args, n1, many, step.max_q_len, g.page_size, self.kernel_window, self.scale,
                                          status=rt.status)
         o = rt.scratch.get("latent_v", (rt.max_tokens, H, dv), rt.dtype)[:T]
-        rt.linear_batched(o.permute(1, 0, 2), ol.permute(1, 0, 2), self.w_uv)
+        if Ta > 0:
+            rt.linear_batched(o[:Ta].permute(1, 0, 2), ol.permute(1, 0, 2), self.w_uv)
+        if span is not None:
+            self._dense(q, rows, span, gate, o, step, g)
         out = rt.scratch.get(self.out_key, (rt.max_tokens, self.hidden), rt.dtype)[:T]
         return rt.linear(out, o.view(T, H * dv), self.w_o)

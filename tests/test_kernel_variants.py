@@ -159,3 +159,112 @@ def test_state_space_recurrence_in_chunks(H, G, N, P):
                                     None, first[slot])
         assert (out[r0:r0 + n].double() - want).abs().max() <= 2.0 ** -14 * want.abs().max()
         assert (state[slot].double() - after).abs().max() <= 2.0 ** -14 * after.abs().max()
+
+
+class _Step:
+    """The arrays of a step whose requests have (cached, new) tokens each, single tokens first, on shuffled pages."""
+
+    def __init__(self, entries, page, seed):
+        from ccinfer_b200.engine.step import GroupStep, StepContext
+        counts = [n for _, n in entries]
+        s = self.step = StepContext()
+
+        def dev(x):
+            return torch.tensor(x, dtype=torch.int32, device="cuda")
+
+        s.n_tokens, s.n_entries, s.n_single = sum(counts), len(entries), sum(n == 1 for n in counts)
+        s.max_q_len, s.max_ctx = max(counts), max(p + n for p, n in entries)
+        s.positions = dev([p + i for p, n in entries for i in range(n)])
+        s.entry_of_token = dev([e for e, n in enumerate(counts) for _ in range(n)])
+        cu = [0]
+        for n in counts:
+            cu.append(cu[-1] + n)
+        s.cu_q, s.pos0, s.state_slot = dev(cu), dev([p for p, _ in entries]), dev(list(range(len(entries))))
+        pages = [-(-(p + n) // page) for p, n in entries]
+        order = torch.randperm(sum(pages), generator=torch.Generator().manual_seed(seed)).tolist()
+        table = torch.full((len(entries), max(pages)), -1, dtype=torch.int32)
+        self.slots, at = [], 0
+        for e, k in enumerate(pages):
+            table[e, :k] = torch.tensor(order[at:at + k])
+            at += k
+            j = torch.arange(sum(entries[e]))
+            self.slots.append((table[e, j // page].long() * page + j % page))
+        new = torch.cat([x[p:] for x, (p, _) in zip(self.slots, entries)]).int()
+        s.groups = [GroupStep(0, page, sum(pages), None, new.cuda(), table.cuda(), new.numpy(), table.numpy())]
+
+
+# d, r, rotated, value and latent sizes: one and two blocks of 64 key and value columns, sizes that fill none; windows
+# that end in a tile, at a tile's edge, none; heads in groups
+@pytest.mark.parametrize("d,r,dims,dv,R,H,window,groups", [
+    (64, 64, 64, 128, 512, 4, 130, False), (128, 64, 64, 128, 64, 3, None, False), (64, 32, 16, 64, 128, 2, 128, False),
+    (40, 16, 0, 24, 48, 5, 256, True), (72, 8, 0, 72, 512, 2, 1, False), (64, 64, 64, 128, 128, 6, 300, True)])
+def test_latent_attention_over_made_keys_and_values(monkeypatch, d, r, dims, dv, R, H, window, groups):
+    """Portions beside single tokens: against float64, no further off than the form that stays in the latent space (both round
+    queries, keys or latent queries, weights and results to bfloat16 once), with a third in hand for their different sums."""
+    from ccinfer_b200 import kernels
+    from ccinfer_b200.engine.runtime import Runtime
+    from ccinfer_b200.engine.step import LayerCache
+    from ccinfer_b200.parts import LatentAttention
+    D, page, scale, base, eps = 96, 16, (d + r) ** -0.5, 10000.0, 1e-5
+    entries = [(0, 1), (300, 1), (0, 2), (0, 33), (127, 128), (250, 129), (129, 200)]
+    g = _gen(d + r + dv + R + H)
+    shapes = {"q": (H * (d + r), D), "dkv": (R + r, D), "uk": (H * d, R), "uv": (H * dv, R), "o": (D, H * dv), "g": (H, D)}
+    w = {k: (torch.randn(s, generator=g, device="cuda") * s[1] ** -0.5).to(torch.bfloat16) for k, s in shapes.items()}
+    w["dkv_norm"], w["sink"] = 1 + 0.1 * torch.randn(R, generator=g, device="cuda"), torch.randn(H, generator=g, device="cuda")
+    made = _Step(entries, page, 5)
+    step, T = made.step, made.step.n_tokens
+    x = torch.randn((T, D), generator=g, device="cuda").to(torch.bfloat16)
+    old = [torch.randn((p, R + r), generator=g, device="cuda").to(torch.bfloat16) for p, _ in entries]
+
+    def run():
+        part = LatentAttention(D, H, d, r, dv, R, window, scale, base, dims, eps, {k: k for k in w})
+        rt = Runtime("cuda:0", torch.bfloat16, T, len(entries))
+        part.bind(rt, w.__getitem__)
+        cache = torch.zeros((step.groups[0].num_pages, page, R + r), dtype=torch.bfloat16, device="cuda")
+        for rows, at in zip(old, made.slots):
+            cache.view(-1, R + r)[at[:rows.shape[0]].cuda()] = rows
+        out = part.forward(x, step, LayerCache({"latent": cache}, step.groups[0], True), None).double()
+        rt.check_status()
+        return out
+
+    launched = []
+    real = kernels.attention_prefill_dense
+    monkeypatch.setattr(kernels, "attention_prefill_dense", lambda *a, **k: (launched.append(a[9]), real(*a, **k)))
+    if groups:   # two heads at a time
+        monkeypatch.setattr(kernels, "LATENT_DENSE_ELEMENTS", 2 * 64 * (-(-d // 64) - (-dv // 64)) * 4096)
+    got = run()
+    assert launched and (not groups or len(launched) > 1)
+    monkeypatch.setattr(kernels, "LATENT_DENSE_MIN_TOKENS", 1 << 30)
+    n = len(launched)
+    before = run()
+    assert len(launched) == n
+    W = {k: v.double() for k, v in w.items()}
+    freq = base ** (-torch.arange(0, dims, 2, device="cuda").double() / max(dims, 1))
+    want, at = torch.empty(T, D, dtype=torch.float64, device="cuda"), 0
+
+    def turn(y, pos):
+        a, h = torch.outer(pos.double(), freq), dims // 2
+        u, v = y[..., :h], y[..., h:dims]
+        a = a.view(a.shape[0], *([1] * (y.dim() - 2)), h)
+        return torch.cat([u * a.cos() - v * a.sin(), v * a.cos() + u * a.sin(), y[..., dims:]], -1)
+
+    for (p, m), rows in zip(entries, old):
+        h = x[at:at + m].double()
+        pos = torch.arange(p, p + m, device="cuda")
+        q = (h @ W["q"].T).view(m, H, d + r)
+        q = torch.cat([q[..., :d], turn(q[..., d:], pos)], -1)
+        c = h @ W["dkv"].T
+        new = torch.cat([c[:, :R] / (c[:, :R].square().mean(-1, keepdim=True) + eps).sqrt() * W["dkv_norm"], turn(c[:, R:], pos)], -1)
+        seen = torch.cat([rows.double(), new])
+        k = torch.cat([(seen[:, :R] @ W["uk"].T).view(-1, H, d), seen[:, None, R:].expand(-1, H, r)], -1)
+        v = (seen[:, :R] @ W["uv"].T).view(-1, H, dv)
+        s = torch.einsum("ihd,jhd->hij", q, k) * scale
+        i, j = pos[:, None], torch.arange(p + m, device="cuda")[None]
+        s.masked_fill_((j > i) | ((i - j >= window) if window else (j < 0)), float("-inf"))
+        s = torch.softmax(torch.cat([s, W["sink"][:, None, None].expand(H, m, 1)], -1), -1)[..., :-1]
+        o = torch.einsum("hij,jhd->ihd", s, v) * torch.sigmoid(h @ W["g"].T)[..., None]
+        want[at:at + m] = o.reshape(m, -1) @ W["o"].T
+        at += m
+    e_new, e_old = ((y - want).norm() / want.norm() for y in (got, before))
+    assert e_new <= 1.33 * e_old and e_old < 0.02
+    assert (got - want).abs().max() <= 2 * max((before - want).abs().max(), 2.0 ** -8 * want.abs().max())

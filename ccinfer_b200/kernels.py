@@ -126,7 +126,7 @@ _SIGNATURES = {
     "ccb_moe_gather_rows": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "ccb_moe_grouped_tc": [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p,
                            c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_float, c_float,
-                           c_int, c_void_p, c_void_p],
+                           c_int, c_int, c_int, c_void_p, c_void_p],
     "ccb_moe_combine": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     "ccb_scaled_residual": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_int, c_int, c_int, c_void_p],
     "ccb_concat_cast": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
@@ -1098,7 +1098,7 @@ def moe_grouped(c, a, src_row, w, w_expert_stride: int, row_w, tile_e, tile_r0, 
                                  mode, *(glu or _SILU_GLU).args, 1 if weight_in else 0, _dt(a), _stream()), "moe_grouped")
 
 
-MOE_TC_ROWS = 128   # rows of a tile of the tcgen05 grouped product
+MOE_TC_ROWS = (64, 320)   # rows of a tile of the tcgen05 grouped product: either
 
 
 def moe_gather_rows(out, x, src_row) -> None:
@@ -1112,8 +1112,8 @@ def moe_gather_rows(out, x, src_row) -> None:
 
 
 def moe_grouped_tc(c, a, w, row_w, tile_e, tile_r0, tile_n, N: int, K: int, F: int, mode: int, status=None,
-                   glu: GluAct = None, weight_in: bool = False) -> None:
-    """``moe_grouped`` on tcgen05 tensor cores for tiles of MOE_TC_ROWS sorted rows (bfloat16).  ``a`` holds the
+                   glu: GluAct = None, weight_in: bool = False, BM: int = MOE_TC_ROWS[0]) -> None:
+    """``moe_grouped`` on tcgen05 tensor cores for tiles of ``BM`` (one of MOE_TC_ROWS) sorted rows (bfloat16).  ``a`` holds the
     sorted rows themselves.  mode 0: ``w`` = all first matrices stacked [E F, K], c bfloat16 [rows, F] =
     relu(a W_e^T)^2 * row_w;  mode 1: ``w`` = all second matrices side by side [N, E F] (K = F), c float;  mode 2:
     as mode 0 with every expert's F = N rows gate and up rows in turn, c bfloat16 [rows, N / 2] as ``moe_grouped``'s."""
@@ -1122,8 +1122,8 @@ def moe_grouped_tc(c, a, w, row_w, tile_e, tile_r0, tile_n, N: int, K: int, F: i
     assert a.shape[1] == K and c.shape == (a.shape[0], N // 2 if mode == 2 else N) and c.is_contiguous()
     _check(lib().ccb_moe_grouped_tc(_p(a), a.stride(0), a.shape[0], _p(w), w.stride(0), w.shape[0], w.shape[1], _p(c),
                                     c.stride(0), _p(row_w), _p(tile_e), _p(tile_r0), _p(tile_n), tile_e.numel(), N, K,
-                                    F, mode, *(glu or _SILU_GLU).args, 1 if weight_in else 0, _p(status), _stream()),
-           "moe_grouped_tc")
+                                    F, mode, *(glu or _SILU_GLU).args, 1 if weight_in else 0, int(BM), sm_count(), _p(status),
+                                    _stream()), "moe_grouped_tc")
 
 
 def moe_combine(out, rows, pair_pos, shared, top: int) -> None:

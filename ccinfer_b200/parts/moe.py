@@ -47,9 +47,17 @@ class MixtureOfExperts(FeedForward):
     # of which 4 are chosen, the whole part in us, dense / sparse at 1, 8, 256, 2,048 tokens: 16.8 M weights
     # 22 / 26, 24 / 31, 37 / 51, 138 / 99; 67 M weights 47 / 33, 48 / 42, 75 / 78, 340 / 187.
     SPARSE_MIN_WEIGHTS = 1 << 25
-    # (token, choice) pairs per expert from which the tcgen05 grouped product runs (402 M weights, 64 tokens, i.e.
-    # 8 pairs an expert: 131 us against 222 us for tiles of 16 rows on mma.sync)
+    # The tcgen05 grouped product runs from this many (token, choice) pairs an expert, or from this many weights of the first
+    # matrices of the experts that a step can choose: below both its walks are too few for pairs of SMs, and a block for
+    # every eight columns on mma.sync (rows16) streams them faster.  Measured on B200, the whole part in us, tcgen05 / rows16
+    # (hidden x F, experts / chosen, tokens): 4096 x 3072, 32 / 4: 90 / 102 (1 token), 129 / 170 (2), 282 / 425 (8); 2048 x
+    # 2048, 32 / 4: 49 / 48 (1), 63 / 71 (2); 2048 x 512, 32 / 4: 45 / 45 (4), 62 / 60 (8), 68 / 81 (32); 1024 x 512, 32 / 4:
+    # 41 / 37 (8), 44 / 51 (32); 2048 x 256, 64 / 6: 47 / 48 (4), 53 / 68 (8); 4096 x 512, 16 / 2: 53 / 45 (4), 57 / 60 (8).
     TC_MIN_ROWS_PER_EXPERT = 8
+    TC_MIN_CHOSEN_WEIGHTS = 48 << 20
+    # ... and from this many pairs an expert with tiles of up to 320 rows instead of 64 (192 tokens of 4096 x 3072, 32 / 4:
+    # 435 / 429 us; 64 tokens 430 / 402; 512 tokens 480 / 596)
+    TC_WIDE_ROWS_PER_EXPERT = 24
 
     def __init__(self, hidden: int, experts: int, top: int, expert_ff: int, names: dict, groups: int = 1,
                  keep: int = 1, shared_ff: int = 0, activation="relu2", sparse=None, rule=None,
@@ -201,10 +209,13 @@ class MixtureOfExperts(FeedForward):
         E, F, D, top = self.E, self.F, self.hidden, self.top
         i32, f32 = torch.int32, torch.float32
         pairs, max_pairs = T * top, rt.max_tokens * top
-        # rows per tile: 16 (a decode step: the chosen experts' weights are streamed once per tile), or 128 on
-        # tcgen05 once an expert gets some rows on average (bfloat16)
-        tc = rt.dtype == torch.bfloat16 and pairs >= self.TC_MIN_ROWS_PER_EXPERT * E
-        BM = kernels.MOE_TC_ROWS if tc else 16
+        # rows per tile: 16 (the chosen experts' weights are streamed once per tile), or those of the tcgen05 product (bfloat16)
+        # the first product's rows an expert and its mode: with gates, gate and up rows in turn and the gated activation as
+        # the epilogue
+        F1, first = (2 * F, 2) if self.glu else (F, 0)
+        tc = rt.dtype == torch.bfloat16 and (pairs >= self.TC_MIN_ROWS_PER_EXPERT * E
+                                             or min(E, pairs) * F1 * D >= self.TC_MIN_CHOSEN_WEIGHTS)
+        BM = kernels.MOE_TC_ROWS[pairs >= self.TC_WIDE_ROWS_PER_EXPERT * E] if tc else 16
         n_tiles = kernels.moe_max_tiles(pairs, E, BM)
         cap = kernels.moe_max_tiles(max_pairs, E, 16)
         # (layers of other sizes have buffers of their own: a buffer that only long steps use must not grow once
@@ -216,15 +227,12 @@ class MixtureOfExperts(FeedForward):
         idx, wts, _ = self.route(x, T, sort_into=(BM, src_row, row_w, pair_pos, *tiles), step=step)
         act = rt.scratch.get(f"moe_act_rows:{top}:{F}", (max_pairs, F), rt.dtype)[:pairs]
         rows = rt.scratch.get(f"moe_out_rows:{top}", (max_pairs, D), f32)[:pairs]
-        # the first product's rows an expert and its mode: with gates, gate and up rows in turn and the gated
-        # activation as the epilogue
-        F1, first = (2 * F, 2) if self.glu else (F, 0)
         act_args = {"glu": self.glu_act, "weight_in": self.weight_on_input}
         if tc:
             xs = rt.scratch.get(f"moe_x_sorted:{top}", (max_pairs, D), rt.dtype)[:pairs]
             kernels.moe_gather_rows(xs, x, src_row)
-            kernels.moe_grouped_tc(act, xs, self.w_up, row_w, *tiles, F1, D, F1, first, status=rt.status, **act_args)
-            kernels.moe_grouped_tc(rows, act, self.w_down, row_w, *tiles, D, F, F, 1, status=rt.status)
+            kernels.moe_grouped_tc(act, xs, self.w_up, row_w, *tiles, F1, D, F1, first, status=rt.status, BM=BM, **act_args)
+            kernels.moe_grouped_tc(rows, act, self.w_down, row_w, *tiles, D, F, F, 1, status=rt.status, BM=BM)
         else:
             kernels.moe_grouped(act, x, src_row, self.w_up, F1 * self.w_up.stride(0), row_w, *tiles, F1, D, BM, first,
                                 **act_args)

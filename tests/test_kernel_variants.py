@@ -268,3 +268,56 @@ def test_latent_attention_over_made_keys_and_values(monkeypatch, d, r, dims, dv,
     e_new, e_old = ((y - want).norm() / want.norm() for y in (got, before))
     assert e_new <= 1.33 * e_old and e_old < 0.02
     assert (got - want).abs().max() <= 2 * max((before - want).abs().max(), 2.0 ** -8 * want.abs().max())
+
+
+@pytest.mark.parametrize("mode", [0, 1, 2])
+@pytest.mark.parametrize("BM", [64, 320])
+@pytest.mark.parametrize("N,K", [(256, 64), (40, 72), (264, 200), (1024, 512)])
+def test_grouped_products_of_experts(mode, N, K, BM):
+    """Experts with no row, one, and numbers around the steps of 32 columns, the accumulators of 256 and the tiles of 64 and 320 rows, against float64: float
+    results to K roundings of the sum of magnitudes, 16-bit ones to theirs (2^-8) beside that."""
+    k, g = _k(), _gen(N + K + mode)
+    counts = [0, 1, 31, 32, 33, 0, 64, 65, 255, 256, 257, 300, 320, 321, 700, 2]
+    E, pairs = len(counts), sum(counts)
+
+    def rnd(*shape):
+        return torch.randn(shape, generator=g, device="cuda")
+
+    idx = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))[torch.randperm(pairs, generator=torch.Generator().manual_seed(1))]
+    idx = idx.to(torch.int32).cuda().view(pairs, 1)
+    wts = torch.rand((pairs, 1), generator=g, device="cuda") + 0.5
+    i32 = dict(dtype=torch.int32, device="cuda")
+    src, pos, row_w = torch.empty(pairs, **i32), torch.empty(pairs, **i32), torch.empty(pairs, device="cuda")
+    tiles = [torch.empty(k.moe_max_tiles(pairs, E, BM), **i32) for _ in range(3)]
+    k.moe_sort(idx, wts, E, BM, src, row_w, pos, *tiles)
+    x = rnd(pairs, K).to(torch.bfloat16)
+    xs = torch.empty_like(x)
+    k.moe_gather_rows(xs, x, src)
+    status = torch.zeros(1, **i32)
+    w = (rnd(N, E * K) if mode == 1 else rnd(E * N, K)).mul(K ** -0.5).to(torch.bfloat16)
+    c = torch.full((pairs, N // 2 if mode == 2 else N), float("nan"), dtype=torch.float32 if mode == 1 else torch.bfloat16, device="cuda")
+    k.moe_grouped_tc(c, xs, w, row_w, *tiles, N, K, K if mode == 1 else N, mode, status=status, BM=BM)
+    assert int(status.item()) == 0
+    order = idx.view(-1)[src.long()].long()   # the expert of every sorted row
+    assert (order[1:] >= order[:-1]).all()
+    for e in range(E):
+        rows = (order == e).nonzero().view(-1)
+        if not rows.numel():
+            continue
+        we = (w[:, e * K:(e + 1) * K] if mode == 1 else w[e * N:(e + 1) * N]).double()
+        a = xs[rows].double()
+        ref, size = a @ we.T, a.abs() @ we.abs().T
+        slack = K * 2.0 ** -24 * size
+        got = c[rows].double()
+        if mode == 1:
+            assert ((got - ref).abs() <= slack).all()
+            continue
+        rw = row_w[rows].double()[:, None]
+        if mode == 0:
+            ref, slack = ref.clamp_min(0) ** 2 * rw, 2 * ref.abs() * slack * rw + slack ** 2 * rw
+        else:
+            gate, up = ref[:, ::2], ref[:, 1::2]
+            sg, su = slack[:, ::2], slack[:, 1::2]
+            ref = torch.nn.functional.silu(gate) * up * rw
+            slack = (1.1 * sg * up.abs() + gate.abs() * su + sg * su) * rw + 2.0 ** -20 * ref.abs()   # (silu's slope is below 1.1)
+        assert ((got - ref).abs() <= 2.0 ** -8 * ref.abs() + slack + 1e-30).all()

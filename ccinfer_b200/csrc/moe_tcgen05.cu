@@ -24,7 +24,9 @@
 //     activation (gate and up are neighbouring lanes, which exchange one of two tokens each) in bfloat16, the second's float.
 // The rows of A must lie in sorted order, so the tokens are gathered first (moe_gather_rows).
 // Every wait on an mbarrier is bounded as in gemm_tcgen05.cu.
-// MOE_FIGURES
+// Bound by the stream of weights up to some 130 rows an expert (32 of 4096 x 3072, 4 chosen, 128 tokens: 2.4 GB in 414 us, 5.9
+// TB/s), by that and the products together at 2,048 tokens (0.62 TFLOP in 750 us).  The whole part, 8 / 2,048 tokens: tiles of
+// 128 x 256 on one SM and 16 rows on mma.sync 413 / 1,161 us; this with four epilogue warps 284 / 956, with eight 280 / 866.
 #include "cluster_common.cuh"
 #include <cuda.h>
 #include <type_traits>
@@ -48,7 +50,7 @@ template <int CAP> struct Ring {
   static constexpr int kStages = CAP == 64 ? 11 : 6;
 };
 constexpr int kBoxes = 4;          // token copies come in boxes of 16, 32, 64 and 128 rows: at most three make up a block's half
-constexpr int kThreads = 224;     // warps: 0 weights, 1 products, 2 .. 5 epilogue, 6 tokens
+constexpr int kThreads = 352;     // warps: 0 weights, 1 products, 2 .. 9 epilogue, 10 tokens
 constexpr int kAcc = 2;            // accumulators of 256 columns in tensor memory
 
 struct TokenMaps {
@@ -90,7 +92,7 @@ moe_grouped_tc_kernel(const __grid_constant__ TokenMaps tmX, const __grid_consta
     }
     for (int b = 0; b < kAcc; ++b) {
       mbar_init(tfull0 + 8 * b, 1);
-      mbar_init(tempty0 + 8 * b, 8);   // four epilogue warps of each block
+      mbar_init(tempty0 + 8 * b, 16);   // eight epilogue warps of each block
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -141,7 +143,7 @@ moe_grouped_tc_kernel(const __grid_constant__ TokenMaps tmX, const __grid_consta
         }
       }
     }
-  } else if (warp == 6) {
+  } else if (warp == 10) {
     if (lane == 0) {  // ---- the same for this block's half of the tokens ----
       int s = 0, ph = 0;
       bool alive = true;
@@ -225,7 +227,9 @@ moe_grouped_tc_kernel(const __grid_constant__ TokenMaps tmX, const __grid_consta
       }
     }
   } else {  // ---- epilogue: this block's 128 weight rows (lanes), all tokens of the tile (columns) ----
-    const int q = warp & 3;
+    // two warps a quarter of the lanes, which take 32 tokens in turn (one warp each left a third of a tile's time exposed
+    // where both accumulators are taken)
+    const int q = warp & 3, turn = (warp - 2) >> 2;
     int local = 0;
     bool alive = true;
     for (int t = pair, n0 = 0; t < items && alive; ++local) {   // an accumulator at a time: tokens n0 .. of item t
@@ -244,7 +248,7 @@ moe_grouped_tc_kernel(const __grid_constant__ TokenMaps tmX, const __grid_consta
       const int col = tf * kFeatures + (int)rank * (kFeatures / 2) + q * 32 + lane;   // this lane's column of the product
       const uint32_t taddr = tmem_base + buf * kTokens + ((uint32_t)(q * 32) << 16);
 #pragma unroll 1
-      for (int c0 = 0; c0 < n; c0 += 32) {
+      for (int c0 = 32 * turn; c0 < n; c0 += 64) {
         uint32_t v[32];
         tc_ld32(taddr + c0, v);
         tc_wait_ld();
@@ -264,20 +268,32 @@ moe_grouped_tc_kernel(const __grid_constant__ TokenMaps tmX, const __grid_consta
         } else {   // columns (2 f, 2 f + 1) are gate f and up f: the even lane takes token j, the odd one token j + 1
           const int odd = lane & 1;
           __nv_bfloat16* dst = (__nv_bfloat16*)Cout + (g0 + c0 + odd) * ldc + (col >> 1);
-#pragma unroll
-          for (int j = 0; j < 32; j += 2) {
+          const bool mine = (col | 1) < N;
+          auto one = [&](int j) {
             const float w = __shfl_sync(0xffffffffu, my_w, j + odd);
             const float wi = w_in ? w : 1.f, wo = w_in ? 1.f : w;
             const float a = __uint_as_float(v[j]), b = __uint_as_float(v[j + 1]);
             const float got = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);   // what the other lane has of this lane's token
-            const float gate = odd ? got : a, up = odd ? b : got;
-            if (c0 + j + odd < n && (col | 1) < N) dst[(size_t)j * ldc] = __float2bfloat16_rn(glu_act(act, gate * wi, up * wi) * wo);
+            return glu_act(act, (odd ? got : a) * wi, (odd ? b : got) * wi) * wo;
+          };
+          if (c0 + 32 <= n) {   // (no condition a token: the activations of several run side by side)
+#pragma unroll
+            for (int j = 0; j < 32; j += 2) {
+              const float y = one(j);
+              if (mine) dst[(size_t)j * ldc] = __float2bfloat16_rn(y);
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; j += 2) {
+              const float y = one(j);
+              if (mine && c0 + j + odd < n) dst[(size_t)j * ldc] = __float2bfloat16_rn(y);
+            }
           }
         }
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) {   // this warp's quarter of this block's accumulator is free again: the leader counts eight
+      if (lane == 0) {   // this warp's quarter of this block's accumulator is free again: the leader counts sixteen
         if (leader) mbar_arrive(tempty0 + 8 * buf);
         else mbar_arrive_remote(map_to_rank(tempty0 + 8 * buf, 0));
       }

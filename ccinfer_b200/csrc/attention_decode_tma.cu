@@ -21,7 +21,6 @@ namespace {
 
 constexpr int kTileKeys = 64;
 constexpr int kStages = 3;
-constexpr int kMinSplitTiles = 4;   // tiles a split should have before another block is worth its start-up
 constexpr int kComputeThreads = 128;
 constexpr int kThreads = 192;  // four compute warps and two producer warps (keys, values)
 constexpr int kHalfBytes = kTileKeys * 128;  // 64 rows x 64 columns of bfloat16
@@ -69,7 +68,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                             const int* __restrict__ positions, const int* __restrict__ entry_of_token,
                             const int* __restrict__ block_table, int bt_stride, int n_entries, int row0, int nq,
                             int nkv, int page_size, int page_shift, int num_pages, int window, float scale,
-                            int num_splits, int* __restrict__ counters, AttnExtra ex, int* status) {
+                            int num_splits, int min_tiles, int* __restrict__ counters, AttnExtra ex, int* status) {
   // The kernel after this one is let in only when this one ends: a product that came in while the last
   // blocks were still merging made the pair slower (measured), not faster.
   // The fused form may itself come in early (programmatic dependent launch): the cached keys and values it
@@ -105,8 +104,8 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
   const int b = entry_of_token[t];
   const int p = positions[t];
   const bool padded = b < 0 || b >= n_entries || p < 0;
-  // The row's tiles and how many of the grid's splits get some.  A split is worth a block only from a few
-  // tiles on: with a short context the first eff_splits splits take kMinSplitTiles tiles each and the
+  // The row's tiles and how many of the grid's splits get some.  A split is worth a block only from
+  // min_tiles tiles on: with a short context the first eff_splits splits take that many each and the
   // others have nothing to do (the grid is sized without knowing the context).  Where the last block
   // merges, they leave at once and are not waited for (measured at one row and 2,048 keys with a grid of
   // 32 splits: 12.1 us when all 32 took a tile and were merged, as against 10.6 us with a grid of 8).
@@ -114,8 +113,9 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
   const KeyTiles kt(j0, ex.keep, kTileKeys);
   const int first_tile = kt.first, last_tile = (padded ? 0 : p) / kTileKeys;
   const int n_tiles = last_tile - first_tile + 1;
-  const int eff_splits = padded ? 1 : min(num_splits, max(1, (n_tiles + kMinSplitTiles - 1) / kMinSplitTiles));
+  const int eff_splits = padded ? 1 : min(num_splits, max(1, (n_tiles + min_tiles - 1) / min_tiles));
   if (counters != nullptr && split >= eff_splits) return;
+  const bool whole = num_splits == 1 || (counters != nullptr && eff_splits == 1);   // this block sees all of the row's keys
   if (tid == 0) {
     for (int s = 0; s < kStages; ++s) {
       mbar_init(bar0 + 8 * s, 2);     // the two producer warps
@@ -466,7 +466,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
       }
     }
     const int h = h0 + row;
-    if (num_splits == 1) {
+    if (whole) {
       a *= attn_sink_fold(ex, h, mm, ll);
       if (!padded) a *= attn_gate<__nv_bfloat16>(ex, t, h);
       out[((size_t)t * nq + h) * HD + d] = __float2bfloat16_rn(ll > 0.f ? a / ll : 0.f);
@@ -479,7 +479,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
       }
     }
   }
-  if (num_splits == 1 || counters == nullptr) return;  // without counters a second kernel merges the splits
+  if (whole || counters == nullptr) return;  // without counters a second kernel merges the splits
   // The block that arrives last at this (row, head group) merges the splits that had tiles, in ascending order whichever
   // block it is, so that no second kernel (and no gap before it) is needed.
   __shared__ int last_flag;
@@ -581,7 +581,7 @@ int launch(const void* q, const FusedQkv& fq, const void* k_cache, const void* v
            float* part_ml,
            const int* positions, const int* entry_of_token, const int* block_table, int bt_stride, int n_entries,
            int row0, int n_rows, int nq, int nkv, int page_size, int num_pages, int window, float scale,
-           int num_splits, int* counters, AttnExtra ex, int* status, cudaStream_t stream) {
+           int num_splits, int min_tiles, int* counters, AttnExtra ex, int* status, cudaStream_t stream) {
   const int G = nq / nkv, gchunks = (G + 15) / 16;
   int page_shift = 0;
   while ((1 << page_shift) < page_size) ++page_shift;
@@ -601,7 +601,7 @@ int launch(const void* q, const FusedQkv& fq, const void* k_cache, const void* v
   dim3 grid(n_rows, nkv * gchunks, num_splits);
   ccb_launch_ex(FUSED && fq.k_cache != nullptr, attention_decode_tma_kernel<HD, FUSED>, grid, kThreads, smem, stream,
                 tmK, tmV, (const __nv_bfloat16*)q, fq, (__nv_bfloat16*)out, part_acc, part_ml, positions, entry_of_token, block_table, bt_stride, n_entries,
-             row0, nq, nkv, page_size, page_shift, num_pages, window, scale, num_splits, counters, ex, status);
+             row0, nq, nkv, page_size, page_shift, num_pages, window, scale, num_splits, min_tiles, counters, ex, status);
   int rc = ccb_launch_status();
   if (rc != 0 || num_splits == 1 || counters != nullptr) return rc;
   ccb_launch(attention_merge_bf16_kernel2, dim3(n_rows, nq), 128, 0, stream, (__nv_bfloat16*)out, part_acc, part_ml,
@@ -613,6 +613,7 @@ int launch(const void* q, const FusedQkv& fq, const void* k_cache, const void* v
 
 // As ccb_attention_decode_mma, for page sizes that are a power of two from 8 to 64 (others: CCB_REFUSE_SIZE).
 // chunk, keep, sink, gate, gate_stride: see AttnExtra (0 / null: none).
+// A row's key range is cut into at most num_splits pieces of at least min_tiles tiles of 64 keys.
 // `counters` (optional): n_rows * kv_heads * ceil(group / 16) ints that are zero before the first launch and
 // are left zero; with them the splits are merged by the attention kernel itself, without them by a second
 // kernel.
@@ -620,13 +621,13 @@ CCB_API int ccb_attention_decode_tma(const void* q, const void* k_cache, const v
                                      float* part_acc, float* part_ml, const int* positions,
                                      const int* entry_of_token, const int* block_table, int bt_stride,
                                      int n_entries, int row0, int n_rows, int nq, int nkv, int hd, int page_size,
-                                     int num_pages, int window, float scale, int num_splits, int* counters,
-                                     int chunk, int keep, const float* sink, const void* gate, int gate_stride,
+                                     int num_pages, int window, float scale, int num_splits, int min_tiles,
+                                     int* counters, int chunk, int keep, const float* sink, const void* gate, int gate_stride,
                                      int* status, cudaStream_t stream) {
   if (n_rows <= 0) return 0;
   if (chunk < 0 || keep < 0 || (gate != nullptr && gate_stride < nq)) return CCB_REFUSE_ARG;
   const AttnExtra ex{chunk, sink, gate, gate_stride, keep};
-  if (nq <= 0 || nkv <= 0 || nq % nkv != 0 || bt_stride <= 0 || num_splits <= 0 || num_splits > 64 ||
+  if (nq <= 0 || nkv <= 0 || nq % nkv != 0 || bt_stride <= 0 || num_splits <= 0 || num_splits > 64 || min_tiles <= 0 ||
       page_size < 8 || page_size > 64 || (page_size & (page_size - 1)) != 0 ||
       ((reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) != 0)
     return CCB_REFUSE_SIZE;
@@ -635,11 +636,11 @@ CCB_API int ccb_attention_decode_tma(const void* q, const void* k_cache, const v
   if (hd == 128)
     return launch<128, false>(q, none, k_cache, v_cache, out, part_acc, part_ml, positions, entry_of_token,
                               block_table, bt_stride, n_entries, row0, n_rows, nq, nkv, page_size, num_pages, window,
-                              scale, num_splits, counters, ex, status, stream);
+                              scale, num_splits, min_tiles, counters, ex, status, stream);
   if (hd == 64)
     return launch<64, false>(q, none, k_cache, v_cache, out, part_acc, part_ml, positions, entry_of_token,
                              block_table, bt_stride, n_entries, row0, n_rows, nq, nkv, page_size, num_pages, window,
-                             scale, num_splits, counters, ex, status, stream);
+                             scale, num_splits, min_tiles, counters, ex, status, stream);
   return CCB_REFUSE_SIZE;
 }
 
@@ -658,13 +659,13 @@ CCB_API int ccb_attention_decode_tma_fused(const void* qkv, int qkv_stride, void
                                            int page_size, int num_pages, int window, float scale, int num_splits,
                                            const float* q_w, const float* k_w, float eps, const float* inv_freq,
                                            int write_kv, const float* bias, float qt_coef, int qt_every,
-                                           int* counters, int chunk, int keep, const float* sink, const void* gate,
+                                           int min_tiles, int* counters, int chunk, int keep, const float* sink, const void* gate,
                                            int gate_stride, int* status, cudaStream_t stream) {
   if (n_rows <= 0) return 0;
   if (chunk < 0 || keep < 0 || (gate != nullptr && gate_stride < nq)) return CCB_REFUSE_ARG;
   const AttnExtra ex{chunk, sink, gate, gate_stride, keep};
   if (qt_every < 0 || (bias != nullptr && !write_kv)) return CCB_REFUSE_ARG;
-  if (nq <= 0 || nkv <= 0 || nq % nkv != 0 || bt_stride <= 0 || num_splits <= 0 || num_splits > 64 ||
+  if (nq <= 0 || nkv <= 0 || nq % nkv != 0 || bt_stride <= 0 || num_splits <= 0 || num_splits > 64 || min_tiles <= 0 ||
       page_size < 8 || page_size > 64 || (page_size & (page_size - 1)) != 0 || (qkv_stride & 1) ||
       qkv_stride < (nq + (write_kv ? 2 * nkv : 0)) * hd ||
       ((reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) != 0 ||
@@ -686,10 +687,10 @@ CCB_API int ccb_attention_decode_tma_fused(const void* qkv, int qkv_stride, void
   if (hd == 128)
     return launch<128, true>(nullptr, fq, k_cache, v_cache, out, part_acc, part_ml, positions, entry_of_token,
                              block_table, bt_stride, n_entries, row0, n_rows, nq, nkv, page_size, num_pages, window,
-                             scale, num_splits, counters, ex, status, stream);
+                             scale, num_splits, min_tiles, counters, ex, status, stream);
   if (hd == 64)
     return launch<64, true>(nullptr, fq, k_cache, v_cache, out, part_acc, part_ml, positions, entry_of_token,
                             block_table, bt_stride, n_entries, row0, n_rows, nq, nkv, page_size, num_pages, window,
-                            scale, num_splits, counters, ex, status, stream);
+                            scale, num_splits, min_tiles, counters, ex, status, stream);
   return CCB_REFUSE_SIZE;
 }

@@ -149,12 +149,12 @@ _SIGNATURES = {
                                  c_float, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p],
     "ccb_attention_decode_tma": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                  c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
-                                 c_float, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p,
+                                 c_float, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p,
                                  c_void_p],
     "ccb_attention_decode_tma_fused": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                        c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                                        c_int, c_int, c_float, c_int, c_void_p, c_void_p, c_float, c_void_p, c_int,
-                                       c_void_p, c_float, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int,
+                                       c_void_p, c_float, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int,
                                        c_void_p, c_void_p],
     "ccb_attention_prefill_mma": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                                   c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int,
@@ -1670,6 +1670,30 @@ def attention_split_plan(n_rows: int, nq: int, nkv: int, hd: int, heads_per_bloc
     return splits, target * gt * hd, target * gt * 2
 
 
+DECODE_MIN_TILES = 4            # tiles of 64 keys that a split of the decode kernels should have: its start-up costs as much
+DECODE_RAGGED_SPLITS = 4
+DECODE_RAGGED_BLOCKS = 384
+
+
+def attention_decode_plan(n_rows: int, nq: int, nkv: int, hd: int):
+    """(num_splits, min_tiles, merged by the kernel, scratch floats for the accumulators, for max and sum) of
+    ``attention_decode_tma``, from the number of rows only, as ``attention_split_plan``.
+
+    Where the rows alone nearly fill the machine, a few long contexts among short ones would be all that runs at the end: up
+    to DECODE_RAGGED_BLOCKS (row, kv head) pairs, contexts are cut into up to four pieces, but only into long ones, so that
+    batches of equal contexts gain no merging that they do not need.  Measured on B200, 8 kv heads of 128, one piece / this,
+    us: 32 rows, contexts of 500 to 8,000 103 / 75, all 2,048 44 / 44, all 8,000 156 / 172; 48 rows 130 / 110, 78 / 78, 279 /
+    258; 16 rows (two pieces / this) 47 / 39, 28 / 28, 82 / 87.  From 8 splits on the block that finishes last merges them,
+    as it does for the cut rows here (a row of one piece is written at once)."""
+    groups = n_rows * nkv * -(-(nq // nkv) // DECODE_MMA_HEADS_PER_BLOCK)
+    splits, _, _ = attention_split_plan(n_rows, nq, nkv, hd, DECODE_MMA_HEADS_PER_BLOCK)
+    blocks = max(split_target_blocks(), DECODE_RAGGED_SPLITS * DECODE_RAGGED_BLOCKS)
+    floats = blocks * DECODE_MMA_HEADS_PER_BLOCK
+    if splits < DECODE_RAGGED_SPLITS - 1 and groups <= DECODE_RAGGED_BLOCKS:
+        return DECODE_RAGGED_SPLITS, 16 if splits > 1 else 32, True, floats * hd, floats * 2
+    return splits, DECODE_MIN_TILES, splits >= 8, floats * hd, floats * 2
+
+
 def attention_split(q, k_cache, v_cache, out, part_acc, part_ml, positions, entry_of_token, block_table,
                     n_entries: int, row0: int, n_rows: int, window: int, scale: float, num_splits: int,
                     status=None, chunk: int = 0, sink=None, gate=None, keep: int = 0) -> None:
@@ -1745,12 +1769,14 @@ def attention_decode_tma_fits(hd: int, page_size: int) -> bool:
 
 def attention_decode_tma(q, k_cache, v_cache, out, part_acc, part_ml, positions, entry_of_token, block_table,
                          n_entries: int, row0: int, n_rows: int, window: int, scale: float, num_splits: int,
-                         status=None, merge_counters=None, chunk: int = 0, sink=None, gate=None, keep: int = 0) -> None:
+                         status=None, merge_counters=None, chunk: int = 0, sink=None, gate=None, keep: int = 0,
+                         min_tiles: int = DECODE_MIN_TILES) -> None:
     """As attention_decode_mma, with keys and values loaded page by page through TMA boxes by a producer warp
     (page size a power of two from 8 to 64).
 
     ``merge_counters`` (int32 zeros, left zero): with them the block that finishes last merges the splits
-    of its row and head group; without them (or where they are too few) a second kernel does."""
+    of its row and head group; without them (or where they are too few) a second kernel does.  ``min_tiles``: tiles of 64
+    keys that a split takes at least."""
     _cuda(q, k_cache, v_cache, out, part_acc, part_ml, positions, entry_of_token, block_table, status, merge_counters)
     T, nq, hd = q.shape
     num_pages, nkv, page_size, hd2 = k_cache.shape
@@ -1769,7 +1795,7 @@ def attention_decode_tma(q, k_cache, v_cache, out, part_acc, part_ml, positions,
     _check(lib().ccb_attention_decode_tma(_p(q), _p(k_cache), _p(v_cache), _p(out), _p(part_acc), _p(part_ml),
                                           _p(positions), _p(entry_of_token), _p(block_table),
                                           block_table.stride(0), n_entries, row0, n_rows, nq, nkv, hd, page_size,
-                                          num_pages, int(window), float(scale), num_splits, _p(merge_counters),
+                                          num_pages, int(window), float(scale), num_splits, int(min_tiles), _p(merge_counters),
                                           *_attn_extra(T, nq, q.dtype, chunk, sink, gate, keep), _p(status), _stream()),
            "attention_decode_tma")
     if num_splits > 1 and merge_counters is None:
@@ -1800,7 +1826,8 @@ def attention_decode_tma_fused(qkv, k_cache, v_cache, out, part_acc, part_ml, po
                                block_table, n_entries: int, row0: int, n_rows: int, nq: int, window: int,
                                scale: float, num_splits: int, q_norm_w, k_norm_w, eps: float, inv_freq,
                                write_kv: bool = True, status=None, merge_counters=None, bias=None,
-                               q_temperature=None, chunk: int = 0, sink=None, gate=None, keep: int = 0) -> None:
+                               q_temperature=None, chunk: int = 0, sink=None, gate=None, keep: int = 0,
+                               min_tiles: int = DECODE_MIN_TILES) -> None:
     """attention_decode_tma for rows of ONE new token each, straight from the q|k|v product ``qkv``
     [T, (nq + 2 nkv) * hd] (only the nq query heads when ``write_kv`` is false): the kernel norms and rotates
     the queries itself and, with ``write_kv``, also the row's key, which it writes with the value to their
@@ -1829,7 +1856,7 @@ def attention_decode_tma_fused(qkv, k_cache, v_cache, out, part_acc, part_ml, po
         _p(entry_of_token), _p(block_table), block_table.stride(0), n_entries, row0, n_rows, nq, nkv, hd, page_size,
         num_pages, int(window), float(scale), num_splits, _p(q_norm_w), _p(k_norm_w), float(eps), _p(inv_freq),
         1 if write_kv else 0, _p(bias), float(q_temperature[0]) if q_temperature else 0.0,
-        int(q_temperature[1]) if q_temperature else 0, _p(merge_counters),
+        int(q_temperature[1]) if q_temperature else 0, int(min_tiles), _p(merge_counters),
         *_attn_extra(T, nq, qkv.dtype, chunk, sink, gate, keep), _p(status), _stream()), "attention_decode_tma_fused")
     if num_splits > 1 and merge_counters is None:
         counters.own += 1  # the merge kernel

@@ -346,20 +346,23 @@ class GroupedQueryAttention(Mixer):
         extra = {"chunk": self.chunk, "sink": self.sink, "gate": gate, "keep": self.keep_first} if self.extras else {}
         n_rows = step.n_single if mma else T
         if n_rows > 0:
-            per_block = kernels.DECODE_MMA_HEADS_PER_BLOCK if mma else 0
-            splits, n_acc, n_ml = kernels.attention_split_plan(n_rows, self.nq, self.nkv, self.hd, per_block)
+            tma = mma and kernels.attention_decode_tma_fits(self.hd, g.page_size)
+            plan = {}
+            if tma:
+                splits, tiles, in_kernel, n_acc, n_ml = kernels.attention_decode_plan(n_rows, self.nq, self.nkv, self.hd)
+                plan = {"min_tiles": tiles, "merge_counters": rt.merge_counters if in_kernel else None}
+            else:
+                per_block = kernels.DECODE_MMA_HEADS_PER_BLOCK if mma else 0
+                splits, n_acc, n_ml = kernels.attention_split_plan(n_rows, self.nq, self.nkv, self.hd, per_block)
             part_acc = rt.scratch.get("attn_part_acc", (n_acc,), torch.float32)
             part_ml = rt.scratch.get("attn_part_ml", (n_ml,), torch.float32)
             args = (q, cache.k, cache.v, o, part_acc, part_ml, step.positions, step.entry_of_token, g.block_table,
                     step.n_entries, 0, n_rows, self.window or 0, self.scale, splits)
-            if mma and kernels.attention_decode_tma_fits(self.hd, g.page_size):
-                # pages arrive as TMA boxes.  Many splits (few rows, long contexts): the last block of a row
-                # and head group merges them; few splits: a second small kernel does, during which the
-                # output projection already loads its first weights (measured: 2 us a layer either way)
-                kernels.attention_decode_tma(*args, status=rt.status, **extra,
-                                             merge_counters=rt.merge_counters if splits >= self.MERGE_IN_KERNEL_MIN_SPLITS else None)
-            else:
-                (kernels.attention_decode_mma if mma else kernels.attention_split)(*args, status=rt.status, **extra)
+            # pages arrive as TMA boxes where they can.  Many splits (few rows, long contexts): the last block of a row
+            # and head group merges them; few splits: a second small kernel does, during which the
+            # output projection already loads its first weights (measured: 2 us a layer either way)
+            (kernels.attention_decode_tma if tma else kernels.attention_decode_mma if mma else kernels.attention_split)(
+                *args, status=rt.status, **extra, **plan)
         if mma and step.n_entries > step.n_single:
             # long portions: 128-token tiles on tcgen05 with the accumulators in tensor memory; short ones
             # (and page sizes a TMA box cannot take): 64-token tiles on mma.sync
@@ -368,7 +371,6 @@ class GroupedQueryAttention(Mixer):
             fn(q, cache.k, cache.v, o, step.cu_q, step.pos0, g.block_table, step.n_single,
                step.n_entries - step.n_single, step.max_q_len, self.window or 0, self.scale, status=rt.status, **extra)
 
-    MERGE_IN_KERNEL_MIN_SPLITS = 8   # from here on the block that finishes last merges the splits itself
     FUSED_DECODE_MAX_ROWS = 48   # measured: 1.3-2.3 us a layer faster up to 32 rows, 1.6 us slower at 64
 
     def _fused_decode(self, step, g) -> bool:
@@ -433,15 +435,14 @@ class GroupedQueryAttention(Mixer):
         elif self._fused_decode(step, g):
             # every row brings one token: the decode attention norms and rotates the queries itself, writes
             # the row's key and value to their page and attends to them: one kernel less in every layer
-            splits, n_acc, n_ml = kernels.attention_split_plan(T, self.nq, self.nkv, self.hd,
-                                                               kernels.DECODE_MMA_HEADS_PER_BLOCK)
+            splits, min_tiles, in_kernel, n_acc, n_ml = kernels.attention_decode_plan(T, self.nq, self.nkv, self.hd)
             kernels.attention_decode_tma_fused(
                 qkv, cache.k, cache.v, o, rt.scratch.get("attn_part_acc", (n_acc,), torch.float32),
                 rt.scratch.get("attn_part_ml", (n_ml,), torch.float32), step.positions, step.entry_of_token,
                 g.block_table, step.n_entries, 0, T, self.nq, self.window or 0, self.scale, splits,
                 self.q_norm_w, self.k_norm_w, self.norm_eps if self.norm_eps is not None else 1.0,
                 self.position.rotary_table(), write_kv=self.own_kv, status=rt.status,
-                merge_counters=rt.merge_counters if splits >= self.MERGE_IN_KERNEL_MIN_SPLITS else None,
+                merge_counters=rt.merge_counters if in_kernel else None, min_tiles=min_tiles,
                 bias=self.bias, q_temperature=self.position.query_temperature(), chunk=self.chunk, sink=self.sink,
                 gate=gate, keep=self.keep_first)
         else:

@@ -321,3 +321,101 @@ def test_grouped_products_of_experts(mode, N, K, BM):
             ref = torch.nn.functional.silu(gate) * up * rw
             slack = (1.1 * sg * up.abs() + gate.abs() * su + sg * su) * rw + 2.0 ** -20 * ref.abs()   # (silu's slope is below 1.1)
         assert ((got - ref).abs() <= 2.0 ** -8 * ref.abs() + slack + 1e-30).all()
+
+
+# rows around the runs of four, requests of one row beside longer ones (their first rows read the convolution's state),
+# heads that fill a warp's 128 channels and that do not; steps of few rows take a warp a row
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("lens,taps,G,H,dk,dv", [
+    ([5], 4, 1, 2, 128, 128), ([1, 1, 2, 4, 9], 4, 2, 2, 64, 32), ([3, 1, 1, 7], 2, 1, 1, 4, 128), ([6, 2], 1, 2, 4, 36, 12),
+    ([1, 8, 3], 3, 1, 3, 128, 4), ([2, 1], 4, 1, 2, 128, 128)])
+def test_delta_rows_in_runs(lens, taps, G, H, dk, dv, dtype):
+    """Against float64: a row's sums of ``taps`` products, one activation and one norm over dk squares."""
+    k, g = _k(), _gen(sum(lens) + taps + dk)
+    T, C = sum(lens), 2 * G * dk + H * dv
+    ob = -(-C // 8) * 8
+    width = ob + -(-H // 8) * 8
+
+    def rnd(*shape):
+        return torch.randn(shape, generator=g, device="cuda")
+
+    proj, a = rnd(T, width).to(dtype), rnd(T, H * dk).to(dtype)
+    state, w = rnd(len(lens), max(taps - 1, 1), C).to(dtype), 0.5 * rnd(taps, C)
+    A_log, dt_bias = rnd(H), rnd(H * dk)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), **i32)
+    entry = torch.tensor([e for e, n in enumerate(lens) for _ in range(n)], **i32)
+    slots = torch.tensor(list(range(len(lens)))[::-1], **i32)
+    qn, kn, vv, gg, bb = (torch.full(s, float("nan"), device="cuda") for s in ((T, G, dk), (T, G, dk), (T, H, dv), (T, H, dk), (T, H)))
+    k.delta_prepare(proj, (0, G * dk, 2 * G * dk, ob), a, w, taps, state, A_log, dt_bias, entry, cu, slots, qn, kn, vv, gg, bb,
+                    G, H, dk, dv, dk ** -0.5, 1e-6)
+    x, rows = proj.double(), []
+    for e, n in enumerate(lens):
+        r0 = int(cu[e])
+        pad = torch.cat([state[len(lens) - 1 - e, :taps - 1].double(), x[r0:r0 + n, :C]])
+        rows.append(torch.nn.functional.silu(sum(pad[j:j + n] * w[j].double() for j in range(taps))))
+    y = torch.cat(rows)
+    q, kk, v = y[:, :G * dk].view(T, G, dk), y[:, G * dk:2 * G * dk].view(T, G, dk), y[:, 2 * G * dk:].view(T, H, dv)
+    q, kk = (t / (t.square().sum(-1, keepdim=True) + 1e-6).sqrt() for t in (q, kk))
+    decay = torch.exp(-torch.exp(A_log.double())[:, None] * torch.nn.functional.softplus(a.double() + dt_bias.double()).view(T, H, dk))
+    for got, want in ((qn, q * dk ** -0.5), (kn, kk), (vv, v), (gg, decay), (bb, torch.sigmoid(x[:, ob:ob + H]))):
+        assert (got.double() - want).abs().max() <= 64 * 2.0 ** -24 * max(1.0, float(want.abs().max()))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,P,parts", [(1, 4, 1), (4, 8, 8), (2, 64, 1), (3, 44, 1), (8, 64, 2), (16, 64, 1), (64, 64, 4), (257, 4, 1)])
+def test_state_space_gate_and_norm(H, P, parts, dtype):
+    """Slices of 4 to 1,024 channels in a warp's registers, a longer one and one that starts nowhere in particular."""
+    k, g = _k(), _gen(H * P + parts)
+    T, inner = 5, H * P
+
+    def rnd(*shape):
+        return torch.randn(shape, generator=g, device="cuda")
+
+    o, xs, proj, skip, w = rnd(T, H, P), rnd(T, H, P), rnd(T, 2 * inner + 8).to(dtype), rnd(H), rnd(inner)
+    z = proj[:, 8:8 + inner].double()
+    v = (o.double() + skip.double()[:, None] * xs.double()).view(T, inner) * torch.nn.functional.silu(z)
+    s = v.view(T, parts, -1)
+    want = (s / (s.square().mean(-1, keepdim=True) + 1e-5).sqrt()).reshape(T, inner) * w.double()
+    for off in (8, 9):
+        moved = proj if off == 8 else torch.cat([proj[:, -1:], proj[:, :-1]], 1).contiguous()
+        y = torch.full((T, inner), float("nan"), dtype=dtype, device="cuda")
+        k.ssm_gate_norm(y, o, xs, moved, off, skip, w, H, P, parts, 1e-5)
+        tol = 2.0 ** -8 if dtype == torch.bfloat16 else 64 * 2.0 ** -24
+        assert ((y.double() - want).abs() <= tol * want.abs() + 64 * 2.0 ** -24 * want.abs().max()).all()
+
+
+# one block a row and group, pieces of at least 4, 16 and 32 tiles of 64 keys: contexts at the pieces' edges beside short ones
+@pytest.mark.parametrize("rows,min_tiles", [(1, None), (8, None), (16, None), (24, None), (48, None), (49, None), (5, 1)])
+def test_decode_of_ragged_contexts(rows, min_tiles):
+    """Every row against float64, split as the plan for so many rows says; counters are left zero."""
+    k, g = _k(), _gen(rows)
+    nq, nkv, hd, page = 8, 2 if rows == 5 else 8, 128, 16
+    edges = [1, 63, 64, 65, 256, 257, 1024, 1025, 2047, 2048, 2049, 4096, 4097, 4160]
+    ctx = [edges[i % len(edges)] for i in range(rows)]
+    pages = [-(-c // page) for c in ctx]
+    order = torch.randperm(sum(pages), generator=torch.Generator().manual_seed(2)).to(torch.int32)
+    table, at = torch.full((rows, max(pages)), -1, dtype=torch.int32), 0
+    for r, n in enumerate(pages):
+        table[r, :n] = order[at:at + n]
+        at += n
+    kc, vc = (torch.randn((sum(pages), nkv, page, hd), generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    q = torch.randn((rows, nq, hd), generator=g, device="cuda").to(torch.bfloat16)
+    splits, tiles, in_kernel, n_acc, n_ml = k.attention_decode_plan(rows, nq, nkv, hd)
+    assert rows != 48 or (splits, tiles, in_kernel) == (4, 32, True)
+    acc, ml = torch.full((n_acc,), float("nan"), device="cuda"), torch.full((n_ml,), float("nan"), device="cuda")
+    count = torch.zeros(8192, dtype=torch.int32, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = torch.full_like(q, float("nan"))
+    i32 = dict(dtype=torch.int32, device="cuda")
+    k.attention_decode_tma(q, kc, vc, out, acc, ml, torch.tensor([c - 1 for c in ctx], **i32), torch.arange(rows, **i32),
+                           table.cuda(), rows, 0, rows, 0, hd ** -0.5, splits, status=status,
+                           merge_counters=count if in_kernel else None, min_tiles=min_tiles or tiles)
+    assert int(status.item()) == 0 and int(count.abs().sum()) == 0
+    for r, c in enumerate(ctx):
+        at = table[r, :pages[r]].long().cuda()
+        keys, values = (t[at].transpose(1, 2).reshape(-1, nkv, hd)[:c].double() for t in (kc, vc))
+        s = torch.einsum("hd,jhd->hj", q[r].double(), keys.repeat_interleave(nq // nkv, 1)) * hd ** -0.5
+        want = torch.einsum("hj,jhd->hd", torch.softmax(s, -1), values.repeat_interleave(nq // nkv, 1))
+        # (weights are rounded to bfloat16 for their product, results once more)
+        assert (out[r].double() - want).abs().max() <= 2.0 ** -7 * values.abs().max()

@@ -178,7 +178,8 @@ class LatentAttention(Mixer):
         kernels.latent_query_rows(qr, q, self.inv_freq, self.rot_dims, self.amp, step.positions, self.d, self.r)
         cols = 64 * (self.nd + self.nv)
         heads = max(1, min(H, kernels.LATENT_DENSE_ELEMENTS // (cap * cols)))
-        kv = rt.scratch.get(f"latent_kv:{cap}:{heads * cols}", (cap * heads * cols,), rt.dtype)
+        size = cap * H * cols if heads == H else kernels.LATENT_DENSE_ELEMENTS   # (one buffer for all that go in groups)
+        kv = rt.scratch.get(f"latent_kv:{size}", (size,), rt.dtype)
         for h0 in range(0, H, heads):
             hn = min(heads, H - h0)
             part = kv[:n * hn * cols].view(n, hn * cols)

@@ -614,8 +614,10 @@ CCB_API int ccb_delta_prepare(const void* proj, int ld, int oq, int ok, int ov, 
                    ((reinterpret_cast<uintptr_t>(qn) | reinterpret_cast<uintptr_t>(kn) | reinterpret_cast<uintptr_t>(vv) |
                      reinterpret_cast<uintptr_t>(gg) | reinterpret_cast<uintptr_t>(dt_bias) |
                      reinterpret_cast<uintptr_t>(conv_w)) & 15) == 0;
-  if (vec && dk <= 128 && dv <= 128 && taps <= 4 && T_ > kPrepRun && (dtype == CCB_F32 || dtype == CCB_BF16)) {
-    // (few rows: a warp each, as below, has more of them under way)
+  // Runs from 16,384 (row, head) units on, 110 an SM: before that a warp a row, as below, has more loads under way (64 heads'
+  // inputs of 128, a warp a row / four rows a warp: 16 rows 22.3 / 25.2 us, 64 rows 25.7 / 25.8, 512 rows 54.6 / 43.4)
+  if (vec && dk <= 128 && dv <= 128 && taps <= 4 && (long long)T_ * (2 * G + 2 * H) >= 16384 &&
+      (dtype == CCB_F32 || dtype == CCB_BF16)) {
     const dim3 run_grid((T_ + kPrepRun - 1) / kPrepRun, grid.y);
 #define CCB_RUN(TT, TAPS)                                                                                                  \
   ccb_launch(delta_prepare_run_kernel<TT, TAPS>, run_grid, dim3(kPrepWarps * 32), 0, stream, (const TT*)proj, ld, oq, ok, ov, \

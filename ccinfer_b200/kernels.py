@@ -646,14 +646,20 @@ def delta_recurrence(qn, kn, vv, gg, bb, state, out, cu_q, state_slot, n_entries
 
 # Tokens of a step's longest portion from which the recurrences run in chunks.  The token-by-token kernel costs half a
 # microsecond a token whatever runs beside it, a chunk of 64 tokens (however few of them are there) 4 us of its walk
-# after some 10 us of preparation.
+# after some 10 us of preparation.  32 heads of 128, token by token / in chunks, us: linear attention, 1 request of 32
+# tokens 19 / 20, of 48 27 / 20, 4 of 32 47 / 21; delta rule 1 of 32 21 / 25, of 48 27 / 33, of 64 35 / 35, of 128 64 / 42,
+# 4 of 16 27 / 31, of 32 48 / 42, 16 of 32 168 / 132: its chunks need 64 tokens, or 128 heads of portions beside one another.
 CHUNK_RECURRENCE_MIN_TOKENS = 32
+CHUNK_DELTA_FEW_HEADS, CHUNK_DELTA_FEW_MIN_TOKENS = 128, 64
 
 
-def chunk_recurrence_fits(dtype, dk: int, dv: int, max_tokens: int) -> bool:
+def chunk_recurrence_fits(dtype, dk: int, dv: int, max_tokens: int, delta_heads: int | None = None) -> bool:
     """Whether portions of prompts, the longest of max_tokens tokens, run as chunks on tensor cores: the 16-bit path (in
-    the 32-bit path every operand stays a float) with the sizes the kernel takes."""
-    return dtype == torch.bfloat16 and dk in (64, 128) and dv % 32 == 0 and max_tokens >= CHUNK_RECURRENCE_MIN_TOKENS
+    the 32-bit path every operand stays a float) with the sizes the kernel takes.  ``delta_heads``: the heads of all
+    portions where the delta rule is to run."""
+    few = delta_heads is not None and delta_heads < CHUNK_DELTA_FEW_HEADS
+    least = CHUNK_DELTA_FEW_MIN_TOKENS if few else CHUNK_RECURRENCE_MIN_TOKENS
+    return dtype == torch.bfloat16 and dk in (64, 128) and dv % 32 == 0 and max_tokens >= least
 
 
 def chunk_recurrence(scratch, qn, kn, vv, gg, bb, state, out, cu_q, state_slot, entry0: int, n_entries: int,
@@ -1453,7 +1459,8 @@ def ssm_prepare(proj, ox: int, odt: int, conv_w, conv_b, taps: int, conv_state, 
                                  _dt(proj), _stream()), "ssm_prepare")
 
 
-# (as CHUNK_RECURRENCE_MIN_TOKENS: a chunk costs what some tokens of the recurrence cost)
+# As CHUNK_RECURRENCE_MIN_TOKENS.  128 heads of 64 x 128, token by token / in chunks, us: 1 request of 16 tokens 15 / 19, of 32
+# 23 / 19, of 64 41 / 17, 4 of 16 38 / 35, of 32 68 / 35; 32 heads 1 of 32 15 / 18, of 48 19 / 18, 4 of 32 23 / 15.
 SSM_CHUNKS_MIN_TOKENS = 32
 
 

@@ -114,7 +114,8 @@ def test_recurrence_in_chunks(H, G, dk, dv, rule, decay):
     assert (state.double() - after).abs().max() <= 2.0 ** -14 * after.abs().max()
 
 
-@pytest.mark.parametrize("H,G,N,P", [(4, 2, 128, 64), (2, 1, 128, 16), (3, 3, 64, 48), (4, 1, 64, 32)])
+# one team of 16 columns, two teams of 16, two of 32 (75 blocks and more)
+@pytest.mark.parametrize("H,G,N,P", [(4, 2, 128, 64), (2, 1, 128, 16), (3, 3, 64, 48), (4, 1, 64, 32), (15, 3, 128, 64), (8, 2, 64, 128)])
 def test_state_space_recurrence_in_chunks(H, G, N, P):
     """Portions of a prompt beside single tokens, from the projection's rows: the chunks' rows and the recurrence in float64.
     An operand as two bfloat16 is right to 2^-17; sums of logarithms over 64 tokens that cancel to 2^-18 of 64 steps."""
@@ -324,13 +325,15 @@ def test_grouped_products_of_experts(mode, N, K, BM):
 
 
 # rows around the runs of four, requests of one row beside longer ones (their first rows read the convolution's state),
-# heads that fill a warp's 128 channels and that do not; steps of few rows take a warp a row
+# heads that fill a warp's 128 channels and that do not; steps of few rows take a warp a row, those with a long request runs
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("more", [0, 1, 3])
 @pytest.mark.parametrize("lens,taps,G,H,dk,dv", [
     ([5], 4, 1, 2, 128, 128), ([1, 1, 2, 4, 9], 4, 2, 2, 64, 32), ([3, 1, 1, 7], 2, 1, 1, 4, 128), ([6, 2], 1, 2, 4, 36, 12),
     ([1, 8, 3], 3, 1, 3, 128, 4), ([2, 1], 4, 1, 2, 128, 128)])
-def test_delta_rows_in_runs(lens, taps, G, H, dk, dv, dtype):
+def test_delta_rows_in_runs(lens, taps, G, H, dk, dv, more, dtype):
     """Against float64: a row's sums of ``taps`` products, one activation and one norm over dk squares."""
+    lens = lens + [16384 // (2 * G + 2 * H) + more] if more else lens
     k, g = _k(), _gen(sum(lens) + taps + dk)
     T, C = sum(lens), 2 * G * dk + H * dv
     ob = -(-C // 8) * 8
@@ -364,10 +367,12 @@ def test_delta_rows_in_runs(lens, taps, G, H, dk, dv, dtype):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("H,P,parts", [(1, 4, 1), (4, 8, 8), (2, 64, 1), (3, 44, 1), (8, 64, 2), (16, 64, 1), (64, 64, 4), (257, 4, 1)])
-def test_state_space_gate_and_norm(H, P, parts, dtype):
-    """Slices of 4 to 1,024 channels in a warp's registers, a longer one and one that starts nowhere in particular."""
+@pytest.mark.parametrize("few", [True, False])
+def test_state_space_gate_and_norm(H, P, parts, few, dtype):
+    """Slices of 4 to 1,024 channels in a warp's registers, a longer one and one that starts nowhere in particular; few
+    slices: a block each."""
     k, g = _k(), _gen(H * P + parts)
-    T, inner = 5, H * P
+    T, inner = 5 if few else 1024 // parts + 1, H * P
 
     def rnd(*shape):
         return torch.randn(shape, generator=g, device="cuda")
@@ -419,3 +424,44 @@ def test_decode_of_ragged_contexts(rows, min_tiles):
         want = torch.einsum("hj,jhd->hd", torch.softmax(s, -1), values.repeat_interleave(nq // nkv, 1))
         # (weights are rounded to bfloat16 for their product, results once more)
         assert (out[r].double() - want).abs().max() <= 2.0 ** -7 * values.abs().max()
+
+
+# one block a head from 16 requests of 32 heads on where key and value sizes are over 64; else a cluster a head
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("E,G,H,dk,dv", [(16, 32, 32, 128, 128), (16, 16, 32, 100, 68), (17, 16, 32, 68, 128), (15, 32, 32, 128, 128),
+                                         (16, 32, 32, 128, 64), (16, 32, 32, 64, 128), (32, 8, 16, 128, 128)])
+def test_delta_step_of_many_heads(E, G, H, dk, dv, dtype):
+    """One token of each request against float64; a request without a slot leaves its row and every state alone."""
+    k, g = _k(), _gen(E + dk + dv)
+    C = 2 * G * dk + H * dv
+    pad = -(-(C + 2 * H) // 8) * 8
+    off, width = (0, G * dk, 2 * G * dk, C, C + H, pad), pad + H * dv
+
+    def rnd(*shape):
+        return torch.randn(shape, generator=g, device="cuda")
+
+    conv_w, A_log, dt_bias, w, S = rnd(1, C), rnd(H), rnd(H), rnd(dv), rnd(E, H, dv, dk)
+    rule = k.HeadDelta(off, conv_w, A_log, dt_bias, G, H, dk, dv, dk ** -0.5, 1e-6)
+    proj, ring, before = rnd(E, width).to(dtype), torch.zeros(E, 1, C, dtype=dtype, device="cuda"), S.double()
+    i32 = dict(dtype=torch.int32, device="cuda")
+    slots = torch.arange(E - 1, -1, -1, **i32)
+    slots[1] = -1
+    y = torch.full((E, H * dv), 7.0, dtype=dtype, device="cuda")
+    k.delta_head_step(rule, proj, ring, S, w, 1e-5, torch.full((E,), 9, **i32), torch.arange(E + 1, **i32), slots, y, E)
+    x = proj.double()
+    c = torch.nn.functional.silu(x[:, :C] * conv_w[0].double())
+    q, key = (t.reshape(E, G, dk).repeat_interleave(H // G, 1) for t in (c[:, :G * dk], c[:, G * dk:2 * G * dk]))
+    q, key = (t / (t.square().sum(-1, keepdim=True) + 1e-6).sqrt() for t in (q, key))
+    v, beta = c[:, 2 * G * dk:].view(E, H, dv), torch.sigmoid(x[:, C:C + H])
+    decay = torch.exp(-torch.exp(A_log.double()) * torch.nn.functional.softplus(x[:, C + H:C + 2 * H] + dt_bias.double()))
+    old = before[slots.long()] * decay[..., None, None]
+    put = beta[..., None] * (v - torch.einsum("ehvk,ehk->ehv", old, key))
+    after = old + put[..., None] * key[:, :, None]
+    o = torch.einsum("ehvk,ehk->ehv", after, q) * dk ** -0.5
+    o = o / (o.square().mean(-1, keepdim=True) + 1e-5).sqrt() * w.double()
+    want = o.reshape(E, H * dv) * torch.nn.functional.silu(x[:, pad:])
+    want[1], after[1] = 7.0, before[E - 2]
+    # (sums of up to 128 products in any order; y is rounded once)
+    assert (S[torch.arange(E - 1, -1, -1)].double() - after).abs().max() <= 128 * 2.0 ** -24 * after.abs().max()
+    tol = 2.0 ** -8 if dtype == torch.bfloat16 else 0.0
+    assert ((y.double() - want).abs() <= tol * want.abs() + 256 * 2.0 ** -24 * want.abs().max()).all()

@@ -19,10 +19,11 @@
 // of the keys: n . q is one more column of o) the first slice takes it as one more block of eight columns.
 // The next chunk's rows arrive through cp.async while this one is computed; two barriers a chunk.
 //
-// A state space layer's recurrence is the same with values that are floats (they enter as two bfloat16 as well, one barrier
-// a chunk more) and with groups of heads that share queries and keys.  2,048 tokens of two requests, 128 heads of 64 x 128:
-// 1,034 us token by token, 459 us in chunks (one block of four warps an SM: the two halves of queries and keys fill its
-// shared memory).
+// A state space layer's recurrence is the same with values that are floats (they enter as two bfloat16 as well) and with
+// groups of heads that share queries and keys.  The two halves of queries and keys fill an SM's shared memory, so one block
+// runs on it: of two teams of four warps, a slice of value columns each, that share the tiles of queries and keys and the
+// weighted scores (a team makes those of every second block of 16 keys and leaves them for the other).  2,048 tokens of two
+// requests, 128 heads of 64 x 128: 1,034 us token by token, 459 us in chunks by one team a block, 225 us by two.
 #include "common.cuh"
 #include "mma_common.cuh"
 #include <math_constants.h>
@@ -32,7 +33,7 @@ using namespace ccb;
 namespace {
 
 constexpr int kChunk = 64;
-constexpr int kThreads = 128;
+constexpr int kThreads = 128;   // of a team
 
 struct ChunkArgs {
   const __nv_bfloat16 *q, *q_lo, *k, *k_lo, *v;
@@ -56,9 +57,10 @@ __device__ __forceinline__ void split2(float x, float y, uint32_t& hi, uint32_t&
   lo = pack_bf16(x - f.x, y - f.y);
 }
 
-template <int DK, int NB, bool SPLIT, bool ONES, bool V32>
-__global__ void __launch_bounds__(kThreads)
+template <int DK, int NB, bool SPLIT, bool ONES, bool V32, int TEAMS>
+__global__ void __launch_bounds__(kThreads * TEAMS)
 memory_chunks_kernel(const ChunkArgs a) {
+  static_assert(TEAMS == 1 || (V32 && TEAMS == 2), "two teams: with float values");
   ccb::pdl_begin();
   constexpr int BN = 8 * NB, VP = BN + 8;      // columns of the slice, pitch of its rows in shared memory (elements)
   constexpr int NT = NB + (ONES ? 1 : 0);      // blocks of eight columns
@@ -68,19 +70,21 @@ memory_chunks_kernel(const ChunkArgs a) {
   constexpr int QK = SPLIT ? 4 : 2;            // tiles of a stage: q, k (, their second halves)
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __nv_bfloat16* tiles = reinterpret_cast<__nv_bfloat16*>(smem_raw);   // [2][QK][64][DK], swizzled
-  __nv_bfloat16* v_s = tiles + 2 * QK * TILE;                          // [2][64][VP] (V32: the values' two halves)
+  constexpr int TEAM = 4 * VT + 2 * DK * VP;                           // elements that a team has for itself
+  const int team = threadIdx.x / kThreads;
+  __nv_bfloat16* v_s = tiles + 2 * QK * TILE + team * TEAM;            // [2][64][VP] (V32: the values' two halves)
   __nv_bfloat16* s_hi = v_s + 2 * VT;                                  // [DK][VP]
   __nv_bfloat16* s_lo = s_hi + DK * VP;
   __nv_bfloat16* w_hi = s_lo + DK * VP;                                // [64][VP]
   __nv_bfloat16* w_lo = w_hi + VT;
-  float* gates = reinterpret_cast<float*>(w_lo + VT);                  // [2][4][64]: c_t, exp(c_t), log b - c, weights
-  float* v32_s = gates + 2 * 4 * kChunk;                               // V32: [2][64][BN]
+  float* gates = reinterpret_cast<float*>(tiles + 2 * QK * TILE + TEAMS * TEAM);   // [2][4][64]: c_t, exp(c_t), log b - c, weights
+  uint4* p_s = reinterpret_cast<uint4*>(gates + 2 * 4 * kChunk);       // two teams: weighted scores, [10 tiles][2][32]
 
-  const int e = a.entry0 + blockIdx.z, h = blockIdx.y, slice = blockIdx.x;
+  const int e = a.entry0 + blockIdx.z, h = blockIdx.y, slice = blockIdx.x * TEAMS + team;
   const int slot = a.state_slot[e];
   const int r0 = a.cu_q[e], n = a.cu_q[e + 1] - r0;
   if (slot < 0 || slot >= a.max_slots || n <= 0) return;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x % kThreads, lane = tid & 31, warp = tid >> 5;   // in the team
   const int gid = lane >> 2, tig = lane & 3;
   const int kvh = h / a.group;
   const int col0 = slice * BN;
@@ -94,25 +98,14 @@ memory_chunks_kernel(const ChunkArgs a) {
 #pragma unroll
     for (int x = 0; x < QK; ++x)
 #pragma unroll
-      for (int i = 0; i < kChunk * (DK / 8) / kThreads; ++i) {
-        const int idx = tid + kThreads * i;
+      for (int i = 0; i < kChunk * (DK / 8) / (kThreads * TEAMS); ++i) {
+        const int idx = threadIdx.x + kThreads * TEAMS * i;
         const int row = idx / (DK / 8), c = idx % (DK / 8);
         const bool ok = t0 + row < n;
         cp_async16(smem_u32(dst + x * TILE + swz<DK>(row, c)),
                    src[x] + (size_t)(r0 + t0 + (ok ? row : 0)) * a.ldqk + kvh * DK + c * 8, ok);
       }
-    if constexpr (V32) {
-#pragma unroll
-      for (int i = 0; i < kChunk * 2 * NB / kThreads; ++i) {
-        const int idx = tid + kThreads * i;
-        const int row = idx / (2 * NB), c = idx % (2 * NB);
-        const bool ok = t0 + row < n;
-        cp_async16(smem_u32(v32_s + (st * kChunk + row) * BN + c * 4),
-                   a.v32 + (size_t)(r0 + t0 + (ok ? row : 0)) * a.ldv + h * a.dv + col0 + c * 4, ok);
-      }
-      cp_async_commit();
-      return;
-    }
+    if constexpr (!V32) {
 #pragma unroll
     for (int i = 0; i < (kChunk * NB + kThreads - 1) / kThreads; ++i) {
       const int idx = tid + kThreads * i;
@@ -121,7 +114,17 @@ memory_chunks_kernel(const ChunkArgs a) {
       cp_async16(smem_u32(v_s + st * VT + row * VP + c * 8),
                  a.v + (size_t)(r0 + t0 + (ok ? row : 0)) * a.ldv + h * a.dv + col0 + c * 8, ok);
     }
+    }
     cp_async_commit();
+  };
+
+  // V32: half a row of the slice a thread, loaded one chunk ahead
+  float4 vv[V32 ? NB : 1];
+  auto load_values = [&](int chunk) {
+    const int t = chunk * kChunk + (tid >> 1);
+    const float4* src = reinterpret_cast<const float4*>(a.v32 + (size_t)(r0 + t) * a.ldv + h * a.dv + col0 + (tid & 1) * (BN / 2));
+#pragma unroll
+    for (int c = 0; c < NB; ++c) vv[c] = t < n ? src[c] : make_float4(0.f, 0.f, 0.f, 0.f);
   };
 
   // The gates of a chunk, two tokens a lane of warp 0: loaded one chunk ahead, summed and left in shared memory.
@@ -156,7 +159,9 @@ memory_chunks_kernel(const ChunkArgs a) {
   };
 
   issue(0, 0);
-  if (warp == 0) {
+  if constexpr (V32) load_values(0);
+  const bool gating = warp == 0 && team == 0;
+  if (gating) {
     load_gates(0);
     write_gates(0);
     load_gates(1);
@@ -216,7 +221,7 @@ memory_chunks_kernel(const ChunkArgs a) {
     cp_async_wait<0>();
     __syncthreads();   // the chunk's rows and gates are there; everybody is done with the chunk before
     if (ch + 1 < chunks) issue(ch + 1, st ^ 1);
-    if (warp == 0 && ch + 1 < chunks) {
+    if (gating && ch + 1 < chunks) {
       write_gates(st ^ 1);
       load_gates(ch + 2);
     }
@@ -228,10 +233,9 @@ memory_chunks_kernel(const ChunkArgs a) {
       const int row = tid >> 1, part = (tid & 1) * (BN / 2);
       const float w = gw[row];
       if constexpr (V32) {
-        const float* v32 = v32_s + (st * kChunk + row) * BN + part;
 #pragma unroll
         for (int c = 0; c < BN / 2; c += 2) {
-          const float2 f = *reinterpret_cast<const float2*>(v32 + c);
+          const float2 f = c & 2 ? make_float2(vv[c / 4].z, vv[c / 4].w) : make_float2(vv[c / 4].x, vv[c / 4].y);
           uint32_t hi, lo;
           split2(f.x, f.y, hi, lo);
           *reinterpret_cast<uint32_t*>(v_s + row * VP + part + c) = hi;
@@ -240,6 +244,7 @@ memory_chunks_kernel(const ChunkArgs a) {
           *reinterpret_cast<uint32_t*>(w_hi + row * VP + part + c) = hi;
           *reinterpret_cast<uint32_t*>(w_lo + row * VP + part + c) = lo;
         }
+        if (ch + 1 < chunks) load_values(ch + 1);
       } else {
 #pragma unroll
       for (int c = 0; c < BN / 2; c += 2) {
@@ -259,11 +264,13 @@ memory_chunks_kernel(const ChunkArgs a) {
     }
 
     // read-out of rows warp * 16 ..: first S0^T q and the raw scores q . k of the keys up to the rows' own block
-    float acc[NT][4], s[2 * 4][4];
+    // (two teams: of every second block of keys each)
+    constexpr int NP = 4 / TEAMS;
+    float acc[NT][4], s[2 * NP][4];
 #pragma unroll
     for (int nb = 0; nb < NT; ++nb) acc[nb][0] = acc[nb][1] = acc[nb][2] = acc[nb][3] = 0.f;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.f;
+    for (int i = 0; i < 2 * NP; ++i) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.f;
     const int arow = warp * 16 + (lane & 7) + 8 * ((lane >> 3) & 1), achunk = lane >> 4;
     const int krow = (lane & 7) + 8 * (lane >> 4), kchunk = (lane >> 3) & 1;
 #pragma unroll 2
@@ -288,22 +295,23 @@ memory_chunks_kernel(const ChunkArgs a) {
         }
       }
 #pragma unroll
-      for (int np = 0; np < 4; ++np) {
+      for (int p = 0; p < NP; ++p) {
+        const int np = TEAMS * p + (TEAMS > 1 ? team : 0);
         if (np > warp) continue;
         uint32_t b[4];
         ldmatrix_x4(b[0], b[1], b[2], b[3], smem_u32(kt + swz<DK>(np * 16 + krow, 2 * ks + kchunk)));
-        mma_bf16_16816(s[2 * np], qa, b[0], b[1]);
-        mma_bf16_16816(s[2 * np + 1], qa, b[2], b[3]);
+        mma_bf16_16816(s[2 * p], qa, b[0], b[1]);
+        mma_bf16_16816(s[2 * p + 1], qa, b[2], b[3]);
         if (SPLIT) {
-          mma_bf16_16816(s[2 * np], qb, b[0], b[1]);
-          mma_bf16_16816(s[2 * np + 1], qb, b[2], b[3]);
+          mma_bf16_16816(s[2 * p], qb, b[0], b[1]);
+          mma_bf16_16816(s[2 * p + 1], qb, b[2], b[3]);
           ldmatrix_x4(b[0], b[1], b[2], b[3], smem_u32(kl + swz<DK>(np * 16 + krow, 2 * ks + kchunk)));
-          mma_bf16_16816(s[2 * np], qa, b[0], b[1]);
-          mma_bf16_16816(s[2 * np + 1], qa, b[2], b[3]);
+          mma_bf16_16816(s[2 * p], qa, b[0], b[1]);
+          mma_bf16_16816(s[2 * p + 1], qa, b[2], b[3]);
         }
       }
     }
-    if (V32) __syncthreads();   // the values' halves are complete
+    if (V32 && TEAMS == 1) __syncthreads();   // the values' halves are complete
     const int t_lo = warp * 16 + gid, t_hi = t_lo + 8;
     const float a_lo = ga[t_lo] * a.q_mult, a_hi = ga[t_hi] * a.q_mult;
     const float c_lo = gc[t_lo], c_hi = gc[t_hi];
@@ -312,13 +320,11 @@ memory_chunks_kernel(const ChunkArgs a) {
       acc[nb][0] *= a_lo; acc[nb][1] *= a_lo;
       acc[nb][2] *= a_hi; acc[nb][3] *= a_hi;
     }
-#pragma unroll
-    for (int np = 0; np < 4; ++np) {
-      if (np > warp) continue;
-      uint32_t ph[4], pl[4];
+    // weights of a block of 16 keys, times its scores, as two bfloat16
+    auto weigh = [&](int np, float (*sc)[4], uint32_t* ph, uint32_t* pl) {
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
-        float* x = s[2 * np + half];
+        float* x = sc[half];
         const int j = np * 16 + half * 8 + 2 * tig;
         const float b0 = gb[j], b1 = gb[j + 1];
         x[0] = j <= t_lo ? x[0] * (__expf(c_lo + b0) * a.q_mult) : 0.f;
@@ -328,6 +334,8 @@ memory_chunks_kernel(const ChunkArgs a) {
         split2(x[0], x[1], ph[2 * half], pl[2 * half]);
         split2(x[2], x[3], ph[2 * half + 1], pl[2 * half + 1]);
       }
+    };
+    auto weighted_values = [&](int np, const uint32_t* ph, const uint32_t* pl) {
 #pragma unroll
       for (int nb = 0; nb < NT; nb += 2) {
         if (nb >= nt) continue;
@@ -346,6 +354,33 @@ memory_chunks_kernel(const ChunkArgs a) {
           if (!single) mma_bf16_16816(acc[nb + 1 < NT ? nb + 1 : nb], ph, b[2], b[3]);
         }
       }
+    };
+    if constexpr (TEAMS == 1) {
+#pragma unroll
+      for (int np = 0; np < 4; ++np) {
+        if (np > warp) continue;
+        uint32_t ph[4], pl[4];
+        weigh(np, s + 2 * np, ph, pl);
+        weighted_values(np, ph, pl);
+      }
+    } else {
+#pragma unroll
+      for (int p = 0; p < NP; ++p) {
+        const int np = 2 * p + team;
+        if (np > warp) continue;
+        uint32_t ph[4], pl[4];
+        weigh(np, s + 2 * p, ph, pl);
+        uint4* to = p_s + (warp * (warp + 1) / 2 + np) * 64 + lane;
+        to[0] = make_uint4(ph[0], ph[1], ph[2], ph[3]);
+        to[32] = make_uint4(pl[0], pl[1], pl[2], pl[3]);
+      }
+      __syncthreads();   // the weighted scores and both forms of the values are complete, and everybody has read S0
+      for (int np = 0; np <= warp; ++np) {
+        const uint4* from = p_s + (warp * (warp + 1) / 2 + np) * 64 + lane;
+        const uint4 x = from[0], y = from[32];
+        const uint32_t ph[4] = {x.x, x.y, x.z, x.w}, pl[4] = {y.x, y.y, y.z, y.w};
+        weighted_values(np, ph, pl);
+      }
     }
     const int left = n - ch * kChunk;
 #pragma unroll
@@ -361,7 +396,7 @@ memory_chunks_kernel(const ChunkArgs a) {
         if (ones && tig == 0) o[a.dv] = acc[NT - 1][2 * x];
       }
     }
-    __syncthreads();   // everybody has read S0, and the weighted values are complete
+    if constexpr (TEAMS == 1) __syncthreads();   // everybody has read S0, and the weighted values are complete
 
     const float keep = ga[kChunk - 1];   // exp(c_64)
 #pragma unroll
@@ -415,21 +450,20 @@ memory_chunks_kernel(const ChunkArgs a) {
       }
 }
 
-template <int DK, int NB, bool SPLIT, bool ONES, bool V32 = false>
+template <int DK, int NB, bool SPLIT, bool ONES, bool V32 = false, int TEAMS = 1>
 int launch_chunks(const ChunkArgs& a, int n_entries, cudaStream_t stream) {
   constexpr int VP = 8 * NB + 8;
-  constexpr size_t smem = (size_t)(2 * (SPLIT ? 4 : 2) * kChunk * DK + 2 * kChunk * VP + 2 * DK * VP + 2 * kChunk * VP) * 2 +
-                          2 * 4 * kChunk * sizeof(float) + (V32 ? (size_t)2 * kChunk * 8 * NB * sizeof(float) : 0);
+  constexpr size_t smem = (size_t)(2 * (SPLIT ? 4 : 2) * kChunk * DK + TEAMS * (4 * kChunk * VP + 2 * DK * VP)) * 2 +
+                          2 * 4 * kChunk * sizeof(float) + (TEAMS > 1 ? 10 * 2 * 32 * sizeof(uint4) : 0);
   static_assert(smem <= 227 * 1024, "shared memory of a block");
+  const auto kernel = memory_chunks_kernel<DK, NB, SPLIT, ONES, V32, TEAMS>;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(memory_chunks_kernel<DK, NB, SPLIT, ONES, V32>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  ccb_launch(memory_chunks_kernel<DK, NB, SPLIT, ONES, V32>, dim3(a.dv / (8 * NB), a.H, n_entries), dim3(kThreads), smem, stream,
-             a);
+  ccb_launch(kernel, dim3(a.dv / (8 * NB * TEAMS), a.H, n_entries), dim3(kThreads * TEAMS), smem, stream, a);
   return ccb_launch_status();
 }
 
@@ -479,7 +513,11 @@ CCB_API int ccb_ssm_chunks(const void* q, const void* q_lo, const void* k, const
   if ((bits(q) | bits(q_lo) | bits(k) | bits(k_lo) | bits(v)) & 15) return CCB_REFUSE_ARG;
   const ChunkArgs a{(const __nv_bfloat16*)q, (const __nv_bfloat16*)q_lo, (const __nv_bfloat16*)k, (const __nv_bfloat16*)k_lo,
                     nullptr, v, ldqk, ldv, H / G, log_a, log_b, state, out, cu_q, state_slot, entry0, H, P, P, max_slots, 1.f};
-  const bool wide = P % 32 == 0 && (long long)(P / 32) * H * n_entries >= 96;
-  if (N == 128) return wide ? launch_chunks<128, 4, true, false, true>(a, n_entries, stream) : launch_chunks<128, 2, true, false, true>(a, n_entries, stream);
-  return wide ? launch_chunks<64, 4, true, false, true>(a, n_entries, stream) : launch_chunks<64, 2, true, false, true>(a, n_entries, stream);
+  // Two teams where P is a multiple of 32, of 32 columns each where that gives half the SMs a block, else (the walk of a request
+  // is a serial chain, and narrower slices have more SMs at it) of 16; one team of 16 for other P.
+  const bool wide = P % 64 == 0 && (long long)(P / 64) * H * n_entries >= 74;
+#define CCB_SSM_CHUNKS(DK)                                                                  return wide          ? launch_chunks<DK, 4, true, false, true, 2>(a, n_entries, stream)          : P % 32 == 0 ? launch_chunks<DK, 2, true, false, true, 2>(a, n_entries, stream)                        : launch_chunks<DK, 2, true, false, true, 1>(a, n_entries, stream)
+  if (N == 128) CCB_SSM_CHUNKS(128);
+  CCB_SSM_CHUNKS(64);
+#undef CCB_SSM_CHUNKS
 }

@@ -70,18 +70,24 @@ __device__ __forceinline__ float dot4(const float4 a, const float4 b) {
 __device__ __forceinline__ float silu_f(float x) { return x * sigmoid_f(x); }
 __device__ __forceinline__ float4 silu4(const float4 x) { return make_float4(silu_f(x.x), silu_f(x.y), silu_f(x.z), silu_f(x.w)); }
 
-constexpr int kStepWarps = 4, kStepThreads = 32 * kStepWarps;
-constexpr int kStepCols = 8;   // columns of S a warp holds at once where a column takes all its lanes
+// Warps of a block, and columns of S a warp holds at once where a column takes all its lanes.  Few requests: four warps and
+// eight columns, four blocks a head of 128, so that every SM has some.  Many: eight warps and sixteen columns, one block a
+// head, which then redoes no q and k and needs no other block's sum of squares; its whole state (64 KB) is in flight at once.
+// A block's chain of waits and not the memory sets the pace, so what it waits for is asked for at its start (state, position,
+// the output's gate), and its sums take few exchanges.  48 requests of 32 heads of 128 x 128, 201 MB: 97 us in clusters of
+// four small blocks, 67 us so.
+constexpr int kStepWarpsFew = 4, kStepColsFew = 8, kStepWarpsMany = 8, kStepColsMany = 16;
 
 // Single tokens.  A cluster of blocks (.x) per (head, request): each redoes the head's q and k and owns a run of
 // `cols` value channels, i.e. columns of S; the sum of squares that the output's norm divides by is made over the cluster.
 // VEC: dk, dv and cols multiples of 4, dk <= 128 X, rows and columns aligned: four channels or key rows a lane, and the
 // block's columns of S are asked for before anything else (an earlier step wrote them: they need not wait for the
 // projection before this kernel).
-template <typename T, bool VEC, int X>
-__global__ void __launch_bounds__(kStepThreads)
+template <typename T, bool VEC, int X, int kStepWarps, int kStepCols>
+__global__ void __launch_bounds__(32 * kStepWarps, kStepWarps == kStepWarpsMany ? 2 : !VEC ? 10 : X == 1 ? 5 : 3)
 delta_head_step_kernel(const T* __restrict__ proj, T* __restrict__ ring, float* __restrict__ state,
                        const float* __restrict__ w, float eps, T* __restrict__ y, int ldy, int cols, const HeadDelta a) {
+  constexpr int kStepThreads = 32 * kStepWarps;
   extern __shared__ __align__(16) float sm[];   // q [dkp], k [dkp], v [cols], o [cols]
   __shared__ float red[3 * kStepWarps + 32];
   __shared__ float slots[kMaxClusterBlocks];
@@ -113,10 +119,13 @@ delta_head_step_kernel(const T* __restrict__ proj, T* __restrict__ ring, float* 
     }
   };
   if (VEC) fetch(0);
+  const int t = a.cu_q[e], pos = live ? a.positions[t] : 0;   // (written with state_slot)
   ccb::pdl_begin();
+  // the thread's first column of the output: its gate and weight are there when the state has been read
+  float gate0 = 0.f, w0 = 0.f;
   if (live) {
-    const int t = a.cu_q[e], pos = a.positions[t];
     const T* row = proj + (size_t)t * a.ld;
+    if (threadIdx.x < n_cols) gate0 = to_f32(row[a.og + h * dv + c_lo + threadIdx.x]), w0 = w[c_lo + threadIdx.x];
     const bool owns_kv = blockIdx.x == 0 && h % per_kv == 0;   // this block writes its group's q and k channels to the ring
     float ssq = 0.f, ssk = 0.f;
     constexpr int W = VEC ? 4 : 1;
@@ -192,7 +201,40 @@ delta_head_step_kernel(const T* __restrict__ proj, T* __restrict__ ring, float* 
     const float g = gates[0], beta = gates[1];
     // a column of S (one value channel): S^T k and S^T q of the decayed state, then the write; the read-out after the
     // write is (g S)^T q + u (k . q)
-    if constexpr (VEC) {
+    if constexpr (kStepCols == kStepColsMany) {
+      // (a column takes all 32 lanes, and the block holds all columns) the 32 sums of the warp's 16 columns, one a lane in
+      // the end: 31 exchanges instead of 160
+      const bool on = 4 * li < dk;
+      const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 kk = on ? *reinterpret_cast<const float4*>(k_s + 4 * li) : none;
+      const float4 qq = on ? *reinterpret_cast<const float4*>(q_s + 4 * li) : none;
+      float m[kStepCols];
+#pragma unroll
+      for (int u = 0; u < kStepCols; ++u) {
+        float4& z = s[u][0];
+        z.x *= g; z.y *= g; z.z *= g; z.w *= g;
+        const float dotk = on ? dot4(z, kk) : 0.f, dotq = on ? dot4(z, qq) : 0.f;
+        m[u] = (lane & 16 ? dotq : dotk) + __shfl_xor_sync(0xffffffffu, lane & 16 ? dotk : dotq, 16);
+      }
+#pragma unroll
+      for (int o = kStepCols / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int u = 0; u < o; ++u)
+          m[u] = (lane & o ? m[u + o] : m[u]) + __shfl_xor_sync(0xffffffffu, lane & o ? m[u] : m[u + o], o);
+      const int mine = warp + (lane & 15) * stride;   // lane u: k's product with column u; lane 16 + u: q's
+      const float other = __shfl_xor_sync(0xffffffffu, m[0], 16);
+      const float put0 = mine < n_cols && lane < 16 ? beta * (v_s[mine] - m[0]) : 0.f;
+#pragma unroll
+      for (int u = 0; u < kStepCols; ++u) {
+        const float put = __shfl_sync(0xffffffffu, put0, u);
+        const int c = warp + u * stride;
+        if (c < n_cols && on) {
+          fma4(s[u][0], kk, make_float4(put, put, put, put));
+          *reinterpret_cast<float4*>(S + (size_t)c * dk + 4 * li) = s[u][0];
+        }
+      }
+      if (mine < n_cols && lane < 16) o_s[mine] = fmaf(put0, kq, other);
+    } else if constexpr (VEC) {
       for (int base = 0; base < n_cols; base += kStepCols * stride) {
         if (base > 0) fetch(base);
 #pragma unroll
@@ -250,10 +292,11 @@ delta_head_step_kernel(const T* __restrict__ proj, T* __restrict__ ring, float* 
   ss = cluster_sum(block_sum<kStepThreads>(ss, red), slots);   // (every block of the cluster, whether its request is live or not)
   if (!live) return;
   const float inv = 1.0f / sqrtf(ss / (float)dv + eps);
-  const int t = a.cu_q[e];
   for (int i = threadIdx.x; i < n_cols; i += kStepThreads) {
     const int c = h * dv + c_lo + i;
-    y[(size_t)t * ldy + c] = from_f32<T>(o_s[i] * inv * w[c_lo + i] * silu_f(to_f32(proj[(size_t)t * a.ld + a.og + c])));
+    const bool first = i == threadIdx.x;
+    const float gate = first ? gate0 : to_f32(proj[(size_t)t * a.ld + a.og + c]), wi = first ? w0 : w[c_lo + i];
+    y[(size_t)t * ldy + c] = from_f32<T>(o_s[i] * inv * wi * silu_f(gate));
   }
 }
 
@@ -463,25 +506,31 @@ CCB_API int ccb_delta_head_step(const void* proj, int ld, const int* offsets, co
   const HeadDelta a = head_delta(ld, offsets, G, H, dk, dv, taps, conv_w, A_log, dt_bias, positions, nullptr, cu_q,
                                  state_slot, q_mult, unit_eps, n_slots);
   if (!sizes_ok(a) || n_entries > 65535 || ldy < H * dv) return CCB_REFUSE_SIZE;
-  // about 32 value channels a block, at most eight blocks a head
-  int n_blocks = (dv + 31) / 32;
+  const int esz = dtype == CCB_F32 ? 4 : 2;
+  const bool vec = dk % 4 == 0 && dv % 4 == 0 && dk <= 256 && ld % 4 == 0 && a.oq % 4 == 0 && a.ok % 4 == 0 && a.ov % 4 == 0 &&
+                   (reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(ring)) % (4 * esz) == 0 &&
+                   ((reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(conv_w)) & 15) == 0;
+  // one block a head where that gives two for every SM and a block holds the head's columns at once (32 heads of 128, L2 cold,
+  // with some 20 us of launch, clusters of four / one block, us: 10 requests 43 / 41, 16 55 / 45, 32 88 / 67, 96 215 / 148;
+  // two blocks do better for heads of 64 columns)
+  const bool many = vec && dk <= 128 && dk > 64 && dv <= kStepWarpsMany * kStepColsMany && dv > 64 && (long long)n_entries * H >= 2 * 148;
+  // else about 32 value channels a block, at most eight blocks a head
+  int n_blocks = many ? 1 : (dv + 31) / 32;
   if (n_blocks > kMaxClusterBlocks) n_blocks = kMaxClusterBlocks;
   const int cols = ((dv + n_blocks - 1) / n_blocks + 3) & ~3;
   n_blocks = (dv + cols - 1) / cols;
   const size_t smem = (size_t)(2 * ((dk + 3) & ~3) + 2 * cols) * sizeof(float);
   if (smem > 44 * 1024) return CCB_REFUSE_SIZE;
-  const int esz = dtype == CCB_F32 ? 4 : 2;
-  const bool vec = dk % 4 == 0 && dv % 4 == 0 && dk <= 256 && ld % 4 == 0 && a.oq % 4 == 0 && a.ok % 4 == 0 && a.ov % 4 == 0 &&
-                   (reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(ring)) % (4 * esz) == 0 &&
-                   ((reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(conv_w)) & 15) == 0;
-#define CCB_STEP(TT, VV, XX)                                                                                          \
-  ccb_launch_cluster(true, n_blocks, delta_head_step_kernel<TT, VV, XX>, dim3(n_blocks, H, n_entries),                \
-                     dim3(kStepThreads), smem, stream, (const TT*)proj, (TT*)ring, state, w, eps, (TT*)y, ldy, cols, a)
+#define CCB_STEP(TT, VV, XX, SIZE)                                                                                    \
+  ccb_launch_cluster(true, n_blocks, delta_head_step_kernel<TT, VV, XX, kStepWarps##SIZE, kStepCols##SIZE>,           \
+                     dim3(n_blocks, H, n_entries), dim3(32 * kStepWarps##SIZE), smem, stream, (const TT*)proj,        \
+                     (TT*)ring, state, w, eps, (TT*)y, ldy, cols, a)
 #define CCB_STEP_X(TT)                                                                                                \
   do {                                                                                                                \
-    if (!vec) CCB_STEP(TT, false, 1);                                                                                 \
-    else if (dk <= 128) CCB_STEP(TT, true, 1);                                                                        \
-    else CCB_STEP(TT, true, 2);                                                                                       \
+    if (many) CCB_STEP(TT, true, 1, Many);                                                                            \
+    else if (!vec) CCB_STEP(TT, false, 1, Few);                                                                       \
+    else if (dk <= 128) CCB_STEP(TT, true, 1, Few);                                                                   \
+    else CCB_STEP(TT, true, 2, Few);                                                                                  \
   } while (0)
   if (dtype == CCB_F32) CCB_STEP_X(float);
   else if (dtype == CCB_BF16) CCB_STEP_X(__nv_bfloat16);

@@ -21,6 +21,7 @@ namespace {
 
 constexpr int kTileKeys = 64;
 constexpr int kStages = 3;
+constexpr int kMergeAtOnce = 10;   // splits of a row whose results a thread holds at once when it merges them
 constexpr int kComputeThreads = 128;
 constexpr int kThreads = 192;  // four compute warps and two producer warps (keys, values)
 constexpr int kHalfBytes = kTileKeys * 128;  // 64 rows x 64 columns of bfloat16
@@ -134,6 +135,8 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
   for (int i = 0; i < 2 * KS; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
   float m0 = -CUDART_INF_F, m1 = -CUDART_INF_F, l0 = 0.f, l1 = 0.f;
   bool owner = false;   // fused form: this block's key range ends at the row's own position
+  constexpr int CPL = HD / 32;
+  __nv_bfloat16 kb[CPL], vb[CPL];   // that position's key and value: columns CPL lane .. of warp 4
 
   if (!padded) {
     // q as A fragments: rows = heads of the group (zero beyond n_heads); the producer warp has none
@@ -277,6 +280,56 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
         issue(my_first + j, st);
       }
     }
+    if (FUSED && warp == 4 && owner) {
+      // The row's own key and value, from the product's row: norm, rotation, rounding as the cache holds them; into their
+      // page for the steps to come, and kept for the result.  A lane has HD / 32 consecutive columns; the partner of a
+      // rotation is 16 lanes away.  Done here, while the compute warps are at the last tiles, and not after them:
+      // 8 rows of 60 keys 10.6 -> 10.3 us, of 256 12.6 -> 12.35.
+      ccb::pdl_wait();   // (only the compute warps have waited)
+      const int col0 = lane * CPL;
+      const __nv_bfloat16* krow = fq.qkv + (size_t)t * fq.stride + (size_t)(nq + kvh) * HD;
+      const __nv_bfloat16* vrow = krow + (size_t)nkv * HD;
+      float kx[CPL];
+      float ss = 0.f;
+#pragma unroll
+      for (int c = 0; c < CPL; ++c) {
+        kx[c] = __bfloat162float(krow[col0 + c]);
+        vb[c] = vrow[col0 + c];
+        if (fq.bias != nullptr) {
+          kx[c] += fq.bias[(size_t)(nq + kvh) * HD + col0 + c];
+          vb[c] = __float2bfloat16_rn(__bfloat162float(vb[c]) + fq.bias[(size_t)(nq + nkv + kvh) * HD + col0 + c]);
+        }
+        ss += kx[c] * kx[c];
+      }
+      if (fq.k_w != nullptr) {
+        ss = warp_sum(ss);
+        const float inv = 1.0f / sqrtf(ss / (float)HD + fq.eps);
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) kx[c] *= inv * fq.k_w[col0 + c];
+      }
+      const bool first_half = lane < 16;
+#pragma unroll
+      for (int c = 0; c < CPL; ++c) {
+        const float other = __shfl_xor_sync(0xffffffffu, kx[c], 16);
+        const int i = (col0 + c) & (HD / 2 - 1);
+        const float2 cs = cs_sm[i];
+        const float a = first_half ? kx[c] : other, bb = first_half ? other : kx[c];
+        kb[c] = __float2bfloat16_rn(first_half ? a * cs.x - bb * cs.y : bb * cs.x + a * cs.y);
+      }
+      const int page = lp_last < bt_stride ? bt[lp_last] : -1;
+      if (page < 0 || page >= num_pages) {
+        if (lane == 0) set_status(status, CCB_ST_BAD_PAGE);
+      } else if (gc == 0) {   // one block per kv head writes, once its own copy of the page is complete
+        if (!mbar_wait(bar0 + 8 * ((my_tiles - 1) % kStages), ((my_tiles - 1) / kStages) & 1) && lane == 0)
+          set_status(status, CCB_ST_WAIT_TIMEOUT);
+        const size_t dst = (((size_t)page * nkv + kvh) * page_size + (p & (page_size - 1))) * HD + col0;
+#pragma unroll
+        for (int c = 0; c < CPL; ++c) {
+          fq.k_cache[dst + c] = kb[c];
+          fq.v_cache[dst + c] = vb[c];
+        }
+      }
+    }
     for (int it = 0; warp < 4 && it < my_tiles; ++it) {
       const int st = it % kStages;
       if (!mbar_wait(bar0 + 8 * st, (it / kStages) & 1)) {
@@ -372,57 +425,8 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
   float* m_s = o_s + 5 * 16 * HD;                   // [5][16]
   float* l_s = m_s + 80;
   const int n_part = owner ? 5 : 4;
-  if (FUSED && warp == 4 && owner) {
-    // The row's own key and value, from the product's row: norm, rotation, rounding as the cache holds them;
-    // into their page for the steps to come, and into the result as a fifth partial (one key: its score is
-    // the maximum, its weight 1, its output the value).  A lane has HD / 32 consecutive columns; the partner
-    // of a rotation is 16 lanes away.
-    constexpr int CPL = HD / 32;
+  if (FUSED && warp == 4 && owner) {   // a fifth partial (one key: its score is the maximum, its weight 1, its output the value)
     const int col0 = lane * CPL;
-    const __nv_bfloat16* krow = fq.qkv + (size_t)t * fq.stride + (size_t)(nq + kvh) * HD;
-    const __nv_bfloat16* vrow = krow + (size_t)nkv * HD;
-    float kx[CPL];
-    __nv_bfloat16 vb[CPL];
-    float ss = 0.f;
-#pragma unroll
-    for (int c = 0; c < CPL; ++c) {
-      kx[c] = __bfloat162float(krow[col0 + c]);
-      vb[c] = vrow[col0 + c];
-      if (fq.bias != nullptr) {
-        kx[c] += fq.bias[(size_t)(nq + kvh) * HD + col0 + c];
-        vb[c] = __float2bfloat16_rn(__bfloat162float(vb[c]) + fq.bias[(size_t)(nq + nkv + kvh) * HD + col0 + c]);
-      }
-      ss += kx[c] * kx[c];
-    }
-    if (fq.k_w != nullptr) {
-      ss = warp_sum(ss);
-      const float inv = 1.0f / sqrtf(ss / (float)HD + fq.eps);
-#pragma unroll
-      for (int c = 0; c < CPL; ++c) kx[c] *= inv * fq.k_w[col0 + c];
-    }
-    const bool first_half = lane < 16;
-    __nv_bfloat16 kb[CPL];
-#pragma unroll
-    for (int c = 0; c < CPL; ++c) {
-      const float other = __shfl_xor_sync(0xffffffffu, kx[c], 16);
-      const int i = (col0 + c) & (HD / 2 - 1);
-      const float2 cs = cs_sm[i];
-      const float a = first_half ? kx[c] : other, bb = first_half ? other : kx[c];
-      kb[c] = __float2bfloat16_rn(first_half ? a * cs.x - bb * cs.y : bb * cs.x + a * cs.y);
-    }
-    const int* bt = block_table + (size_t)b * bt_stride;
-    const int lp = p >> page_shift;
-    const int page = lp < bt_stride ? bt[lp] : -1;
-    if (page < 0 || page >= num_pages) {
-      if (lane == 0) set_status(status, CCB_ST_BAD_PAGE);
-    } else if (gc == 0) {   // one block per kv head writes
-      const size_t dst = (((size_t)page * nkv + kvh) * page_size + (p & (page_size - 1))) * HD + col0;
-#pragma unroll
-      for (int c = 0; c < CPL; ++c) {
-        fq.k_cache[dst + c] = kb[c];
-        fq.v_cache[dst + c] = vb[c];
-      }
-    }
     for (int hh = 0; hh < n_heads; ++hh) {
       float dot = 0.f;
 #pragma unroll
@@ -485,15 +489,47 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
   __shared__ int last_flag;
   __syncthreads();
   if (tid == 0) {
-    __threadfence();  // cumulative: the whole block's partial results are visible before its count is
+    // cumulative: the whole block's partial results are visible before its count is, and all counted blocks' after it
     int* c = counters + (size_t)r * gridDim.y + blockIdx.y;
-    const int old = atomicAdd(c, 1);
+    int old;
+    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(old) : "l"(c) : "memory");
     last_flag = old == eff_splits - 1;
     if (last_flag) *c = 0;  // ready for the next launch
-    __threadfence();
   }
   __syncthreads();
   if (!last_flag) return;
+  if (eff_splits <= kMergeAtOnce) {
+    // few splits: every thread asks for their maxima, sums and its columns at once, and makes the weights by itself (weights
+    // first, through shared memory as below, is one more trip to L2: 8 rows of 2,048 keys 18.3 us, so 16.2, with a kernel
+    // of its own for the merge 16.9; 32 rows of 8,000 181 / 177)
+    for (int idx = tid; idx < n_heads * (HD / 4); idx += kThreads) {
+      const int h = h0 + idx / (HD / 4), d = 4 * (idx % (HD / 4));
+      const size_t base = ((size_t)r * nq + h) * num_splits;
+      float2 ml[kMergeAtOnce];
+      float4 av[kMergeAtOnce];
+#pragma unroll
+      for (int s = 0; s < kMergeAtOnce; ++s) {
+        ml[s] = s < eff_splits ? __ldcg(reinterpret_cast<const float2*>(part_ml) + base + s) : make_float2(-CUDART_INF_F, 0.f);
+        av[s] = s < eff_splits ? __ldcg(reinterpret_cast<const float4*>(&part_acc[(base + s) * HD + d])) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      const float gt = attn_gate<__nv_bfloat16>(ex, t, h);
+      float mm = ml[0].x, ll = 0.f;
+#pragma unroll
+      for (int s = 1; s < kMergeAtOnce; ++s) mm = fmaxf(mm, ml[s].x);
+      float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int s = 0; s < kMergeAtOnce; ++s) {
+        const float f = mm == -CUDART_INF_F ? 0.f : __expf(ml[s].x - mm);   // 0 for splits that do not exist
+        ll += ml[s].y * f;
+        a.x += av[s].x * f; a.y += av[s].y * f; a.z += av[s].z * f; a.w += av[s].w * f;
+      }
+      const float k = attn_sink_fold(ex, h, mm, ll) * gt, inv = ll > 0.f ? k / ll : 0.f;
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(a.x * inv, a.y * inv), hi = __floats2bfloat162_rn(a.z * inv, a.w * inv);
+      *reinterpret_cast<uint2*>(&out[((size_t)t * nq + h) * HD + d]) =
+          make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    }
+    return;
+  }
   float* f_s = reinterpret_cast<float*>(smem);  // [16 heads][splits]: each split's weight, then 1 / sum
   float* inv_s = f_s + 16 * 64;
   // a warp per head, a lane per split (two beyond 32): every load of the head is in flight at once

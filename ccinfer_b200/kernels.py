@@ -1690,15 +1690,16 @@ def attention_decode_plan(n_rows: int, nq: int, nkv: int, hd: int):
     to DECODE_RAGGED_BLOCKS (row, kv head) pairs, contexts are cut into up to four pieces, but only into long ones, so that
     batches of equal contexts gain no merging that they do not need.  Measured on B200, 8 kv heads of 128, one piece / this,
     us: 32 rows, contexts of 500 to 8,000 103 / 75, all 2,048 44 / 44, all 8,000 156 / 172; 48 rows 130 / 110, 78 / 78, 279 /
-    258; 16 rows (two pieces / this) 47 / 39, 28 / 28, 82 / 87.  From 8 splits on the block that finishes last merges them,
-    as it does for the cut rows here (a row of one piece is written at once)."""
+    258; 16 rows (two pieces / this) 47 / 39, 28 / 28, 82 / 87.  The block of a row that finishes last merges its pieces, and a
+    row of one piece is written at once (8 rows, kernel of its own / so: 60 keys 10.6 / 8.5 us, 256 12.4 / 9.8, 2,048 16.9 /
+    16.4, 4,100 29.4 / 28.9)."""
     groups = n_rows * nkv * -(-(nq // nkv) // DECODE_MMA_HEADS_PER_BLOCK)
     splits, _, _ = attention_split_plan(n_rows, nq, nkv, hd, DECODE_MMA_HEADS_PER_BLOCK)
     blocks = max(split_target_blocks(), DECODE_RAGGED_SPLITS * DECODE_RAGGED_BLOCKS)
     floats = blocks * DECODE_MMA_HEADS_PER_BLOCK
     if splits < DECODE_RAGGED_SPLITS - 1 and groups <= DECODE_RAGGED_BLOCKS:
         return DECODE_RAGGED_SPLITS, 16 if splits > 1 else 32, True, floats * hd, floats * 2
-    return splits, DECODE_MIN_TILES, splits >= 8, floats * hd, floats * 2
+    return splits, DECODE_MIN_TILES, splits > 1, floats * hd, floats * 2
 
 
 def attention_split(q, k_cache, v_cache, out, part_acc, part_ml, positions, entry_of_token, block_table,

@@ -358,9 +358,7 @@ class GroupedQueryAttention(Mixer):
             part_ml = rt.scratch.get("attn_part_ml", (n_ml,), torch.float32)
             args = (q, cache.k, cache.v, o, part_acc, part_ml, step.positions, step.entry_of_token, g.block_table,
                     step.n_entries, 0, n_rows, self.window or 0, self.scale, splits)
-            # pages arrive as TMA boxes where they can.  Many splits (few rows, long contexts): the last block of a row
-            # and head group merges them; few splits: a second small kernel does, during which the
-            # output projection already loads its first weights (measured: 2 us a layer either way)
+            # pages arrive as TMA boxes where they can; the last block of a row and head group then merges its splits
             (kernels.attention_decode_tma if tma else kernels.attention_decode_mma if mma else kernels.attention_split)(
                 *args, status=rt.status, **extra, **plan)
         if mma and step.n_entries > step.n_single:

@@ -391,7 +391,7 @@ def test_state_space_gate_and_norm(H, P, parts, few, dtype):
 
 
 # one block a row and group, pieces of at least 4, 16 and 32 tiles of 64 keys: contexts at the pieces' edges beside short ones
-@pytest.mark.parametrize("rows,min_tiles", [(1, None), (8, None), (16, None), (24, None), (48, None), (49, None), (5, 1)])
+@pytest.mark.parametrize("rows,min_tiles", [(1, None), (4, None), (8, None), (12, None), (16, None), (24, None), (48, None), (49, None), (5, 1)])
 def test_decode_of_ragged_contexts(rows, min_tiles):
     """Every row against float64, split as the plan for so many rows says; counters are left zero."""
     k, g = _k(), _gen(rows)
@@ -465,3 +465,62 @@ def test_delta_step_of_many_heads(E, G, H, dk, dv, dtype):
     assert (S[torch.arange(E - 1, -1, -1)].double() - after).abs().max() <= 128 * 2.0 ** -24 * after.abs().max()
     tol = 2.0 ** -8 if dtype == torch.bfloat16 else 0.0
     assert ((y.double() - want).abs() <= tol * want.abs() + 256 * 2.0 ** -24 * want.abs().max()).all()
+
+
+# enough rows that a thread takes four of them: requests of one row (their state moves on) before long ones that end within a
+# run and beside its edges; rows of no request, and a request without a slot
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("taps,H,P,G,N,last", [(4, 4, 64, 1, 64, 0), (3, 8, 16, 2, 4, 1), (2, 2, 128, 2, 128, 2), (1, 4, 64, 1, 64, 3)])
+def test_state_space_rows_in_runs(taps, H, P, G, N, last, dtype):
+    """Against float64: a row's sum of ``taps`` products and its activation, a head's step and decay."""
+    k, g = _k(), _gen(taps + H + N)
+    C = H * P + 2 * G * N
+    lens = [1, 1, 1, 2, 3, 9, 1 << 10, 1000000 // (C // 4 + H) + last]
+    T = sum(lens) + 2   # (two rows that pad the step)
+    first = 5           # rows from the fourth request on go to the chunks
+
+    def rnd(*shape):
+        return torch.randn(shape, generator=g, device="cuda")
+
+    proj, width = rnd(T, C + 8 + -(-H // 8) * 8).to(dtype), C + 8
+    conv_w, conv_b, dt_bias, A_log = 0.5 * rnd(taps, C), rnd(C), rnd(H) - 2, torch.log(1 + rnd(H).abs())
+    conv = rnd(len(lens), max(taps - 1, 1), C).to(dtype)
+    old = conv.double()
+    i32 = dict(dtype=torch.int32, device="cuda")
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), **i32)
+    entry = torch.tensor([e for e, n in enumerate(lens) for _ in range(n)] + [-1, -1], **i32)
+    slots = torch.arange(len(lens) - 1, -1, -1, **i32)
+    slots[4] = -1
+    nan = float("nan")
+    xs, bs, cs = (torch.full(s, nan, device="cuda") for s in ((T, H, P), (T, G, N), (T, G, N)))
+    dts, decay, log_a, log_dt = (torch.full((T, H), nan, device="cuda") for _ in range(4))
+    halves = [torch.full((T, G, N), nan, dtype=torch.bfloat16, device="cuda") for _ in range(4)]
+    chunk = (first, *halves, log_a, log_dt) if dtype == torch.bfloat16 else None
+    k.ssm_prepare(proj, 8, width, conv_w, conv_b, taps, conv if taps > 1 else None, A_log, dt_bias, entry, cu, slots, xs, bs, cs,
+                  dts, decay, H, P, G, N, shift_single=True, chunk=chunk)
+    x, rows, after = proj.double(), [], old.clone()
+    for e, n in enumerate(lens):
+        r0, at = int(cu[e]), len(lens) - 1 - e
+        part = x[r0:r0 + n, 8:8 + C]
+        before = old[at, :taps - 1] if e != 4 else torch.zeros_like(old[0, :taps - 1])
+        pad = torch.cat([before, part])
+        rows.append(torch.nn.functional.silu(conv_b.double() + sum(pad[j:j + n] * conv_w[j].double() for j in range(taps))))
+        if n == 1 and taps > 1:
+            after[at, :taps - 1] = pad[1:]
+    want = torch.cat(rows + [torch.zeros_like(x[:2, :C])])
+    tol = 64 * 2.0 ** -24 * float(want.abs().max())
+    b, c = want[:, H * P:H * P + G * N].view(T, G, N), want[:, H * P + G * N:].view(T, G, N)
+    dt = torch.nn.functional.softplus(x[:, width:width + H] + dt_bias.double())
+    n1 = first if chunk is not None else T
+    assert (xs.double() - want[:, :H * P].view(T, H, P)).abs().max() <= tol
+    assert (bs[:n1].double() - b[:n1]).abs().max() <= tol and (cs[:n1].double() - c[:n1]).abs().max() <= tol
+    live = entry[:n1] >= 0
+    assert (dts[:n1][live].double() - dt[:n1][live]).abs().max() <= 64 * 2.0 ** -24 * dt.max()
+    assert (decay[:n1][live].double() - torch.exp(-A_log.double().exp() * dt[:n1][live])).abs().max() <= 64 * 2.0 ** -24 * 8
+    if chunk is not None:
+        for hi, lo, w in ((halves[0], halves[1], b), (halves[2], halves[3], c)):   # (two bfloat16: 2^-17)
+            assert (hi[n1:].double() + lo[n1:].double() - w[n1:]).abs().max() <= 2.0 ** -17 * w.abs().max() + tol
+        s = slice(n1, T - 2)
+        assert (log_a[s].double() + A_log.double().exp() * dt[s]).abs().max() <= 64 * 2.0 ** -24 * 16 * dt.max()
+        assert (log_dt[s].double() - dt[s].log()).abs().max() <= 64 * 2.0 ** -24 * 16
+    assert torch.equal(conv.double(), after)

@@ -850,8 +850,10 @@ def latent_attention_mma_fits(dtype, R: int, r: int) -> bool:
 
 
 # Tokens of a step's longest portion from which the heads' keys and values are made from the cached rows for the step.  Per
-# cached row and head that costs (64 nd + 64 nv) R products once, and saves 2 R + r - 64 (nd + nv + 1) a query; with the
-# rates of the two attention kernels (0.18 against 0.6 PFLOP/s) and of the product some twenty queries pay for a row.
+# cached row and head that costs (64 nd + 64 nv) R products once, and saves 2 R + r - 64 (nd + nv + 1) a query.  A layer of 32
+# heads, in the latent space / over made keys and values, us: 32 tokens after 200 56 / 43, after 1,500 (window 1,024) 131 / 64,
+# after 3,000 307 / 95, 4 portions of about 32 after 200 70 / 56; 128 tokens after 200 83 / 51.  (20 tokens gain as much as
+# 32; fewer were not measured.)
 LATENT_DENSE_MIN_TOKENS = 32
 LATENT_DENSE_ELEMENTS = 96 << 20   # of the made keys and values at most: heads go in groups where all would be more
 LATENT_DENSE_ROWS = 1 << 16        # cached rows at most

@@ -9,10 +9,12 @@
 //   S   = exp(c_64) S0 + sum_s exp(c_64 - c_s + log b_s) k_s v_s^T
 //
 // so a chunk is four small products, and only S is carried from chunk to chunk.  What the model computes in 32 bits
-// stays so to about 2^-17: the logarithms, their sums and the exponentials are float; the memory lives in float
-// registers for the whole portion; and every float that must become an operand (the memory, the weighted scores, the
-// weighted values, queries and keys that were rotated) goes in as TWO bfloat16, its rounding and what the rounding
-// left, each with a product of its own.  Queries, keys and values straight from a projection are bfloat16 already.
+// stays so to about 2^-17: the logarithms and the exponentials are float, sums of logarithms are made in double and kept
+// as two floats each (c_t - c_s of strong decays cancels: with 16 a token a single float left 1e-4 in the weight that a
+// token gives itself, with 80 a token 9e-4); the memory lives in float registers for the whole portion; and every float
+// that must become an operand (the memory, the weighted scores, the weighted values, queries and keys that were
+// rotated) goes in as TWO bfloat16, its rounding and what the rounding left, each with a product of its own.  Queries,
+// keys and values straight from a projection are bfloat16 already.
 //
 // A block: one request, one head, a slice of 8 NB value columns; four warps.  A warp takes 16 query rows of the chunk
 // for the read-out and DK / 4 key channels of S for the update.  With a column of ones after the values (a running sum
@@ -34,6 +36,8 @@ namespace {
 
 constexpr int kChunk = 64;
 constexpr int kThreads = 128;   // of a team
+constexpr int kGates = 5;       // numbers that a token's gates leave for a chunk
+constexpr float kLeastLog = -200.f;   // a token's log decay at least: exp(-200) is zero in a float
 
 struct ChunkArgs {
   const __nv_bfloat16 *q, *q_lo, *k, *k_lo, *v;
@@ -77,8 +81,8 @@ memory_chunks_kernel(const ChunkArgs a) {
   __nv_bfloat16* s_lo = s_hi + DK * VP;
   __nv_bfloat16* w_hi = s_lo + DK * VP;                                // [64][VP]
   __nv_bfloat16* w_lo = w_hi + VT;
-  float* gates = reinterpret_cast<float*>(tiles + 2 * QK * TILE + TEAMS * TEAM);   // [2][4][64]: c_t, exp(c_t), log b - c, weights
-  uint4* p_s = reinterpret_cast<uint4*>(gates + 2 * 4 * kChunk);       // two teams: weighted scores, [10 tiles][2][32]
+  float* gates = reinterpret_cast<float*>(tiles + 2 * QK * TILE + TEAMS * TEAM);   // [2][kGates][64]: see write_gates
+  uint4* p_s = reinterpret_cast<uint4*>(gates + 2 * kGates * kChunk);  // two teams: weighted scores, [10 tiles][2][32]
 
   const int e = a.entry0 + blockIdx.z, h = blockIdx.y, slice = blockIdx.x * TEAMS + team;
   const int slot = a.state_slot[e];
@@ -134,28 +138,33 @@ memory_chunks_kernel(const ChunkArgs a) {
     for (int i = 0; i < 2; ++i) {
       const int t = chunk * kChunk + 2 * lane + i;
       const bool ok = t < n;
-      la[i] = ok ? a.log_a[(size_t)(r0 + t) * a.H + h] : 0.f;
+      const float x = ok ? a.log_a[(size_t)(r0 + t) * a.H + h] : 0.f;
+      la[i] = x < kLeastLog ? kLeastLog : x;
       lb[i] = ok ? (a.log_b ? a.log_b[(size_t)(r0 + t) * a.H + h] : 0.f) : -CUDART_INF_F;
     }
   };
+  // c_t (its float and what that left), exp(c_t), log b_t, exp(c_64 - c_t) b_t
   auto write_gates = [&](int st) {
-    float* g = gates + st * 4 * kChunk;
-    float sum = la[0] + la[1];
+    float* g = gates + st * kGates * kChunk + 2 * lane;
+    double sum = (double)la[0] + (double)la[1];
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const float p = __shfl_up_sync(0xffffffffu, sum, o);
+      const double p = __shfl_up_sync(0xffffffffu, sum, o);
       if (lane >= o) sum += p;
     }
-    const float total = __shfl_sync(0xffffffffu, sum, 31);
-    const float c1 = sum, c0 = sum - la[1];
-    g[2 * lane] = c0;
-    g[2 * lane + 1] = c1;
-    g[kChunk + 2 * lane] = expf(c0);
-    g[kChunk + 2 * lane + 1] = expf(c1);
-    g[2 * kChunk + 2 * lane] = lb[0] - c0;
-    g[2 * kChunk + 2 * lane + 1] = lb[1] - c1;
-    g[3 * kChunk + 2 * lane] = expf(total + (lb[0] - c0));
-    g[3 * kChunk + 2 * lane + 1] = expf(total + (lb[1] - c1));
+    const double total = __shfl_sync(0xffffffffu, sum, 31);
+    double before = __shfl_up_sync(0xffffffffu, sum, 1);
+    if (lane == 0) before = 0.;
+    const double c[2] = {before + (double)la[0], sum};
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float hi = (float)c[i];
+      g[i] = hi;
+      g[kChunk + i] = (float)(c[i] - (double)hi);
+      g[2 * kChunk + i] = expf(hi);
+      g[3 * kChunk + i] = lb[i];
+      g[4 * kChunk + i] = expf((float)(total - c[i]) + lb[i]);
+    }
   };
 
   issue(0, 0);
@@ -227,7 +236,7 @@ memory_chunks_kernel(const ChunkArgs a) {
     }
     const __nv_bfloat16 *qt = tiles + st * QK * TILE, *kt = qt + TILE, *ql = qt + 2 * TILE, *kl = qt + 3 * TILE;
     const __nv_bfloat16* vt = v_s + (V32 ? 0 : st * VT);
-    const float *gc = gates + st * 4 * kChunk, *ga = gc + kChunk, *gb = ga + kChunk, *gw = gb + kChunk;
+    const float *gc = gates + st * kGates * kChunk, *gl = gc + kChunk, *ga = gl + kChunk, *gb = ga + kChunk, *gw = gb + kChunk;
 
     {   // the values times their weights in the chunk's contribution to S
       const int row = tid >> 1, part = (tid & 1) * (BN / 2);
@@ -314,7 +323,7 @@ memory_chunks_kernel(const ChunkArgs a) {
     if (V32 && TEAMS == 1) __syncthreads();   // the values' halves are complete
     const int t_lo = warp * 16 + gid, t_hi = t_lo + 8;
     const float a_lo = ga[t_lo] * a.q_mult, a_hi = ga[t_hi] * a.q_mult;
-    const float c_lo = gc[t_lo], c_hi = gc[t_hi];
+    const float c_lo = gc[t_lo], c_hi = gc[t_hi], cl_lo = gl[t_lo], cl_hi = gl[t_hi];
 #pragma unroll
     for (int nb = 0; nb < NT; ++nb) {
       acc[nb][0] *= a_lo; acc[nb][1] *= a_lo;
@@ -326,11 +335,12 @@ memory_chunks_kernel(const ChunkArgs a) {
       for (int half = 0; half < 2; ++half) {
         float* x = sc[half];
         const int j = np * 16 + half * 8 + 2 * tig;
-        const float b0 = gb[j], b1 = gb[j + 1];
-        x[0] = j <= t_lo ? x[0] * (__expf(c_lo + b0) * a.q_mult) : 0.f;
-        x[1] = j + 1 <= t_lo ? x[1] * (__expf(c_lo + b1) * a.q_mult) : 0.f;
-        x[2] = j <= t_hi ? x[2] * (__expf(c_hi + b0) * a.q_mult) : 0.f;
-        x[3] = j + 1 <= t_hi ? x[3] * (__expf(c_hi + b1) * a.q_mult) : 0.f;
+#pragma unroll
+        for (int y = 0; y < 2; ++y) {
+          const float c = gc[j + y], l = gl[j + y], b = gb[j + y];
+          x[y] = j + y <= t_lo ? x[y] * (expf(((c_lo - c) + (cl_lo - l)) + b) * a.q_mult) : 0.f;
+          x[2 + y] = j + y <= t_hi ? x[2 + y] * (expf(((c_hi - c) + (cl_hi - l)) + b) * a.q_mult) : 0.f;
+        }
         split2(x[0], x[1], ph[2 * half], pl[2 * half]);
         split2(x[2], x[3], ph[2 * half + 1], pl[2 * half + 1]);
       }
@@ -454,7 +464,7 @@ template <int DK, int NB, bool SPLIT, bool ONES, bool V32 = false, int TEAMS = 1
 int launch_chunks(const ChunkArgs& a, int n_entries, cudaStream_t stream) {
   constexpr int VP = 8 * NB + 8;
   constexpr size_t smem = (size_t)(2 * (SPLIT ? 4 : 2) * kChunk * DK + TEAMS * (4 * kChunk * VP + 2 * DK * VP)) * 2 +
-                          2 * 4 * kChunk * sizeof(float) + (TEAMS > 1 ? 10 * 2 * 32 * sizeof(uint4) : 0);
+                          2 * kGates * kChunk * sizeof(float) + (TEAMS > 1 ? 10 * 2 * 32 * sizeof(uint4) : 0);
   static_assert(smem <= 227 * 1024, "shared memory of a block");
   const auto kernel = memory_chunks_kernel<DK, NB, SPLIT, ONES, V32, TEAMS>;
   static bool configured = false;

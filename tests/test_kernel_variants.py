@@ -162,6 +162,44 @@ def test_state_space_recurrence_in_chunks(H, G, N, P):
         assert (state[slot].double() - after).abs().max() <= 2.0 ** -14 * after.abs().max()
 
 
+# steps and rates up to where a token keeps nothing; three such tokens before slow ones; steps of nothing; whole chunks of both
+@pytest.mark.parametrize("decay", ["strong", "then slow", "extreme"])
+@pytest.mark.parametrize("H,G,N,P", [(4, 2, 128, 64), (2, 1, 64, 48), (40, 1, 64, 128)])
+def test_state_space_chunks_under_strong_decays(H, G, N, P, decay):
+    """Every output against float64, within what rounds on its way: queries, keys, weighted scores or memory, and values, each
+    right to 2^-17, and one more 2^-17 for the weights, of the sum of magnitudes."""
+    k, g = _k(), _gen(H + N + len(decay))
+    lens = [1, 64, 65, 150, 200]
+    T = sum(lens)
+
+    def rnd(*shape):
+        return torch.randn(shape, generator=g, device="cuda")
+
+    def dev(x):
+        return torch.tensor(x, dtype=torch.int32, device="cuda")
+
+    b, c, v, state = rnd(T, G, N), rnd(T, G, N), rnd(T, H, P), rnd(len(lens), H, P, N)
+    u = torch.rand((T, H), generator=g, device="cuda")
+    dt = {"strong": 20 * u, "then slow": torch.where(torch.arange(T, device="cuda")[:, None] % 29 < 3, 15 + 5 * u, 1e-3 * u),
+          "extreme": torch.where(u < 0.1, 0 * u, torch.where(u < 0.2, 1e6 * u, u))}[decay]
+    log_a, log_dt = -16 * dt, dt.log()
+    halves = []
+    for x in (b, c):
+        halves += [x.to(torch.bfloat16), (x - x.to(torch.bfloat16).float()).to(torch.bfloat16)]
+    first = state.double()
+    out = torch.full((T, H, P), float("nan"), device="cuda")
+    cu = [0] + torch.tensor(lens).cumsum(0).tolist()
+    k.ssm_chunks((0, *halves, log_a, log_dt), v, state, out, dev(cu), dev(list(range(len(lens)))), 0, len(lens), G, H, N, P)
+    for e, n in enumerate(lens):
+        s, rep = slice(cu[e], cu[e + 1]), H // G
+        args = [c[s].double().repeat_interleave(rep, 1), b[s].double().repeat_interleave(rep, 1),
+                v[s].double() * log_dt[s].double().exp()[..., None], log_a[s].double().exp()[..., None], None, first[e]]
+        want, after = _recurrence64(*args)
+        size, size_after = _recurrence64(*(x if x is None else x.abs() for x in args))
+        assert ((out[s].double() - want).abs() <= 5 * 2.0 ** -17 * size + 1e-35).all()
+        assert ((state[e].double() - after).abs() <= 5 * 2.0 ** -17 * size_after + 1e-35).all()
+
+
 class _Step:
     """The arrays of a step whose requests have (cached, new) tokens each, single tokens first, on shuffled pages."""
 

@@ -25,12 +25,16 @@
 // logarithms, sums, exponentials, the solve and the memory are float, and every operand of a product (rows, scores,
 // memory) goes in as TWO bfloat16, its rounding and what the rounding left, in three products.  A decay below 2^-115
 // counts as that: it keeps nothing that a float can tell from zero.
+// A number that is not finite must not reach the tokens before it, whose share of it is a zero that would still be
+// multiplied by it: among the operands whose sum runs over tokens (the solve's right sides, u) it enters as zero, and what
+// it belongs to, from its token on, is made NaN afterwards.
 //
 // Bound by: the walk by the chain of its products (one block of eight warps an SM, an instruction on 0.31 of the cycles),
 // the preparation by what it issues (0.42).  Measured on B200, 2,048 tokens of one request, 32 heads of 128 x 128 with a
 // decay per channel and the delta rule: 189 + 103 us; token by token 959 us.
 #include "common.cuh"
 #include "mma_common.cuh"
+#include <math_constants.h>
 #include <type_traits>
 
 using namespace ccb;
@@ -59,6 +63,9 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+
+// Finite, also as two bfloat16 (the largest floats round to infinity).
+__device__ __forceinline__ bool is_finite(float x) { return fabsf(x) < 3.38e38f; }
 
 // bfloat16 pair of (x, y) and of what their rounding left
 __device__ __forceinline__ void split2(float x, float y, uint32_t& hi, uint32_t& lo) {
@@ -418,6 +425,24 @@ chunk_prepare_kernel(const ChunkRows a) {
             mma3(x[nb], xh[j], xl[j], bh[0], bh[1], bl[0], bl[1]);
           }
         }
+        int bad[2] = {kRun, kRun};   // by column: the first token of the run with no finite right side
+        const bool finite = is_finite(x[0][0]) && is_finite(x[0][1]) && is_finite(x[0][2]) && is_finite(x[0][3]) &&
+                            is_finite(x[1][0]) && is_finite(x[1][1]) && is_finite(x[1][2]) && is_finite(x[1][3]);
+        if (__any_sync(0xffffffffu, !finite)) {
+#pragma unroll
+          for (int nb = 0; nb < 2; ++nb)
+#pragma unroll
+            for (int y = 0; y < 4; ++y)
+              if (!is_finite(x[nb][y])) {
+                bad[y >> 1] = min(bad[y >> 1], nb * 8 + 2 * tig + (y & 1));
+                x[nb][y] = 0.f;
+              }
+#pragma unroll
+          for (int up = 0; up < 2; ++up) {   // (the four lanes of a column)
+            bad[up] = min(bad[up], __shfl_xor_sync(0xffffffffu, bad[up], 1));
+            bad[up] = min(bad[up], __shfl_xor_sync(0xffffffffu, bad[up], 2));
+          }
+        }
         uint32_t ah[4], al[4];
 #pragma unroll
           for (int nb = 0; nb < 2; ++nb)
@@ -436,6 +461,11 @@ chunk_prepare_kernel(const ChunkRows a) {
           }
           mma3(x[nb], ah, al, bh[0], bh[1], bl[0], bl[1]);
         }
+#pragma unroll
+        for (int nb = 0; nb < 2; ++nb)
+#pragma unroll
+          for (int y = 0; y < 4; ++y)
+            if (nb * 8 + 2 * tig + (y & 1) >= bad[y >> 1]) x[nb][y] = CUDART_NAN_F;
 #pragma unroll
           for (int nb = 0; nb < 2; ++nb)
 #pragma unroll
@@ -490,6 +520,8 @@ chunk_walk_kernel(const ChunkRows a) {
   __nv_bfloat16* u_hi = s_lo + DK * kPitch;                          // [64][kPitch]
   __nv_bfloat16* u_lo = u_hi + kChunk * kPitch;
 
+  // by column of the slice: the first token of a chunk whose u is not finite (64: none); and whether there is one
+  __shared__ int bad_col[kCols], bad_any;
   const int e = a.entry0 + blockIdx.z, h = blockIdx.y, col0 = blockIdx.x * kCols;
   const int slot = a.state_slot[e];
   const int r0 = a.cu_q[e], n = a.cu_q[e + 1] - r0;
@@ -524,6 +556,8 @@ chunk_walk_kernel(const ChunkRows a) {
     cp_async_commit();
   };
   issue_read(0);
+  if (tid < kCols) bad_col[tid] = kChunk;   // (read and written behind the barriers of a chunk)
+  if (tid == 0) bad_any = 0;
 
   // S: key channels 16 warp .. + 15 (with 64 channels only the first four warps have some), all columns of the slice
   constexpr int SW = DK / 16;   // warps with channels
@@ -605,13 +639,21 @@ chunk_walk_kernel(const ChunkRows a) {
 #pragma unroll
       for (int up = 0; up < 2; ++up) {
         uint32_t hi, lo;
-        split2(u[nb][2 * up] - d[nb][2 * up], u[nb][2 * up + 1] - d[nb][2 * up + 1], hi, lo);
+        float x0 = u[nb][2 * up] - d[nb][2 * up], x1 = u[nb][2 * up + 1] - d[nb][2 * up + 1];
+        if (!(is_finite(x0) && is_finite(x1))) {
+          const int t = wr * 16 + gid + 8 * up, c = wc * 16 + nb * 8 + 2 * tig;
+          bad_any = 1;
+          if (!is_finite(x0)) atomicMin(&bad_col[c], t), x0 = 0.f;
+          if (!is_finite(x1)) atomicMin(&bad_col[c + 1], t), x1 = 0.f;
+        }
+        split2(x0, x1, hi, lo);
         const int pos = (wr * 16 + gid + 8 * up) * kPitch + wc * 16 + nb * 8 + 2 * tig;
         *reinterpret_cast<uint32_t*>(u_hi + pos) = hi;
         *reinterpret_cast<uint32_t*>(u_lo + pos) = lo;
       }
     cp_async_wait<0>();
     __syncthreads();   // u, p and k are there; q, w and the memory's halves have been read
+    const bool bad = bad_any != 0;
     if (ch + 1 < chunks) issue_read(ch + 1);
 
 #pragma unroll
@@ -646,7 +688,21 @@ chunk_walk_kernel(const ChunkRows a) {
           mma3(S[2 * np + 1], xh, xl, bh[2], bh[3], bl[2], bl[3]);
         }
       }
+      if (bad) {   // (for good: what the column's memory is multiplied by later stays NaN)
+#pragma unroll
+        for (int nb = 0; nb < 4; ++nb)
+#pragma unroll
+          for (int x = 0; x < 4; ++x)
+            if (bad_col[nb * 8 + 2 * tig + (x & 1)] < kChunk) S[nb][x] = CUDART_NAN_F;
+      }
       if (ch + 1 < chunks) store_s();
+    }
+    if (bad) {
+#pragma unroll
+      for (int nb = 0; nb < 2; ++nb)
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+          if (bad_col[wc * 16 + nb * 8 + 2 * tig + (x & 1)] <= wr * 16 + gid + 8 * (x >> 1)) o[nb][x] = CUDART_NAN_F;
     }
 #pragma unroll
     for (int up = 0; up < 2; ++up) {

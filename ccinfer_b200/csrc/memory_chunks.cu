@@ -26,6 +26,9 @@
 // runs on it: of two teams of four warps, a slice of value columns each, that share the tiles of queries and keys and the
 // weighted scores (a team makes those of every second block of 16 keys and leaves them for the other).  2,048 tokens of two
 // requests, 128 heads of 64 x 128: 1,034 us token by token, 459 us in chunks by one team a block, 225 us by two.
+// A value that is no finite number must not reach the tokens before it, whose weight of it is a zero that would still
+// be multiplied by it: such a value enters the products as zero, and its column, from its token on, is made NaN
+// afterwards.  (Values of 16 bits are multiplied where they lie: there it reaches up to 15 tokens before it.)
 #include "common.cuh"
 #include "mma_common.cuh"
 #include <math_constants.h>
@@ -61,6 +64,9 @@ __device__ __forceinline__ void split2(float x, float y, uint32_t& hi, uint32_t&
   lo = pack_bf16(x - f.x, y - f.y);
 }
 
+// Finite, also as two bfloat16 (the largest floats round to infinity).
+__device__ __forceinline__ bool is_finite(float x) { return fabsf(x) < 3.38e38f; }
+
 template <int DK, int NB, bool SPLIT, bool ONES, bool V32, int TEAMS>
 __global__ void __launch_bounds__(kThreads * TEAMS)
 memory_chunks_kernel(const ChunkArgs a) {
@@ -83,6 +89,8 @@ memory_chunks_kernel(const ChunkArgs a) {
   __nv_bfloat16* w_lo = w_hi + VT;
   float* gates = reinterpret_cast<float*>(tiles + 2 * QK * TILE + TEAMS * TEAM);   // [2][kGates][64]: see write_gates
   uint4* p_s = reinterpret_cast<uint4*>(gates + 2 * kGates * kChunk);  // two teams: weighted scores, [10 tiles][2][32]
+  // V32: by column of the slice, the first token of a chunk whose value is not finite (64: none); and whether there is one
+  __shared__ int bad_col[V32 ? TEAMS * BN : 1], bad_any[TEAMS];
 
   const int e = a.entry0 + blockIdx.z, h = blockIdx.y, slice = blockIdx.x * TEAMS + team;
   const int slot = a.state_slot[e];
@@ -168,7 +176,11 @@ memory_chunks_kernel(const ChunkArgs a) {
   };
 
   issue(0, 0);
-  if constexpr (V32) load_values(0);
+  if constexpr (V32) {
+    load_values(0);
+    if (tid < BN) bad_col[team * BN + tid] = kChunk;
+    if (tid == 0) bad_any[team] = 0;
+  }
   const bool gating = warp == 0 && team == 0;
   if (gating) {
     load_gates(0);
@@ -242,6 +254,21 @@ memory_chunks_kernel(const ChunkArgs a) {
       const int row = tid >> 1, part = (tid & 1) * (BN / 2);
       const float w = gw[row];
       if constexpr (V32) {
+        bool finite = true;
+#pragma unroll
+        for (int c = 0; c < NB; ++c)
+          finite = finite && is_finite(vv[c].x) && is_finite(vv[c].y) && is_finite(vv[c].z) && is_finite(vv[c].w);
+        if (!finite) {
+          bad_any[team] = 1;
+#pragma unroll
+          for (int c = 0; c < BN / 2; ++c) {
+            float& x = c % 4 == 0 ? vv[c / 4].x : c % 4 == 1 ? vv[c / 4].y : c % 4 == 2 ? vv[c / 4].z : vv[c / 4].w;
+            if (!is_finite(x)) {
+              atomicMin(&bad_col[team * BN + part + c], row);
+              x = 0.f;
+            }
+          }
+        }
 #pragma unroll
         for (int c = 0; c < BN / 2; c += 2) {
           const float2 f = c & 2 ? make_float2(vv[c / 4].z, vv[c / 4].w) : make_float2(vv[c / 4].x, vv[c / 4].y);
@@ -392,6 +419,15 @@ memory_chunks_kernel(const ChunkArgs a) {
         weighted_values(np, ph, pl);
       }
     }
+    // (the barrier before the weighted values has passed)
+    const bool bad = V32 && bad_any[team] != 0;
+    if (V32 && bad) {
+#pragma unroll
+      for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+          if (bad_col[team * BN + nb * 8 + 2 * tig + (x & 1)] <= (x < 2 ? t_lo : t_hi)) acc[nb][x] = CUDART_NAN_F;
+    }
     const int left = n - ch * kChunk;
 #pragma unroll
     for (int x = 0; x < 2; ++x) {
@@ -445,6 +481,15 @@ memory_chunks_kernel(const ChunkArgs a) {
           }
         }
       }
+    }
+    if (V32 && bad) {   // (for good: what the column's memory is multiplied by later stays NaN)
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+          for (int x = 0; x < 4; ++x)
+            if (bad_col[team * BN + nb * 8 + 2 * tig + (x & 1)] < kChunk) S[mt][nb][x] = CUDART_NAN_F;
     }
     if (ch + 1 < chunks) store_s();
   }

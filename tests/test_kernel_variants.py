@@ -200,6 +200,88 @@ def test_state_space_chunks_under_strong_decays(H, G, N, P, decay):
         assert ((state[e].double() - after).abs() <= 5 * 2.0 ** -17 * size_after + 1e-35).all()
 
 
+def _same_where_finite(got, want, bound):
+    """Numbers where the reference has numbers, within ``bound`` of the largest; none where it has none."""
+    ok = torch.isfinite(want)
+    assert not torch.isfinite(got[~ok]).any()
+    assert torch.isfinite(got[ok]).all()
+    assert (got.double() - want)[ok].abs().max() <= bound * want[ok].abs().max()
+
+
+# one number that is none, within a run, at its first and at its last token, in the first and in a later chunk
+@pytest.mark.parametrize("at", [0, 37, 47, 64, 90])
+@pytest.mark.parametrize("what", ["q", "k", "v", "decay", "beta"])
+@pytest.mark.parametrize("rule", ["delta", "head delta", "linear", "head linear"])
+def test_recurrence_in_chunks_keeps_what_is_no_number_to_later_tokens(rule, what, at):
+    """Tokens before it, requests, heads and value columns beside it stay what they are, as token by token in float64."""
+    delta, head = "delta" in rule, "head" in rule
+    if what == "beta" and not delta:
+        pytest.skip("no such factor")
+    H, dk, dv, lens, g = 2, 64, 64, [70, 130], _gen(at + len(what))
+    T, row = sum(lens), 70 + at
+
+    def rnd(*shape):
+        return torch.randn(shape, generator=g, device="cuda")
+
+    def dev(x):
+        return torch.tensor(x, dtype=torch.int32, device="cuda")
+
+    q, k = (torch.nn.functional.normalize(rnd(T, H, dk), dim=-1) for _ in range(2))
+    v, state, beta = rnd(T, H, dv), rnd(2, H, dv, dk), torch.rand((T, H), generator=g, device="cuda") if delta else None
+    a = 1 - 0.1 * torch.rand((T, H) if head else (T, H, dk), generator=g, device="cuda")
+    if what == "beta":
+        beta[row, 1] = float("nan")
+    elif what == "decay" and head:
+        a[row, 1] = float("nan")
+    else:
+        {"q": q, "k": k, "v": v, "decay": a}[what][row, 1, 21] = float("nan") if what == "decay" or at % 2 else float("inf")
+    want, after, cu = torch.empty(T, H, dv, dtype=torch.float64, device="cuda"), state.double(), [0, 70, 200]
+    for e in range(2):
+        s = slice(cu[e], cu[e + 1])
+        want[s], after[e] = _recurrence64(q[s].double(), k[s].double(), v[s].double(), (a[s, :, None] if head else a[s]).double(),
+                                          beta[s].double() if delta else None, after[e])
+    assert torch.isfinite(want[:row]).all() and torch.isfinite(want[:, 0]).all() and not torch.isfinite(want[row, 1]).all()
+
+    def scratch(key, per, shape, dtype):
+        return torch.full((T,) + tuple(shape), float("nan"), dtype=dtype, device="cuda")
+
+    out = torch.zeros(T, H, dv, device="cuda")
+    _k().chunk_recurrence(scratch, q, k, v, a, beta, state, out, dev(cu), dev([0, 1]), 0, 2, 130, H, H, dk, dv)
+    _same_where_finite(out, want, 2.0 ** -14)
+    _same_where_finite(state, after, 2.0 ** -14)
+
+
+@pytest.mark.parametrize("at", [0, 37, 47, 64, 90])
+@pytest.mark.parametrize("what", ["b", "c", "x", "log_a", "log_dt"])
+@pytest.mark.parametrize("P", [16, 32, 64])
+def test_state_space_chunks_keep_what_is_no_number_to_later_tokens(P, what, at):
+    """As above; one team, two teams of 16 and (with enough heads) of 32 columns."""
+    H, N, lens, g = 40, 64, [70, 130], _gen(at + P + len(what))
+    T, row = sum(lens), 70 + at
+
+    def rnd(*shape):
+        return torch.randn(shape, generator=g, device="cuda")
+
+    def dev(x):
+        return torch.tensor(x, dtype=torch.int32, device="cuda")
+
+    b, c, x, state = rnd(T, 2, N).to(torch.bfloat16), rnd(T, 2, N).to(torch.bfloat16), rnd(T, H, P), rnd(2, H, P, N)
+    log_dt = torch.log(0.1 + torch.rand((T, H), generator=g, device="cuda"))
+    log_a = -0.1 * log_dt.exp()
+    {"b": b, "c": c, "x": x, "log_a": log_a, "log_dt": log_dt}[what].view(T, -1)[row, 11] = float("nan") if what[0] == "l" or at % 2 else float("inf")
+    want, after, cu = torch.empty(T, H, P, dtype=torch.float64, device="cuda"), state.double(), [0, 70, 200]
+    for e in range(2):
+        s = slice(cu[e], cu[e + 1])
+        want[s], after[e] = _recurrence64(c[s].double().repeat_interleave(H // 2, 1), b[s].double().repeat_interleave(H // 2, 1),
+                                          x[s].double() * log_dt[s].double().exp()[..., None], log_a[s].double().exp()[..., None],
+                                          None, after[e])
+    assert torch.isfinite(want[:row]).all() and not torch.isfinite(want[row]).all() and torch.isfinite(want[row]).any()
+    out, zero = torch.full((T, H, P), 7.0, device="cuda"), torch.zeros_like(b)
+    _k().ssm_chunks((0, b, zero, c, zero, log_a, log_dt), x, state, out, dev(cu), dev([0, 1]), 0, 2, 2, H, N, P)
+    _same_where_finite(out, want, 2.0 ** -14)
+    _same_where_finite(state, after, 2.0 ** -14)
+
+
 class _Step:
     """The arrays of a step whose requests have (cached, new) tokens each, single tokens first, on shuffled pages."""
 

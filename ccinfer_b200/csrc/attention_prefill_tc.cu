@@ -789,8 +789,9 @@ int launch_dense(const CUtensorMap& tmQ, const CUtensorMap& tmKV, const CUtensor
   constexpr size_t smem = (size_t)((1 + kKvStages) * NK + kKvStages * NV) * 128 * 128 + 20 * 8 + 1024;
   static_assert(smem <= 227 * 1024, "shared memory of a block");
   auto kernel = attention_prefill_tc_kernel<NK, NV, true>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return (int)e;
+  static std::atomic<unsigned long long> done{0};
+  const int rc = ccb_allow_smem(kernel, (int)smem, done);
+  if (rc != 0) return rc;
   ccb_launch(kernel, dim3(heads, (max_new + kTQ - 1) / kTQ, n_entries), kTcThreads, smem, stream, tmQ, tmKV, tmKV, tmShared,
              dense, (__nv_bfloat16*)out, cu_q, pos0, (const int*)nullptr, 0, entry0, nq, 1, 1, 0, 1, window,
              scale * 1.4426950408889634f, ex, status);

@@ -728,12 +728,13 @@ int launch_chunked(const ChunkRows& a, int n_entries, int max_tokens, cudaStream
   auto walk = chunk_walk_kernel<DK, DELTA>;
   constexpr int prep_bytes = PrepShape<DK, DELTA, HEAD>::kBytes, walk_bytes = WalkShape<DK, DELTA>::kBytes;
   static_assert(walk_bytes <= 227 * 1024 && prep_bytes <= 227 * 1024, "shared memory of a block");
-  cudaError_t err = cudaFuncSetAttribute(prepare, cudaFuncAttributeMaxDynamicSharedMemorySize, prep_bytes);
-  if (err == cudaSuccess) err = cudaFuncSetAttribute(walk, cudaFuncAttributeMaxDynamicSharedMemorySize, walk_bytes);
-  if (err != cudaSuccess) return (int)err;
+  static std::atomic<unsigned long long> prep_done{0}, walk_done{0};
+  int rc = ccb_allow_smem(prepare, prep_bytes, prep_done);
+  if (rc == 0) rc = ccb_allow_smem(walk, walk_bytes, walk_done);
+  if (rc != 0) return rc;
   ccb_launch(prepare, dim3((max_tokens + kChunk - 1) / kChunk, a.H, n_entries), kThreads, prep_bytes, stream, a);
-  err = cudaGetLastError();
-  if (err != cudaSuccess) return (int)err;
+  rc = ccb_launch_status();
+  if (rc != 0) return rc;
   ccb_launch(walk, dim3(a.dv / kCols, a.H, n_entries), kThreads, walk_bytes, stream, a);
   return ccb_launch_status();
 }

@@ -8,6 +8,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <atomic>
 #include <utility>
 
 #define CCB_API extern "C" __attribute__((visibility("default")))
@@ -205,6 +206,21 @@ __device__ __forceinline__ void set_status(int* status, int bit) {
 #define CCB_REFUSE_ARG (-4)
 
 static inline int ccb_launch_status() { return (int)cudaGetLastError(); }
+
+// More dynamic shared memory than a block gets unasked: allowed once per kernel and device (`done`: a bit per device, one
+// word per kernel), not before each of its launches.
+template <typename... KArgs>
+static inline int ccb_allow_smem(void (*kernel)(KArgs...), int bytes, std::atomic<unsigned long long>& done) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return (int)e;
+  const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+  if (done.load(std::memory_order_relaxed) & bit) return 0;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e != cudaSuccess) return (int)cudaGetLastError();   // (and cleared)
+  done.fetch_or(bit, std::memory_order_relaxed);
+  return 0;
+}
 
 // One switch per kernel family (ccb_set_pdl of its shared object; kernels.set_pdl tells every loaded family and every
 // family loaded later): launch kernels with programmatic stream serialization.

@@ -359,8 +359,9 @@ struct F32Product {
 
 template <int MR> int rows_go(const F32Product& p, int vec, cudaStream_t stream) {
   auto kernel = gemm_f32_rows_kernel<MR>;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RowsStage<MR>::kBytes) != cudaSuccess)
-    return (int)cudaGetLastError();
+  static std::atomic<unsigned long long> done{0};
+  const int rc = ccb_allow_smem(kernel, RowsStage<MR>::kBytes, done);
+  if (rc != 0) return rc;
   ccb_launch(kernel, dim3((p.N + kRowW - 1) / kRowW, 1, p.batch), kRowWarps * 32, RowsStage<MR>::kBytes, stream, p.C, p.A, p.W,
              p.M, p.N, p.K, p.lda, p.ldw, p.ldc, p.sa, p.sw, p.sc, vec);
   return ccb_launch_status();
@@ -375,8 +376,9 @@ template <int BM> int tiles_go(const F32Product& p, int vec_a, int vec_w, cudaSt
   const bool cluster = tiles < 2 * 148 && p.K >= 512;
   constexpr int bytes = TileShape<BM>::kBytes;
   auto kernel = cluster ? gemm_f32_tiles_kernel<BM, true> : gemm_f32_tiles_kernel<BM, false>;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
-    return (int)cudaGetLastError();
+  static std::atomic<unsigned long long> done[2];
+  const int rc = ccb_allow_smem(kernel, bytes, done[cluster]);
+  if (rc != 0) return rc;
   if (cluster)
     ccb_launch_cluster(false, kSegments, kernel, dim3(gx * kSegments, gy, p.batch), TileShape<BM>::kThreads, bytes, stream, p.C, p.A, p.W,
                        p.M, p.N, p.K, p.lda, p.ldw, p.ldc, p.sa, p.sw, p.sc, vec_a, vec_w);

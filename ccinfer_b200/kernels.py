@@ -644,22 +644,32 @@ def delta_recurrence(qn, kn, vv, gg, bb, state, out, cu_q, state_slot, n_entries
                                       _p(state_slot), n_entries, G, H, dk, dv, _stream()), "delta_recurrence")
 
 
-# Tokens of a step's longest portion from which the recurrences run in chunks.  The token-by-token kernel costs half a
-# microsecond a token whatever runs beside it, a chunk of 64 tokens (however few of them are there) 4 us of its walk
-# after some 10 us of preparation.  32 heads of 128, token by token / in chunks, us: linear attention, 1 request of 32
-# tokens 19 / 20, of 48 27 / 20, 4 of 32 47 / 21; delta rule 1 of 32 21 / 25, of 48 27 / 33, of 64 35 / 35, of 128 64 / 42,
-# 4 of 16 27 / 31, of 32 48 / 42, 16 of 32 168 / 132: its chunks need 64 tokens, or 128 heads of portions beside one another.
-CHUNK_RECURRENCE_MIN_TOKENS = 32
-CHUNK_DELTA_FEW_HEADS, CHUNK_DELTA_FEW_MIN_TOKENS = 128, 64
+# When the recurrences of a step's portions run in chunks: from so many (token, head) pairs of portions on with the longest
+# portion at least so long, or from a longest portion of CHUNK_LONG on.  What decides is the LAYER as a portion's step
+# launches it, kernel by kernel: its chunks take the host 9 us more (of some 110 to 170), which the device has to make up.
+# Token by token is a chain of half a microsecond a token; a chunk of 64 (however few of them are there) is 10 us of
+# preparation and 4 of its walk.  Time of the layer token by token / in chunks, alone and among others:
+#   linear attention, 16 heads of 128: 2 portions of 96 tokens 1.08, 0.94, of 200 1.47, 1.18; 8 of 32 1.10, 0.94, of 64
+#     1.40, 1.13; 1 of 128 1.07, 0.93, of 200 1.26, 0.96.  32 heads: 2 of 64 1.10, 0.95; 8 of 16 1.04, 0.94, of 24 1.17,
+#     1.16; 16 of 8 0.92, 0.93, of 12 1.02, 1.05
+#   delta rule, decay a channel, 16 heads: 2 of 200 1.17, 0.97; 8 of 64 1.06, 0.96, of 96 1.14, 1.16; 1 of 128 0.98, 0.95, of
+#     200 1.06, 0.97.  32 heads: 4 of 48 1.00, 0.96, of 64 1.04, 1.00; 16 of 16 0.89, 0.89, of 24 0.99, 1.00, of 32 1.10, 1.12
+#   decay a head, 32 heads: 2 of 96 1.04, 1.07; 8 of 24 0.95, 0.96, of 32 1.02, 1.05; 1 of 128 1.05, 0.98, of 200 1.19, 1.26
+CHUNK_LINEAR_MIN = (4096, 12)
+CHUNK_DELTA_MIN = (8192, 32)
+CHUNK_LONG = 160
 
 
-def chunk_recurrence_fits(dtype, dk: int, dv: int, max_tokens: int, delta_heads: int | None = None) -> bool:
-    """Whether portions of prompts, the longest of max_tokens tokens, run as chunks on tensor cores: the 16-bit path (in
-    the 32-bit path every operand stays a float) with the sizes the kernel takes.  ``delta_heads``: the heads of all
-    portions where the delta rule is to run."""
-    few = delta_heads is not None and delta_heads < CHUNK_DELTA_FEW_HEADS
-    least = CHUNK_DELTA_FEW_MIN_TOKENS if few else CHUNK_RECURRENCE_MIN_TOKENS
-    return dtype == torch.bfloat16 and dk in (64, 128) and dv % 32 == 0 and max_tokens >= least
+def _chunks_pay(least, units: int, longest: int) -> bool:
+    return longest >= CHUNK_LONG or (units >= least[0] and longest >= least[1])
+
+
+def chunk_recurrence_fits(dtype, dk: int, dv: int, longest: int, units: int, delta: bool) -> bool:
+    """Whether portions of prompts, the longest of ``longest`` tokens and ``units`` (token, head) pairs in all, run as chunks
+    on tensor cores: the 16-bit path (in the 32-bit path every operand stays a float) with the sizes the kernel takes.
+    ``delta``: with the delta rule's correction."""
+    return (dtype == torch.bfloat16 and dk in (64, 128) and dv % 32 == 0
+            and _chunks_pay(CHUNK_DELTA_MIN if delta else CHUNK_LINEAR_MIN, units, longest))
 
 
 def chunk_recurrence(scratch, qn, kn, vv, gg, bb, state, out, cu_q, state_slot, entry0: int, n_entries: int,
@@ -669,21 +679,23 @@ def chunk_recurrence(scratch, qn, kn, vv, gg, bb, state, out, cu_q, state_slot, 
     between the two kernels goes into the memory of qn, kn, vv and gg where sizes allow.  ``scratch(key, tokens_or_chunks,
     shape, dtype)``: a workspace of shape [tokens or chunks, *shape]."""
     _cuda(qn, kn, vv, gg, bb, state, out, cu_q, state_slot)
-    assert all(t.dtype == torch.float32 for t in (qn, kn, vv, gg, state, out)) and state.shape[1:] == (H, dv, dk)
+    f32, bf = torch.float32, torch.bfloat16
+    assert qn.dtype == kn.dtype == vv.dtype == gg.dtype == state.dtype == out.dtype == f32
     T, head = vv.shape[0], gg.dim() == 2
-    assert qn.shape == kn.shape == (T, G, dk) and vv.shape == out.shape == (T, H, dv)
-    assert tuple(gg.shape) == ((T, H) if head else (T, H, dk)) and (bb is None or bb.shape == (T, H))
-    bf = torch.bfloat16
+    assert qn.shape == kn.shape == (T, G, dk) and vv.shape == out.shape == (T, H, dv) and state.shape[1:] == (H, dv, dk)
+    assert gg.shape == ((T, H) if head else (T, H, dk)) and (bb is None or bb.shape == (T, H))
     qs = qn if G == H else scratch("chunk_q", "tokens", (H, 2, dk), bf)
     ks = kn if G == H else scratch("chunk_k", "tokens", (H, 2, dk), bf)
     w = None if bb is None else (scratch("chunk_w", "tokens", (H, 2, dk), bf) if head else gg)
     p = scratch("chunk_p", "tokens", (H, 2, 64), bf)
-    keep = scratch("chunk_keep", "chunks", (H, dk), torch.float32)
-    assert all(t is None or t.shape[0] >= T for t in (qs, ks, w, p)) and keep.shape[0] >= T // 64 + entry0 + n_entries
-    _check(lib().ccb_chunk_recurrence(_p(qn), _p(kn), _p(vv), _p(gg), _p(bb), _p(qs), _p(ks), _p(w),
-                                      _p(vv if bb is not None else None), _p(p), _p(keep), _p(state), _p(out), _p(cu_q),
-                                      _p(state_slot), int(entry0), int(n_entries), int(max_tokens), G, H, dk, dv,
-                                      state.shape[0], 1 if head else 0, _stream()), "chunk_recurrence")
+    keep = scratch("chunk_keep", "chunks", (H, dk), f32)
+    assert qs.shape[0] >= T and ks.shape[0] >= T and (w is None or w.shape[0] >= T) and p.shape[0] >= T
+    assert keep.shape[0] >= T // 64 + entry0 + n_entries
+    pv = vv.data_ptr()
+    _check(lib().ccb_chunk_recurrence(qn.data_ptr(), kn.data_ptr(), pv, gg.data_ptr(), _p(bb), qs.data_ptr(), ks.data_ptr(),
+                                      _p(w), pv if bb is not None else 0, p.data_ptr(), keep.data_ptr(), state.data_ptr(),
+                                      out.data_ptr(), cu_q.data_ptr(), state_slot.data_ptr(), entry0, n_entries, max_tokens,
+                                      G, H, dk, dv, state.shape[0], 1 if head else 0, _stream()), "chunk_recurrence")
     counters.own += 1   # two kernels
 
 
@@ -1447,7 +1459,7 @@ def ssm_prepare(proj, ox: int, odt: int, conv_w, conv_b, taps: int, conv_state, 
     and decay [T, H].  ``shift_single``: a request that brings one token has its convolution state moved on here
     (then ``conv_state_shift`` is for the others only).  ``chunk`` = (first row, b_hi, b_lo, c_hi, c_lo, log_a, log_dt):
     from that row on B and C go to bfloat16 [T, G, N], their values and what the rounding left, and dt and decay as
-    their logarithms, float [T, H] (``ssm_chunks`` takes them)."""
+    their logarithms, float [T, H] (``ssm_chunks`` takes them; the six may have more rows than T)."""
     _cuda(conv_w, conv_b, conv_state, A_log, dt_bias, entry_of_token, cu_q, state_slot, xs, bs, cs, dts, decay)
     T = xs.shape[0]
     C = H * P + 2 * G * N
@@ -1461,15 +1473,16 @@ def ssm_prepare(proj, ox: int, odt: int, conv_w, conv_b, taps: int, conv_state, 
                                  _dt(proj), _stream()), "ssm_prepare")
 
 
-# As CHUNK_RECURRENCE_MIN_TOKENS.  128 heads of 64 x 128, token by token / in chunks, us: 1 request of 16 tokens 15 / 19, of 32
-# 23 / 19, of 64 41 / 17, 4 of 16 38 / 35, of 32 68 / 35; 32 heads 1 of 32 15 / 18, of 48 19 / 18, 4 of 32 23 / 15.
-SSM_CHUNKS_MIN_TOKENS = 32
+# As CHUNK_LINEAR_MIN (heads of 64 x 128), the layer token by token / in chunks, alone and among others: 64 heads, 2 portions of
+# 48 tokens 1.00, 0.94, of 128 1.35, 1.07; 8 of 20 1.01, 0.96, of 32 1.15, 1.01; 1 of 128 1.18, 0.97.  128 heads: 1 of 64 1.07,
+# 0.97, of 96 1.20, 1.16; 4 of 16 0.96, 0.99, of 20 1.01, 1.06; 16 of 12 0.91, 0.90, of 16 1.01, 1.00, of 20 1.11, 1.13.
+SSM_CHUNKS_MIN = (8192, 20)
 
 
-def ssm_chunks_fits(dtype, N: int, P: int, max_tokens: int) -> bool:
-    """Whether portions of prompts, the longest of max_tokens tokens, run as chunks on tensor cores: the 16-bit path with
-    the sizes the kernel takes."""
-    return dtype == torch.bfloat16 and N in (64, 128) and P % 16 == 0 and max_tokens >= SSM_CHUNKS_MIN_TOKENS
+def ssm_chunks_fits(dtype, N: int, P: int, longest: int, units: int) -> bool:
+    """Whether portions of prompts, the longest of ``longest`` tokens and ``units`` (token, head) pairs in all, run as chunks
+    on tensor cores: the 16-bit path with the sizes the kernel takes."""
+    return dtype == torch.bfloat16 and N in (64, 128) and P % 16 == 0 and _chunks_pay(SSM_CHUNKS_MIN, units, longest)
 
 
 def ssm_chunks(chunk, xs, state, out, cu_q, state_slot, entry0: int, n_entries: int, G: int, H: int, N: int, P: int) -> None:
@@ -1477,13 +1490,15 @@ def ssm_chunks(chunk, xs, state, out, cu_q, state_slot, entry0: int, n_entries: 
     ``ssm_prepare`` left in ``chunk``."""
     _, b_hi, b_lo, c_hi, c_lo, log_a, log_dt = chunk
     _cuda(b_hi, b_lo, c_hi, c_lo, log_a, log_dt, xs, state, out, cu_q, state_slot)
-    T = xs.shape[0]
-    assert all(t.dtype == torch.bfloat16 and t.shape == (T, G, N) for t in (b_hi, b_lo, c_hi, c_lo))
-    assert log_a.shape == log_dt.shape == (T, H) and state.shape[1:] == (H, P, N) and out.shape == xs.shape == (T, H, P)
-    assert all(t.dtype == torch.float32 for t in (log_a, log_dt, xs, state, out))
-    _check(lib().ccb_ssm_chunks(_p(c_hi), _p(c_lo), _p(b_hi), _p(b_lo), G * N, _p(xs), H * P, _p(log_a), _p(log_dt), _p(state),
-                                _p(out), _p(cu_q), _p(state_slot), int(entry0), int(n_entries), G, H, N, P, state.shape[0],
-                                _stream()), "ssm_chunks")
+    T, f32 = xs.shape[0], torch.float32
+    assert b_hi.dtype == b_lo.dtype == c_hi.dtype == c_lo.dtype == torch.bfloat16
+    assert b_hi.shape == b_lo.shape == c_hi.shape == c_lo.shape and b_hi.shape[1:] == (G, N) and b_hi.shape[0] >= T
+    assert log_a.shape == log_dt.shape and log_a.shape[1:] == (H,) and log_a.shape[0] >= T
+    assert state.shape[1:] == (H, P, N) and out.shape == xs.shape == (T, H, P)
+    assert log_a.dtype == log_dt.dtype == xs.dtype == state.dtype == out.dtype == f32
+    _check(lib().ccb_ssm_chunks(c_hi.data_ptr(), c_lo.data_ptr(), b_hi.data_ptr(), b_lo.data_ptr(), G * N, xs.data_ptr(), H * P,
+                                log_a.data_ptr(), log_dt.data_ptr(), state.data_ptr(), out.data_ptr(), cu_q.data_ptr(),
+                                state_slot.data_ptr(), entry0, n_entries, G, H, N, P, state.shape[0], _stream()), "ssm_chunks")
 
 
 def conv_state_shift(rows, taps: int, state, cu_q, state_slot, n_entries: int, entry0: int = 0) -> None:

@@ -141,9 +141,10 @@ class ChannelGatedDelta(Mixer):
                                   G, H, dk, dv)
         o = rt.scratch.get("delta_o", (rt.max_tokens, H, dv), f32)[:T]
         # (a step lists its single tokens first: they, and short portions, go token by token)
-        chunks = kernels.chunk_recurrence_fits(rt.dtype, dk, dv, step.max_q_len, (step.n_entries - step.n_single) * H)
+        chunks = kernels.chunk_recurrence_fits(rt.dtype, dk, dv, step.max_q_len, (T - step.n_single) * H, True)
         n1 = step.n_single if chunks else step.n_entries
-        kernels.delta_recurrence(qn, kn, vv, gg, bb, S, o, step.cu_q, step.state_slot, n1, G, H, dk, dv)
+        if n1:
+            kernels.delta_recurrence(qn, kn, vv, gg, bb, S, o, step.cu_q, step.state_slot, n1, G, H, dk, dv)
         if step.n_entries > n1:
             kernels.chunk_recurrence(rt.chunk_scratch, qn, kn, vv, gg, bb, S, o, step.cu_q, step.state_slot, n1,
                                      step.n_entries - n1, step.max_q_len, G, H, dk, dv)
@@ -242,7 +243,7 @@ class HeadGatedDelta(Mixer):
             kernels.delta_head_prepare(self.rule, proj, ring, step.positions, step.entry_of_token, step.cu_q,
                                        step.state_slot, qn, kn, vv, gg, bb, n1, T - n1)
             kernels.conv_ring_write(self.rule, proj, ring, step.positions, step.cu_q, step.state_slot, n1, many)
-            if kernels.chunk_recurrence_fits(rt.dtype, dk, dv, step.max_q_len, many * H):
+            if kernels.chunk_recurrence_fits(rt.dtype, dk, dv, step.max_q_len, (T - n1) * H, True):
                 kernels.chunk_recurrence(rt.chunk_scratch, qn, kn, vv, gg, bb, S, o, step.cu_q, step.state_slot, n1, many,
                                          step.max_q_len, G, H, dk, dv)
             else:

@@ -93,8 +93,10 @@ class GatedLinearAttention(Mixer):
                             dk ** -0.5, self.tau)
         o = rt.scratch.get("delta_o", (rt.max_tokens, H, dv), f32)[:T]
         # (a step lists its single tokens first: they, and short portions, go token by token)
-        n1 = step.n_single if kernels.chunk_recurrence_fits(rt.dtype, dk, dv, step.max_q_len) else step.n_entries
-        kernels.gated_linear_recurrence(qn, kn, vv, gg, state, o, step.cu_q, step.state_slot, n1, H, dk, dv)
+        chunks = kernels.chunk_recurrence_fits(rt.dtype, dk, dv, step.max_q_len, (T - step.n_single) * H, False)
+        n1 = step.n_single if chunks else step.n_entries
+        if n1:
+            kernels.gated_linear_recurrence(qn, kn, vv, gg, state, o, step.cu_q, step.state_slot, n1, H, dk, dv)
         if step.n_entries > n1:
             kernels.chunk_recurrence(rt.chunk_scratch, qn, kn, vv, gg, None, state, o, step.cu_q, step.state_slot, n1,
                                      step.n_entries - n1, step.max_q_len, H, H, dk, dv)

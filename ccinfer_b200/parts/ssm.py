@@ -61,6 +61,7 @@ class SelectiveStateSpace(Mixer):
 
     def bind(self, rt, fetch):
         self.rt = rt
+        self.chunk_rows = None
         n = self.names
         self.w_in = fetch(n["in"])
         if self.proj_width != self.in_width:   # zero rows: columns that nobody reads
@@ -91,12 +92,15 @@ class SelectiveStateSpace(Mixer):
         S, conv = state["S"], state["conv"]
         # portions of prompts go in chunks on tensor cores (a step lists its single tokens first: they, and short portions,
         # go token by token).  The chunks' rows take the places of those that the recurrence would read.
-        n1 = step.n_single if kernels.ssm_chunks_fits(rt.dtype, N, P, step.max_q_len) else step.n_entries
+        chunks = kernels.ssm_chunks_fits(rt.dtype, N, P, step.max_q_len, (T - step.n_single) * H)
+        n1 = step.n_single if chunks else step.n_entries
         chunk = None
         if step.n_entries > n1:
-            halves = [rt.scratch.get(f"ssm_chunk{i}:{G * N}", (rt.max_tokens, G, N), rt.dtype)[:T] for i in range(4)]
-            logs = [rt.scratch.get(f"ssm_log{i}:{H}", (rt.max_tokens, H), f32)[:T] for i in range(2)]
-            chunk = (n1, *halves, *logs)   # (single tokens: one row each)
+            if self.chunk_rows is None:   # (of constant sizes: looked up once)
+                halves = [rt.scratch.get(f"ssm_chunk{i}:{G}:{N}", (rt.max_tokens, G, N), rt.dtype) for i in range(4)]
+                logs = [rt.scratch.get(f"ssm_log{i}:{H}", (rt.max_tokens, H), f32) for i in range(2)]
+                self.chunk_rows = (*halves, *logs)
+            chunk = (n1, *self.chunk_rows)   # (single tokens: one row each)
         ox, odt = self.inner, self.inner + self.conv_width
         kernels.ssm_prepare(proj, ox, odt, self.conv_w, self.conv_b, self.taps, conv, self.A_log, self.dt_bias,
                             step.entry_of_token, step.cu_q, step.state_slot, xs, bs, cs, dts, decay, H, P, G, N,
@@ -105,7 +109,8 @@ class SelectiveStateSpace(Mixer):
         kernels.conv_state_shift(proj[:, ox:ox + self.conv_width], self.taps, conv, step.cu_q, step.state_slot,
                                  step.n_entries - step.n_single, entry0=step.n_single)
         o = rt.scratch.get("ssm_o", (rt.max_tokens, H, P), f32)[:T]
-        kernels.ssm_recurrence(cs, bs, xs, decay, dts, S, o, step.cu_q, step.state_slot, n1, G, H, N, P)
+        if n1:
+            kernels.ssm_recurrence(cs, bs, xs, decay, dts, S, o, step.cu_q, step.state_slot, n1, G, H, N, P)
         if chunk is not None:
             kernels.ssm_chunks(chunk, xs, S, o, step.cu_q, step.state_slot, n1, step.n_entries - n1, G, H, N, P)
         y = rt.scratch.get("ssm_y", (rt.max_tokens, self.inner), rt.dtype)[:T]

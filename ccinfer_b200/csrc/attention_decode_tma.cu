@@ -60,6 +60,13 @@ __device__ __forceinline__ float2 angle_cs(const float* inv_freq, float fpos, in
   return make_float2(cs, sn);
 }
 
+// How a row's key range is cut: into at most num_splits (the grid's) pieces of at least min_tiles tiles; or, with
+// ragged_percent > 0 and the step's rows alike (the longest less than so many hundredths of their mean), into at most
+// even_splits of at least even_tiles.
+struct RowPieces {
+  int num_splits, min_tiles, even_splits, even_tiles, ragged_percent;
+};
+
 template <int HD, bool FUSED>
 __global__ void __launch_bounds__(kThreads)
 attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
@@ -69,7 +76,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                             const int* __restrict__ positions, const int* __restrict__ entry_of_token,
                             const int* __restrict__ block_table, int bt_stride, int n_entries, int row0, int nq,
                             int nkv, int page_size, int page_shift, int num_pages, int window, float scale,
-                            int num_splits, int min_tiles, int* __restrict__ counters, AttnExtra ex, int* status) {
+                            const RowPieces pieces, int* __restrict__ counters, AttnExtra ex, int* status) {
   // The kernel after this one is let in only when this one ends: a product that came in while the last
   // blocks were still merging made the pair slower (measured), not faster.
   // The fused form may itself come in early (programmatic dependent launch): the cached keys and values it
@@ -79,6 +86,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
   // the kernel before this one wrote: everybody waits first.
   const bool early = FUSED && fq.k_cache != nullptr;
   if (!early) ccb::pdl_wait();
+  const int num_splits = pieces.num_splits;
   constexpr int NH = HD / 64;
   constexpr int KS = HD / 16;
   constexpr int TILE_BYTES = NH * kHalfBytes;        // one K or V tile
@@ -104,17 +112,43 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
 
   const int b = entry_of_token[t];
   const int p = positions[t];
+  // (asked for with the block's own row, for the lengths below)
+  const bool in_lane = pieces.ragged_percent > 0 && lane < (int)gridDim.x;
+  const int b_lane = in_lane ? entry_of_token[row0 + lane] : -1, p_lane = in_lane ? positions[row0 + lane] : -1;
   const bool padded = b < 0 || b >= n_entries || p < 0;
   // The row's tiles and how many of the grid's splits get some.  A split is worth a block only from
-  // min_tiles tiles on: with a short context the first eff_splits splits take that many each and the
+  // min_tiles (even_tiles) tiles on: with a short context the first eff_splits splits take that many each and the
   // others have nothing to do (the grid is sized without knowing the context).  Where the last block
   // merges, they leave at once and are not waited for (measured at one row and 2,048 keys with a grid of
   // 32 splits: 12.1 us when all 32 took a tile and were merged, as against 10.6 us with a grid of 8).
+  auto tiles_of = [&](int pos) { return KeyTiles(first_visible_key(pos, window, ex.chunk), ex.keep, kTileKeys); };
   const int j0 = padded ? 0 : first_visible_key(p, window, ex.chunk);
-  const KeyTiles kt(j0, ex.keep, kTileKeys);
+  const KeyTiles kt = tiles_of(padded ? 0 : p);
   const int first_tile = kt.first, last_tile = (padded ? 0 : p) / kTileKeys;
   const int n_tiles = last_tile - first_tile + 1;
-  const int eff_splits = padded ? 1 : min(num_splits, max(1, (n_tiles + min_tiles - 1) / min_tiles));
+  int most_splits = num_splits, min_tiles = pieces.min_tiles;
+  if (pieces.ragged_percent > 0) {   // the rows' lengths, a lane a row (every warp for itself)
+    unsigned longest = 0, total = 0, live = 0;
+    auto count = [&](int bi, int pi) {
+      const bool is_row = bi >= 0 && bi < n_entries && pi >= 0;
+      const unsigned n = is_row ? pi / kTileKeys - tiles_of(pi).first + 1 : 0;
+      longest = max(longest, n);
+      total += n;
+      live += __popc(__ballot_sync(0xffffffffu, is_row));
+    };
+    count(b_lane, p_lane);
+    for (int i0 = 32; i0 < (int)gridDim.x; i0 += 32) {
+      const int i = i0 + lane;
+      count(i < (int)gridDim.x ? entry_of_token[row0 + i] : -1, i < (int)gridDim.x ? positions[row0 + i] : -1);
+    }
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    total = __reduce_add_sync(0xffffffffu, total);
+    if (100ull * longest * live < (unsigned long long)pieces.ragged_percent * total) {
+      most_splits = pieces.even_splits;
+      min_tiles = pieces.even_tiles;
+    }
+  }
+  const int eff_splits = padded ? 1 : min(most_splits, max(1, (n_tiles + min_tiles - 1) / min_tiles));
   if (counters != nullptr && split >= eff_splits) return;
   const bool whole = num_splits == 1 || (counters != nullptr && eff_splits == 1);   // this block sees all of the row's keys
   if (tid == 0) {
@@ -617,7 +651,8 @@ int launch(const void* q, const FusedQkv& fq, const void* k_cache, const void* v
            float* part_ml,
            const int* positions, const int* entry_of_token, const int* block_table, int bt_stride, int n_entries,
            int row0, int n_rows, int nq, int nkv, int page_size, int num_pages, int window, float scale,
-           int num_splits, int min_tiles, int* counters, AttnExtra ex, int* status, cudaStream_t stream) {
+           const RowPieces& pieces, int* counters, AttnExtra ex, int* status, cudaStream_t stream) {
+  const int num_splits = pieces.num_splits;
   const int G = nq / nkv, gchunks = (G + 15) / 16;
   int page_shift = 0;
   while ((1 << page_shift) < page_size) ++page_shift;
@@ -637,7 +672,7 @@ int launch(const void* q, const FusedQkv& fq, const void* k_cache, const void* v
   dim3 grid(n_rows, nkv * gchunks, num_splits);
   ccb_launch_ex(FUSED && fq.k_cache != nullptr, attention_decode_tma_kernel<HD, FUSED>, grid, kThreads, smem, stream,
                 tmK, tmV, (const __nv_bfloat16*)q, fq, (__nv_bfloat16*)out, part_acc, part_ml, positions, entry_of_token, block_table, bt_stride, n_entries,
-             row0, nq, nkv, page_size, page_shift, num_pages, window, scale, num_splits, min_tiles, counters, ex, status);
+             row0, nq, nkv, page_size, page_shift, num_pages, window, scale, pieces, counters, ex, status);
   int rc = ccb_launch_status();
   if (rc != 0 || num_splits == 1 || counters != nullptr) return rc;
   ccb_launch(attention_merge_bf16_kernel2, dim3(n_rows, nq), 128, 0, stream, (__nv_bfloat16*)out, part_acc, part_ml,
@@ -645,11 +680,17 @@ int launch(const void* q, const FusedQkv& fq, const void* k_cache, const void* v
   return ccb_launch_status();
 }
 
+bool pieces_ok(const RowPieces& p) {
+  if (p.num_splits <= 0 || p.num_splits > 64 || p.min_tiles <= 0 || p.ragged_percent < 0) return false;
+  return p.ragged_percent == 0 || (p.even_splits > 0 && p.even_splits <= p.num_splits && p.even_tiles > 0);
+}
+
 }  // namespace
 
 // As ccb_attention_decode_mma, for page sizes that are a power of two from 8 to 64 (others: CCB_REFUSE_SIZE).
 // chunk, keep, sink, gate, gate_stride: see AttnExtra (0 / null: none).
-// A row's key range is cut into at most num_splits pieces of at least min_tiles tiles of 64 keys.
+// A row's key range is cut into at most num_splits pieces of at least min_tiles tiles of 64 keys; with ragged_percent > 0 and
+// rows whose longest is less than so many hundredths of their mean, into at most even_splits of at least even_tiles.
 // `counters` (optional): n_rows * kv_heads * ceil(group / 16) ints that are zero before the first launch and
 // are left zero; with them the splits are merged by the attention kernel itself, without them by a second
 // kernel.
@@ -658,12 +699,14 @@ CCB_API int ccb_attention_decode_tma(const void* q, const void* k_cache, const v
                                      const int* entry_of_token, const int* block_table, int bt_stride,
                                      int n_entries, int row0, int n_rows, int nq, int nkv, int hd, int page_size,
                                      int num_pages, int window, float scale, int num_splits, int min_tiles,
-                                     int* counters, int chunk, int keep, const float* sink, const void* gate, int gate_stride,
-                                     int* status, cudaStream_t stream) {
+                                     int even_splits, int even_tiles, int ragged_percent, int* counters, int chunk, int keep,
+                                     const float* sink, const void* gate, int gate_stride, int* status, cudaStream_t stream) {
   if (n_rows <= 0) return 0;
+  const RowPieces pieces{num_splits, min_tiles, even_splits, even_tiles, ragged_percent};
+  if (!pieces_ok(pieces)) return CCB_REFUSE_SIZE;
   if (chunk < 0 || keep < 0 || (gate != nullptr && gate_stride < nq)) return CCB_REFUSE_ARG;
   const AttnExtra ex{chunk, sink, gate, gate_stride, keep};
-  if (nq <= 0 || nkv <= 0 || nq % nkv != 0 || bt_stride <= 0 || num_splits <= 0 || num_splits > 64 || min_tiles <= 0 ||
+  if (nq <= 0 || nkv <= 0 || nq % nkv != 0 || bt_stride <= 0 ||
       page_size < 8 || page_size > 64 || (page_size & (page_size - 1)) != 0 ||
       ((reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) != 0)
     return CCB_REFUSE_SIZE;
@@ -672,11 +715,11 @@ CCB_API int ccb_attention_decode_tma(const void* q, const void* k_cache, const v
   if (hd == 128)
     return launch<128, false>(q, none, k_cache, v_cache, out, part_acc, part_ml, positions, entry_of_token,
                               block_table, bt_stride, n_entries, row0, n_rows, nq, nkv, page_size, num_pages, window,
-                              scale, num_splits, min_tiles, counters, ex, status, stream);
+                              scale, pieces, counters, ex, status, stream);
   if (hd == 64)
     return launch<64, false>(q, none, k_cache, v_cache, out, part_acc, part_ml, positions, entry_of_token,
                              block_table, bt_stride, n_entries, row0, n_rows, nq, nkv, page_size, num_pages, window,
-                             scale, num_splits, min_tiles, counters, ex, status, stream);
+                             scale, pieces, counters, ex, status, stream);
   return CCB_REFUSE_SIZE;
 }
 
@@ -695,13 +738,16 @@ CCB_API int ccb_attention_decode_tma_fused(const void* qkv, int qkv_stride, void
                                            int page_size, int num_pages, int window, float scale, int num_splits,
                                            const float* q_w, const float* k_w, float eps, const float* inv_freq,
                                            int write_kv, const float* bias, float qt_coef, int qt_every,
-                                           int min_tiles, int* counters, int chunk, int keep, const float* sink, const void* gate,
-                                           int gate_stride, int* status, cudaStream_t stream) {
+                                           int min_tiles, int even_splits, int even_tiles, int ragged_percent, int* counters,
+                                           int chunk, int keep, const float* sink, const void* gate, int gate_stride, int* status,
+                                           cudaStream_t stream) {
   if (n_rows <= 0) return 0;
+  const RowPieces pieces{num_splits, min_tiles, even_splits, even_tiles, ragged_percent};
+  if (!pieces_ok(pieces)) return CCB_REFUSE_SIZE;
   if (chunk < 0 || keep < 0 || (gate != nullptr && gate_stride < nq)) return CCB_REFUSE_ARG;
   const AttnExtra ex{chunk, sink, gate, gate_stride, keep};
   if (qt_every < 0 || (bias != nullptr && !write_kv)) return CCB_REFUSE_ARG;
-  if (nq <= 0 || nkv <= 0 || nq % nkv != 0 || bt_stride <= 0 || num_splits <= 0 || num_splits > 64 || min_tiles <= 0 ||
+  if (nq <= 0 || nkv <= 0 || nq % nkv != 0 || bt_stride <= 0 ||
       page_size < 8 || page_size > 64 || (page_size & (page_size - 1)) != 0 || (qkv_stride & 1) ||
       qkv_stride < (nq + (write_kv ? 2 * nkv : 0)) * hd ||
       ((reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15) != 0 ||
@@ -723,10 +769,10 @@ CCB_API int ccb_attention_decode_tma_fused(const void* qkv, int qkv_stride, void
   if (hd == 128)
     return launch<128, true>(nullptr, fq, k_cache, v_cache, out, part_acc, part_ml, positions, entry_of_token,
                              block_table, bt_stride, n_entries, row0, n_rows, nq, nkv, page_size, num_pages, window,
-                             scale, num_splits, min_tiles, counters, ex, status, stream);
+                             scale, pieces, counters, ex, status, stream);
   if (hd == 64)
     return launch<64, true>(nullptr, fq, k_cache, v_cache, out, part_acc, part_ml, positions, entry_of_token,
                             block_table, bt_stride, n_entries, row0, n_rows, nq, nkv, page_size, num_pages, window,
-                            scale, num_splits, min_tiles, counters, ex, status, stream);
+                            scale, pieces, counters, ex, status, stream);
   return CCB_REFUSE_SIZE;
 }

@@ -149,13 +149,13 @@ _SIGNATURES = {
                                  c_float, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p],
     "ccb_attention_decode_tma": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                  c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
-                                 c_float, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p,
-                                 c_void_p],
+                                 c_float, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p,
+                                 c_int, c_void_p, c_void_p],
     "ccb_attention_decode_tma_fused": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                        c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                                        c_int, c_int, c_float, c_int, c_void_p, c_void_p, c_float, c_void_p, c_int,
-                                       c_void_p, c_float, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int,
-                                       c_void_p, c_void_p],
+                                       c_void_p, c_float, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_int,
+                                       c_void_p, c_void_p, c_int, c_void_p, c_void_p],
     "ccb_attention_prefill_mma": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                                   c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int,
                                   c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p],
@@ -1686,7 +1686,7 @@ def attention_split_plan(n_rows: int, nq: int, nkv: int, hd: int, heads_per_bloc
     """(num_splits, scratch floats for the accumulators, scratch floats for max and sum).
 
     The number of splits depends on the number of token rows only, so a step of a given size always
-    launches the same grid (and its results do not depend on the lengths in the batch)."""
+    launches the same grid (and, but for ``attention_decode_even``, its results do not depend on the lengths in the batch)."""
     gt = heads_per_block or attention_split_heads_per_block(nq, nkv, hd)
     per_split = n_rows * nkv * -(-(nq // nkv) // gt)
     target = split_target_blocks()
@@ -1697,6 +1697,7 @@ def attention_split_plan(n_rows: int, nq: int, nkv: int, hd: int, heads_per_bloc
 DECODE_MIN_TILES = 4            # tiles of 64 keys that a split of the decode kernels should have: its start-up costs as much
 DECODE_RAGGED_SPLITS = 4
 DECODE_RAGGED_BLOCKS = 384
+DECODE_RAGGED_PERCENT = 145     # of the rows' mean length that the longest of a ragged batch has at least
 
 
 def attention_decode_plan(n_rows: int, nq: int, nkv: int, hd: int):
@@ -1704,12 +1705,11 @@ def attention_decode_plan(n_rows: int, nq: int, nkv: int, hd: int):
     ``attention_decode_tma``, from the number of rows only, as ``attention_split_plan``.
 
     Where the rows alone nearly fill the machine, a few long contexts among short ones would be all that runs at the end: up
-    to DECODE_RAGGED_BLOCKS (row, kv head) pairs, contexts are cut into up to four pieces, but only into long ones, so that
-    batches of equal contexts gain no merging that they do not need.  Measured on B200, 8 kv heads of 128, one piece / this,
-    us: 32 rows, contexts of 500 to 8,000 103 / 75, all 2,048 44 / 44, all 8,000 156 / 172; 48 rows 130 / 110, 78 / 78, 279 /
-    258; 16 rows (two pieces / this) 47 / 39, 28 / 28, 82 / 87.  The block of a row that finishes last merges its pieces, and a
-    row of one piece is written at once (8 rows, kernel of its own / so: 60 keys 10.6 / 8.5 us, 256 12.4 / 9.8, 2,048 16.9 /
-    16.4, 4,100 29.4 / 28.9)."""
+    to DECODE_RAGGED_BLOCKS (row, kv head) pairs, long contexts are cut into up to four pieces.  A layer of 8 kv heads of 128,
+    rows in one piece (16 rows: two) / cut, us: contexts of 500 to 8,000, 16 rows 76 / 72, 24 131 / 88, 32 143 / 115, 48 164 /
+    130; all of 8,000, 40 rows 313 / 247, 48 315 / 292.  Up to two blocks an SM, rows whose lengths are alike are not:
+    ``attention_decode_even``.  The block of a row that finishes last merges its pieces, and a row of one piece is written at
+    once (8 rows, kernel of its own / so: 60 keys 10.6 / 8.5 us, 256 12.4 / 9.8, 2,048 16.9 / 16.4, 4,100 29.4 / 28.9)."""
     groups = n_rows * nkv * -(-(nq // nkv) // DECODE_MMA_HEADS_PER_BLOCK)
     splits, _, _ = attention_split_plan(n_rows, nq, nkv, hd, DECODE_MMA_HEADS_PER_BLOCK)
     blocks = max(split_target_blocks(), DECODE_RAGGED_SPLITS * DECODE_RAGGED_BLOCKS)
@@ -1717,6 +1717,23 @@ def attention_decode_plan(n_rows: int, nq: int, nkv: int, hd: int):
     if splits < DECODE_RAGGED_SPLITS - 1 and groups <= DECODE_RAGGED_BLOCKS:
         return DECODE_RAGGED_SPLITS, 16 if splits > 1 else 32, True, floats * hd, floats * 2
     return splits, DECODE_MIN_TILES, splits > 1, floats * hd, floats * 2
+
+
+def attention_decode_even(n_rows: int, nq: int, nkv: int, hd: int):
+    """(pieces, tiles of a piece at least, DECODE_RAGGED_PERCENT) for ``even`` of ``attention_decode_tma`` beside the plan
+    above, or None: how rows are cut whose lengths are alike.
+
+    All rows then run side by side, and cutting them costs start-ups and a merge.  The kernel looks at the step's lengths, as
+    a captured launch cannot: of so many rows, a row's pieces (not their order or merge) depend on its neighbours' lengths.
+    The layer in one piece (16 rows: two) / cut, us, by the longest row over the mean.  1.0, all of 4,000: 16 rows 75 / 81, 20 90
+    / 107, 24 95 / 109, 32 111 / 117; all of 8,000: 16 113 / 117, 32 189 / 204, 36 206 / 219.  1.26: 20 136 / 134, 32 171 / 183,
+    36 181 / 190.  1.45: 16 98 / 99, 20 134 / 107, 24 142 / 135, 32 160 / 160, 36 171 / 180.  1.7: 20 131 / 101, 24 139 / 108, 32
+    153 / 142, 36 160 / 164.  2.0: 20 131 / 97, 32 148 / 134, 36 156 / 141.  Looking takes 0.5 us of a launch."""
+    groups = n_rows * nkv * -(-(nq // nkv) // DECODE_MMA_HEADS_PER_BLOCK)
+    splits, _, _ = attention_split_plan(n_rows, nq, nkv, hd, DECODE_MMA_HEADS_PER_BLOCK)
+    if splits >= DECODE_RAGGED_SPLITS - 1 or groups > split_target_blocks():
+        return None
+    return splits, DECODE_MIN_TILES, DECODE_RAGGED_PERCENT
 
 
 def attention_split(q, k_cache, v_cache, out, part_acc, part_ml, positions, entry_of_token, block_table,
@@ -1795,13 +1812,14 @@ def attention_decode_tma_fits(hd: int, page_size: int) -> bool:
 def attention_decode_tma(q, k_cache, v_cache, out, part_acc, part_ml, positions, entry_of_token, block_table,
                          n_entries: int, row0: int, n_rows: int, window: int, scale: float, num_splits: int,
                          status=None, merge_counters=None, chunk: int = 0, sink=None, gate=None, keep: int = 0,
-                         min_tiles: int = DECODE_MIN_TILES) -> None:
+                         min_tiles: int = DECODE_MIN_TILES, even=None) -> None:
     """As attention_decode_mma, with keys and values loaded page by page through TMA boxes by a producer warp
     (page size a power of two from 8 to 64).
 
     ``merge_counters`` (int32 zeros, left zero): with them the block that finishes last merges the splits
     of its row and head group; without them (or where they are too few) a second kernel does.  ``min_tiles``: tiles of 64
-    keys that a split takes at least."""
+    keys that a split takes at least.  ``even`` = (splits, min_tiles, percent): these where the longest row has less than
+    so many hundredths of the rows' mean."""
     _cuda(q, k_cache, v_cache, out, part_acc, part_ml, positions, entry_of_token, block_table, status, merge_counters)
     T, nq, hd = q.shape
     num_pages, nkv, page_size, hd2 = k_cache.shape
@@ -1820,7 +1838,8 @@ def attention_decode_tma(q, k_cache, v_cache, out, part_acc, part_ml, positions,
     _check(lib().ccb_attention_decode_tma(_p(q), _p(k_cache), _p(v_cache), _p(out), _p(part_acc), _p(part_ml),
                                           _p(positions), _p(entry_of_token), _p(block_table),
                                           block_table.stride(0), n_entries, row0, n_rows, nq, nkv, hd, page_size,
-                                          num_pages, int(window), float(scale), num_splits, int(min_tiles), _p(merge_counters),
+                                          num_pages, int(window), float(scale), num_splits, int(min_tiles),
+                                          *(even or (1, 1, 0)), _p(merge_counters),
                                           *_attn_extra(T, nq, q.dtype, chunk, sink, gate, keep), _p(status), _stream()),
            "attention_decode_tma")
     if num_splits > 1 and merge_counters is None:
@@ -1852,12 +1871,13 @@ def attention_decode_tma_fused(qkv, k_cache, v_cache, out, part_acc, part_ml, po
                                scale: float, num_splits: int, q_norm_w, k_norm_w, eps: float, inv_freq,
                                write_kv: bool = True, status=None, merge_counters=None, bias=None,
                                q_temperature=None, chunk: int = 0, sink=None, gate=None, keep: int = 0,
-                               min_tiles: int = DECODE_MIN_TILES) -> None:
+                               min_tiles: int = DECODE_MIN_TILES, even=None) -> None:
     """attention_decode_tma for rows of ONE new token each, straight from the q|k|v product ``qkv``
     [T, (nq + 2 nkv) * hd] (only the nq query heads when ``write_kv`` is false): the kernel norms and rotates
     the queries itself and, with ``write_kv``, also the row's key, which it writes with the value to their
     page and attends to.  qk_norm_rope_kv_write is not needed for these rows.  ``bias`` and ``q_temperature``
-    as for ``qkv_bias_rope_kv_write``; ``chunk``, ``sink``, ``gate`` as for ``attention_split``."""
+    as for ``qkv_bias_rope_kv_write``; ``chunk``, ``sink``, ``gate`` as for ``attention_split``; ``min_tiles`` and ``even``
+    as for ``attention_decode_tma``."""
     _cuda(qkv, k_cache, v_cache, out, part_acc, part_ml, positions, entry_of_token, block_table, status,
           merge_counters, q_norm_w, k_norm_w, inv_freq, bias)
     assert bias is None or (write_kv and bias.dtype == torch.float32
@@ -1881,7 +1901,7 @@ def attention_decode_tma_fused(qkv, k_cache, v_cache, out, part_acc, part_ml, po
         _p(entry_of_token), _p(block_table), block_table.stride(0), n_entries, row0, n_rows, nq, nkv, hd, page_size,
         num_pages, int(window), float(scale), num_splits, _p(q_norm_w), _p(k_norm_w), float(eps), _p(inv_freq),
         1 if write_kv else 0, _p(bias), float(q_temperature[0]) if q_temperature else 0.0,
-        int(q_temperature[1]) if q_temperature else 0, int(min_tiles), _p(merge_counters),
+        int(q_temperature[1]) if q_temperature else 0, int(min_tiles), *(even or (1, 1, 0)), _p(merge_counters),
         *_attn_extra(T, nq, qkv.dtype, chunk, sink, gate, keep), _p(status), _stream()), "attention_decode_tma_fused")
     if num_splits > 1 and merge_counters is None:
         counters.own += 1  # the merge kernel

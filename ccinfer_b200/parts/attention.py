@@ -350,7 +350,8 @@ class GroupedQueryAttention(Mixer):
             plan = {}
             if tma:
                 splits, tiles, in_kernel, n_acc, n_ml = kernels.attention_decode_plan(n_rows, self.nq, self.nkv, self.hd)
-                plan = {"min_tiles": tiles, "merge_counters": rt.merge_counters if in_kernel else None}
+                plan = {"min_tiles": tiles, "merge_counters": rt.merge_counters if in_kernel else None,
+                        "even": kernels.attention_decode_even(n_rows, self.nq, self.nkv, self.hd)}
             else:
                 per_block = kernels.DECODE_MMA_HEADS_PER_BLOCK if mma else 0
                 splits, n_acc, n_ml = kernels.attention_split_plan(n_rows, self.nq, self.nkv, self.hd, per_block)
@@ -441,6 +442,7 @@ class GroupedQueryAttention(Mixer):
                 self.q_norm_w, self.k_norm_w, self.norm_eps if self.norm_eps is not None else 1.0,
                 self.position.rotary_table(), write_kv=self.own_kv, status=rt.status,
                 merge_counters=rt.merge_counters if in_kernel else None, min_tiles=min_tiles,
+                even=kernels.attention_decode_even(T, self.nq, self.nkv, self.hd),
                 bias=self.bias, q_temperature=self.position.query_temperature(), chunk=self.chunk, sink=self.sink,
                 gate=gate, keep=self.keep_first)
         else:

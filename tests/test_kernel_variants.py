@@ -546,6 +546,43 @@ def test_decode_of_ragged_contexts(rows, min_tiles):
         assert (out[r].double() - want).abs().max() <= 2.0 ** -7 * values.abs().max()
 
 
+# rows whose lengths are alike stay in one piece (or two: 16 rows), a long one among short ones is cut; 40 rows: always
+@pytest.mark.parametrize("rows,even_pieces,ragged_pieces", [(16, 2, 4), (24, 1, 3), (36, 1, 3), (40, 3, 3)])
+@pytest.mark.parametrize("window", [0, 3000])
+def test_decode_cuts_long_rows_of_ragged_batches_only(rows, even_pieces, ragged_pieces, window):
+    """Every row against float64, and how many pieces left results (a row of one piece leaves none)."""
+    k, g = _k(), _gen(rows)
+    nq, nkv, hd, page, most = 16, 8, 128, 64, 4160
+    n = -(-most // page)
+    kc, vc = (torch.randn((n, nkv, page, hd), generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    table = torch.stack([torch.randperm(n, generator=torch.Generator().manual_seed(r)) for r in range(rows)]).to(torch.int32)
+    q = torch.randn((rows, nq, hd), generator=g, device="cuda").to(torch.bfloat16)
+    splits, tiles, in_kernel, n_acc, n_ml = k.attention_decode_plan(rows, nq, nkv, hd)
+    even = k.attention_decode_even(rows, nq, nkv, hd)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    count, status = torch.zeros(8192, **i32), torch.zeros(1, **i32)
+    for ragged in (False, True):
+        ctx = [most - 5 * r for r in range(rows)] if not ragged else [most if r == 7 else 100 + 3 * r for r in range(rows)]
+        acc, ml, out = torch.full((n_acc,), float("nan"), device="cuda"), torch.full((n_ml,), float("nan"), device="cuda"), torch.full_like(q, float("nan"))
+        entry = torch.arange(rows, **i32)
+        entry[3] = -1   # a row that pads the step
+        k.attention_decode_tma(q, kc, vc, out, acc, ml, torch.tensor([c - 1 for c in ctx], **i32), entry, table.cuda(), rows, 0, rows,
+                               window, hd ** -0.5, splits, status=status, merge_counters=count, min_tiles=tiles, even=even)
+        assert int(status.item()) == 0 and int(count.abs().sum()) == 0
+        left = torch.isfinite(ml[:2 * rows * nq * splits].view(rows, nq, splits, 2)).all(-1).sum(-1)
+        if not window:
+            assert (left[7] == (ragged_pieces if ragged else even_pieces if even_pieces > 1 else 0)).all()
+        for r in (0, 3, 7, rows - 1):
+            if r == 3:
+                assert not out[r].any()
+                continue
+            at = table[r].long().cuda()
+            keys, values = (t[at].transpose(1, 2).reshape(-1, nkv, hd)[max(0, ctx[r] - window) if window else 0:ctx[r]].double() for t in (kc, vc))
+            s = torch.einsum("hd,jhd->hj", q[r].double(), keys.repeat_interleave(nq // nkv, 1)) * hd ** -0.5
+            want = torch.einsum("hj,jhd->hd", torch.softmax(s, -1), values.repeat_interleave(nq // nkv, 1))
+            assert (out[r].double() - want).abs().max() <= 2.0 ** -7 * values.abs().max()
+
+
 # one block a head from 16 requests of 32 heads on where key and value sizes are over 64; else a cluster a head
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("E,G,H,dk,dv", [(16, 32, 32, 128, 128), (16, 16, 32, 100, 68), (17, 16, 32, 68, 128), (15, 32, 32, 128, 128),

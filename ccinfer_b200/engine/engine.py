@@ -165,7 +165,8 @@ class Engine:
         # first ones where those are kept (None: all of them)
         spans = [min(x for x in (w, c) if x is not None) + -(-k // P) * P if (w is not None or c is not None) else None
                  for w, c, k in zip(windows, chunks, kept)]
-        pages = self._pages_per_group(opt, group_keys, spans, token_bytes)
+        late = max((getattr(part, "late_bytes", int)() for part in plan.parts()), default=0)   # (their layers share the buffers)
+        pages = self._pages_per_group(opt, group_keys, spans, token_bytes, late)
         for i, need in owners.items():
             n = pages[self._entry_group[i]]
             self._cache[i] = {t.name: torch.zeros((n,) + t.page_shape(P), dtype=t.dtype or self.dtype, device=rt.device)
@@ -221,7 +222,7 @@ class Engine:
         kv_tokens = opt.kv_tokens if opt.kv_tokens is not None else 1024 * P
         return max(1, -(-kv_tokens // P))
 
-    def _pages_per_group(self, opt, group_keys, windows, token_bytes) -> List[int]:
+    def _pages_per_group(self, opt, group_keys, windows, token_bytes, late=0) -> List[int]:
         """Pages of each cache group's pool, from what a token costs there and a budget.
 
         A group that keeps every token gets ``kv_tokens`` tokens (default 1024 pages, the reference's pool:
@@ -242,7 +243,8 @@ class Engine:
         if opt.kv_memory_fraction is not None:
             if not (0.0 < opt.kv_memory_fraction <= 1.0):
                 raise InvalidArgument("kv_memory_fraction lies in (0, 1]")
-            budget = int(torch.cuda.mem_get_info(self.rt.device)[0] * opt.kv_memory_fraction)
+            # (what parts ask for only when a long prompt comes must be free then)
+            budget = int(max(0, torch.cuda.mem_get_info(self.rt.device)[0] - late) * opt.kv_memory_fraction)
             page_bytes = [b * P for b in token_bytes]
             capped = [window_cap(w) if w is not None else None for w in windows]
             fixed = sum(c * pb for c, pb in zip(capped, page_bytes) if c is not None)
@@ -649,7 +651,7 @@ class Engine:
     def stats(self) -> dict:
         s = self.cache.stats()
         s["steps"] = self.steps_run
-        s["scratch_bytes"] = self.rt.scratch.bytes()
+        s["scratch_bytes"] = self.rt.scratch_bytes()
         return s
 
 

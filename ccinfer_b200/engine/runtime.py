@@ -78,6 +78,7 @@ class Runtime:
         self.sm_count = torch.cuda.get_device_properties(self.device).multi_processor_count
         self.tc_counters = torch.zeros(4096, dtype=torch.int32, device=self.device)  # split-K tile counters
         self._chunk_scratch: Dict[tuple, torch.Tensor] = {}
+        self._late: Dict[str, torch.Tensor] = {}
         self.merge_counters = torch.zeros(8192, dtype=torch.int32, device=self.device)  # attention split counters
         self._sink_turn = 0
 
@@ -90,6 +91,23 @@ class Runtime:
             name = ":".join([key] + [str(d) for d in shape])
             t = self._chunk_scratch[key, shape] = self.scratch.get(name, (n,) + tuple(shape), dtype)
         return t
+
+    def late(self, key: str, n: int, dtype: torch.dtype) -> torch.Tensor:
+        """A flat buffer of at least n elements for steps that no graph of the engine holds (portions of prompts) and whose
+        need follows the lengths in the step: ONE buffer a key, which a larger one takes the place of (a part says how
+        large it can get: ``Part.late_bytes``)."""
+        if torch.cuda.is_current_stream_capturing():   # (somebody's own graph: this address must stay)
+            return self.scratch.get(f"{key}:{n}", (n,), dtype)
+        buf = self._late.get(key)
+        if buf is None or buf.numel() < n:
+            if buf is not None:
+                buf.record_stream(torch.cuda.current_stream())
+                del self._late[key], buf   # given back before the larger one is asked for
+            buf = self._late[key] = torch.empty(n, dtype=dtype, device=self.device)
+        return buf
+
+    def scratch_bytes(self) -> int:
+        return self.scratch.bytes() + sum(b.numel() * b.element_size() for b in self._late.values())
 
     @staticmethod
     def rows(x):

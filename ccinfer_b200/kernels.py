@@ -861,12 +861,20 @@ def latent_attention_mma_fits(dtype, R: int, r: int) -> bool:
     return dtype == torch.bfloat16 and R % 16 == 0 and r % 16 == 0 and 0 < R <= 512
 
 
-# Tokens of a step's longest portion from which the heads' keys and values are made from the cached rows for the step.  Per
-# cached row and head that costs (64 nd + 64 nv) R products once, and saves 2 R + r - 64 (nd + nv + 1) a query.  A layer of 32
-# heads, in the latent space / over made keys and values, us: 32 tokens after 200 56 / 43, after 1,500 (window 1,024) 131 / 64,
-# after 3,000 307 / 95, 4 portions of about 32 after 200 70 / 56; 128 tokens after 200 83 / 51.  (20 tokens gain as much as
-# 32; fewer were not measured.)
-LATENT_DENSE_MIN_TOKENS = 32
+# When the heads' keys and values are made from the cached rows that a step's portions see.  Per row and head that costs
+# (64 nd + 64 nv) R products once, and saves 2 R + r - 64 (nd + nv + 1) a query; but the kernel over the latent rows walks a
+# portion's keys one after another, whatever the portion brings, so that few tokens after many gain most and many portions
+# beside one another least.  Times by kernel, ns: over the latent rows 100 a key of the longest walk, or 0.022 a (row, token,
+# head) triple where those keep the machine busy; over made ones 0.25 a row and head and 8 a key of the longest walk and
+# group of heads.  And below LATENT_DENSE_MIN_NS a layer waits for its launches, of which made keys and values take 13 us
+# more, unless a portion brings LATENT_DENSE_MIN_TOKENS.  Layers in the latent space / over made keys and values, us, alone
+# and among others.  16 heads: 24 tokens after 20 151 / 166, 142 / 155; after 400 158 / 166, 142 / 156; after 1,500 (window
+# 1,024) 213 / 164, 147 / 154; after 1,500 254 / 165, 179 / 155; after 6,000 662 / 206, 582 / 160; 128 after 400 169 / 165, 143
+# / 154; 15 portions of 2 after 2,000 304 / 327, 232 / 210, after 4,000 491 / 394, 426 / 338.  32 heads: 4 of 64 after 400
+# 180 / 173, 147 / 159, after 1,500 280 / 203, 224 / 160; 4 of 2 after 4,000 501 / 325, 426 / 254, after 16,000 1,600 / 1,062,
+# 1,516 / 1,003; 15 of 2 after 300 171 / 217, 159 / 177, after 4,000 509 / 671, 435 / 609.
+LATENT_DENSE_MIN_NS = 70_000
+LATENT_DENSE_MIN_TOKENS = 192
 LATENT_DENSE_ELEMENTS = 96 << 20   # of the made keys and values at most: heads go in groups where all would be more
 LATENT_DENSE_ROWS = 1 << 16        # cached rows at most
 
@@ -880,6 +888,23 @@ def latent_dense_fits(dtype, d: int, r: int, rot_dims: int, dv: int, R: int) -> 
 def latent_dense_rows(pos0: int, n: int, window: int) -> int:
     """Rows of a request with ``pos0`` cached and ``n`` new tokens (see ``csrc/dense_rows.cuh``)."""
     return -(-(pos0 + n) // 128) * 128 - max(0, pos0 - window + 1) // 128 * 128
+
+
+def latent_dense_heads(rows: int, heads: int, cols: int) -> int:
+    """Heads of ``cols`` columns of keys and values that are made at once for ``rows`` rows (a power of two)."""
+    return max(1, min(heads, LATENT_DENSE_ELEMENTS // (rows * cols)))
+
+
+def latent_dense_pays(rows, tokens, heads: int, cols: int) -> bool:
+    """Whether a step's portions, which see so many ``rows`` and bring so many ``tokens`` each, run over made keys and
+    values (``cols`` columns a head): all of them or none."""
+    seen, longest = sum(rows), max(rows)
+    if seen > LATENT_DENSE_ROWS:
+        return False
+    groups = -(-heads // latent_dense_heads(1 << (seen - 1).bit_length(), heads, cols))
+    walk = max(100 * longest, 0.022 * heads * sum(r * n for r, n in zip(rows, tokens)))
+    return (walk >= 0.25 * heads * seen + 8 * groups * longest
+            and (walk >= LATENT_DENSE_MIN_NS or max(tokens) >= LATENT_DENSE_MIN_TOKENS))
 
 
 def latent_rows(dst, max_rows: int, cache, cu_q, pos0, block_table, entry0: int, n_entries: int, window: int,

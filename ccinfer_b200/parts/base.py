@@ -19,6 +19,9 @@ A mixer further says what it needs to remember between steps:
 * ``cache_need()``: the tensors it keeps per token, in pages (of all tokens, or
   of a window of them), or None;
 * ``state_need()``: a tensor of fixed size per request, or None.
+
+A part may say how much memory it asks for only in some steps (``late_bytes()``, once bound), which is kept free when
+pages are counted.
 """
 from __future__ import annotations
 

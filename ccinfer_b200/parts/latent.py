@@ -135,7 +135,8 @@ class LatentAttention(Mixer):
         self.w_kv = None
         if kernels.latent_dense_fits(rt.dtype, self.d, self.r, self.rot_dims, self.dv, self.R):
             self.nd, self.nv = -(-self.d // 64), -(-self.dv // 64)
-            w_kv = torch.zeros((H, 64 * (self.nd + self.nv), self.R), dtype=rt.dtype, device=rt.device)
+            self.kv_cols = 64 * (self.nd + self.nv)
+            w_kv = torch.zeros((H, self.kv_cols, self.R), dtype=rt.dtype, device=rt.device)
             w_kv[:, :self.d] = fetch(n["uk"]).view(H, self.d, self.R)
             w_kv[:, 64 * self.nd:64 * self.nd + self.dv] = self.w_uv
             self.w_kv = w_kv.view(-1, self.R)
@@ -151,35 +152,41 @@ class LatentAttention(Mixer):
 
     def _dense_rows(self, step):
         """(rows in all, rows of a request at most) that the step's portions see, or None where they do not run over made keys
-        and values: no portion is long enough, or the rows are too many.  From the host's arrays where the step has them,
-        else a bound."""
+        and values (``kernels.latent_dense_pays``).  From the host's arrays where the step has them, else from bounds."""
         n1, many = step.n_single, step.n_entries - step.n_single
-        if self.w_kv is None or many == 0 or step.max_q_len < kernels.LATENT_DENSE_MIN_TOKENS:
+        if self.w_kv is None or many == 0:
             return None
         if step.host is not None:
-            spans = [kernels.latent_dense_rows(int(p), int(c) - int(p), self.kernel_window)
-                     for p, c in zip(step.host.pos0[n1:step.n_entries], step.host.ctx_after[n1:step.n_entries])]
-            rows, most = sum(spans), max(spans)
+            pos0 = step.host.pos0[n1:step.n_entries].tolist()
+            counts = [c - p for p, c in zip(pos0, step.host.ctx_after[n1:step.n_entries].tolist())]
+            spans = [kernels.latent_dense_rows(p, n, self.kernel_window) for p, n in zip(pos0, counts)]
         else:
-            most = -(-min(step.max_ctx, step.max_q_len + self.kernel_window + 126) // 128) * 128
-            rows = many * most
-        return (rows, most) if rows <= kernels.LATENT_DENSE_ROWS else None
+            spans = [-(-min(step.max_ctx, step.max_q_len + self.kernel_window + 126) // 128) * 128] * many
+            counts = [step.max_q_len] + [(step.n_tokens - n1 - step.max_q_len) // max(1, many - 1)] * (many - 1)
+        return (sum(spans), max(spans)) if kernels.latent_dense_pays(spans, counts, self.H, self.kv_cols) else None
+
+    def late_bytes(self) -> int:
+        """Of the buffers of ``_dense`` at most."""
+        if self.w_kv is None:
+            return 0
+        rows = kernels.LATENT_DENSE_ROWS
+        return 2 * (rows * (self.R + self.r) + min(kernels.LATENT_DENSE_ELEMENTS, rows * self.H * self.kv_cols))
 
     def _dense(self, q, rows, span, gate, o, step, g):
         """Attention of the step's portions over keys and values of every head, made from the cached rows they see."""
         rt, H, R, W = self.rt, self.H, self.R, self.R + self.r
         T, n1, many = q.shape[0], step.n_single, step.n_entries - step.n_single
         n, most = span
-        cap = 1 << (n - 1).bit_length()   # (buffers of the next power of two: no graph holds their addresses)
-        seen = rt.scratch.get(f"latent_seen:{cap}:{W}", (cap, W), rt.dtype)[:n]
+        cap = 1 << (n - 1).bit_length()   # (buffers of the next power of two)
+        seen = rt.late("latent_seen", cap * W, rt.dtype)[:n * W].view(n, W)
         kernels.latent_rows(seen, most, rows, step.cu_q, step.pos0, g.block_table, n1, many, self.kernel_window,
                             status=rt.status)
         qr = rt.scratch.get(f"latent_query:{H}:{self.nd}", (rt.max_tokens, H, 64 * self.nd + 64), rt.dtype)[:T]
         kernels.latent_query_rows(qr, q, self.inv_freq, self.rot_dims, self.amp, step.positions, self.d, self.r)
-        cols = 64 * (self.nd + self.nv)
-        heads = max(1, min(H, kernels.LATENT_DENSE_ELEMENTS // (cap * cols)))
+        cols = self.kv_cols
+        heads = kernels.latent_dense_heads(cap, H, cols)
         size = cap * H * cols if heads == H else kernels.LATENT_DENSE_ELEMENTS   # (one buffer for all that go in groups)
-        kv = rt.scratch.get(f"latent_kv:{size}", (size,), rt.dtype)
+        kv = rt.late("latent_kv", size, rt.dtype)
         for h0 in range(0, H, heads):
             hn = min(heads, H - h0)
             part = kv[:n * hn * cols].view(n, hn * cols)

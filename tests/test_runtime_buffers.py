@@ -42,3 +42,40 @@ def test_portions_run_in_chunks_where_the_layer_gains():
     assert not delta(1, 64, 32) and not delta(16, 31, 32) and delta(4, 64, 32) and delta(16, 32, 32) and delta(1, 160, 4)
     assert not space(1, 40, 64) and not space(16, 19, 128) and space(16, 20, 128) and space(2, 64, 64)
     assert not kernels.ssm_chunks_fits(bf, 96, 64, 512, 1 << 20) and not kernels.ssm_chunks_fits(bf, 64, 24, 512, 1 << 20)
+
+
+def test_latent_portions_run_over_made_keys_where_that_is_shorter():
+    """(rows seen, tokens brought by each portion, heads of 192 columns)"""
+    def pays(rows, tokens, heads):
+        return kernels.latent_dense_pays(rows, tokens, heads, 192)
+
+    assert not pays([128], [32], 32) and not pays([640] * 4, [24] * 4, 16)   # short walks: the layer waits for its launches
+    assert pays([768], [2], 16) and pays([128, 768], [64, 2], 16) and pays([6016], [2], 32)
+    assert pays([512] * 4, [100] * 4, 32) and pays([256], [192], 1)          # many tokens, or one portion of many
+    assert not pays([128] + [2048] * 15, [32] + [2] * 15, 32)                # many portions that see much
+    assert not pays([4224] * 15, [2] * 15, 32)                               # ... its heads in groups
+    assert pays([128] + [4224] * 4, [32] + [2] * 4, 32) and pays([128] + [16128] * 4, [32] + [2] * 4, 32)
+    assert not pays([32768, 32768, 128], [400] * 3, 32)                      # more rows than the buffers hold
+
+
+def test_pages_leave_room_for_what_comes_late(monkeypatch):
+    """With kv_memory_fraction the pools share what is free beside the buffers that a long prompt will ask for."""
+    from types import SimpleNamespace
+
+    from ccinfer_b200.engine.engine import Engine, EngineOptions
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda device: (1 << 30, 2 << 30))
+    opt = EngineOptions(page_size=16, kv_memory_fraction=0.5)
+    me = SimpleNamespace(rt=SimpleNamespace(device="cuda:0"))
+    for late in (0, 1 << 28, 1 << 31):
+        pages, = Engine._pages_per_group(me, opt, [("all",)], [None], [1024], late)
+        assert pages == max(1, max(0, (1 << 30) - late) // 2 // (16 * 1024))
+
+
+@pytest.mark.gpu
+def test_one_buffer_for_portions_of_any_length():
+    rt = Runtime("cuda:0", torch.bfloat16, 64, 4)
+    small = rt.late("seen", 1 << 16, torch.bfloat16)
+    assert rt.late("seen", 1 << 10, torch.bfloat16).data_ptr() == small.data_ptr()
+    before = rt.scratch_bytes()
+    assert rt.late("seen", 1 << 20, torch.bfloat16).numel() >= 1 << 20
+    assert rt.scratch_bytes() - before == (1 << 21) - (1 << 17)   # the larger one alone

@@ -66,6 +66,13 @@ __device__ __forceinline__ void split2(float x, float y, uint32_t& hi, uint32_t&
 
 // Finite, also as two bfloat16 (the largest floats round to infinity).
 __device__ __forceinline__ bool is_finite(float x) { return fabsf(x) < 3.38e38f; }
+// The largest magnitude of m, x and y, NaN if there is one: is_finite of it is that of all of them, at half an instruction a
+// number.
+__device__ __forceinline__ float largest(float m, float x, float y) {
+  float d;
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(m), "f"(x), "f"(y));
+  return d;
+}
 
 template <int DK, int NB, bool SPLIT, bool ONES, bool V32, int TEAMS>
 __global__ void __launch_bounds__(kThreads * TEAMS)
@@ -254,11 +261,10 @@ memory_chunks_kernel(const ChunkArgs a) {
       const int row = tid >> 1, part = (tid & 1) * (BN / 2);
       const float w = gw[row];
       if constexpr (V32) {
-        bool finite = true;
+        float most = 0.f;
 #pragma unroll
-        for (int c = 0; c < NB; ++c)
-          finite = finite && is_finite(vv[c].x) && is_finite(vv[c].y) && is_finite(vv[c].z) && is_finite(vv[c].w);
-        if (!finite) {
+        for (int c = 0; c < NB; ++c) most = largest(largest(most, vv[c].x, vv[c].y), vv[c].z, vv[c].w);
+        if (!is_finite(most)) {
           bad_any[team] = 1;
 #pragma unroll
           for (int c = 0; c < BN / 2; ++c) {

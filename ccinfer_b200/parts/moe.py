@@ -47,14 +47,17 @@ class MixtureOfExperts(FeedForward):
     # of which 4 are chosen, the whole part in us, dense / sparse at 1, 8, 256, 2,048 tokens: 16.8 M weights
     # 22 / 26, 24 / 31, 37 / 51, 138 / 99; 67 M weights 47 / 33, 48 / 42, 75 / 78, 340 / 187.
     SPARSE_MIN_WEIGHTS = 1 << 25
-    # The tcgen05 grouped product runs from this many (token, choice) pairs an expert, or from this many weights of the first
-    # matrices of the experts that a step can choose: below both its walks are too few for pairs of SMs, and a block for
-    # every eight columns on mma.sync (rows16) streams them faster.  Measured on B200, the whole part in us, tcgen05 / rows16
-    # (hidden x F, experts / chosen, tokens): 4096 x 3072, 32 / 4: 90 / 102 (1 token), 129 / 170 (2), 282 / 425 (8); 2048 x
-    # 2048, 32 / 4: 49 / 48 (1), 63 / 71 (2); 2048 x 512, 32 / 4: 45 / 45 (4), 62 / 60 (8), 68 / 81 (32); 1024 x 512, 32 / 4:
-    # 41 / 37 (8), 44 / 51 (32); 2048 x 256, 64 / 6: 47 / 48 (4), 53 / 68 (8); 4096 x 512, 16 / 2: 53 / 45 (4), 57 / 60 (8).
+    # The tcgen05 grouped product runs from this many (token, choice) pairs an expert, or from so many weights of the first
+    # matrices of the experts that a step chooses (as many as chance makes different), fewer with more tokens: below, its
+    # walks are too few for pairs of SMs, and a block for every eight columns on mma.sync (rows16) streams them faster.
+    # Measured on B200 with cold weights, the whole part in us, rows16 / tcgen05 (hidden x F, experts / chosen; tokens): 4096 x
+    # 3072, 32 / 4: 1 (96 Mi) 117 / 111, 8 408 / 297; 2048 x 2048, 32 / 4: 1 (32 Mi) 59 / 63, 2 (60) 80 / 78, 4 117 / 107; 2048 x
+    # 1024, 32 / 4: 3 (42) 70 / 80, 4 (53) 78 / 80, 5 (62) 86 / 80; 2048 x 768, 64 / 8: 2 (45) 76 / 80, 3 (63) 94 / 84; 4096 x 1024,
+    # 8 / 2: 4 (44) 59 / 64, 6 (53) 74 / 72, 8 (58) 84 / 76; 4096 x 512, 16 / 2: 6 (35) 61 / 66, 7 (39) 66 / 68, 8 (42) 72 / 70, 16
+    # 90 / 80; 2048 x 512, 32 / 4: 6 (35) 64 / 61, 8 (42) 72 / 76, 9 (45) 80 / 76, 16 88 / 80; 2048 x 256, 64 / 6: 4 (21) 59 / 57, 8
+    # (35) 78 / 68; 1024 x 512, 32 / 4: 8 (21) 47 / 57, 16 (28) 55 / 57, 32 (32) 95 / 108.
     TC_MIN_ROWS_PER_EXPERT = 8
-    TC_MIN_CHOSEN_WEIGHTS = 48 << 20
+    TC_MIN_CHOSEN_WEIGHTS = ((8, 32 << 20), (6, 48 << 20), (0, 56 << 20))   # (from tokens on, weights)
     # ... and from this many pairs an expert with tiles of up to 320 rows instead of 64 (192 tokens of 4096 x 3072, 32 / 4:
     # 435 / 429 us; 64 tokens 430 / 402; 512 tokens 480 / 596)
     TC_WIDE_ROWS_PER_EXPERT = 24
@@ -204,18 +207,26 @@ class MixtureOfExperts(FeedForward):
             kernels.moe_sort(idx, wts, self.E, *sort_into)
         return idx, wts, dense
 
+    def tile_rows(self, T: int, dtype) -> int:
+        """Sorted rows of a tile for a step of T tokens: 16 (the chosen experts' weights are streamed once per tile), or those
+        of the tcgen05 product (bfloat16)."""
+        pairs = T * self.top
+        chosen = self.E * (1.0 - (1.0 - self.top / self.E) ** T) * self.F * self.hidden * (2 if self.glu else 1)
+        least = next(w for t, w in self.TC_MIN_CHOSEN_WEIGHTS if T >= t)
+        if dtype != torch.bfloat16 or not (pairs >= self.TC_MIN_ROWS_PER_EXPERT * self.E or chosen >= least):
+            return 16
+        return kernels.MOE_TC_ROWS[pairs >= self.TC_WIDE_ROWS_PER_EXPERT * self.E]
+
     def _forward_sparse(self, x, T, step):
         rt = self.rt
         E, F, D, top = self.E, self.F, self.hidden, self.top
         i32, f32 = torch.int32, torch.float32
         pairs, max_pairs = T * top, rt.max_tokens * top
-        # rows per tile: 16 (the chosen experts' weights are streamed once per tile), or those of the tcgen05 product (bfloat16)
         # the first product's rows an expert and its mode: with gates, gate and up rows in turn and the gated activation as
         # the epilogue
         F1, first = (2 * F, 2) if self.glu else (F, 0)
-        tc = rt.dtype == torch.bfloat16 and (pairs >= self.TC_MIN_ROWS_PER_EXPERT * E
-                                             or min(E, pairs) * F1 * D >= self.TC_MIN_CHOSEN_WEIGHTS)
-        BM = kernels.MOE_TC_ROWS[pairs >= self.TC_WIDE_ROWS_PER_EXPERT * E] if tc else 16
+        BM = self.tile_rows(T, rt.dtype)
+        tc = BM != 16
         n_tiles = kernels.moe_max_tiles(pairs, E, BM)
         cap = kernels.moe_max_tiles(max_pairs, E, 16)
         # (layers of other sizes have buffers of their own: a buffer that only long steps use must not grow once

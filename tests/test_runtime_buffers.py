@@ -58,6 +58,24 @@ def test_latent_portions_run_over_made_keys_where_that_is_shorter():
     assert not pays([32768, 32768, 128], [400] * 3, 32)                      # more rows than the buffers hold
 
 
+def test_experts_of_few_tokens_keep_the_tiles_that_suit_them():
+    """(hidden, F, experts, chosen, tokens): 16 rows a tile until the chosen weights fill the pairs of SMs."""
+    from ccinfer_b200.parts import MixtureOfExperts
+
+    def rows(D, F, E, top, T, dtype=torch.bfloat16):
+        return MixtureOfExperts(D, E, top, F, {"router": "r", "gate": "g{e}", "up": "u{e}", "down": "d{e}"},
+                                activation="swiglu").tile_rows(T, dtype)
+
+    for D, F, E, top, T in ((2048, 1024, 32, 4, 4), (2048, 768, 64, 8, 2), (4096, 1024, 8, 2, 4), (4096, 512, 16, 2, 6),
+                            (2048, 2048, 32, 4, 1), (1024, 512, 32, 4, 32)):
+        assert rows(D, F, E, top, T) == 16
+    for D, F, E, top, T in ((4096, 3072, 32, 4, 1), (2048, 2048, 32, 4, 2), (2048, 1024, 32, 4, 5), (4096, 1024, 8, 2, 6), (2048, 768, 64, 8, 3), (4096, 512, 16, 2, 8),
+                            (2048, 256, 64, 6, 8), (1024, 512, 32, 4, 64)):
+        assert rows(D, F, E, top, T) == 64
+        assert rows(D, F, E, top, T, torch.float32) == 16
+    assert rows(4096, 3072, 32, 4, 192) == 320
+
+
 def test_pages_leave_room_for_what_comes_late(monkeypatch):
     """With kv_memory_fraction the pools share what is free beside the buffers that a long prompt will ask for."""
     from types import SimpleNamespace

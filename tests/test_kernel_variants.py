@@ -546,6 +546,52 @@ def test_decode_of_ragged_contexts(rows, min_tiles):
         assert (out[r].double() - want).abs().max() <= 2.0 ** -7 * values.abs().max()
 
 
+# ten pieces of a row, whose results a thread of the merging block holds at once, eleven and more, which go through shared
+# memory; heads of one group and of two blocks of a group
+@pytest.mark.parametrize("fused", [False, True])
+@pytest.mark.parametrize("extras", [False, True])
+@pytest.mark.parametrize("nq,nkv", [(8, 2), (40, 2)])
+@pytest.mark.parametrize("ctx,pieces", [(2304, 9), (2560, 10), (2561, 11), (4160, 17), (8192, 32)])
+def test_decode_merges_pieces_of_a_long_context(ctx, pieces, nq, nkv, extras, fused):
+    """One request against float64, with a sink and a gate of the output's heads or without."""
+    k, g = _k(), _gen(ctx + nq + extras)
+    hd, page = 128, 16
+    n = ctx // page + 1
+
+    def rnd(*shape):
+        return torch.randn(shape, generator=g, device="cuda").to(torch.bfloat16)
+
+    table = torch.randperm(n, generator=torch.Generator().manual_seed(2)).to(torch.int32).view(1, n)
+    kc, vc, qkv = rnd(n, nkv, page, hd), rnd(n, nkv, page, hd), rnd(1, (nq + 2 * nkv) * hd)
+    q = qkv[:, :nq * hd].view(1, nq, hd).contiguous()
+    at = table[0].long().cuda()
+    keys, values = (t[at].transpose(1, 2).reshape(-1, nkv, hd)[:ctx].double() for t in (kc, vc))
+    if fused:   # (the row's own key and value come with it)
+        keys[-1], values[-1] = (qkv[0, (nq + i * nkv) * hd:(nq + (i + 1) * nkv) * hd].view(nkv, hd).double() for i in (0, 1))
+    sink, gate = (4 * torch.randn(nq, generator=g, device="cuda"), rnd(1, nq + 8)) if extras else (None, None)
+    splits, tiles, in_kernel, n_acc, n_ml = k.attention_decode_plan(1, nq, nkv, hd)
+    assert in_kernel and min(splits, -(-(-(-ctx // 64)) // tiles)) == pieces
+    i32 = dict(dtype=torch.int32, device="cuda")
+    acc, ml = torch.full((n_acc,), float("nan"), device="cuda"), torch.full((n_ml,), float("nan"), device="cuda")
+    count, status, out = torch.zeros(8192, **i32), torch.zeros(1, **i32), torch.full_like(q, float("nan"))
+    args = (kc, vc, out, acc, ml, torch.tensor([ctx - 1], **i32), torch.zeros(1, **i32), table.cuda(), 1, 0, 1)
+    more = dict(status=status, merge_counters=count, sink=sink, gate=gate, min_tiles=tiles)
+    if fused:
+        k.attention_decode_tma_fused(qkv, *args, nq, 0, hd ** -0.5, splits, None, None, 1e-6, torch.zeros(hd // 2, device="cuda"), **more)
+    else:
+        k.attention_decode_tma(q, *args, 0, hd ** -0.5, splits, **more)
+    assert int(status.item()) == 0 and int(count.abs().sum()) == 0
+    assert (torch.isfinite(ml[:2 * nq * splits].view(nq, splits, 2)).all(-1).sum(-1) == pieces).all()
+    s = torch.einsum("hd,jhd->hj", q[0].double(), keys.repeat_interleave(nq // nkv, 1)) * hd ** -0.5
+    if extras:
+        s = torch.cat([s, sink.double()[:, None]], 1)
+    want = torch.einsum("hj,jhd->hd", torch.softmax(s, -1)[:, :ctx], values.repeat_interleave(nq // nkv, 1))
+    if extras:
+        want *= torch.sigmoid(gate[0, :nq].double())[:, None]
+    # (weights are rounded to bfloat16 for their product, results once more)
+    assert (out[0].double() - want).abs().max() <= 2.0 ** -7 * values.abs().max()
+
+
 # rows whose lengths are alike stay in one piece (or two: 16 rows), a long one among short ones is cut; 40 rows: always
 @pytest.mark.parametrize("rows,even_pieces,ragged_pieces", [(16, 2, 4), (24, 1, 3), (36, 1, 3), (40, 3, 3)])
 @pytest.mark.parametrize("window", [0, 3000])

@@ -692,8 +692,8 @@ bool pieces_ok(const RowPieces& p) {
 // A row's key range is cut into at most num_splits pieces of at least min_tiles tiles of 64 keys; with ragged_percent > 0 and
 // rows whose longest is less than so many hundredths of their mean, into at most even_splits of at least even_tiles.
 // `counters` (optional): n_rows * kv_heads * ceil(group / 16) ints that are zero before the first launch and
-// are left zero; with them the splits are merged by the attention kernel itself, without them by a second
-// kernel.
+// are left zero; with them the splits are merged by the attention kernel itself, without them (a caller of this
+// interface that has none; the package's own parts always have) by a second kernel.
 CCB_API int ccb_attention_decode_tma(const void* q, const void* k_cache, const void* v_cache, void* out,
                                      float* part_acc, float* part_ml, const int* positions,
                                      const int* entry_of_token, const int* block_table, int bt_stride,

@@ -60,4 +60,14 @@ template <int HD> __device__ __forceinline__ int swz(int row, int chunk) {
   return row * HD + ((chunk ^ (row & 7)) << 3);
 }
 
+// Finite, also as two bfloat16 (the largest floats round to infinity).
+__device__ __forceinline__ bool is_finite(float x) { return fabsf(x) < 3.38e38f; }
+// The largest magnitude of m, x and y, NaN if there is one: is_finite of it is that of all of them, at half an instruction a
+// number.
+__device__ __forceinline__ float largest(float m, float x, float y) {
+  float d;
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(m), "f"(x), "f"(y));
+  return d;
+}
+
 }  // namespace ccb

@@ -5,7 +5,6 @@
 // an expert with 260 rows costs 288 columns, not three tiles of 128 rows, and one with eight reads its weights past 32
 // columns.  A cluster of two blocks works on a tile (tcgen05 cta_group::2, as gemm_tc_pair.cu: each block holds 128 of the
 // weight rows and half of the tokens), one cluster per pair of SMs walks over (token tile, 256 weight rows), weight rows
-// weight rows and half of the tokens), one cluster per pair of SMs walks over (token tile, 256 weight rows), weight rows
 // fastest, so that the clusters running at one time share a few tokens in L2 and read every weight once.  The ring of
 // stages (64 k) and the two accumulators of 256 columns run on from tile to tile.  Weights and tokens have a producer warp
 // each: one thread for both set the pace (one instruction more in its loop, a copy to L2 ahead of the ring, made 64 tokens

@@ -76,6 +76,12 @@ class SelectiveStateSpace(Mixer):
         self.norm_w = fetch(n["norm"]).float().contiguous()
         self.w_o = fetch(n["o"])
 
+    def runs_in_chunks(self, conv, longest: int, units: int) -> bool:
+        """As ``kernels.ssm_chunks_fits``; the kernel that makes the chunks' rows has 16-byte loads only, so that weights or a
+        convolution state from elsewhere in somebody's buffer go token by token."""
+        return (kernels.ssm_chunks_fits(self.rt.dtype, self.N, self.P, longest, units)
+                and not (self.conv_w.data_ptr() | self.conv_b.data_ptr() | conv.data_ptr()) & 15)
+
     def forward(self, x, step, cache, state):
         rt = self.rt
         x = rt.rows(x)
@@ -92,7 +98,7 @@ class SelectiveStateSpace(Mixer):
         S, conv = state["S"], state["conv"]
         # portions of prompts go in chunks on tensor cores (a step lists its single tokens first: they, and short portions,
         # go token by token).  The chunks' rows take the places of those that the recurrence would read.
-        chunks = kernels.ssm_chunks_fits(rt.dtype, N, P, step.max_q_len, (T - step.n_single) * H)
+        chunks = self.runs_in_chunks(conv, step.max_q_len, (T - step.n_single) * H)
         n1 = step.n_single if chunks else step.n_entries
         chunk = None
         if step.n_entries > n1:

@@ -44,6 +44,28 @@ def test_portions_run_in_chunks_where_the_layer_gains():
     assert not kernels.ssm_chunks_fits(bf, 96, 64, 512, 1 << 20) and not kernels.ssm_chunks_fits(bf, 64, 24, 512, 1 << 20)
 
 
+@pytest.mark.parametrize("moved,taps", [(None, 4), ("conv_bias", 4), ("conv", 1), ("state", 4)])
+def test_state_space_rows_for_chunks_start_on_16_bytes(moved, taps):
+    """The kernel that makes them takes nothing else; weights and states from elsewhere in a buffer go token by token."""
+    from types import SimpleNamespace
+
+    from ccinfer_b200.parts import SelectiveStateSpace
+    part = SelectiveStateSpace(64, 4, 32, 64, 2, taps, 2, 1e-5,
+                               {k: k for k in ("in", "conv", "conv_bias", "dt_bias", "A_log", "D", "norm", "o")})
+    shapes = {s.name: s.shape for s in part.tensor_specs()}
+
+    def place(name, shape, dtype):
+        n = torch.Size(shape).numel()
+        return torch.zeros(n + 1, dtype=dtype)[1:].view(shape) if name == moved else torch.zeros(shape, dtype=dtype)
+
+    bf = torch.bfloat16
+    part.bind(SimpleNamespace(dtype=bf, device="cpu"), lambda n: place(n, shapes[n], bf if n in ("in", "o") else torch.float32))
+    conv = place("state", (3, max(taps - 1, 1), part.conv_width), bf)
+    assert kernels.ssm_chunks_fits(bf, 64, 32, 200, 4 * 200)
+    assert part.runs_in_chunks(conv, 200, 4 * 200) == (moved is None)
+    assert not part.runs_in_chunks(conv, 20, 4 * 20)
+
+
 def test_latent_portions_run_over_made_keys_where_that_is_shorter():
     """(rows seen, tokens brought by each portion, heads of 192 columns)"""
     def pays(rows, tokens, heads):

@@ -162,6 +162,45 @@ def test_state_space_recurrence_in_chunks(H, G, N, P):
         assert (state[slot].double() - after).abs().max() <= 2.0 ** -14 * after.abs().max()
 
 
+# what the rows of chunks are made from, on no 16 bytes: the bias of the convolution, its one tap's weights, its state
+@pytest.mark.parametrize("moved,taps", [("conv_bias", 4), ("conv", 1), ("state", 4)])
+def test_state_space_portions_whose_weights_or_state_start_anywhere(moved, taps):
+    """The layer takes them token by token.  Against the layer that has them on 16 bytes: rows between differ by their last
+    bfloat16 place at most, 2^-8, and so do the results; the memory by what chunks leave, as above."""
+    from ccinfer_b200.engine.runtime import Runtime
+    from ccinfer_b200.parts import SelectiveStateSpace
+    D, H, P, N, G = 64, 4, 32, 64, 2
+    lens, g = [1, 170, 200], _gen(taps)
+    part = SelectiveStateSpace(D, H, P, N, G, taps, 2, 1e-5, {k: k for k in ("in", "conv", "conv_bias", "dt_bias", "A_log", "D", "norm", "o")})
+    w = {s.name: torch.randn(s.shape, generator=g, device="cuda") * (0.125 if len(s.shape) == 2 else 0.5) for s in part.tensor_specs()}
+    w = {n: t.to(torch.bfloat16) if n in ("in", "o") else t for n, t in w.items()}
+    x = torch.randn((sum(lens), D), generator=g, device="cuda").to(torch.bfloat16)
+    memory = torch.randn((len(lens), H, P, N), generator=g, device="cuda")
+    ring = torch.randn((len(lens), max(taps - 1, 1), part.conv_width), generator=g, device="cuda").to(torch.bfloat16)
+
+    def elsewhere(t, name):
+        if name != moved:
+            return t.clone()
+        out = torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")[1:].view(t.shape)
+        out.copy_(t)
+        assert out.data_ptr() & 15
+        return out
+
+    def run(place):
+        rt = Runtime("cuda:0", torch.bfloat16, sum(lens), len(lens))
+        part.bind(rt, lambda n: place(w[n], n))
+        state = {"S": memory.clone(), "conv": place(ring, "state")}
+        step = _Step([(3, n) for n in lens], 16, 1).step
+        out = part.forward(x, step, None, state).double()
+        rt.check_status()
+        return out, state["S"].double(), state["conv"].clone()
+
+    (want, after, rows), (got, got_after, got_rows) = run(lambda t, n: t.clone()), run(elsewhere)
+    assert (got - want).norm() <= 2.0 ** -8 * want.norm()
+    assert (got_after - after).abs().max() <= 2.0 ** -14 * after.abs().max()
+    assert torch.equal(got_rows, rows)
+
+
 # steps and rates up to where a token keeps nothing; three such tokens before slow ones; steps of nothing; whole chunks of both
 @pytest.mark.parametrize("decay", ["strong", "then slow", "extreme"])
 @pytest.mark.parametrize("H,G,N,P", [(4, 2, 128, 64), (2, 1, 64, 48), (40, 1, 64, 128)])

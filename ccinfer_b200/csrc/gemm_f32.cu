@@ -13,15 +13,17 @@
 //   rows   M <= 16: the product is a stream of W.  A block takes 16 rows of W and its eight half-warps a segment
 //          each, so that 64 blocks already keep eight streams an SM going: cp.async into a ring that each warp owns,
 //          a lane per row of W, A's values broadcast from the same ring.
-//   tiles  M > 16: BM x 128 tiles, 8 x 8 places a thread whatever BM is (six 16-byte reads of shared memory for 64
-//          multiply-adds; with 4 x 8 places the reads set the pace), two multiply-adds an instruction (fma.rn.f32x2).
-//          Where the tiles do not fill the machine a cluster of eight blocks takes a tile, a segment each, and adds up
-//          through distributed shared memory.
+//   tiles  M > 16: tiles of 12 to 128 rows x 128 columns, two multiply-adds an instruction (fma.rn.f32x2); `choose_tiles`
+//          picks their height, so that few rows of a tile are empty and few SMs idle in the last round.  Where the tiles do
+//          not fill the machine a cluster of eight blocks takes a tile, a segment each, and adds up through distributed
+//          shared memory.
 // What bounds them: the rows kernel the stream of W (2 x 16,384 x 2,048: 34 us, 3.9 TB/s; 2 x 32,000 x 2,048: 57 us, 4.6
-// TB/s) until many rows make it the reads of A (16 x 16,384 x 2,048: 66 us); the tiles kernel the multiply-adds (300 x
-// 16,384 x 2,048: 515 us, 39 TFLOP/s; 1,024 rows: 48 TFLOP/s of 72).  One tile kernel for every M, without segments or
-// pipelining, took 562 us on average for the products of 2-3 rows of a model of width 2,048 and 771 us for those of some
-// 200 rows; a call of that model (two prompts of some 100 tokens, three more tokens each) went from 22.7 to 3.0 ms.
+// TB/s) until many rows make it the reads of A (16 x 16,384 x 2,048: 66 us); the tiles kernel the multiply-adds, of which
+// registers alone reach 65 TFLOP/s, with reads of shared memory beside them.  us, tiles of 32, 64 or 128 rows with 8 x 8 places
+// a thread, one block an SM / so: 17 x 16,384 x 2,048 77 / 60, 64 x 4,096 x 2,048 35 / 35, 100 x 16,384 x 2,048 267 / 187,
+// 210 x 2,048 x 8,192 307 / 174, 210 x 16,384 x 2,048 524 / 349 (40 TFLOP/s), 300 x 16,384 x 2,048 511 / 501, 2,048 x 4,096 x
+// 4,096 1,593 / 1,452 (47).  Sums of even and of odd k side by side (no element stored by itself, eight columns a thread) took
+// 419 us for 210 x 16,384 x 2,048.
 #include "cluster_common.cuh"
 #include "mma_common.cuh"
 
@@ -153,19 +155,36 @@ gemm_f32_rows_kernel(float* __restrict__ C, const float* __restrict__ A, const f
 }
 
 // ---------------------------------------------------------------------------------------------
+// A block: a tile of WR x WC warps, 128 columns; a thread TM rows x TN columns, two columns a multiply-add.  What it reads from
+// shared memory comes back at 128 bytes a cycle and SM whether lanes read the same or not, so TM + TN cycles a k and warp stand
+// against TM TN / 4 of multiply-adds: sixteen columns a thread where there are rows enough for four warps below one another
+// (eight left the reads the bound), eight and warps side by side for fewer rows.  Several blocks an SM: one's first loads and
+// last exchange run under another's multiply-adds.
 constexpr int kTileK = 16;
 constexpr int kTileN = 128;
-constexpr int TM = 8;            // rows a thread
-constexpr int kWPitch = kTileN + 4;
+constexpr int kTilePitch = kTileN + 4;   // floats from k to k
+constexpr int kTileMinRows = 3, kTileMaxRows = 8;   // TM
 
-template <int BM> struct TileShape {
-  static constexpr int kThreads = 2 * BM;
-  static constexpr int kBlocks = BM == 128 ? 1 : BM == 64 ? 3 : 6;   // an SM, so that no register spills
-  static constexpr int kPitch = BM + 4;
-  static constexpr int kA = kTileK * kPitch;                       // floats of a stage
-  static constexpr int kW = kTileK * kWPitch;
-  static constexpr int kTotals = BM * kTileN;                      // a segment's tile, or the total so far
-  static constexpr int kBytes = (2 * (kA + kW) + kTotals) * 4;
+template <int TM_, int TN_, int WR_, int WC_> struct TileShape {
+  static constexpr int TM = TM_, TN = TN_, WR = WR_, WC = WC_;
+  static_assert(WC * 8 * TN == kTileN, "128 columns");
+  static constexpr int kThreads = 32 * WR * WC;
+  static constexpr int kBlocks = TN == 16 ? 2 : WR == 2 ? 3 : 5;   // an SM
+  static constexpr int kWarpRows = 4 * TM, kRows = WR * kWarpRows;
+  static constexpr int kPlaces = TM > 4 ? 32 : 16;                 // of a warp's rows in shared memory
+  static constexpr int kPitchA = WR * kPlaces + 4;
+  static constexpr int kStage = kTileK * (kPitchA + kTilePitch);   // floats
+  static constexpr int kTotals = kRows * kTileN;                   // a segment's tile, or the total so far
+  static constexpr int kQuads = TM * TN / 4;                       // fours of sums a thread has
+  // where a warp's row lies: four to a lane's quarter first, then the quarter's others from place 16 on
+  static __device__ __forceinline__ int place(int row) {
+    constexpr int kFirst = TM < 4 ? TM : 4, kRest = TM > 4 ? TM - 4 : 1;
+    if (row < 4 * kFirst) return row / kFirst * 4 + row % kFirst;
+    return 16 + (row - 16) / kRest * 4 + (row - 16) % kRest;
+  }
+  static constexpr int bytes(bool cluster) {   // (a cluster's block has one segment: its sums take the stages' place)
+    return 4 * (cluster ? (2 * kStage > kTotals ? 2 * kStage : kTotals) : 2 * kStage + kTotals);
+  }
 };
 
 __device__ __forceinline__ unsigned long long twice(float x) {
@@ -179,28 +198,29 @@ __device__ __forceinline__ void fma2(unsigned long long& c, unsigned long long a
 }
 
 // grid.x: column tiles x cluster blocks (1 or 8), grid.y: row tiles, grid.z: products of a batch
-template <int BM, bool CLUSTER>
-__global__ void __launch_bounds__(TileShape<BM>::kThreads, TileShape<BM>::kBlocks)
+template <class Sh, bool CLUSTER>
+__global__ void __launch_bounds__(Sh::kThreads, Sh::kBlocks)
 gemm_f32_tiles_kernel(float* __restrict__ C, const float* __restrict__ A, const float* __restrict__ W, int M, int N, int K,
                       int lda, int ldw, int ldc, long long sa, long long sw, long long sc, int vec_a, int vec_w) {
   ccb::pdl_begin();
-  using Sh = TileShape<BM>;
-  constexpr int kTileThreads = Sh::kThreads;
+  constexpr int TM = Sh::TM, TN = Sh::TN, kThreads = Sh::kThreads;
   extern __shared__ __align__(16) float smem[];
-  float* a_s = smem;                    // [2][kTileK][kPitch]
-  float* w_s = smem + 2 * Sh::kA;       // [2][kTileK][kWPitch]
-  float4* totals = reinterpret_cast<float4*>(smem + 2 * (Sh::kA + Sh::kW));   // [2 TM][threads]
+  float4* totals = reinterpret_cast<float4*>(smem + (CLUSTER ? 0 : 2 * Sh::kStage));   // [kQuads][threads]
   C += (size_t)blockIdx.z * sc;
   A += (size_t)blockIdx.z * sa;
   W += (size_t)blockIdx.z * sw;
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+  const int tid = threadIdx.x, wr = (tid >> 5) % Sh::WR, wc = (tid >> 5) / Sh::WR, ty = (tid >> 3) & 3, tx = tid & 7;
   const int rank = CLUSTER ? blockIdx.x % kSegments : 0;
-  const int n0 = (CLUSTER ? blockIdx.x / kSegments : blockIdx.x) * kTileN, m0 = blockIdx.y * BM;
+  const int n0 = (CLUSTER ? blockIdx.x / kSegments : blockIdx.x) * kTileN, m0 = blockIdx.y * Sh::kRows;
   const int seg = segment_of(K);
   const int k_begin = rank * seg, k_end = min(K, CLUSTER ? k_begin + seg : K);
-  constexpr int LA = BM * 4 / kTileThreads, LW = kTileN * 4 / kTileThreads;
-  float4 ra[LA], rw[LW];
+  const int steps = k_begin < k_end ? (k_end - k_begin + kTileK - 1) / kTileK : 0;
 
+  // A thread takes four k of some rows, to registers and from there to shared memory; for the second eight k the rows lie
+  // with eights exchanged, so that a warp's stores fall into different banks.
+  const int q4 = 4 * (tid & 3), cr = tid >> 2, flip = q4 & 8;
+  constexpr int kPass = kThreads / 4, LA = (Sh::kRows + kPass - 1) / kPass, LW = kTileN / kPass;
+  float4 ra[LA], rw[LW];
   auto piece = [&](const float* base, int ld, int row, int rows, int k, int vec) {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (row < rows) {
@@ -216,112 +236,106 @@ gemm_f32_tiles_kernel(float* __restrict__ C, const float* __restrict__ A, const 
     }
     return v;
   };
-  auto load = [&](int k0) {
+  auto load = [&](int step) {
+    const int k = k_begin + step * kTileK + q4;
 #pragma unroll
-    for (int i = 0; i < LA; ++i) {
-      const int idx = tid + kTileThreads * i;
-      ra[i] = piece(A, lda, m0 + (idx >> 2), M, k0 + 4 * (idx & 3), vec_a);
-    }
+    for (int i = 0; i < LA; ++i)
+      if (Sh::kRows % kPass == 0 || cr + kPass * i < Sh::kRows) ra[i] = piece(A, lda, m0 + cr + kPass * i, M, k, vec_a);
 #pragma unroll
-    for (int i = 0; i < LW; ++i) {
-      const int idx = tid + kTileThreads * i;
-      rw[i] = piece(W, ldw, n0 + (idx >> 2), N, k0 + 4 * (idx & 3), vec_w);
-    }
+    for (int i = 0; i < LW; ++i) rw[i] = piece(W, ldw, n0 + cr + kPass * i, N, k, vec_w);
   };
-  auto store = [&](int st) {
-    float* as = a_s + st * Sh::kA;
-    float* ws = w_s + st * Sh::kW;
+  auto put = [&](float* to, int pitch, float4 v) {
+    to[0] = v.x;
+    to[pitch] = v.y;
+    to[2 * pitch] = v.z;
+    to[3 * pitch] = v.w;
+  };
+  auto store = [&](int step) {
+    float* a_s = smem + (step & 1) * Sh::kStage + q4 * Sh::kPitchA;
+    float* w_s = smem + (step & 1) * Sh::kStage + kTileK * Sh::kPitchA + q4 * kTilePitch;
 #pragma unroll
     for (int i = 0; i < LA; ++i) {
-      const int idx = tid + kTileThreads * i, row = idx >> 2, k = 4 * (idx & 3);
-      as[(k + 0) * Sh::kPitch + row] = ra[i].x;
-      as[(k + 1) * Sh::kPitch + row] = ra[i].y;
-      as[(k + 2) * Sh::kPitch + row] = ra[i].z;
-      as[(k + 3) * Sh::kPitch + row] = ra[i].w;
+      const int row = cr + kPass * i;
+      if (Sh::kRows % kPass == 0 || row < Sh::kRows)
+        put(a_s + row / Sh::kWarpRows * Sh::kPlaces + (Sh::place(row % Sh::kWarpRows) ^ flip), Sh::kPitchA, ra[i]);
     }
 #pragma unroll
-    for (int i = 0; i < LW; ++i) {
-      const int idx = tid + kTileThreads * i, row = idx >> 2, k = 4 * (idx & 3);
-      ws[(k + 0) * kWPitch + row] = rw[i].x;
-      ws[(k + 1) * kWPitch + row] = rw[i].y;
-      ws[(k + 2) * kWPitch + row] = rw[i].z;
-      ws[(k + 3) * kWPitch + row] = rw[i].w;
-    }
+    for (int i = 0; i < LW; ++i) put(w_s + ((cr + kPass * i) ^ flip), kTilePitch, rw[i]);
   };
 
-  // columns tx * 4 .. + 3 (pairs 0, 1) and 64 + tx * 4 .. + 3 (pairs 2, 3) of rows ty * TM ..
-  unsigned long long acc[TM][4];
+  // columns col0 + 32 j .. + 3 (pairs 2 j, 2 j + 1)
+  const int col0 = wc * 8 * TN + 4 * tx;
+  unsigned long long acc[TM][TN / 2];
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+    for (int j = 0; j < TN / 2; ++j) acc[i][j] = 0ull;
 
   // the sums of the segment that has ended, into (or onto) the totals; a thread only touches its own places
   auto fold = [&](bool first) {
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        float4& t = totals[(2 * i + h) * kTileThreads + tid];
-        const float2 lo = *reinterpret_cast<const float2*>(&acc[i][2 * h]), hi = *reinterpret_cast<const float2*>(&acc[i][2 * h + 1]);
+      for (int j = 0; j < TN / 4; ++j) {
+        float4& t = totals[(TN / 4 * i + j) * kThreads + tid];
+        const float2 lo = *reinterpret_cast<const float2*>(&acc[i][2 * j]), hi = *reinterpret_cast<const float2*>(&acc[i][2 * j + 1]);
         float4 v = make_float4(lo.x, lo.y, hi.x, hi.y);
         if (!first) {
           const float4 o = t;
           v = make_float4(o.x + v.x, o.y + v.y, o.z + v.z, o.w + v.w);
         }
         t = v;
-        acc[i][2 * h] = acc[i][2 * h + 1] = 0ull;
+        acc[i][2 * j] = acc[i][2 * j + 1] = 0ull;
       }
   };
 
-  bool first = true;
-  int st = 0, left = seg;
-  if (k_begin < k_end) {
-    load(k_begin);
+  if (steps > 0) {
+    load(0);
     store(0);
   }
   __syncthreads();
-  for (int k0 = k_begin; k0 < k_end; k0 += kTileK) {
-    const bool more = k0 + kTileK < k_end;
-    if (more) load(k0 + kTileK);
-    const float* as = a_s + st * Sh::kA + TM * ty;
-    const float* ws = w_s + st * Sh::kW + 4 * tx;
+  bool first = true;
+  int left = seg;
+  for (int step = 0; step < steps; ++step) {
+    if (step + 1 < steps) load(step + 1);
+    const float* stage = smem + (step & 1) * Sh::kStage;
 #pragma unroll
     for (int k = 0; k < kTileK; ++k) {
-      unsigned long long a[TM], b[4];
+      const float* a_s = stage + wr * Sh::kPlaces + ((4 * ty) ^ (k & 8)) + k * Sh::kPitchA;
+      const float* w_s = stage + kTileK * Sh::kPitchA + (col0 ^ (k & 8)) + k * kTilePitch;
+      unsigned long long b[TN / 2];
 #pragma unroll
-      for (int i = 0; i < TM; i += 4) {
-        const float4 v = *reinterpret_cast<const float4*>(as + k * Sh::kPitch + i);
-        a[i] = twice(v.x);
-        a[i + 1] = twice(v.y);
-        a[i + 2] = twice(v.z);
-        a[i + 3] = twice(v.w);
+      for (int j = 0; j < TN / 4; ++j) {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(w_s + 32 * j);
+        b[2 * j] = v.x;
+        b[2 * j + 1] = v.y;
       }
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(ws + k * kWPitch + 64 * h);
-        b[2 * h] = v.x;
-        b[2 * h + 1] = v.y;
+      for (int g = 0; g < (TM + 3) / 4; ++g) {
+        const float4 v = *reinterpret_cast<const float4*>(a_s + 16 * g);
+        const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 4 * g; i < TM && i < 4 * g + 4; ++i) {
+          const unsigned long long a = twice(x[i & 3]);
+#pragma unroll
+          for (int j = 0; j < TN / 2; ++j) fma2(acc[i][j], a, b[j]);
+        }
       }
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) fma2(acc[i][j], a[i], b[j]);
     }
-    if (more) store(st ^ 1);
-    __syncthreads();
-    st ^= 1;
+    if (step + 1 < steps) store(step + 1);
+    __syncthreads();   // the next stage is there, and everybody has read this one
     left -= kTileK;
-    if (left == 0 || !more) {
+    if (left == 0 || step + 1 == steps) {
       fold(first);
       first = false;
       left = seg;
     }
   }
-  if (CLUSTER && k_begin >= k_end) fold(true);   // a segment past K: zeros
+  if (CLUSTER && steps == 0) fold(true);   // a segment past K: zeros
 
-  auto write = [&](int q, float4 v) {   // place q of this thread's: row q / 2, column half q % 2
-    const int gm = m0 + ty * TM + (q >> 1), gn = n0 + (q & 1) * 64 + tx * 4;
+  auto write = [&](int q, float4 v) {   // the thread's four q: a row, four neighbouring columns
+    const int i = q / (TN / 4), row = i < 4 ? ty * (TM < 4 ? TM : 4) + i : 16 + ty * (TM - 4) + (i - 4);
+    const int gm = m0 + wr * Sh::kWarpRows + row, gn = n0 + col0 + 32 * (q % (TN / 4));
     if (gm >= M) return;
     float* dst = C + (size_t)gm * ldc + gn;
     if (gn < N) dst[0] = v.x;
@@ -333,11 +347,11 @@ gemm_f32_tiles_kernel(float* __restrict__ C, const float* __restrict__ A, const 
     namespace cg = cooperative_groups;
     const cg::cluster_group cluster = cg::this_cluster();
     cluster.sync();
-    for (int q = rank; q < 2 * TM; q += kSegments) {
-      float4 v = cluster.map_shared_rank(totals, 0)[q * kTileThreads + tid];
+    for (int q = rank; q < Sh::kQuads; q += kSegments) {
+      float4 v = cluster.map_shared_rank(totals, 0)[q * kThreads + tid];
       float4 o[kSegments - 1];
 #pragma unroll
-      for (int s = 1; s < kSegments; ++s) o[s - 1] = cluster.map_shared_rank(totals, s)[q * kTileThreads + tid];
+      for (int s = 1; s < kSegments; ++s) o[s - 1] = cluster.map_shared_rank(totals, s)[q * kThreads + tid];
 #pragma unroll
       for (int s = 0; s < kSegments - 1; ++s) v = make_float4(v.x + o[s].x, v.y + o[s].y, v.z + o[s].z, v.w + o[s].w);
       write(q, v);
@@ -345,7 +359,7 @@ gemm_f32_tiles_kernel(float* __restrict__ C, const float* __restrict__ A, const 
     cluster.sync();   // nobody leaves while its sums are read
   } else {
 #pragma unroll
-    for (int q = 0; q < 2 * TM; ++q) write(q, totals[q * kTileThreads + tid]);
+    for (int q = 0; q < Sh::kQuads; ++q) write(q, totals[q * kThreads + tid]);
   }
 }
 
@@ -367,25 +381,69 @@ template <int MR> int rows_go(const F32Product& p, int vec, cudaStream_t stream)
   return ccb_launch_status();
 }
 
-template <int BM> int tiles_go(const F32Product& p, int vec_a, int vec_w, cudaStream_t stream) {
-  const int gx = (p.N + kTileN - 1) / kTileN, gy = (p.M + BM - 1) / BM;
-  // A block an SM computes as fast as two do (the multiply-adds are the bound), so tiles run in rounds of 148.  A
-  // cluster's rounds are an eighth as long: it is taken where the tiles fill fewer than two rounds, and where a segment
-  // is long enough to pay for the exchange.
-  const long long tiles = (long long)gx * gy * p.batch;
-  const bool cluster = tiles < 2 * 148 && p.K >= 512;
-  constexpr int bytes = TileShape<BM>::kBytes;
-  auto kernel = cluster ? gemm_f32_tiles_kernel<BM, true> : gemm_f32_tiles_kernel<BM, false>;
+template <class Sh> int tiles_go(const F32Product& p, int vec_a, int vec_w, bool cluster, cudaStream_t stream) {
+  const int bytes = Sh::bytes(cluster);
+  const int gx = (p.N + kTileN - 1) / kTileN, gy = (p.M + Sh::kRows - 1) / Sh::kRows;
+  auto kernel = cluster ? gemm_f32_tiles_kernel<Sh, true> : gemm_f32_tiles_kernel<Sh, false>;
   static std::atomic<unsigned long long> done[2];
   const int rc = ccb_allow_smem(kernel, bytes, done[cluster]);
   if (rc != 0) return rc;
   if (cluster)
-    ccb_launch_cluster(false, kSegments, kernel, dim3(gx * kSegments, gy, p.batch), TileShape<BM>::kThreads, bytes, stream, p.C, p.A, p.W,
+    ccb_launch_cluster(false, kSegments, kernel, dim3(gx * kSegments, gy, p.batch), Sh::kThreads, bytes, stream, p.C, p.A, p.W,
                        p.M, p.N, p.K, p.lda, p.ldw, p.ldc, p.sa, p.sw, p.sc, vec_a, vec_w);
   else
-    ccb_launch(kernel, dim3(gx, gy, p.batch), TileShape<BM>::kThreads, bytes, stream, p.C, p.A, p.W, p.M, p.N, p.K, p.lda, p.ldw, p.ldc,
+    ccb_launch(kernel, dim3(gx, gy, p.batch), Sh::kThreads, bytes, stream, p.C, p.A, p.W, p.M, p.N, p.K, p.lda, p.ldw, p.ldc,
                p.sa, p.sw, p.sc, vec_a, vec_w);
   return ccb_launch_status();
+}
+
+// The rows of a tile and whether a cluster shares it, by the cycles that the busiest SM would need: its blocks go round by
+// round, a k of a block costs an SM its multiply-adds or its reads and stores of shared memory, whichever is more, and a
+// round no less than one thread's chain of instructions; a block multiplies some 16 k more than it has, and not every SM can
+// be part of a cluster.  The constants are fitted to 66 shapes of 17 to 2,048 rows, each timed with every tile: what is
+// chosen takes 3 per cent longer than the best on average (5 and 9 of 66 more than that beyond 5 and 10 per cent).
+struct TileChoice {
+  int family, tm;   // family 0: 16 columns a thread, 4 x 1 warps; 1: 8, 2 x 2; 2: 8, 1 x 2
+  bool cluster;
+};
+TileChoice choose_tiles(int M, int N, int K, int batch) {
+  TileChoice best{0, kTileMaxRows, false};
+  double least = 0;
+  for (int family = 0; family < 3; ++family) {
+    const int tn = family == 0 ? 16 : 8, wr = 4 >> family, warps = family == 2 ? 2 : 4, blocks = family == 0 ? 2 : family == 1 ? 3 : 5;
+    for (int tm = kTileMaxRows; tm >= kTileMinRows; --tm) {
+      const int rows = 4 * wr * tm;
+      const double adds = warps * tm * tn / 4., moves = warps * (0.8 * tm + tn) + (rows + kTileN) / 20.;
+      const double cost = adds > moves ? adds : moves, chain = 1.2 * tm * tn + 80;
+      const long long tiles = (long long)((N + kTileN - 1) / kTileN) * ((M + rows - 1) / rows) * batch;
+      for (int cluster = 0; cluster < 2; ++cluster) {
+        const long long units = cluster ? tiles * kSegments : tiles, sms = cluster ? 136 : 148;
+        const long long full = units / (sms * blocks), rest = (units % (sms * blocks) + sms - 1) / sms;
+        double cycles = full * (blocks * cost > chain ? blocks * cost : chain);
+        if (rest) cycles += rest * cost > chain ? rest * cost : chain;
+        cycles = cycles * ((cluster ? segment_of(K) : K) + 16) + (cluster ? 2000 : 0);
+        if (least == 0 || cycles < least) least = cycles, best = {family, tm, cluster != 0};
+      }
+    }
+  }
+  return best;
+}
+
+template <int TM> int tiles_of(const F32Product& p, int vec_a, int vec_w, const TileChoice& t, cudaStream_t stream) {
+  if (t.family == 0) return tiles_go<TileShape<TM, 16, 4, 1>>(p, vec_a, vec_w, t.cluster, stream);
+  if (t.family == 1) return tiles_go<TileShape<TM, 8, 2, 2>>(p, vec_a, vec_w, t.cluster, stream);
+  return tiles_go<TileShape<TM, 8, 1, 2>>(p, vec_a, vec_w, t.cluster, stream);
+}
+
+int tiles_any(const F32Product& p, int vec_a, int vec_w, const TileChoice& t, cudaStream_t stream) {
+  switch (t.tm) {
+    case 3: return tiles_of<3>(p, vec_a, vec_w, t, stream);
+    case 4: return tiles_of<4>(p, vec_a, vec_w, t, stream);
+    case 5: return tiles_of<5>(p, vec_a, vec_w, t, stream);
+    case 6: return tiles_of<6>(p, vec_a, vec_w, t, stream);
+    case 7: return tiles_of<7>(p, vec_a, vec_w, t, stream);
+    default: return tiles_of<8>(p, vec_a, vec_w, t, stream);
+  }
 }
 
 int gemm_f32_launch(const F32Product& p, cudaStream_t stream) {
@@ -399,11 +457,13 @@ int gemm_f32_launch(const F32Product& p, cudaStream_t stream) {
   if (p.M <= 4) return rows_go<4>(p, vec_a && vec_w, stream);
   if (p.M <= 8) return rows_go<8>(p, vec_a && vec_w, stream);
   if (p.M <= 16) return rows_go<16>(p, vec_a && vec_w, stream);
-  if (p.M <= 32) return tiles_go<32>(p, vec_a, vec_w, stream);
-  // tiles of 64 rows where 128 would leave more than an eighth of the rows empty that 64 does not
-  const int r64 = (p.M + 63) / 64 * 64, r128 = (p.M + 127) / 128 * 128;
-  if (8 * (r128 - r64) > r128) return tiles_go<64>(p, vec_a, vec_w, stream);
-  return tiles_go<128>(p, vec_a, vec_w, stream);
+  constexpr int kMost = 65535 * 4 * kTileMinRows;   // rows of a launch, whatever the tile's height
+  for (F32Product q = p;; q.M -= kMost, q.A += (size_t)kMost * q.lda, q.C += (size_t)kMost * q.ldc) {
+    F32Product part = q;
+    part.M = q.M < kMost ? q.M : kMost;
+    const int rc = tiles_any(part, vec_a, vec_w, choose_tiles(part.M, part.N, part.K, part.batch), stream);
+    if (rc != 0 || q.M <= kMost) return rc;
+  }
 }
 
 }  // namespace

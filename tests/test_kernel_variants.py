@@ -50,6 +50,24 @@ def test_float_product_of_every_shape_is_one_order_of_sums(M, N, K, pad, batch):
         assert torch.equal(c1, c[0, M - n:])
 
 
+# every height of a tile, whole and with rows left over, whole tiles and shared ones
+@pytest.mark.parametrize("M", [20, 21, 23, 29, 31, 41, 47, 50, 57, 63, 77, 79, 90, 96, 101, 107, 112, 125, 140, 175, 223])
+@pytest.mark.parametrize("N,K", [(200, 1030), (3001, 96), (640, 2048)])
+def test_float_product_of_every_tile_height(M, N, K):
+    """As above, beside the rows by themselves: sixteen at a time have a kernel without tiles."""
+    g = _gen(M + 7 * N + 13 * K)
+    a, w = torch.randn((M, K), generator=g, device="cuda"), torch.randn((N, K), generator=g, device="cuda")
+    k = _k()
+    c = torch.full((M, N), float("nan"), device="cuda")
+    k.gemm_f32(c, a, w)
+    ref, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    assert ((c.double() - ref).abs() <= (K / 8 + 8) * 2.0 ** -24 * size).all()
+    for r in range(0, M, 16):
+        c1 = torch.empty((min(16, M - r), N), device="cuda")
+        k.gemm_f32(c1, a[r:r + 16], w)
+        assert torch.equal(c1, c[r:r + 16])
+
+
 def _recurrence64(q, k, v, g, beta, S):
     """Token by token in float64: q, k [n, H, dk], v [n, H, dv], g [n, H, dk or 1], beta [n, H] or None, S [H, dv, dk]."""
     out = torch.empty_like(v)

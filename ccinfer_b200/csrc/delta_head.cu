@@ -11,11 +11,13 @@
 // before its own and writes its own, so blocks that share a request's channels need not wait for one another, and what
 // lies before the sequence's start is known by its position alone.
 //
-//   delta_head_step     single tokens: everything above in one kernel, a cluster of blocks per (request, head)
+//   delta_head_step     single tokens: everything above in one kernel, a cluster of blocks per (request, head), or the stream
+//                       of states (state_stream.cuh)
 //   delta_head_prepare  portions: a warp per (head of q / k / v, run of tokens) -> float rows of q, k, v and per head g and
 //                       beta (the recurrence itself is delta_rule.cu's)
 //   conv_ring_write     portions: their last rows into the ring, after delta_head_prepare has read it
 #include "cluster_common.cuh"
+#include "state_stream.cuh"
 
 using namespace ccb;
 
@@ -70,21 +72,85 @@ __device__ __forceinline__ float dot4(const float4 a, const float4 b) {
 __device__ __forceinline__ float silu_f(float x) { return x * sigmoid_f(x); }
 __device__ __forceinline__ float4 silu4(const float4 x) { return make_float4(silu_f(x.x), silu_f(x.y), silu_f(x.z), silu_f(x.w)); }
 
-// Warps of a block, and columns of S a warp holds at once where a column takes all its lanes.  Few requests: four warps and
-// eight columns, four blocks a head of 128, so that every SM has some.  Many: eight warps and sixteen columns, one block a
-// head, which then redoes no q and k and needs no other block's sum of squares; its whole state (64 KB) is in flight at once.
-// A block's chain of waits and not the memory sets the pace, so what it waits for is asked for at its start (state, position,
-// the output's gate), and its sums take few exchanges.  48 requests of 32 heads of 128 x 128, 201 MB: 97 us in clusters of
-// four small blocks, 67 us so.
-constexpr int kStepWarpsFew = 4, kStepColsFew = 8, kStepWarpsMany = 8, kStepColsMany = 16;
+// Many single tokens: what state_stream.cuh needs of a head.  A warp each makes q, k and v, four channels a lane.
+template <typename T> struct HeadDeltaJob {
+  static constexpr bool DELTA = true, CHANNEL = false, NORM = true;
+  const T* proj;
+  T* ring;
+  const float* w;
+  T* y;
+  int ldy;
+  float eps;
+  HeadDelta a;
+
+  template <class Wait>
+  __device__ __forceinline__ bool prepare(int part, int lane, int t, int e, int h, int slot, StreamRows& rows, Wait wait) const {
+    using R4 = Row4<T>;
+    const int pos = a.positions[t], C = 2 * a.G * a.dk + a.H * a.dv, per_kv = a.H / a.G, kvh = h / per_kv, i = 4 * lane;
+    const int width = part == 2 ? a.dv : a.dk, at = (part == 2 ? h * a.dv : kvh * a.dk) + i;
+    const int c = (part == 2 ? 2 * a.G * a.dk : (part == 1 ? a.G * a.dk : 0)) + at;
+    const T* row = proj + (size_t)t * a.ld;
+    const bool on = i < width;
+    const typename R4::Raw now = on ? R4::load(row + (part == 2 ? a.ov : (part == 1 ? a.ok : a.oq)) + at) : R4::zero();
+    float gate[4], wi[4], decay = 0.f, beta = 0.f;
+    if (part == 2) {
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        gate[x] = on ? to_f32(row[a.og + at + x]) : 0.f;
+        wi[x] = on ? w[i + x] : 0.f;
+      }
+      if (lane == 0) {
+        decay = expf(-expf(a.A_log[h]) * softplus_f(to_f32(row[a.oa + h]) + a.dt_bias[h]));
+        beta = sigmoid_f(to_f32(row[a.ob + h]));
+      }
+    }
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    // four taps at a time, their loads in flight together; tap j multiplies the input taps - 1 - j tokens back
+    for (int j0 = 0; on && j0 < a.taps; j0 += 4) {
+      typename R4::Raw x[4];
+      float4 cw[4];
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) {
+        const int j = j0 + jj, p = pos - (a.taps - 1 - j);
+        const bool there = j < a.taps && p >= 0;
+        x[jj] = there ? (p == pos ? now : R4::load(ring + ring_at<T>(slot, p, a.taps, C) + c)) : R4::zero();
+        cw[jj] = there ? *reinterpret_cast<const float4*>(a.conv_w + (size_t)j * C + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int jj = 0; jj < 4; ++jj) fma4(acc, cw[jj], R4::value(x[jj]));
+    }
+    // (one head of a group writes the group's q and k channels to the ring)
+    if (on && a.taps > 1 && (part == 2 || h % per_kv == 0)) R4::store(ring + ring_at<T>(slot, pos, a.taps, C) + c, now);
+    acc = silu4(acc);
+    if (part < 2) {
+      const float f = (part == 0 ? a.q_mult : 1.0f) / sqrtf(warp_sum(dot4(acc, acc)) + a.unit_eps);
+      acc.x *= f; acc.y *= f; acc.z *= f; acc.w *= f;
+    }
+    if (!wait()) return false;
+    *reinterpret_cast<float4*>((part == 2 ? rows.v : (part == 1 ? rows.k : rows.q)) + i) = acc;
+    if (part == 2) {
+      *reinterpret_cast<float4*>(rows.w + i) =
+          make_float4(wi[0] * silu_f(gate[0]), wi[1] * silu_f(gate[1]), wi[2] * silu_f(gate[2]), wi[3] * silu_f(gate[3]));
+      if (lane == 0) rows.decay = decay, rows.beta = beta;
+    }
+    return true;
+  }
+  __device__ __forceinline__ void store(int t, int h, int c, float v) const {
+    y[(size_t)t * ldy + h * a.dv + c] = from_f32<T>(v);
+  }
+};
+
+// Few single tokens: warps of a block, and columns of S a warp holds at once where a column takes all its lanes.  Four
+// blocks a head of 128, so that every SM has some; what a block waits for is asked for at its start.
+constexpr int kStepWarps = 4, kStepCols = 8;
 
 // Single tokens.  A cluster of blocks (.x) per (head, request): each redoes the head's q and k and owns a run of
 // `cols` value channels, i.e. columns of S; the sum of squares that the output's norm divides by is made over the cluster.
 // VEC: dk, dv and cols multiples of 4, dk <= 128 X, rows and columns aligned: four channels or key rows a lane, and the
 // block's columns of S are asked for before anything else (an earlier step wrote them: they need not wait for the
 // projection before this kernel).
-template <typename T, bool VEC, int X, int kStepWarps, int kStepCols>
-__global__ void __launch_bounds__(32 * kStepWarps, kStepWarps == kStepWarpsMany ? 2 : !VEC ? 10 : X == 1 ? 5 : 3)
+template <typename T, bool VEC, int X>
+__global__ void __launch_bounds__(32 * kStepWarps, !VEC ? 10 : X == 1 ? 5 : 3)
 delta_head_step_kernel(const T* __restrict__ proj, T* __restrict__ ring, float* __restrict__ state,
                        const float* __restrict__ w, float eps, T* __restrict__ y, int ldy, int cols, const HeadDelta a) {
   constexpr int kStepThreads = 32 * kStepWarps;
@@ -201,40 +267,7 @@ delta_head_step_kernel(const T* __restrict__ proj, T* __restrict__ ring, float* 
     const float g = gates[0], beta = gates[1];
     // a column of S (one value channel): S^T k and S^T q of the decayed state, then the write; the read-out after the
     // write is (g S)^T q + u (k . q)
-    if constexpr (kStepCols == kStepColsMany) {
-      // (a column takes all 32 lanes, and the block holds all columns) the 32 sums of the warp's 16 columns, one a lane in
-      // the end: 31 exchanges instead of 160
-      const bool on = 4 * li < dk;
-      const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
-      const float4 kk = on ? *reinterpret_cast<const float4*>(k_s + 4 * li) : none;
-      const float4 qq = on ? *reinterpret_cast<const float4*>(q_s + 4 * li) : none;
-      float m[kStepCols];
-#pragma unroll
-      for (int u = 0; u < kStepCols; ++u) {
-        float4& z = s[u][0];
-        z.x *= g; z.y *= g; z.z *= g; z.w *= g;
-        const float dotk = on ? dot4(z, kk) : 0.f, dotq = on ? dot4(z, qq) : 0.f;
-        m[u] = (lane & 16 ? dotq : dotk) + __shfl_xor_sync(0xffffffffu, lane & 16 ? dotk : dotq, 16);
-      }
-#pragma unroll
-      for (int o = kStepCols / 2; o > 0; o >>= 1)
-#pragma unroll
-        for (int u = 0; u < o; ++u)
-          m[u] = (lane & o ? m[u + o] : m[u]) + __shfl_xor_sync(0xffffffffu, lane & o ? m[u] : m[u + o], o);
-      const int mine = warp + (lane & 15) * stride;   // lane u: k's product with column u; lane 16 + u: q's
-      const float other = __shfl_xor_sync(0xffffffffu, m[0], 16);
-      const float put0 = mine < n_cols && lane < 16 ? beta * (v_s[mine] - m[0]) : 0.f;
-#pragma unroll
-      for (int u = 0; u < kStepCols; ++u) {
-        const float put = __shfl_sync(0xffffffffu, put0, u);
-        const int c = warp + u * stride;
-        if (c < n_cols && on) {
-          fma4(s[u][0], kk, make_float4(put, put, put, put));
-          *reinterpret_cast<float4*>(S + (size_t)c * dk + 4 * li) = s[u][0];
-        }
-      }
-      if (mine < n_cols && lane < 16) o_s[mine] = fmaf(put0, kq, other);
-    } else if constexpr (VEC) {
+    if constexpr (VEC) {
       for (int base = 0; base < n_cols; base += kStepCols * stride) {
         if (base > 0) fetch(base);
 #pragma unroll
@@ -478,6 +511,8 @@ __global__ void conv_ring_write_kernel(const T* __restrict__ proj, T* __restrict
     ring[ring_at<T>(slot, a.positions[r0 + i], a.taps, C) + c] = proj[(size_t)(r0 + i) * a.ld + col];
 }
 
+constexpr int kStreamItems = 148;   // (requests x heads) from which on single tokens go through the stream of states
+
 bool sizes_ok(const HeadDelta& a) {
   return a.G > 0 && a.H > 0 && a.H % a.G == 0 && a.dk > 0 && a.dv > 0 && a.taps >= 1;
 }
@@ -501,7 +536,7 @@ CCB_API int ccb_delta_head_step(const void* proj, int ld, const int* offsets, co
                                 float* state, const float* A_log, const float* dt_bias, const float* w, float eps,
                                 const int* positions, const int* cu_q, const int* state_slot, void* y, int ldy,
                                 int n_entries, int G, int H, int dk, int dv, int n_slots, float q_mult, float unit_eps,
-                                int dtype, cudaStream_t stream) {
+                                int dtype, int* status, cudaStream_t stream) {
   if (n_entries <= 0) return 0;
   const HeadDelta a = head_delta(ld, offsets, G, H, dk, dv, taps, conv_w, A_log, dt_bias, positions, nullptr, cu_q,
                                  state_slot, q_mult, unit_eps, n_slots);
@@ -510,27 +545,30 @@ CCB_API int ccb_delta_head_step(const void* proj, int ld, const int* offsets, co
   const bool vec = dk % 4 == 0 && dv % 4 == 0 && dk <= 256 && ld % 4 == 0 && a.oq % 4 == 0 && a.ok % 4 == 0 && a.ov % 4 == 0 &&
                    (reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(ring)) % (4 * esz) == 0 &&
                    ((reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(conv_w)) & 15) == 0;
-  // one block a head where that gives two for every SM and a block holds the head's columns at once (32 heads of 128, L2 cold,
-  // with some 20 us of launch, clusters of four / one block, us: 10 requests 43 / 41, 16 55 / 45, 32 88 / 67, 96 215 / 148;
-  // two blocks do better for heads of 64 columns)
-  const bool many = vec && dk <= 128 && dk > 64 && dv <= kStepWarpsMany * kStepColsMany && dv > 64 && (long long)n_entries * H >= 2 * 148;
+  // The stream of states where every SM has one (16 heads of 128 x 128, the layer, blocks / stream: 8 requests 23.4 / 23.9 us
+  // with 128 states; 12 33.1 / 27.2; 32 heads, 5 requests 51.3 / 51.5, 8 61.2 / 52.5, 48 112 / 86)
+  if (vec && (long long)n_entries * H >= kStreamItems && state_stream_fits(dk, dv, state) && (dtype == CCB_F32 || dtype == CCB_BF16)) {
+    const StateStream st{state, state_slot, cu_q, n_slots, n_entries, H, dk, dv, 0, status};
+    if (dtype == CCB_F32)
+      return state_stream_launch(true, st, HeadDeltaJob<float>{(const float*)proj, (float*)ring, w, (float*)y, ldy, eps, a}, stream);
+    return state_stream_launch(true, st, HeadDeltaJob<__nv_bfloat16>{(const __nv_bfloat16*)proj, (__nv_bfloat16*)ring, w,
+                                                                     (__nv_bfloat16*)y, ldy, eps, a}, stream);
+  }
   // else about 32 value channels a block, at most eight blocks a head
-  int n_blocks = many ? 1 : (dv + 31) / 32;
+  int n_blocks = (dv + 31) / 32;
   if (n_blocks > kMaxClusterBlocks) n_blocks = kMaxClusterBlocks;
   const int cols = ((dv + n_blocks - 1) / n_blocks + 3) & ~3;
   n_blocks = (dv + cols - 1) / cols;
   const size_t smem = (size_t)(2 * ((dk + 3) & ~3) + 2 * cols) * sizeof(float);
   if (smem > 44 * 1024) return CCB_REFUSE_SIZE;
-#define CCB_STEP(TT, VV, XX, SIZE)                                                                                    \
-  ccb_launch_cluster(true, n_blocks, delta_head_step_kernel<TT, VV, XX, kStepWarps##SIZE, kStepCols##SIZE>,           \
-                     dim3(n_blocks, H, n_entries), dim3(32 * kStepWarps##SIZE), smem, stream, (const TT*)proj,        \
-                     (TT*)ring, state, w, eps, (TT*)y, ldy, cols, a)
+#define CCB_STEP(TT, VV, XX)                                                                                          \
+  ccb_launch_cluster(true, n_blocks, delta_head_step_kernel<TT, VV, XX>, dim3(n_blocks, H, n_entries),                \
+                     dim3(32 * kStepWarps), smem, stream, (const TT*)proj, (TT*)ring, state, w, eps, (TT*)y, ldy, cols, a)
 #define CCB_STEP_X(TT)                                                                                                \
   do {                                                                                                                \
-    if (many) CCB_STEP(TT, true, 1, Many);                                                                            \
-    else if (!vec) CCB_STEP(TT, false, 1, Few);                                                                       \
-    else if (dk <= 128) CCB_STEP(TT, true, 1, Few);                                                                   \
-    else CCB_STEP(TT, true, 2, Few);                                                                                  \
+    if (!vec) CCB_STEP(TT, false, 1);                                                                                 \
+    else if (dk <= 128) CCB_STEP(TT, true, 1);                                                                        \
+    else CCB_STEP(TT, true, 2);                                                                                       \
   } while (0)
   if (dtype == CCB_F32) CCB_STEP_X(float);
   else if (dtype == CCB_BF16) CCB_STEP_X(__nv_bfloat16);

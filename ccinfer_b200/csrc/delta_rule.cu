@@ -20,6 +20,7 @@
 // contiguous), and the convolution's last (taps - 1) inputs as [taps - 1, channels] in the compute type.
 // Rows whose request has no slot (padding of a replayed step) are skipped.
 #include "common.cuh"
+#include "state_stream.cuh"
 
 using namespace ccb;
 
@@ -525,6 +526,37 @@ delta_recurrence_kernel(const float* __restrict__ qn, const float* __restrict__ 
     }
 }
 
+// Many single tokens: what state_stream.cuh needs of a head, whose rows are there already.
+template <bool DELTA_, bool CHANNEL_> struct RowsJob {
+  static constexpr bool DELTA = DELTA_, CHANNEL = CHANNEL_, NORM = false;
+  const float *q, *k, *v, *g, *beta;   // as in delta_recurrence_kernel
+  float* out;
+  int G, H, dk, dv;
+  float eps;   // (of a norm: there is none)
+
+  template <class Wait>
+  __device__ __forceinline__ bool prepare(int part, int lane, int t, int e, int h, int slot, StreamRows& rows, Wait wait) const {
+    const int i = 4 * lane, kvh = h / (H / G);
+    const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 x = none, decay = none;
+    float b = 1.f, d = 0.f;
+    if (part < 2) {
+      if (i < dk) x = load4((part == 0 ? q : k) + ((size_t)t * G + kvh) * dk + i);
+      if (CHANNEL && part == 0 && i < dk) decay = load4(g + ((size_t)t * H + h) * dk + i);
+    } else {
+      if (i < dv) x = load4(v + ((size_t)t * H + h) * dv + i);
+      if (lane == 0 && beta != nullptr) b = beta[(size_t)t * H + h];
+      if (!CHANNEL && lane == 0) d = g[(size_t)t * H + h];
+    }
+    if (!wait()) return false;
+    *reinterpret_cast<float4*>((part == 2 ? rows.v : (part == 1 ? rows.k : rows.q)) + i) = x;
+    if (CHANNEL && part == 0) *reinterpret_cast<float4*>(rows.g + i) = decay;
+    if (part == 2 && lane == 0) rows.decay = d, rows.beta = b;
+    return true;
+  }
+  __device__ __forceinline__ void store(int t, int h, int c, float x) const { out[((size_t)t * H + h) * dv + c] = x; }
+};
+
 // ---------------------------------------------------------------------------------------------
 // y[t, h, :] = o[t, h, :] / sqrt(mean(o^2) + eps) * w[:] * sigmoid(gate[t, h, :]); one warp per (t, h).
 // SILU: the gate is gate * sigmoid(gate) instead.
@@ -693,12 +725,25 @@ static void launch_recurrence(const float* qn, const float* kn, const float* vv,
              state, out, cu_q, state_slot, entry0, G, H, dk, dv, tch);
 }
 
+// From so many value channels on, of all heads and requests together, single tokens go through the stream of states: an SM has
+// a whole state of 128 channels then (the layers of state_stream.cuh, before / with it: 32 heads of 128 x 128, 5 requests 67.3 / 65.3
+// us; 16 heads, 12 requests 44.9 / 41.0; 64 heads of 64 x 128, 5 requests 34.9 / 32.8).
+constexpr long long kStreamColumns = 148 * 128;
+
+// single_slots > 0: every entry brings one token, and the state has so many slots.
 template <bool DELTA, bool HEAD>
 static int pick_recurrence(const float* qn, const float* kn, const float* vv, const float* gg, const float* bb,
                            float* state, float* out, const int* cu_q, const int* state_slot, int n_entries, int G,
-                           int H, int dk, int dv, cudaStream_t stream, int entry0 = 0) {
+                           int H, int dk, int dv, cudaStream_t stream, int entry0 = 0, int single_slots = 0,
+                           int* status = nullptr) {
   if (n_entries <= 0) return 0;
   if (G <= 0 || H <= 0 || H % G || dk <= 0 || dk > 256 || dv <= 0) return CCB_REFUSE_SIZE;
+  const auto bits = [](const void* p) { return reinterpret_cast<uintptr_t>(p); };
+  if (single_slots > 0 && entry0 == 0 && (long long)n_entries * H * dv >= kStreamColumns && state_stream_fits(dk, dv, state) &&
+      ((bits(qn) | bits(kn) | bits(vv) | (HEAD ? 0 : bits(gg))) & 15) == 0) {
+    const StateStream st{state, state_slot, cu_q, single_slots, n_entries, H, dk, dv, 0, status};
+    return state_stream_launch(true, st, RowsJob<DELTA, !HEAD>{qn, kn, vv, gg, bb, out, G, H, dk, dv, 0.f}, stream);
+  }
   int R = 1;
   while (R * kLanes < dk) R *= 2;
   // One column per thread.  Two (the rows of q, k, g read once for both) were slower: 1.11 against 0.99 ms
@@ -721,10 +766,13 @@ static int pick_recurrence(const float* qn, const float* kn, const float* vv, co
   return ccb_launch_status();
 }
 
+// single_slots (here and below): 0, or the state's slots where every entry brings one token; status: as everywhere, or null
 CCB_API int ccb_delta_recurrence(const float* qn, const float* kn, const float* vv, const float* gg,
                                  const float* bb, float* state, float* out, const int* cu_q, const int* state_slot,
-                                 int n_entries, int G, int H, int dk, int dv, cudaStream_t stream) {
-  return pick_recurrence<true, false>(qn, kn, vv, gg, bb, state, out, cu_q, state_slot, n_entries, G, H, dk, dv, stream);
+                                 int n_entries, int G, int H, int dk, int dv, int single_slots, int* status,
+                                 cudaStream_t stream) {
+  return pick_recurrence<true, false>(qn, kn, vv, gg, bb, state, out, cu_q, state_slot, n_entries, G, H, dk, dv, stream, 0,
+                                      single_slots, status);
 }
 
 // The same with one decay per head and token (gg [T, H]), for the entries entry0 .. entry0 + n_entries - 1.
@@ -740,9 +788,10 @@ CCB_API int ccb_delta_head_recurrence(const float* qn, const float* kn, const fl
 // The plain gated recurrence (no correction by what the state already holds): S <- diag(g) S + k v^T, o = S^T q.
 CCB_API int ccb_gated_linear_recurrence(const float* qn, const float* kn, const float* vv, const float* gg,
                                         float* state, float* out, const int* cu_q, const int* state_slot,
-                                        int n_entries, int G, int H, int dk, int dv, cudaStream_t stream) {
+                                        int n_entries, int G, int H, int dk, int dv, int single_slots, int* status,
+                                        cudaStream_t stream) {
   return pick_recurrence<false, false>(qn, kn, vv, gg, nullptr, state, out, cu_q, state_slot, n_entries, G, H, dk, dv,
-                                       stream);
+                                       stream, 0, single_slots, status);
 }
 
 // The plain recurrence with ONE decay per head and token and a step size on the write (a selective state space
@@ -750,9 +799,10 @@ CCB_API int ccb_gated_linear_recurrence(const float* qn, const float* kn, const 
 // a and dt float [T, H]; q and k have G groups of dk channels.
 CCB_API int ccb_ssm_recurrence(const float* qn, const float* kn, const float* vv, const float* a, const float* dt,
                                float* state, float* out, const int* cu_q, const int* state_slot, int n_entries,
-                               int G, int H, int dk, int dv, cudaStream_t stream) {
+                               int G, int H, int dk, int dv, int single_slots, int* status, cudaStream_t stream) {
   if (a == nullptr) return CCB_REFUSE_ARG;   // (dt null: every step size is one)
-  return pick_recurrence<false, true>(qn, kn, vv, a, dt, state, out, cu_q, state_slot, n_entries, G, H, dk, dv, stream);
+  return pick_recurrence<false, true>(qn, kn, vv, a, dt, state, out, cu_q, state_slot, n_entries, G, H, dk, dv, stream, 0,
+                                      single_slots, status);
 }
 
 template <typename T, bool SILU>

@@ -74,11 +74,11 @@ _SIGNATURES = {
     "ccb_conv_state_update": [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int,
                               c_int, c_int, c_int, c_int, c_int, c_void_p],
     "ccb_delta_recurrence": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                             c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
+                             c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "ccb_gated_head_rmsnorm": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_float, c_int,
                                c_int, c_void_p],
     "ccb_gated_linear_recurrence": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                                    c_int, c_int, c_int, c_int, c_int, c_void_p],
+                                    c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "ccb_gla_prepare": [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                         c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_int, c_void_p],
     "ccb_latent_prepare": [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_float, c_void_p,
@@ -89,7 +89,7 @@ _SIGNATURES = {
     "ccb_moe_table_route": [c_void_p] * 4 + [c_int] * 4 + [c_float, c_void_p, c_int, c_void_p, c_void_p],
     "ccb_moe_table_sort": [c_void_p] * 4 + [c_int] * 4 + [c_float, c_int, c_int, c_int] + [c_void_p] * 8,
     "ccb_delta_head_step": [c_void_p, c_int, c_void_p, c_void_p, c_int] + [c_void_p] * 5 + [c_float] + [c_void_p] * 4
-                           + [c_int] * 7 + [c_float, c_float, c_int, c_void_p],
+                           + [c_int] * 7 + [c_float, c_float, c_int, c_void_p, c_void_p],
     "ccb_delta_head_prepare": [c_void_p, c_int, c_void_p, c_void_p, c_int] + [c_void_p] * 12 + [c_int] * 7
                               + [c_float, c_float, c_int, c_void_p],
     "ccb_conv_ring_write": [c_void_p, c_int, c_void_p, c_int] + [c_void_p] * 4 + [c_int] * 8 + [c_void_p],
@@ -185,7 +185,7 @@ _SIGNATURES = {
                                     c_void_p, c_void_p],
     "ccb_ssm_gate_norm": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int,
                           c_int, c_float, c_int, c_void_p],
-    "ccb_ssm_recurrence": [c_void_p] * 9 + [c_int] * 5 + [c_void_p],
+    "ccb_ssm_recurrence": [c_void_p] * 9 + [c_int] * 6 + [c_void_p, c_void_p],
     "ccb_attention_talking_fits": [c_int, c_int, c_int],
     "ccb_attention_talking": [c_void_p] * 10 + [c_int] * 9 + [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p],
     "ccb_attention_talking_mma_fits": [c_int, c_int, c_int],
@@ -635,13 +635,15 @@ def conv_state_rows(rows, taps: int, C: int, state, cu_q, state_slot, entry0: in
 
 
 def delta_recurrence(qn, kn, vv, gg, bb, state, out, cu_q, state_slot, n_entries: int, G: int, H: int, dk: int,
-                     dv: int) -> None:
+                     dv: int, single: bool = False, status=None) -> None:
     """The gated delta rule over each request's tokens of the step, from and into ``state``
-    [slots, H, dv, dk] (float); out float [T, H, dv]."""
+    [slots, H, dv, dk] (float); out float [T, H, dv].  ``single`` (here and in the recurrences below): every entry brings
+    one token, so that many of them may go through the stream of states (``csrc/state_stream.cuh``)."""
     _cuda(qn, kn, vv, gg, bb, state, out, cu_q, state_slot)
     assert state.dtype == torch.float32 and state.shape[1:] == (H, dv, dk) and out.dtype == torch.float32
     _check(lib().ccb_delta_recurrence(_p(qn), _p(kn), _p(vv), _p(gg), _p(bb), _p(state), _p(out), _p(cu_q),
-                                      _p(state_slot), n_entries, G, H, dk, dv, _stream()), "delta_recurrence")
+                                      _p(state_slot), n_entries, G, H, dk, dv, state.shape[0] if single else 0, _p(status),
+                                      _stream()), "delta_recurrence")
 
 
 # When the recurrences of a step's portions run in chunks: from so many (token, head) pairs of portions on with the longest
@@ -718,7 +720,8 @@ class HeadDelta:
         assert tuple(ring.shape[1:]) == (self.taps, 2 * G * dk + H * dv)
 
 
-def delta_head_step(rule: HeadDelta, proj, ring, state, w, eps: float, positions, cu_q, state_slot, y, n_entries: int) -> None:
+def delta_head_step(rule: HeadDelta, proj, ring, state, w, eps: float, positions, cu_q, state_slot, y, n_entries: int,
+                    status=None) -> None:
     """A step's first ``n_entries`` entries, one token each, through the whole mixer between its projections: y [T, H dv]
     = o / rms(o) * w * silu(gate); the convolution's ``ring`` [slots, taps, channels] and ``state`` float [slots, H, dv, dk]
     move on."""
@@ -730,7 +733,7 @@ def delta_head_step(rule: HeadDelta, proj, ring, state, w, eps: float, positions
     _check(lib().ccb_delta_head_step(_p(proj), proj.stride(0), rule.offsets, _p(rule.conv_w), rule.taps, _p(ring), _p(state),
                                      _p(rule.A_log), _p(rule.dt_bias), _p(w), float(eps), _p(positions), _p(cu_q),
                                      _p(state_slot), _p(y), y.stride(0), int(n_entries), G, H, dk, dv, ring.shape[0],
-                                     rule.q_mult, rule.unit_eps, _dt(proj), _stream()), "delta_head_step")
+                                     rule.q_mult, rule.unit_eps, _dt(proj), _p(status), _stream()), "delta_head_step")
 
 
 def delta_head_prepare(rule: HeadDelta, proj, ring, positions, entry_of_token, cu_q, state_slot, qn, kn, vv, gg, bb,
@@ -781,15 +784,15 @@ def gated_head_rmsnorm(y, o, gate, w, H: int, dv: int, eps: float, silu_gate: bo
 
 
 def gated_linear_recurrence(qn, kn, vv, gg, state, out, cu_q, state_slot, n_entries: int, H: int, dk: int,
-                            dv: int) -> None:
+                            dv: int, single: bool = False, status=None) -> None:
     """S <- diag(g_t) S + k_t v_t^T, out_t = S^T q_t over each request's tokens of the step, from and into
     ``state`` [slots, H, dv, dk] (float); the rows float [T, H, dk] (q, k, g) and [T, H, dv] (v, out)."""
     _cuda(qn, kn, vv, gg, state, out, cu_q, state_slot)
     assert state.dtype == torch.float32 and state.shape[1:] == (H, dv, dk) and out.dtype == torch.float32
     assert qn.dtype == kn.dtype == vv.dtype == gg.dtype == torch.float32
     _check(lib().ccb_gated_linear_recurrence(_p(qn), _p(kn), _p(vv), _p(gg), _p(state), _p(out), _p(cu_q),
-                                             _p(state_slot), n_entries, H, H, dk, dv, _stream()),
-           "gated_linear_recurrence")
+                                             _p(state_slot), n_entries, H, H, dk, dv, state.shape[0] if single else 0,
+                                             _p(status), _stream()), "gated_linear_recurrence")
 
 
 def gla_prepare(proj, offsets, a, bias, qn, kn, vv, gg, H: int, dk: int, dv: int, q_mult: float, tau: float) -> None:
@@ -1441,7 +1444,7 @@ def memory_recurrence(qn, kn, vv, decay, put, state, out, cu_q, state_slot, n_en
     cu_q, state_slot = cu_q[entry0:], state_slot[entry0:]
     _cuda(qn, kn, vv, decay, put, state, out, cu_q, state_slot)
     _check(lib().ccb_ssm_recurrence(_p(qn), _p(kn), _p(vv), _p(decay), _p(put), _p(state), _p(out), _p(cu_q),
-                                    _p(state_slot), int(n_entries), H, H, dk, dv, _stream()), "memory_recurrence")
+                                    _p(state_slot), int(n_entries), H, H, dk, dv, 0, 0, _stream()), "memory_recurrence")
 
 
 def memory_output(y, o, gate, H: int, dv: int, eps: float, weight=None, floor=None, den_eps: float = 0.0,
@@ -1543,13 +1546,14 @@ def conv_state_shift(rows, taps: int, state, cu_q, state_slot, n_entries: int, e
 
 
 def ssm_recurrence(cs, bs, xs, decay, dts, state, out, cu_q, state_slot, n_entries: int, G: int, H: int, N: int,
-                   P: int) -> None:
+                   P: int, single: bool = False, status=None) -> None:
     """S <- decay_t S + B_t (dt_t x_t)^T, out_t = S^T C_t per head over each request's tokens of the step, from and
     into ``state`` [slots, H, P, N] (float); cs, bs float [T, G, N], xs and out [T, H, P], decay and dts [T, H]."""
     _cuda(cs, bs, xs, decay, dts, state, out, cu_q, state_slot)
     assert state.dtype == torch.float32 and state.shape[1:] == (H, P, N) and out.dtype == torch.float32
     _check(lib().ccb_ssm_recurrence(_p(cs), _p(bs), _p(xs), _p(decay), _p(dts), _p(state), _p(out), _p(cu_q),
-                                    _p(state_slot), n_entries, G, H, N, P, _stream()), "ssm_recurrence")
+                                    _p(state_slot), n_entries, G, H, N, P, state.shape[0] if single else 0, _p(status),
+                                    _stream()), "ssm_recurrence")
 
 
 def ssm_gate_norm(y, o, xs, proj, oz: int, skip, w, H: int, P: int, parts: int, eps: float) -> None:

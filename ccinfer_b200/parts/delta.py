@@ -144,7 +144,8 @@ class ChannelGatedDelta(Mixer):
         chunks = kernels.chunk_recurrence_fits(rt.dtype, dk, dv, step.max_q_len, (T - step.n_single) * H, True)
         n1 = step.n_single if chunks else step.n_entries
         if n1:
-            kernels.delta_recurrence(qn, kn, vv, gg, bb, S, o, step.cu_q, step.state_slot, n1, G, H, dk, dv)
+            kernels.delta_recurrence(qn, kn, vv, gg, bb, S, o, step.cu_q, step.state_slot, n1, G, H, dk, dv,
+                                     single=n1 == step.n_single, status=rt.status)
         if step.n_entries > n1:
             kernels.chunk_recurrence(rt.chunk_scratch, qn, kn, vv, gg, bb, S, o, step.cu_q, step.state_slot, n1,
                                      step.n_entries - n1, step.max_q_len, G, H, dk, dv)
@@ -230,7 +231,7 @@ class HeadGatedDelta(Mixer):
         n1, many = step.n_single, step.n_entries - step.n_single
         if n1 > 0:
             kernels.delta_head_step(self.rule, proj, ring, S, self.norm_w, self.eps, step.positions, step.cu_q,
-                                    step.state_slot, y, n1)
+                                    step.state_slot, y, n1, status=rt.status)
         if many > 0:
             # (layers of other sizes have buffers of their own: what only portions use must not grow once graphs hold the
             # pool's addresses)

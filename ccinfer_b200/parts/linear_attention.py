@@ -96,7 +96,8 @@ class GatedLinearAttention(Mixer):
         chunks = kernels.chunk_recurrence_fits(rt.dtype, dk, dv, step.max_q_len, (T - step.n_single) * H, False)
         n1 = step.n_single if chunks else step.n_entries
         if n1:
-            kernels.gated_linear_recurrence(qn, kn, vv, gg, state, o, step.cu_q, step.state_slot, n1, H, dk, dv)
+            kernels.gated_linear_recurrence(qn, kn, vv, gg, state, o, step.cu_q, step.state_slot, n1, H, dk, dv,
+                                            single=n1 == step.n_single, status=rt.status)
         if step.n_entries > n1:
             kernels.chunk_recurrence(rt.chunk_scratch, qn, kn, vv, gg, None, state, o, step.cu_q, step.state_slot, n1,
                                      step.n_entries - n1, step.max_q_len, H, H, dk, dv)

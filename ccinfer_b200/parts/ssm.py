@@ -116,7 +116,8 @@ class SelectiveStateSpace(Mixer):
                                  step.n_entries - step.n_single, entry0=step.n_single)
         o = rt.scratch.get("ssm_o", (rt.max_tokens, H, P), f32)[:T]
         if n1:
-            kernels.ssm_recurrence(cs, bs, xs, decay, dts, S, o, step.cu_q, step.state_slot, n1, G, H, N, P)
+            kernels.ssm_recurrence(cs, bs, xs, decay, dts, S, o, step.cu_q, step.state_slot, n1, G, H, N, P,
+                                   single=n1 == step.n_single, status=rt.status)
         if chunk is not None:
             kernels.ssm_chunks(chunk, xs, S, o, step.cu_q, step.state_slot, n1, step.n_entries - n1, G, H, N, P)
         y = rt.scratch.get("ssm_y", (rt.max_tokens, self.inner), rt.dtype)[:T]

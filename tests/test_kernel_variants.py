@@ -784,3 +784,90 @@ def test_state_space_rows_in_runs(taps, H, P, G, N, last, dtype):
         assert (log_a[s].double() + A_log.double().exp() * dt[s]).abs().max() <= 64 * 2.0 ** -24 * 16 * dt.max()
         assert (log_dt[s].double() - dt[s].log()).abs().max() <= 64 * 2.0 ** -24 * 16
     assert torch.equal(conv.double(), after)
+
+
+# sizes of a state that fill no lane's four, no warp's eight or sixteen channels; more requests than SMs; slots that are none
+@pytest.mark.parametrize("kind", ["delta", "linear", "state space"])
+@pytest.mark.parametrize("E,H,G,dk,dv", [(9, 17, 17, 128, 128), (160, 2, 1, 68, 64), (75, 8, 4, 100, 36), (40, 10, 5, 124, 68),
+                                        (150, 1, 1, 128, 128), (3, 50, 25, 72, 128)])
+def test_single_tokens_of_many_requests_stream_their_states(kind, E, H, G, dk, dv):
+    """One token each against float64: sums of dk products, sizes of some 1; a state that no request of the step has stays."""
+    from ccinfer_b200 import kernels as k
+    if kind == "linear":
+        G = H
+    assert E * H * dv >= 148 * 128   # (from here on)
+    g = _gen(E + H + dk + dv)
+
+    def rnd(*shape):
+        return torch.randn(shape, generator=g, device="cuda")
+
+    def dev(x):
+        return torch.tensor(x, dtype=torch.int32, device="cuda")
+
+    q, kk = (torch.nn.functional.normalize(rnd(E, G, dk), dim=-1) for _ in range(2))
+    v, beta = rnd(E, H, dv), torch.rand((E, H), generator=g, device="cuda")
+    decay = torch.rand((E, H) if kind == "state space" else (E, H, dk), generator=g, device="cuda")
+    state = rnd(E + 3, H, dv, dk)
+    slots = torch.randperm(E + 3, generator=torch.Generator().manual_seed(E)).tolist()[:E]
+    dead = {1, E - 1}
+    before, out = state.double(), torch.full((E, H, dv), float("nan"), device="cuda")
+    args = (dev(list(range(E + 1))), dev([-1 if e in dead else s for e, s in enumerate(slots)]), E)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    if kind == "delta":
+        k.delta_recurrence(q, kk, v, decay, beta, state, out, *args, G, H, dk, dv, single=True, status=status)
+    elif kind == "linear":
+        k.gated_linear_recurrence(q, kk, v, decay, state, out, *args, H, dk, dv, single=True, status=status)
+    else:
+        k.ssm_recurrence(q, kk, v, decay, beta, state, out, *args, G, H, dk, dv, single=True, status=status)
+    rep = H // G
+    want, after = out.double(), before.clone()
+    for e, s in enumerate(slots):
+        if e in dead:
+            continue
+        put = v[e:e + 1].double() * (beta[e:e + 1, :, None].double() if kind == "state space" else 1)
+        want[e:e + 1], after[s] = _recurrence64(
+            q[e:e + 1].double().repeat_interleave(rep, 1), kk[e:e + 1].double().repeat_interleave(rep, 1), put,
+            (decay[e:e + 1, :, None] if kind == "state space" else decay[e:e + 1]).double(),
+            beta[e:e + 1].double() if kind == "delta" else None, before[s])
+    live = [e for e in range(E) if e not in dead]
+    assert int(status) == 0 and torch.isnan(out[list(dead)]).all()   # (nobody writes the others)
+    # a sum of dk terms in float, in some ten additions one after another, and few operations around it
+    assert (out[live].double() - want[live]).abs().max() <= 2.0 ** -20 * want[live].abs().max()
+    assert (state.double() - after).abs().max() <= 2.0 ** -20 * after.abs().max()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("E,H,G,dk,dv,taps", [(5, 37, 37, 128, 128, 4), (150, 2, 1, 68, 36, 1), (30, 10, 5, 100, 64, 6), (40, 8, 2, 72, 100, 2)])
+def test_one_token_of_the_head_delta_rule_beside_its_blocks(E, H, G, dk, dv, taps, dtype):
+    """The stream of states beside the blocks of few requests (the same step in parts small enough for them)."""
+    from ccinfer_b200 import kernels as k
+    g = _gen(E + H + dk + dv)
+
+    def rnd(*shape):
+        return torch.randn(shape, generator=g, device="cuda")
+
+    C = 2 * G * dk + H * dv
+    offsets = [0, G * dk, 2 * G * dk, C, C + H, C + 2 * H]
+    width = -(-(C + 2 * H + H * dv) // 8) * 8
+    proj, w = rnd(E, width).to(dtype), rnd(dv)
+    rule = k.HeadDelta(tuple(offsets), 0.5 * rnd(taps, C), torch.log(1 + 15 * torch.rand(H, generator=g, device="cuda")), rnd(H) - 2,
+                       G, H, dk, dv, dk ** -0.5, 1e-6)
+    ring, state = rnd(E, taps, C).to(dtype), rnd(E, H, dv, dk)
+    i32 = {"dtype": torch.int32, "device": "cuda"}
+    pos, slots = torch.arange(E, **i32) % 7, torch.randperm(E, generator=torch.Generator().manual_seed(1)).to(**i32)
+    slots[2] = -1
+    status = torch.zeros(1, **i32)
+    got = [t.clone() for t in (ring, state)] + [torch.zeros(E, H * dv, dtype=dtype, device="cuda")]
+    want = [t.clone() for t in (ring, state)] + [torch.zeros(E, H * dv, dtype=dtype, device="cuda")]
+    assert E * H >= 148
+    k.delta_head_step(rule, proj, got[0], got[1], w, 1e-5, pos, torch.arange(E + 1, **i32), slots, got[2], E, status=status)
+    n = 147 // H   # (requests of a part)
+    for e in range(0, E, n):
+        m = min(n, E - e)
+        k.delta_head_step(rule, proj[e:e + m], want[0], want[1], w, 1e-5, pos[e:e + m].contiguous(), torch.arange(m + 1, **i32),
+                          slots[e:e + m].contiguous(), want[2][e:e + m], m)
+    assert int(status) == 0 and torch.equal(got[0], want[0])
+    # the same float operations but for the order of sums of dk and dv terms; rows rounded to the compute type
+    assert (got[1] - want[1]).abs().max() <= 2.0 ** -19 * want[1].abs().max()
+    near = 2.0 ** -19 if dtype == torch.float32 else 2.0 ** -7
+    assert (got[2].float() - want[2].float()).abs().max() <= near * want[2].float().abs().max()

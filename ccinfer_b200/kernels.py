@@ -270,7 +270,8 @@ def lib(group: str = None):
     """The kernels (see ``_Kernels``), or with ``group`` the loaded shared object of that one family."""
     if group is not None:
         return _load(group)
-    _load("base")   # (what every model needs: a missing compiler shows here, before anything else happens)
+    if "base" not in _libs:
+        _load("base")   # (what every model needs: a missing compiler shows here, before anything else happens)
     return _kernels
 
 
@@ -296,7 +297,9 @@ def set_pdl(on) -> None:
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream of the current device (as ``torch.cuda.current_stream``, which makes an object that takes the host
+    some 4 us; a portion's layer asks six to ten times)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 class _Counters:

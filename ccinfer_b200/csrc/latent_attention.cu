@@ -27,6 +27,8 @@
 #include "common.cuh"
 #include "mma_common.cuh"
 #include "dense_rows.cuh"
+#include "tc_common.cuh"
+#include "tma_host.h"
 #include <math_constants.h>
 
 using namespace ccb;
@@ -600,6 +602,286 @@ latent_attention_mma_kernel(const float* __restrict__ qa, const __nv_bfloat16* _
     }
 }
 
+// ---------------------------------------------------------------------------------------------
+// Single tokens: a block per (request, 16 MTL heads, piece of the key range) walks the keys 32 at a time, four warps a tile of
+// 16 heads and one that copies.
+//   copies     whole pages of rows, one copy each, a lane a page: lines of 128 bytes in the 128-byte swizzle by lines (a copy
+//              a row holds its warp some 130 cycles: 32 of them set the pace)
+//   S          warp w takes every fourth 16 of the W coordinates for all 32 keys, its queries' parts in registers for good; the
+//              four warps' sums meet in shared memory (two places in turn: one barrier a tile)
+//   softmax    every warp makes all 16 x 32 weights itself and has them as the operand of
+//   O += P C   warp w takes the columns 16 (w + 4 i) .. + 15
+// So a tile's chain is a copy that came long ago, a product of W / 64 steps, one exchange and a second product.  Looked up and
+// copied by the warps that compute, with the keys of a tile shared among them, a tile waits for the look-ups, the copies and
+// four barriers.  4 requests of 16 heads, 3,000 keys of 576 in 47 pieces: 15.4 us so, 8.8 with this; 40 requests of 32 heads, some
+// 2,250 keys each: 159 and 67 us (the layers 41 / 35 and 207 / 110).  What bounds it: instructions and reads of shared memory, some
+// 3,000 cycles a tile of 32 heads.
+constexpr int kSingleKeys = 32, kSingleWarps = 4, kSingleStages = 6;   // (at most)
+constexpr float kLog2e = 1.44269504088896f, kLn2 = 0.693147180559945f;
+
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// Pieces of a token's keys: no more than the launch has, of at least kSingleTiles tiles each (tokens of few keys are finished by
+// one block, and the merge passes them over; with four the pieces of 3,000 keys take 12.3 us in place of 8.8).
+constexpr int kSingleTiles = 2;
+__device__ __forceinline__ int single_pieces(int p, int window, int num_splits) {
+  const int n_tiles = p / kSingleKeys - max(0, p - window + 1) / kSingleKeys + 1;
+  return min(num_splits, (n_tiles + kSingleTiles - 1) / kSingleTiles);
+}
+
+template <int SEGS, int MTL>   // SEGS: rows of 64 SEGS coordinates, the last 64 of them (and maybe more) rotated ones
+__global__ void __launch_bounds__((kSingleWarps * MTL + 1) * 32, MTL == 1 ? 2 : 1)
+latent_single_kernel(const __grid_constant__ CUtensorMap tm_rows, const float* __restrict__ qa, const float* __restrict__ sink,
+                     const __nv_bfloat16* __restrict__ gate, int ldg, __nv_bfloat16* __restrict__ out,
+                     float* __restrict__ part_acc, float* __restrict__ part_ml, int num_splits, const int* __restrict__ cu_q,
+                     const int* __restrict__ pos0, const int* __restrict__ entry_of_token, const int* __restrict__ block_table,
+                     int bt_stride, int entry0, int H, int R, int page_size, int num_pages, int window, float scale, int box_rows,
+                     int stages, int* status) {
+  ccb::pdl_begin();
+  constexpr int KEYS = kSingleKeys, W = 64 * SEGS, STAGE = KEYS * W * 2, NPW = SEGS - 1, KPW = SEGS;
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ __align__(8) uint64_t bars[2 * kSingleStages];
+  unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);   // [stages][KEYS][SEGS] lines
+  float2* part_s = reinterpret_cast<float2*>(ring + stages * STAGE);              // [2][MTL][4 warps][8][32 lanes]
+  const uint32_t full0 = s32(bars), empty0 = full0 + 8 * kSingleStages;
+  const int e = entry0 + blockIdx.y / num_splits, split = blockIdx.y % num_splits;
+  const int t = cu_q[e], p = pos0[e];
+  if (cu_q[e + 1] == t || entry_of_token[t] < 0) return;
+  const int pieces = single_pieces(p, window, num_splits);
+  if (split >= pieces) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
+  const int j_lo = max(0, p - window + 1);
+  const int tile0 = j_lo / KEYS, n_tiles = p / KEYS - tile0 + 1;
+  const int per = (n_tiles + pieces - 1) / pieces;
+  const int t_begin = tile0 + split * per, tiles = max(0, min(per, tile0 + n_tiles - t_begin));
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < stages; ++s) {
+      mbar_init(full0 + 8 * s, 1);
+      mbar_init(empty0 + 8 * s, kSingleWarps * MTL);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+
+  if (warp == kSingleWarps * MTL) {   // ---- copies
+    const int* bt = block_table + (size_t)e * bt_stride;
+    const int boxes = KEYS / box_rows;
+    // the first row of this lane's box (keys past the token's: the box with its own, whose copies get no weight)
+    auto source = [&](int tile) {
+      if (lane >= boxes) return 0;
+      const int j = min((t_begin + tile) * KEYS + lane * box_rows, p / box_rows * box_rows);
+      const int lp = j / page_size;
+      int page = lp < bt_stride ? bt[lp] : -1;
+      if (page < 0 || page >= num_pages) {
+        if (j + box_rows > j_lo) set_status(status, CCB_ST_BAD_PAGE);   // (a page before the window may be gone)
+        else page = bt[p / page_size];
+      }
+      if (page < 0 || page >= num_pages) page = 0;
+      return page * page_size + (j - lp * page_size);
+    };
+    int row = tiles > 0 ? source(0) : 0;
+    int issued = 0;
+    for (int i = 0; i < tiles; ++i) {
+      const int s = i % stages;
+      if (!__all_sync(0xffffffffu, mbar_wait(empty0 + 8 * s, ((i / stages) & 1) ^ 1))) {
+        if (lane == 0) set_status(status, CCB_ST_WAIT_TIMEOUT);
+        break;
+      }
+      fence_async_smem();   // (the stage was read by ordinary loads and is written by the copy engine)
+      if (lane == 0) mbar_expect_tx(full0 + 8 * s, STAGE);
+      __syncwarp();
+      if (lane < boxes) tma_load_3d(s32(ring + s * STAGE) + lane * box_rows * W * 2, &tm_rows, 0, 0, row, full0 + 8 * s);
+      ++issued;
+      if (i + 1 < tiles) row = source(i + 1);
+    }
+    for (int i = max(0, issued - stages); i < issued; ++i) mbar_wait(full0 + 8 * (i % stages), (i / stages) & 1);   // (none is under way when the block goes)
+    return;
+  }
+  const int rt = warp / kSingleWarps, w = warp % kSingleWarps;
+  const int h0 = (blockIdx.x * MTL + rt) * 16;
+  const float scale2 = scale * kLog2e;
+  const bool ok[2] = {h0 + gid < H, h0 + gid + 8 < H};   // this lane's heads
+  // the queries' coordinates of this warp, as the A operand
+  const int n_pairs = R >> 4;
+  uint32_t qf[KPW][4];
+  {
+    float2 x[KPW][4];
+#pragma unroll
+    for (int kk = 0; kk < KPW; ++kk)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int ks = w + kSingleWarps * kk, hh = i & 1;
+        const float* src = qa + ((size_t)t * H + (ok[hh] ? h0 + gid + 8 * hh : 0)) * W + ks * 16 + 2 * tig + 8 * (i >> 1);
+        x[kk][i] = ok[hh] && tiles > 0 ? *reinterpret_cast<const float2*>(src) : make_float2(0.f, 0.f);
+      }
+#pragma unroll
+    for (int kk = 0; kk < KPW; ++kk)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) qf[kk][i] = pack_bf16(x[kk][i].x, x[kk][i].y);
+  }
+  float m[2], l[2], acc[NPW][2][4];
+#pragma unroll
+  for (int hh = 0; hh < 2; ++hh) {   // the sink: one term exp(sink) with no key and no value
+    const bool first = split == 0 && ok[hh];
+    m[hh] = first ? sink[h0 + gid + 8 * hh] * kLog2e : -CUDART_INF_F;   // (of base 2, as the scores)
+    l[hh] = first && tig == 0 ? 1.f : 0.f;   // (of this lane's keys)
+  }
+#pragma unroll
+  for (int i = 0; i < NPW; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) acc[i][j][k] = 0.f;
+
+  bool alive = true;
+  for (int it = 0; it < tiles; ++it) {
+    const int s = it % stages;
+    if (alive) {
+      alive = mbar_wait(full0 + 8 * s, (it / stages) & 1);
+      if (!alive) set_status(status, CCB_ST_WAIT_TIMEOUT);
+    }
+    const uint32_t C = s32(ring + s * STAGE);
+    const int first_key = (t_begin + it) * KEYS;
+    const bool edge = first_key < j_lo || first_key + KEYS - 1 > p;
+    if (edge) {
+      // rows that this token does not see may hold anything, also what is no number: zeros (each tile of heads by itself)
+      const int below = max(0, j_lo - first_key), seen = min(KEYS, p + 1 - first_key) - below, n = (KEYS - seen) * W / 8;
+      for (int i = w * 32 + lane; i < n; i += 32 * kSingleWarps) {
+        const int at = i < below * W / 8 ? i : i + seen * W / 8;
+        reinterpret_cast<uint4*>(ring + s * STAGE)[at] = make_uint4(0u, 0u, 0u, 0u);
+      }
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + rt), "n"(32 * kSingleWarps) : "memory");
+    }
+    float sc[4][4];
+#pragma unroll
+    for (int nb = 0; nb < 4; ++nb) sc[nb][0] = sc[nb][1] = sc[nb][2] = sc[nb][3] = 0.f;
+    // (coordinates 16 w + 64 kk of a row: two 16-byte pieces of its segment kk)
+    const int k_line = ((lane & 7) + 8 * (lane >> 4)) * SEGS, k_piece = 2 * w + ((lane >> 3) & 1);
+#pragma unroll
+    for (int kk = 0; kk < KPW; ++kk) {
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int line = k_line + half * 16 * SEGS + kk;
+        uint32_t b[4];
+        ldmatrix_x4(b[0], b[1], b[2], b[3], C + line * 128 + ((k_piece ^ (line & 7)) << 4));
+        mma_bf16_16816(sc[2 * half], qf[kk], b[0], b[1]);
+        mma_bf16_16816(sc[2 * half + 1], qf[kk], b[2], b[3]);
+      }
+    }
+    float2* mine = part_s + (((it & 1) * MTL + rt) * kSingleWarps + w) * 256 + lane;
+#pragma unroll
+    for (int nb = 0; nb < 4; ++nb)
+#pragma unroll
+      for (int hh = 0; hh < 2; ++hh) mine[(2 * nb + hh) * 32] = make_float2(sc[nb][2 * hh], sc[nb][2 * hh + 1]);
+    asm volatile("bar.sync %0, %1;" ::"r"(1 + rt), "n"(32 * kSingleWarps) : "memory");
+    const float2* all = part_s + ((it & 1) * MTL + rt) * kSingleWarps * 256 + lane;
+#pragma unroll
+    for (int nb = 0; nb < 4; ++nb)
+#pragma unroll
+      for (int hh = 0; hh < 2; ++hh) {
+        float2 x[kSingleWarps];
+#pragma unroll
+        for (int i = 0; i < kSingleWarps; ++i) x[i] = all[i * 256 + (2 * nb + hh) * 32];
+        sc[nb][2 * hh] = (x[0].x + x[1].x) + (x[2].x + x[3].x);
+        sc[nb][2 * hh + 1] = (x[0].y + x[1].y) + (x[2].y + x[3].y);
+      }
+    const int jk = first_key + 2 * tig;
+    float corr[2];
+    uint32_t pa[2][4];
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh) {
+      float v = -CUDART_INF_F;
+#pragma unroll
+      for (int nb = 0; nb < 4; ++nb)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int j = jk + 8 * nb + c;
+          float& x = sc[nb][2 * hh + c];
+          x *= scale2;
+          if (edge && (j < j_lo || j > p)) x = -CUDART_INF_F;
+          v = fmaxf(v, x);
+        }
+      v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
+      v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 2));
+      const float most = fmaxf(m[hh], v), mn = most == -CUDART_INF_F ? 0.f : most;   // (no key with a weight so far: all weights zero)
+      corr[hh] = ex2(m[hh] - mn);
+      m[hh] = most;
+      float ps = 0.f;
+#pragma unroll
+      for (int nb = 0; nb < 4; ++nb) {
+        const float p0 = ex2(sc[nb][2 * hh] - mn), p1 = ex2(sc[nb][2 * hh + 1] - mn);
+        ps += p0 + p1;
+        pa[nb >> 1][2 * (nb & 1) + hh] = pack_bf16(p0, p1);
+      }
+      l[hh] = l[hh] * corr[hh] + ps;
+    }
+    if (!__all_sync(0xffffffffu, corr[0] == 1.f && corr[1] == 1.f)) {
+#pragma unroll
+      for (int i = 0; i < NPW; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          acc[i][j][0] *= corr[0]; acc[i][j][1] *= corr[0];
+          acc[i][j][2] *= corr[1]; acc[i][j][3] *= corr[1];
+        }
+    }
+    const int v_line = ((lane & 7) + ((lane >> 3) & 1) * 8) * SEGS, v_piece = 2 * w + (lane >> 4);
+#pragma unroll
+    for (int i = 0; i < NPW; ++i) {   // columns 16 w + 64 i ..
+      if (w + kSingleWarps * i < n_pairs) {
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) {
+          const int line = v_line + ks * 16 * SEGS + i;
+          uint32_t b[4];
+          ldmatrix_x4_trans(b[0], b[1], b[2], b[3], C + line * 128 + ((v_piece ^ (line & 7)) << 4));
+          mma_bf16_16816(acc[i][0], pa[ks], b[0], b[1]);
+          mma_bf16_16816(acc[i][1], pa[ks], b[2], b[3]);
+        }
+      }
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(empty0 + 8 * s);
+  }
+#pragma unroll
+  for (int hh = 0; hh < 2; ++hh) {
+    l[hh] += __shfl_xor_sync(0xffffffffu, l[hh], 1);
+    l[hh] += __shfl_xor_sync(0xffffffffu, l[hh], 2);
+    if (!ok[hh]) continue;
+    const int h = h0 + gid + 8 * hh;
+    const size_t row = (size_t)t * H + h;
+    if (pieces == 1) {
+      const float g = gate ? 1.0f / (1.0f + expf(-to_f32(gate[(size_t)t * ldg + h]))) : 1.0f;
+      const float f = g / l[hh];
+#pragma unroll
+      for (int i = 0; i < NPW; ++i) {
+        const int np = w + kSingleWarps * i;
+        if (np < n_pairs)
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+            *reinterpret_cast<uint32_t*>(out + row * R + np * 16 + j * 8 + 2 * tig) =
+                pack_bf16(acc[i][j][2 * hh] * f, acc[i][j][2 * hh + 1] * f);
+      }
+    } else {
+      float* pa_out = part_acc + (row * num_splits + split) * R;
+#pragma unroll
+      for (int i = 0; i < NPW; ++i) {
+        const int np = w + kSingleWarps * i;
+        if (np < n_pairs)
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+            *reinterpret_cast<float2*>(pa_out + np * 16 + j * 8 + 2 * tig) = make_float2(acc[i][j][2 * hh], acc[i][j][2 * hh + 1]);
+      }
+      if (w == 0 && tig == 0) {
+        part_ml[(row * num_splits + split) * 2] = m[hh] * kLn2;
+        part_ml[(row * num_splits + split) * 2 + 1] = l[hh];
+      }
+    }
+  }
+}
+
 // out[t, h, :] = sigmoid(gate) * sum_s acc_s exp(m_s - M) / sum_s l_s exp(m_s - M); a block per (token, head),
 // a thread per column; the pieces' factors are worked out once, by the first warp
 constexpr int kMergeThreads = 128;
@@ -608,20 +890,26 @@ constexpr int kMergeMaxSplits = 64;
 __global__ void __launch_bounds__(kMergeThreads)
 latent_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml, int num_splits,
                     const __nv_bfloat16* __restrict__ gate, int ldg, __nv_bfloat16* __restrict__ out,
-                    const int* __restrict__ entry_of_token, int row_begin, int H, int R) {
+                    const int* __restrict__ entry_of_token, const int* __restrict__ pos0, int window, int row_begin, int H, int R) {
   ccb::pdl_begin();
   __shared__ float f[kMergeMaxSplits];
   const int t = row_begin + blockIdx.x / H, h = blockIdx.x % H;
-  if (entry_of_token[t] < 0) return;
+  const int e_row = entry_of_token[t];
+  if (e_row < 0) return;
   const size_t row = (size_t)t * H + h;
+  const int places = num_splits;   // of a row's pieces
+  if (pos0 != nullptr) {   // (after latent_single_kernel: what it wrote)
+    num_splits = single_pieces(pos0[e_row], window, num_splits);
+    if (num_splits == 1) return;
+  }
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
     float ms[2], ls[2];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int s = lane + 32 * i;
-      ms[i] = s < num_splits ? part_ml[(row * num_splits + s) * 2] : -CUDART_INF_F;
-      ls[i] = s < num_splits ? part_ml[(row * num_splits + s) * 2 + 1] : 0.f;
+      ms[i] = s < num_splits ? part_ml[(row * places + s) * 2] : -CUDART_INF_F;
+      ls[i] = s < num_splits ? part_ml[(row * places + s) * 2 + 1] : 0.f;
     }
     const float M = warp_max(fmaxf(ms[0], ms[1]));   // finite: piece 0 holds the sink
     float e[2];
@@ -634,7 +922,7 @@ latent_merge_kernel(const float* __restrict__ part_acc, const float* __restrict_
       if (lane + 32 * i < num_splits) f[lane + 32 * i] = e[i] * g / L;
   }
   __syncthreads();
-  const float* pa = part_acc + row * num_splits * R;
+  const float* pa = part_acc + row * places * R;
   const int c = blockIdx.y * kMergeThreads + threadIdx.x;   // a column a thread
   if (c < R) {
     float v0 = 0.f, v1 = 0.f;
@@ -792,6 +1080,35 @@ int launch_mma(const float* qa, const void* cache, const float* sink, const void
              window, scale, hpb, status);
   return ccb_launch_status();
 }
+
+// Single tokens whose rows are 64 SEGS coordinates, of pages of 8, 16 or a multiple of 32 rows.
+template <int SEGS, int MTL>
+int launch_single(const float* qa, const void* cache, const float* sink, const void* gate, int ldg, void* out, float* part_acc,
+                  float* part_ml, int num_splits, const int* cu_q, const int* pos0, const int* eot, const int* block_table,
+                  int bt_stride, int entry0, int n_entries, int H, int R, int page_size, int num_pages, int window, float scale,
+                  int* status, cudaStream_t stream) {
+  const int stage = kSingleKeys * 128 * SEGS, exchange = 2 * MTL * kSingleWarps * 256 * 8 + 1024;
+  const int room = (MTL == 1 ? 112 : 225) * 1024 - exchange;   // (two blocks an SM, or one)
+  const int stages = room / stage < kSingleStages ? room / stage : kSingleStages, bytes = stages * stage + exchange;
+  const int box_rows = page_size < kSingleKeys ? page_size : kSingleKeys;
+  CUtensorMap tm;
+  if (!ccb_tensor_map_rows(cache, (unsigned long long)num_pages * page_size, SEGS, box_rows, &tm)) return CCB_REFUSE_ARG;
+  const auto kernel = latent_single_kernel<SEGS, MTL>;
+  static std::atomic<unsigned long long> done{0};
+  const int rc = ccb_allow_smem(kernel, (MTL == 1 ? 112 : 225) * 1024, done);
+  if (rc != 0) return rc;
+  ccb_launch(kernel, dim3((H + 16 * MTL - 1) / (16 * MTL), n_entries * num_splits), dim3((kSingleWarps * MTL + 1) * 32), bytes,
+             stream, tm, qa, sink, (const __nv_bfloat16*)gate, ldg, (__nv_bfloat16*)out, part_acc, part_ml, num_splits, cu_q,
+             pos0, eot, block_table, bt_stride, entry0, H, R, page_size, num_pages, window, scale, box_rows, stages, status);
+  return ccb_launch_status();
+}
+
+// Whether single tokens go through latent_single_kernel.
+bool single_fits(const float* qa, const void* cache, int R, int W, int page_size, int num_pages) {
+  return (W == 192 || W == 320 || W == 576) && W - R >= 64 && (page_size == 8 || page_size == 16 || page_size % kSingleKeys == 0) && num_pages > 0 &&
+         (long long)num_pages * page_size < 0x7fffffffll &&
+         ((reinterpret_cast<uintptr_t>(cache) & 15) | (reinterpret_cast<uintptr_t>(qa) & 7)) == 0;
+}
 }  // namespace
 
 // Whether the tensor-core form takes these sizes (bfloat16 only).
@@ -821,7 +1138,21 @@ CCB_API int ccb_latent_attention_mma(const float* qa, const void* cache, const f
   rc = launch_mma<NPW, MTL, WARPS>(qa, cache, sink, gate, ldg, out, part_acc, part_ml, num_splits, cu_q, pos0,     \
                                    entry_of_token, block_table, bt_stride, entry0, n_entries, max_q, H, R, r,      \
                                    page_size, num_pages, window, scale, status, stream)
-  if (wide) {
+  const int W = R + r;
+  const bool single = max_q == 1 && single_fits(qa, cache, R, W, page_size, num_pages);
+  if (single) {
+#define CCB_LSINGLE(SEGS)                                                                                             \
+  rc = H <= 16 ? launch_single<SEGS, 1>(qa, cache, sink, gate, ldg, out, part_acc, part_ml, num_splits, cu_q, pos0,    \
+                                        entry_of_token, block_table, bt_stride, entry0, n_entries, H, R, page_size,   \
+                                        num_pages, window, scale, status, stream)                                     \
+               : launch_single<SEGS, 2>(qa, cache, sink, gate, ldg, out, part_acc, part_ml, num_splits, cu_q, pos0,    \
+                                        entry_of_token, block_table, bt_stride, entry0, n_entries, H, R, page_size,   \
+                                        num_pages, window, scale, status, stream)
+    if (W == 192) CCB_LSINGLE(3);
+    else if (W == 320) CCB_LSINGLE(5);
+    else CCB_LSINGLE(9);
+#undef CCB_LSINGLE
+  } else if (wide) {
     if (pairs_per_warp <= 1) CCB_LMMA(1, 2, 8);
     else if (pairs_per_warp <= 2) CCB_LMMA(2, 2, 8);
     else CCB_LMMA(4, 2, 8);
@@ -834,6 +1165,6 @@ CCB_API int ccb_latent_attention_mma(const float* qa, const void* cache, const f
 #undef CCB_LMMA
   if (rc != 0 || num_splits == 1) return rc;
   ccb_launch(latent_merge_kernel, dim3(n_entries * H, (R + kMergeThreads - 1) / kMergeThreads), dim3(kMergeThreads), 0, stream, part_acc, part_ml, num_splits,
-             (const __nv_bfloat16*)gate, ldg, (__nv_bfloat16*)out, entry_of_token, entry0, H, R);
+             (const __nv_bfloat16*)gate, ldg, (__nv_bfloat16*)out, entry_of_token, single ? pos0 : nullptr, window, entry0, H, R);
   return ccb_launch_status();
 }

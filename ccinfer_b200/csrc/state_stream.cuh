@@ -42,6 +42,7 @@ struct StateStream {
   int* status;
 };
 
+// bytes (a multiple of 16) side by side, both ends on 16 bytes
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
                "r"(bytes), "r"(bar)

@@ -60,6 +60,31 @@ bool ccb_tensor_map_2d(const void* ptr, unsigned long long rows, unsigned long l
   return tensor_map_2d(ptr, rows, cols, ld, box_cols, box_rows, true, out);
 }
 
+bool ccb_tensor_map_rows(const void* ptr, unsigned long long rows, unsigned segments, unsigned box_rows, CUtensorMap* out) {
+  const auto key = std::make_tuple(ptr, rows, 64ull * segments, 64ull * segments, segments, box_rows, 2);
+  std::lock_guard<std::mutex> lock(g_mu);
+  auto it = g_maps.find(key);
+  if (it != g_maps.end()) {
+    *out = it->second;
+    return true;
+  }
+  auto fn = encode_fn();
+  if (fn == nullptr) return false;
+  CUtensorMap tm;
+  const cuuint64_t dims[3] = {64, segments, (cuuint64_t)rows};
+  const cuuint64_t strides[2] = {128, 128ull * segments};
+  const cuuint32_t box[3] = {64, segments, box_rows};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = fn(&tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return false;
+  if (g_maps.size() > 4096) g_maps.clear();
+  g_maps[key] = tm;
+  *out = tm;
+  return true;
+}
+
 bool ccb_tensor_map_2d_plain(const void* ptr, unsigned long long rows, unsigned long long cols, unsigned long long ld,
                              unsigned box_cols, unsigned box_rows, CUtensorMap* out) {
   return tensor_map_2d(ptr, rows, cols, ld, box_cols, box_rows, false, out);

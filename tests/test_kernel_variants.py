@@ -871,3 +871,54 @@ def test_one_token_of_the_head_delta_rule_beside_its_blocks(E, H, G, dk, dv, tap
     assert (got[1] - want[1]).abs().max() <= 2.0 ** -19 * want[1].abs().max()
     near = 2.0 ** -19 if dtype == torch.float32 else 2.0 ** -7
     assert (got[2].float() - want[2].float()).abs().max() <= near * want[2].float().abs().max()
+
+
+# one and two tiles of heads, whole and in part; pages smaller than, as and larger than a tile of 32 keys; rows in one piece and many
+@pytest.mark.parametrize("H,R,r,page,window,splits", [
+    (16, 512, 64, 16, 1 << 30, 1), (5, 512, 64, 8, 1 << 30, 7), (32, 512, 64, 32, 100, 3), (17, 256, 64, 64, 1 << 30, 64), (1, 128, 64, 16, 33, 2),
+    (48, 128, 64, 8, 1 << 30, 1), (16, 112, 80, 16, 64, 5)])
+def test_latent_attention_of_single_tokens(H, R, r, page, window, splits):
+    """Against float64, in pages anywhere.  What a token does not see (rows after it, pages before its window) is no number.
+    Weights and results are rounded to bfloat16: 2^-9 of the largest coordinate each."""
+    k, g = _k(), _gen(H + R + page + splits)
+    ctx = [1, 31, 32, 33, 64, 200, 999]   # (keys that a token sees without a window, its own among them)
+    E, W, scale = len(ctx) + 1, R + r, 0.06
+    pages = [-(-n // page) for n in ctx] + [1]
+    order = torch.randperm(sum(pages), generator=torch.Generator().manual_seed(splits)).tolist()
+    cache = torch.full((sum(pages), page, W), float("nan"), dtype=torch.bfloat16, device="cuda")
+    table = torch.full((E, max(pages)), -1, dtype=torch.int32)
+    qa = torch.randn((E, H, W), generator=g, device="cuda").to(torch.bfloat16).float()
+    sink = torch.randn(H, generator=g, device="cuda")
+    gate = torch.randn((E, H + 3), generator=g, device="cuda").to(torch.bfloat16)[:, :H]
+    want, largest = torch.zeros(E, H, R, dtype=torch.float64, device="cuda"), 0.0
+    at = 0
+    for e, n in enumerate(ctx):
+        lo = max(0, n - window)
+        rows = torch.randn((n, W), generator=g, device="cuda").to(torch.bfloat16)
+        for i in range(pages[e]):
+            if (i + 1) * page <= lo:
+                continue   # (a page before the window is gone)
+            table[e, i] = order[at + i]
+            a, b = max(lo, i * page), min(n, (i + 1) * page)
+            cache[order[at + i], a - i * page:b - i * page] = rows[a:b]
+        at += pages[e]
+        c = rows[lo:].double()
+        s = torch.cat([qa[e].double() @ c.T * scale, sink.double()[:, None]], 1)
+        want[e] = torch.softmax(s, -1)[:, :-1] @ c[:, :R] * torch.sigmoid(gate[e].double())[:, None]
+        largest = max(largest, float(c[:, :R].abs().max()))
+
+    def dev(x):
+        return torch.tensor(x, dtype=torch.int32, device="cuda")
+
+    out = torch.full((E, H, R), 7.0, dtype=torch.bfloat16, device="cuda")
+    want[E - 1] = 7.0   # (a row that pads the step)
+    acc, ml = (torch.full((E * H * splits * m,), float("nan"), device="cuda") for m in (R, 2))
+    status = dev([0])
+    k.latent_attention_mma(qa, cache, sink, gate, out, dev(list(range(E + 1))), dev([n - 1 for n in ctx] + [0]),
+                           dev(list(range(E - 1)) + [-1]), table.cuda(), 0, E, 1, page, window, scale, splits, acc, ml, status)
+    assert int(status) == 0
+    assert (out.double() - want).abs().max() <= 2.0 ** -8 * largest
+    table[5, (ctx[5] - 1) // page] = sum(pages)   # a page that does not exist
+    k.latent_attention_mma(qa, cache, sink, gate, out, dev(list(range(E + 1))), dev([n - 1 for n in ctx] + [0]),
+                           dev(list(range(E - 1)) + [-1]), table.cuda(), 0, E, 1, page, window, scale, splits, acc, ml, status)
+    assert int(status) == 4

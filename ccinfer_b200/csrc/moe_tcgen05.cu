@@ -6,15 +6,19 @@
 // columns.  A cluster of two blocks works on a tile (tcgen05 cta_group::2, as gemm_tc_pair.cu: each block holds 128 of the
 // weight rows and half of the tokens), one cluster per pair of SMs walks over (token tile, 256 weight rows), weight rows
 // fastest, so that the clusters running at one time share a few tokens in L2 and read every weight once.  The ring of
-// stages (64 k) and the two accumulators of 256 columns run on from tile to tile.  Weights and tokens have a producer warp
+// stages (64 k) runs on from tile to tile, and so does tensor memory: its 512 columns are a ring of sixteen slots of 32, a tile
+// takes as many as it has columns, and the next one's products begin as soon as the slots that it needs have been read.  (Two
+// accumulators of 256 columns, both of which a tile of more tokens took, left its whole epilogue without products beside it.)
+// Weights and tokens have a producer warp
 // each: one thread for both set the pace (one instruction more in its loop, a copy to L2 ahead of the ring, made 64 tokens
 // 506 us in place of 430).
 //
 // What counts is bytes in flight: with four stages of 48 KB every size was a third slower than with six of 32, at any number
 // of tokens.  So CAP, the tokens of a tile at most, is 64 (11 stages of 20 KB: steps of few tokens are a stream of weights)
 // or 320 (six of 36 KB): where experts get some 256 tokens, which a prompt's step of 2,048 with 4 of 32 experts means, a
-// tile of 256 would leave half of them with a second one that reads all weights again.  More than 256 tokens are two parts of
-// about the same size, an accumulator each (256 and a few: the few cost what some hundred do).
+// tile of 256 would leave half of them with a second one that reads all weights again.  A product has neighbouring columns and 256
+// at most, so a tile is up to three of them (`TileParts`); each block of the pair holds one half of the tile's tokens, and the
+// columns of a product are some tokens of the one half and then as many of the other.
 //   * the weight operand is ONE tensor map over all experts' matrices, and the expert moves the box: down the rows (the
 //     first matrices, stacked [E F, D]) or along the columns (the second ones, side by side [D, E F]; what a box reads
 //     beyond the expert's F columns meets zeros of A, whose map ends at F);
@@ -24,8 +28,10 @@
 // The rows of A must lie in sorted order, so the tokens are gathered first (moe_gather_rows).
 // Every wait on an mbarrier is bounded as in gemm_tcgen05.cu.
 // Bound by the stream of weights up to some 130 rows an expert (32 of 4096 x 3072, 4 chosen, 128 tokens: 2.4 GB in 414 us, 5.9
-// TB/s), by that and the products together at 2,048 tokens (0.62 TFLOP in 750 us).  The whole part, 8 / 2,048 tokens: tiles of
-// 128 x 256 on one SM and 16 rows on mma.sync 413 / 1,161 us; this with four epilogue warps 284 / 956, with eight 280 / 866.
+// TB/s), by that and the products together at 2,048 tokens (0.62 TFLOP in 580 us).  The whole part, 8 / 2,048 tokens: tiles of
+// 128 x 256 on one SM and 16 rows on mma.sync 413 / 1,161 us; this with two accumulators and four epilogue warps 284 / 956, with
+// eight 280 / 770, with the ring of slots 280 / 665 (width 2,048, 2,048 tokens: 357 / 285).  A warp's signal that a slot has been
+// read does not wait for its stores (with a releasing one, 1,100 tokens of width 2,048 took 127 us in the first product, 109 so).
 #include "cluster_common.cuh"
 #include <cuda.h>
 #include <type_traits>
@@ -38,19 +44,34 @@ using namespace ccb;
 namespace {
 
 constexpr int kFeatures = 256;     // weight rows of a tile; each block loads 128 of them
-constexpr int kTokens = 256;       // tokens of an accumulator at most; each block loads half of them
-constexpr int kTokenStep = 32;     // what their number is rounded up to
+constexpr int kTokenStep = 32;     // what the number of a tile's tokens is rounded up to; each block loads half of them
+constexpr int kSlots = 16;         // of kTokenStep columns of tensor memory
+constexpr int kMostSlots = 8;      // of a product
 constexpr int kK = 64;
 constexpr int kWBytes = (kFeatures / 2) * kK * 2;   // 16 KB
 template <int CAP> struct Ring {
-  static constexpr int kParts = (CAP + kTokens - 1) / kTokens;
-  static constexpr int kPartBytes = CAP / 4 * kK * 2;         // of the first of two parts, at most
   static constexpr int kBytes = kWBytes + CAP / 2 * kK * 2;   // a stage: the weights, then the tokens
   static constexpr int kStages = CAP == 64 ? 11 : 6;
 };
 constexpr int kBoxes = 4;          // token copies come in boxes of 16, 32, 64 and 128 rows: at most three make up a block's half
 constexpr int kThreads = 352;     // warps: 0 weights, 1 products, 2 .. 9 epilogue, 10 tokens
-constexpr int kAcc = 2;            // accumulators of 256 columns in tensor memory
+
+// Where a tile's slots begin: behind the ones before, but a tile of one product is not cut by the ring's end.
+__device__ __forceinline__ int tile_place(int at, int slots) { return slots <= kMostSlots && at + slots > kSlots ? 0 : at; }
+
+// The products of a tile of `slots` slots from slot `at` on: runs that neither pass the ring's end nor have more than 256
+// columns, of about the same size where a run is cut; at most three (slots of the first, second, third).
+struct TileParts {
+  int len[3];
+  __device__ __forceinline__ TileParts(int at, int slots) {
+    const int head = min(slots, kSlots - at), tail = slots - head;
+    const int h = head > kMostSlots ? (head + 1) / 2 : head, t = tail > kMostSlots ? (tail + 1) / 2 : tail;
+    len[0] = h;
+    len[1] = head > h ? head - h : t;
+    len[2] = head > h ? t : tail - t;
+  }
+  __device__ __forceinline__ int count() const { return 1 + (len[1] > 0) + (len[2] > 0); }
+};
 
 struct TokenMaps {
   CUtensorMap box[kBoxes];   // 16 << i rows
@@ -71,12 +92,11 @@ moe_grouped_tc_kernel(const __grid_constant__ TokenMaps tmX, const __grid_consta
                       int F, const CcbGluAct act, int w_in, int* status) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  constexpr int kStages = Ring<CAP>::kStages, kBytes = Ring<CAP>::kBytes, XT = Ring<CAP>::kParts,
-                kPartBytes = Ring<CAP>::kPartBytes;
+  constexpr int kStages = Ring<CAP>::kStages, kBytes = Ring<CAP>::kBytes;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kStages * kBytes);
   const uint32_t full0 = s32(bars), empty0 = s32(bars + kStages), tfull0 = s32(bars + 2 * kStages),
-                 tempty0 = s32(bars + 2 * kStages + 2);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 4);
+                 tempty0 = s32(bars + 2 * kStages + kSlots);   // of a tile (in turn), of a slot
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 2 * kSlots);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();
   const bool leader = rank == 0;
@@ -84,20 +104,20 @@ moe_grouped_tc_kernel(const __grid_constant__ TokenMaps tmX, const __grid_consta
   const int nkb = (K + kK - 1) / kK;
   const int items = tiles.max_tiles * tiles.tiles_f;
 
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) {
-      mbar_init(full0 + 8 * s, 1);
-      mbar_init(empty0 + 8 * s, 1);
+  if (warp == 0) {   // a lane a barrier of each kind
+    if (lane < kStages) {
+      mbar_init(full0 + 8 * lane, 1);
+      mbar_init(empty0 + 8 * lane, 1);
     }
-    for (int b = 0; b < kAcc; ++b) {
-      mbar_init(tfull0 + 8 * b, 1);
-      mbar_init(tempty0 + 8 * b, 16);   // eight epilogue warps of each block
+    if (lane < kSlots) {
+      mbar_init(tfull0 + 8 * lane, 1);
+      mbar_init(tempty0 + 8 * lane, 16);   // eight epilogue warps of each block
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {   // a warp of EACH block of the pair allocates: the columns are taken in both
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s32(tmem_slot)),
-                 "r"((uint32_t)(kAcc * kTokens))
+                 "r"((uint32_t)(kSlots * kTokenStep))
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
@@ -109,26 +129,34 @@ moe_grouped_tc_kernel(const __grid_constant__ TokenMaps tmX, const __grid_consta
   pdl_wait();
   if (threadIdx.x == 0) pdl_trigger();
 
-  // every role walks over the same items: (token tile, 256 weight rows); the first token tile without rows ends the walk
-  auto columns = [](int n) { return (n + kTokenStep - 1) / kTokenStep * kTokenStep; };
-  auto part_columns = [&](int n, int parts, int a) {   // of part a of a tile of n tokens: two parts are as alike as steps allow
-    const int all = columns(n), first = parts == 1 ? all : columns((all + 1) / 2);
-    return a == 0 ? first : all - first;
+  // every role walks over the same items: (token tile, 256 weight rows); the first token tile without rows ends the walk.  Of
+  // wide tiles an item is asked for one ahead, since nobody should stop between two of them (2,048 tokens: 406 -> 399 us in the
+  // first product); a stream of weights alone has no use for it (8 tokens 169.6 with, 169.0 without).
+  constexpr bool kAhead = CAP != 64;
+  struct Item {
+    int tf, e, r0, n;
   };
+  auto item = [&](int t) {
+    Item x{0, 0, 0, 0};
+    if (t < items) {
+      const int ti = t / tiles.tiles_f;
+      x = Item{t - ti * tiles.tiles_f, tiles.e[ti], tiles.r0[ti], min(tiles.n[ti], CAP)};
+    }
+    return x;
+  };
+  auto columns = [](int n) { return (n + kTokenStep - 1) / kTokenStep * kTokenStep; };
   // (the ring's waits have the block's scope: what they order are copies and products, which the barriers count themselves)
   if (warp == 0) {
     if (lane == 0) {  // ---- TMA producer: this block's half of the weight rows ----
       int s = 0, ph = 0;
       bool alive = true;
       const uint32_t full_leader = map_to_rank(full0, 0);
-      for (int t = pair; t < items && alive; t += n_pairs) {
-        const int ti = t / tiles.tiles_f, tf = t - ti * tiles.tiles_f;
-        const int n = min(tiles.n[ti], CAP);
-        if (n <= 0) break;
-        const int e = tiles.e[ti];
-        const int w_row = (MODE != 1 ? e * F : 0) + tf * kFeatures + (int)rank * (kFeatures / 2);
-        const int w_col = MODE != 1 ? 0 : e * F;
-        const uint32_t bytes = 2 * kWBytes + columns(n) * kK * 2;   // of both blocks, the tokens' copies too
+      Item now = item(pair), next = now;
+      for (int t = pair; now.n > 0 && alive; t += n_pairs, now = kAhead ? next : item(t)) {
+        if (kAhead) next = item(t + n_pairs);
+        const int w_row = (MODE != 1 ? now.e * F : 0) + now.tf * kFeatures + (int)rank * (kFeatures / 2);
+        const int w_col = MODE != 1 ? 0 : now.e * F;
+        const uint32_t bytes = 2 * kWBytes + columns(now.n) * kK * 2;   // of both blocks, the tokens' copies too
         for (int kb = 0; kb < nkb; ++kb) {
           if (!mbar_wait(empty0 + 8 * s, ph ^ 1)) {
             set_status(status, CCB_ST_WAIT_TIMEOUT);
@@ -147,157 +175,188 @@ moe_grouped_tc_kernel(const __grid_constant__ TokenMaps tmX, const __grid_consta
       int s = 0, ph = 0;
       bool alive = true;
       const uint32_t full_leader = map_to_rank(full0, 0);
-      for (int t = pair; t < items && alive; t += n_pairs) {
-        const int ti = t / tiles.tiles_f;
-        const int n = min(tiles.n[ti], CAP);
-        if (n <= 0) break;
-        const int r0 = tiles.r0[ti];
-        // (tiles of one accumulator and of two have loops of their own: conditions inside cost every step of both)
-        auto walk = [&](auto parts) {
-          constexpr int P = decltype(parts)::value;
-          int half[P], x_row[P];
-#pragma unroll
-          for (int a = 0; a < P; ++a) {
-            half[a] = part_columns(n, P, a) / 2;
-            x_row[a] = r0 + (a ? part_columns(n, P, 0) : 0) + (int)rank * half[a];
+      Item now = item(pair), next = now;
+      for (int t = pair; now.n > 0 && alive; t += n_pairs, now = kAhead ? next : item(t)) {
+        if (kAhead) next = item(t + n_pairs);
+        const int half = columns(now.n) / 2, x_row = now.r0 + (int)rank * half;
+        for (int kb = 0; kb < nkb; ++kb) {
+          if (!mbar_wait(empty0 + 8 * s, ph ^ 1)) {
+            set_status(status, CCB_ST_WAIT_TIMEOUT);
+            alive = false;
+            break;
           }
-          for (int kb = 0; kb < nkb; ++kb) {
-            if (!mbar_wait(empty0 + 8 * s, ph ^ 1)) {
-              set_status(status, CCB_ST_WAIT_TIMEOUT);
-              alive = false;
-              return;
-            }
-            const uint32_t bar = full_leader + 8 * s, at = s32(smem + s * kBytes) + kWBytes;
+          const uint32_t bar = full_leader + 8 * s, at = s32(smem + s * kBytes) + kWBytes;
+          int x = 0;   // (one instruction a box sets the pace: eight boxes of 16 rows halved the rate of full tiles)
 #pragma unroll
-            for (int a = 0; a < P; ++a) {
-              int x = 0;   // (one instruction a box sets the pace: eight boxes of 16 rows halved the rate of full tiles)
-#pragma unroll
-              for (int b = kBoxes - 1; b >= 0; --b)
-                if (half[a] & (16 << b)) {
-                  tma_load_2d_pair(at + a * kPartBytes + x * kK * 2, &tmX.box[b], kb * kK, x_row[a] + x, bar);
-                  x += 16 << b;
-                }
+          for (int b = kBoxes - 1; b >= 0; --b)
+            if (half & (16 << b)) {
+              tma_load_2d_pair(at + x * kK * 2, &tmX.box[b], kb * kK, x_row + x, bar);
+              x += 16 << b;
             }
-            if (++s == kStages) s = 0, ph ^= 1;
-          }
-        };
-        if (XT == 1 || n <= kTokens) walk(std::integral_constant<int, 1>{});
-        else walk(std::integral_constant<int, XT>{});
+          if (++s == kStages) s = 0, ph ^= 1;
+        }
       }
     }
   } else if (warp == 1) {
     if (lane == 0 && leader) {  // ---- MMA issuer (the leader's): products of M = 256 over both blocks ----
-      int s = 0, ph = 0, local = 0;
+      int s = 0, ph = 0, local = 0, at = 0;
+      uint32_t used = 0;   // a bit a slot: how often it has been used, its last place
       bool alive = true;
-      for (int t = pair; t < items && alive; t += n_pairs) {
-        const int n = min(tiles.n[t / tiles.tiles_f], CAP);
-        if (n <= 0) break;
-        auto walk = [&](auto parts) {
-          constexpr int P = decltype(parts)::value;
-          uint32_t idesc[P], acc[P];
+      Item now = item(pair), next = now;
+      for (int t = pair; now.n > 0 && alive; t += n_pairs, now = kAhead ? next : item(t), ++local) {
+        if (kAhead) next = item(t + n_pairs);
+        const int slots = columns(now.n) / kTokenStep;
+        at = tile_place(at, slots);
+        // Warps read tiles in order, and a tile's even and odd slots in order, so that where the last two slots have been read
+        // all have (a wait for each of ten slots would take longer than the products of a short tile leave).
+        for (int i = max(0, slots - 2); i < slots && alive; ++i) {
+          const int b = at + i < kSlots ? at + i : at + i - kSlots;
+          alive = mbar_wait_cluster(tempty0 + 8 * b, (used >> b & 1) ^ 1);
+        }
+        const uint32_t taken = ((1u << slots) - 1) << at;
+        used ^= (taken | taken >> kSlots) & 0xffffu;
+        if (!alive) {
+          set_status(status, CCB_ST_WAIT_TIMEOUT);
+          break;
+        }
+        tc_fence_after();
+        const TileParts parts(at, slots);
+        auto walk = [&](auto count) {
+          constexpr int P = decltype(count)::value;
+          uint32_t idesc[P], acc[P], from[P];
 #pragma unroll
-          for (int a = 0; a < P; ++a) {
-            idesc[a] = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(part_columns(n, P, a) >> 3) << 17) |
+          for (int a = 0, first = 0; a < P; first += parts.len[a++]) {
+            idesc[a] = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(parts.len[a] * kTokenStep >> 3) << 17) |
                        ((uint32_t)(kFeatures >> 4) << 24);
-            acc[a] = tmem_base + ((local + a) % kAcc) * kTokens;
-            if (!mbar_wait_cluster(tempty0 + 8 * ((local + a) % kAcc), (((local + a) / kAcc) & 1) ^ 1)) return false;
+            acc[a] = tmem_base + (at + first) % kSlots * kTokenStep;
+            from[a] = first * (kTokenStep / 2) * kK * 2;
           }
-          tc_fence_after();
           for (int kb = 0; kb < nkb; ++kb) {
             if (!mbar_wait(full0 + 8 * s, ph)) return false;
             tc_fence_after();
             const uint64_t da = smem_desc(s32(smem + s * kBytes));
 #pragma unroll
             for (int a = 0; a < P; ++a) {
-              const uint64_t db = smem_desc(s32(smem + s * kBytes + kWBytes + a * kPartBytes));
+              const uint64_t db = smem_desc(s32(smem + s * kBytes + kWBytes) + from[a]);
 #pragma unroll
               for (int k = 0; k < kK / 16; ++k) tc_mma2(acc[a], da + 2 * k, db + 2 * k, idesc[a], (kb > 0 || k > 0) ? 1u : 0u);
             }
             tc_commit2(empty0 + 8 * s);
             if (++s == kStages) s = 0, ph ^= 1;
           }
-#pragma unroll
-          for (int a = 0; a < P; ++a) tc_commit2(tfull0 + 8 * ((local + a) % kAcc));
-          local += P;
+          tc_commit2(tfull0 + 8 * (local % kSlots));
           return true;
         };
-        alive = XT == 1 || n <= kTokens ? walk(std::integral_constant<int, 1>{}) : walk(std::integral_constant<int, XT>{});
+        const int count = CAP <= kMostSlots * kTokenStep ? 1 : parts.count();
+        alive = count == 1   ? walk(std::integral_constant<int, 1>{})
+                : count == 2 ? walk(std::integral_constant<int, 2>{})
+                             : walk(std::integral_constant<int, 3>{});
         if (!alive) set_status(status, CCB_ST_WAIT_TIMEOUT);
+        at = (at + slots) % kSlots;
       }
     }
   } else {  // ---- epilogue: this block's 128 weight rows (lanes), all tokens of the tile (columns) ----
-    // two warps a quarter of the lanes, which take 32 tokens in turn (one warp each left a third of a tile's time exposed
-    // where both accumulators are taken)
+    // two warps a quarter of the lanes, which take a slot in turn
     const int q = warp & 3, turn = (warp - 2) >> 2;
-    int local = 0;
-    bool alive = true;
-    for (int t = pair, n0 = 0; t < items && alive; ++local) {   // an accumulator at a time: tokens n0 .. of item t
-      const int ti = t / tiles.tiles_f, tf = t - ti * tiles.tiles_f;
-      const int n_tile = min(tiles.n[ti], CAP);
-      if (n_tile <= 0) break;
-      const int n = min(n_tile - n0, XT == 1 || n_tile <= kTokens ? kTokens : part_columns(n_tile, 2, n0 ? 1 : 0));
-      const int buf = local % kAcc;
-      alive = mbar_wait_cluster(tfull0 + 8 * buf, (local / kAcc) & 1);
-      if (!alive) {
+    int local = 0, at = 0;
+    Item now = item(pair), next = now;
+    for (int t = pair; now.n > 0; t += n_pairs, now = kAhead ? next : item(t), ++local) {
+      if (kAhead) next = item(t + n_pairs);
+      const int n = now.n;
+      if (!mbar_wait_cluster(tfull0 + 8 * (local % kSlots), (local / kSlots) & 1)) {
         if (lane == 0) set_status(status, CCB_ST_WAIT_TIMEOUT);
         break;
       }
       tc_fence_after();
-      const size_t g0 = (size_t)tiles.r0[ti] + n0;
-      const int col = tf * kFeatures + (int)rank * (kFeatures / 2) + q * 32 + lane;   // this lane's column of the product
-      const uint32_t taddr = tmem_base + buf * kTokens + ((uint32_t)(q * 32) << 16);
+      const int slots = columns(n) / kTokenStep, half = slots * (kTokenStep / 2);
+      at = tile_place(at, slots);
+      const TileParts parts(at, slots);
+      const size_t g0 = (size_t)now.r0;
+      const int col = now.tf * kFeatures + (int)rank * (kFeatures / 2) + q * 32 + lane;   // this lane's column of the product
+      auto done_with = [&](int i) {   // the leader counts all sixteen warps, so that none is a turn of the ring behind
+        const uint32_t bar = tempty0 + 8 * ((at + i) % kSlots);
+        if (leader) mbar_arrive(bar);
+        else mbar_arrive_remote_relaxed(map_to_rank(bar, 0));
+      };
+      if (lane == 0)
+        for (int i = turn ^ 1; i < slots; i += 2) done_with(i);
 #pragma unroll 1
-      for (int c0 = 32 * turn; c0 < n; c0 += 64) {
-        uint32_t v[32];
-        tc_ld32(taddr + c0, v);
-        tc_wait_ld();
-        const float my_w = MODE != 1 && c0 + lane < n ? row_w[g0 + c0 + lane] : 1.f;
-        if (MODE == 1) {
-          float* dst = (float*)Cout + (g0 + c0) * ldc + col;
+      for (int i = turn; i < slots; i += 2) {
+        const int b = (at + i) % kSlots;
+        // the tokens of the slot's columns, sixteen neighbours twice: of the product's columns the first half are tokens of the
+        // tile's first half
+        int tok[2];
+        {
+          const int second = parts.len[0], third = second + parts.len[1];   // where the products begin
+          const int first = i < second ? 0 : i < third ? second : third;
+          const int width = (i < second ? parts.len[0] : i < third ? parts.len[1] : parts.len[2]) * (kTokenStep / 2);   // of a half
 #pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (c0 + j < n && col < N) dst[(size_t)j * ldc] = __uint_as_float(v[j]);
-        } else if (MODE == 0) {
-          __nv_bfloat16* dst = (__nv_bfloat16*)Cout + (g0 + c0) * ldc + col;
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const float w = __shfl_sync(0xffffffffu, my_w, j), a = fmaxf(__uint_as_float(v[j]), 0.f);
-            if (c0 + j < n && col < N) dst[(size_t)j * ldc] = __float2bfloat16_rn(a * a * w);
+          for (int x = 0; x < 2; ++x) {
+            const int j = (i - first) * kTokenStep + 16 * x;
+            tok[x] = first * (kTokenStep / 2) + (j < width ? j : half + j - width);
           }
-        } else {   // columns (2 f, 2 f + 1) are gate f and up f: the even lane takes token j, the odd one token j + 1
+        }
+        const int mine = tok[lane >> 4] + (lane & 15);
+        const float my_w = MODE != 1 && mine < n ? row_w[g0 + mine] : 1.f;
+        uint32_t v[32];
+        tc_ld32(tmem_base + b * kTokenStep + ((uint32_t)(q * 32) << 16), v);
+        tc_wait_ld();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) done_with(i);
+        if (MODE == 2 && tok[0] + 16 <= n && tok[1] + 16 <= n) {   // (no condition a token: the activations of many run side by side)
           const int odd = lane & 1;
-          __nv_bfloat16* dst = (__nv_bfloat16*)Cout + (g0 + c0 + odd) * ldc + (col >> 1);
-          const bool mine = (col | 1) < N;
-          auto one = [&](int j) {
+          __nv_bfloat16* dst[2];
+#pragma unroll
+          for (int x = 0; x < 2; ++x) dst[x] = (__nv_bfloat16*)Cout + (g0 + tok[x] + odd) * ldc + (col >> 1);
+          const bool mine_col = (col | 1) < N;
+#pragma unroll
+          for (int j = 0; j < 32; j += 2) {
             const float w = __shfl_sync(0xffffffffu, my_w, j + odd);
             const float wi = w_in ? w : 1.f, wo = w_in ? 1.f : w;
-            const float a = __uint_as_float(v[j]), b = __uint_as_float(v[j + 1]);
-            const float got = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);   // what the other lane has of this lane's token
-            return glu_act(act, (odd ? got : a) * wi, (odd ? b : got) * wi) * wo;
-          };
-          if (c0 + 32 <= n) {   // (no condition a token: the activations of several run side by side)
+            const float a = __uint_as_float(v[j]), c = __uint_as_float(v[j + 1]);
+            const float got = __shfl_xor_sync(0xffffffffu, odd ? a : c, 1);
+            const float y = glu_act(act, (odd ? got : a) * wi, (odd ? c : got) * wi) * wo;
+            if (mine_col) dst[j >> 4][(size_t)(j & 15) * ldc] = __float2bfloat16_rn(y);
+          }
+          continue;
+        }
 #pragma unroll
-            for (int j = 0; j < 32; j += 2) {
-              const float y = one(j);
-              if (mine) dst[(size_t)j * ldc] = __float2bfloat16_rn(y);
+        for (int x = 0; x < 2; ++x) {
+          const size_t row = g0 + tok[x];
+          const int left = n - tok[x];   // of the sixteen tokens
+          if (MODE == 1) {
+            float* dst = (float*)Cout + row * ldc + col;
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+              if (j < left && col < N) dst[(size_t)j * ldc] = __uint_as_float(v[16 * x + j]);
+          } else if (MODE == 0) {
+            __nv_bfloat16* dst = (__nv_bfloat16*)Cout + row * ldc + col;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              const float w = __shfl_sync(0xffffffffu, my_w, 16 * x + j), a = fmaxf(__uint_as_float(v[16 * x + j]), 0.f);
+              if (j < left && col < N) dst[(size_t)j * ldc] = __float2bfloat16_rn(a * a * w);
             }
-          } else {
+          } else {   // columns (2 f, 2 f + 1) are gate f and up f: the even lane takes token j, the odd one token j + 1
+            const int odd = lane & 1;
+            __nv_bfloat16* dst = (__nv_bfloat16*)Cout + (row + odd) * ldc + (col >> 1);
+            const bool mine_col = (col | 1) < N;
+            auto one = [&](int j) {
+              const float w = __shfl_sync(0xffffffffu, my_w, 16 * x + j + odd);
+              const float wi = w_in ? w : 1.f, wo = w_in ? 1.f : w;
+              const float a = __uint_as_float(v[16 * x + j]), c = __uint_as_float(v[16 * x + j + 1]);
+              const float got = __shfl_xor_sync(0xffffffffu, odd ? a : c, 1);   // what the other lane has of this lane's token
+              return glu_act(act, (odd ? got : a) * wi, (odd ? c : got) * wi) * wo;
+            };
 #pragma unroll
-            for (int j = 0; j < 32; j += 2) {
+            for (int j = 0; j < 16; j += 2) {
               const float y = one(j);
-              if (mine && c0 + j + odd < n) dst[(size_t)j * ldc] = __float2bfloat16_rn(y);
+              if (mine_col && j + odd < left) dst[(size_t)j * ldc] = __float2bfloat16_rn(y);
             }
           }
         }
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) {   // this warp's quarter of this block's accumulator is free again: the leader counts sixteen
-        if (leader) mbar_arrive(tempty0 + 8 * buf);
-        else mbar_arrive_remote(map_to_rank(tempty0 + 8 * buf, 0));
-      }
-      n0 += n;
-      if (n0 >= n_tile) n0 = 0, t += n_pairs;
+      at = (at + slots) % kSlots;
     }
   }
   tc_fence_before();
@@ -305,7 +364,7 @@ moe_grouped_tc_kernel(const __grid_constant__ TokenMaps tmX, const __grid_consta
   cluster_sync_all();   // nobody leaves while the other block may still signal it or read its shared memory
   if (warp == 1) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)(kAcc * kTokens))
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)(kSlots * kTokenStep))
                  : "memory");
   }
 }
@@ -325,7 +384,7 @@ moe_gather_rows_kernel(uint4* __restrict__ out, const uint4* __restrict__ x, con
 template <int MODE, int CAP>
 int launch(const TokenMaps& tmX, const CUtensorMap& tmW, void* C, int ldc, const float* row_w, const GroupedTiles& tiles, int N,
            int K, int F, const CcbGluAct& act, int w_in, int sms, int* status, cudaStream_t stream) {
-  constexpr size_t smem = (size_t)Ring<CAP>::kStages * Ring<CAP>::kBytes + (2 * Ring<CAP>::kStages + 4) * 8 + 16 + 1024;
+  constexpr size_t smem = (size_t)Ring<CAP>::kStages * Ring<CAP>::kBytes + (2 * Ring<CAP>::kStages + 2 * kSlots) * 8 + 16 + 1024;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(moe_grouped_tc_kernel<MODE, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -31,7 +31,8 @@
 //
 // Bound by: the walk by the chain of its products (one block of eight warps an SM, an instruction on 0.30 of the cycles),
 // the preparation by what it issues (0.42).  Measured on B200, 2,048 tokens of one request, 32 heads of 128 x 128 with a
-// decay per channel and the delta rule: 193 + 105 us; token by token 959 us.  Outputs and memory are right to 5e-6 in the
+// decay per channel and the delta rule: 188 + 105 us (196 with the solve's operands split again by every 16 columns); token by
+// token 959 us.  Outputs and memory are right to 5e-6 in the
 // 2-norm, token by token to 1e-7 to 4e-7; in a layer's results, whose rows are bfloat16 (3.7e-3), neither shows.
 #include "common.cuh"
 #include "mma_common.cuh"
@@ -390,6 +391,7 @@ chunk_prepare_kernel(const ChunkRows a) {
   // ---- the triangular solve for X = [W | U]: with L the strictly lower blocks, X_i = (I + L_ii)^-1 (B_i - sum L_ij X_j)
   if constexpr (DELTA) {
     __syncthreads();
+    // (as operands, two neighbouring columns as their two bfloat16 in the place of two floats: every 16 columns of X read them)
     if (tid < kChunk) {   // a thread a column of an inverse, which takes its block's place
       const int run = tid / kRun, c = tid % kRun;
       float y[kRun];
@@ -404,7 +406,23 @@ chunk_prepare_kernel(const ChunkRows a) {
       }
       __syncwarp();
 #pragma unroll
-      for (int t = 0; t < kRun; ++t) l_s[lat(run * kRun + t, run * kRun + c)] = y[t];
+      for (int t = 0; t < kRun; ++t) {
+        const float right = __shfl_xor_sync(0xffffffffu, y[t], 1);
+        uint2 both;
+        split2(y[t], right, both.x, both.y);
+        if ((c & 1) == 0) *reinterpret_cast<uint2*>(l_s + lat(run * kRun + t, run * kRun + c)) = both;
+      }
+    } else {   // the blocks below them, negated
+      constexpr int kRest = kThreads - kChunk;
+      for (int x = tid - kChunk; x < 6 * kRun * kRun / 2; x += kRest) {
+        const int b = x / (kRun * kRun / 2), i = b < 1 ? 1 : b < 3 ? 2 : 3, j = b - i * (i - 1) / 2;
+        const int t = i * kRun + x % (kRun * kRun / 2) / (kRun / 2), s = j * kRun + 2 * (x % (kRun / 2));
+        float* at = l_s + lat(t, s);
+        const float2 l = *reinterpret_cast<const float2*>(at);
+        uint2 both;
+        split2(t < cnt ? -l.x : 0.f, t < cnt ? -l.y : 0.f, both.x, both.y);
+        *reinterpret_cast<uint2*>(at) = both;
+      }
     }
     __syncthreads();
     const int runs = (cnt + kRun - 1) / kRun;
@@ -441,8 +459,9 @@ chunk_prepare_kernel(const ChunkRows a) {
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
               const int t = i * kRun + nb * 8 + gid;
-              const float2 l = *reinterpret_cast<const float2*>(l_s + lat(t, j * kRun + 8 * half + 2 * tig));
-              split2(t < cnt ? -l.x : 0.f, t < cnt ? -l.y : 0.f, bh[half], bl[half]);
+              const uint2 l = *reinterpret_cast<const uint2*>(l_s + lat(t, j * kRun + 8 * half + 2 * tig));
+              bh[half] = l.x;
+              bl[half] = l.y;
             }
             mma3(x[nb], xh[j], xl[j], bh[0], bh[1], bl[0], bl[1]);
           }
@@ -474,8 +493,9 @@ chunk_prepare_kernel(const ChunkRows a) {
           uint32_t bh[2], bl[2];
 #pragma unroll
           for (int half = 0; half < 2; ++half) {
-            const float2 l = *reinterpret_cast<const float2*>(l_s + lat(i * kRun + nb * 8 + gid, i * kRun + 8 * half + 2 * tig));
-            split2(l.x, l.y, bh[half], bl[half]);
+            const uint2 l = *reinterpret_cast<const uint2*>(l_s + lat(i * kRun + nb * 8 + gid, i * kRun + 8 * half + 2 * tig));
+            bh[half] = l.x;
+            bl[half] = l.y;
           }
           mma3(x[nb], ah, al, bh[0], bh[1], bl[0], bl[1]);
         }

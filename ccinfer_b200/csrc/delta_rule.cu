@@ -28,6 +28,12 @@ namespace {
 
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + expf(-x)); }
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log1pf(expf(x)); }
+// The sigmoid in steps of many rows: the accurate form in 32 bits; where inputs and results of the layer are bfloat16 anyway,
+// the fast exponential and division (a few units of the last place of a float), an eighth of the instructions.
+template <typename T> __device__ __forceinline__ float silu_of(float x) { return x * sigmoid_f(x); }
+template <> __device__ __forceinline__ float silu_of<__nv_bfloat16>(float x) { return __fdividef(x, 1.f + __expf(-x)); }
+template <typename T> __device__ __forceinline__ float sigmoid_of(float x) { return sigmoid_f(x); }
+template <> __device__ __forceinline__ float sigmoid_of<__nv_bfloat16>(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
 
 // ---------------------------------------------------------------------------------------------
 // proj [T, ld]: columns q (at oq, G*dk), k (at ok, G*dk), v (at ov, H*dv), b (at ob, H); a [T, lda]: H*dk
@@ -203,7 +209,7 @@ delta_prepare_vec_kernel(const T* __restrict__ proj, int ld, int oq, int ok, int
 
 // The same with four neighbouring rows a warp as well: the taps' weights are loaded once for all of them, a row once for all
 // the taps it meets, and all loads are in flight together.  dk, dv <= 128, TAPS taps.  A warp a row set what it issued by
-// its loads: 140 us for 2,048 tokens of 32 heads of 128 with four taps, 87 us.
+// its loads: 140 us for 2,048 tokens of 32 heads of 128 with four taps, 87 us with the accurate sigmoid, 77 so.
 constexpr int kPrepRun = 4;
 
 template <typename T> struct Raw4;   // four neighbouring elements as they are stored
@@ -299,8 +305,7 @@ delta_prepare_run_kernel(const T* __restrict__ proj, int ld, int oq, int ok, int
       acc[2] += cw[j].z * win[j].z;
       acc[3] += cw[j].w * win[j].w;
     }
-    const float4 y = make_float4(acc[0] * sigmoid_f(acc[0]), acc[1] * sigmoid_f(acc[1]), acc[2] * sigmoid_f(acc[2]),
-                                 acc[3] * sigmoid_f(acc[3]));
+    const float4 y = make_float4(silu_of<T>(acc[0]), silu_of<T>(acc[1]), silu_of<T>(acc[2]), silu_of<T>(acc[3]));
     float f = 1.f;
     if (!is_v)   // (zeros beyond the head's channels)
       f = (is_q ? q_mult : 1.0f) / sqrtf(warp_sum((y.x * y.x + y.y * y.y) + (y.z * y.z + y.w * y.w)) + unit_eps);
@@ -627,6 +632,39 @@ __global__ void gated_head_rmsnorm_vec_kernel(T* __restrict__ y, const float* __
   }
 }
 
+// The same for value sizes up to 128 and many rows: four neighbouring heads a warp, their loads in flight together (2,048 rows of
+// 32 heads of 128, 67 MB: 28 us a head a warp with the accurate sigmoid, 21 so).
+constexpr int kNormRun = 4;
+template <typename T, bool SILU>
+__global__ void __launch_bounds__(256)
+gated_head_rmsnorm_run_kernel(T* __restrict__ y, const float* __restrict__ o, const T* __restrict__ gate, int ldg,
+                              const float* __restrict__ w, int units, int H, int dv, float eps) {
+  ccb::pdl_begin();
+  const int u0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * kNormRun, i = 4 * (threadIdx.x & 31);
+  const bool on = i < dv;
+  const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 x[kNormRun], g[kNormRun];
+#pragma unroll
+  for (int r = 0; r < kNormRun; ++r) {
+    const int u = u0 + r, t = u / H, h = u - t * H;
+    x[r] = g[r] = none;
+    if (on && u < units) {
+      x[r] = load4(o + (size_t)u * dv + i);
+      g[r] = load4(gate + (size_t)t * ldg + (size_t)h * dv + i);
+    }
+  }
+  const float4 ww = on ? load4(w + i) : none;
+#pragma unroll
+  for (int r = 0; r < kNormRun; ++r) {
+    const float ss = warp_sum(x[r].x * x[r].x + x[r].y * x[r].y + x[r].z * x[r].z + x[r].w * x[r].w);
+    const float inv = 1.0f / sqrtf(ss / (float)dv + eps);
+    auto act = [](float z) { return SILU ? silu_of<T>(z) : sigmoid_of<T>(z); };
+    if (on && u0 + r < units)
+      store4<T>(y + (size_t)(u0 + r) * dv + i, make_float4(x[r].x * inv * ww.x * act(g[r].x), x[r].y * inv * ww.y * act(g[r].y),
+                                                           x[r].z * inv * ww.z * act(g[r].z), x[r].w * inv * ww.w * act(g[r].w)));
+  }
+}
+
 }  // namespace
 
 CCB_API int ccb_delta_prepare(const void* proj, int ld, int oq, int ok, int ov, int ob, const void* a, int lda,
@@ -805,10 +843,16 @@ CCB_API int ccb_ssm_recurrence(const float* qn, const float* kn, const float* vv
                                       single_slots, status);
 }
 
+// rows x heads from which on a warp takes four; before, one head a warp has more loads under way (heads of 128, a head / four a
+// warp, us alone: 4,800 3.65 / 4.11, 9,600 5.05 / 4.68, 38,400 13.9 / 10.6, 65,536 22.3 / 15.8)
+constexpr int kNormRunUnits = 148 * 56;
 template <typename T, bool SILU>
 static void launch_head_norm(bool vec, dim3 grid, void* y, const float* o, const void* gate, int ldg, const float* w,
                              int rows, int H, int dv, float eps, cudaStream_t stream) {
-  if (vec)
+  if (vec && dv <= 128 && rows * H >= kNormRunUnits)
+    ccb_launch(gated_head_rmsnorm_run_kernel<T, SILU>, dim3((rows * H + 8 * kNormRun - 1) / (8 * kNormRun)), dim3(256), 0, stream,
+               (T*)y, o, (const T*)gate, ldg, w, rows * H, H, dv, eps);
+  else if (vec)
     ccb_launch(gated_head_rmsnorm_vec_kernel<T, SILU>, grid, dim3(256), 0, stream, (T*)y, o, (const T*)gate, ldg, w,
                rows, H, dv, eps);
   else

@@ -64,11 +64,10 @@ gla_prepare_vec_kernel(const T* __restrict__ proj, int ld, int oq, int ok, int o
                        float inv_tau) {
   ccb::pdl_begin();
   const int qk = H * dk, vw = H * dv;
-  const int per_row = (3 * qk + vw) >> 2;
-  const size_t total = (size_t)rows * per_row;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-    const size_t t = i / per_row;
-    int c = (int)(i - t * per_row) * 4;
+  const int c4 = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+  if (c4 >= 3 * qk + vw) return;
+  for (size_t t = blockIdx.y; t < (size_t)rows; t += gridDim.y) {   // (a row a block: no thread divides to find its place)
+    int c = c4;
     const T* row = proj + t * ld;
     if (c < qk) {
       const float4 x = ld4<T>(row + oq + c);
@@ -103,13 +102,12 @@ CCB_API int ccb_gla_prepare(const void* proj, int ld, int oq, int ok, int ov, co
                           reinterpret_cast<uintptr_t>(kn) | reinterpret_cast<uintptr_t>(vv) |
                           reinterpret_cast<uintptr_t>(gg);
   if (((H * dk) | (H * dv) | ld | lda | oq | ok | ov) % 4 == 0 && (bases & 15) == 0) {
-    const size_t total4 = (size_t)rows * ((3 * H * dk + H * dv) / 4);
-    const int blocks4 = (int)((total4 + 255) / 256 < 65535 * 8 ? (total4 + 255) / 256 : 65535 * 8);
+    const dim3 blocks4(((3 * H * dk + H * dv) / 4 + 255) / 256, rows < 65535 ? rows : 65535);
     if (dtype == CCB_F32)
-      ccb_launch(gla_prepare_vec_kernel<float>, dim3(blocks4), dim3(256), 0, stream, (const float*)proj, ld, oq, ok, ov,
+      ccb_launch(gla_prepare_vec_kernel<float>, blocks4, dim3(256), 0, stream, (const float*)proj, ld, oq, ok, ov,
                  (const float*)a, lda, bias, qn, kn, vv, gg, rows, H, dk, dv, q_mult, 1.0f / tau);
     else
-      ccb_launch(gla_prepare_vec_kernel<__nv_bfloat16>, dim3(blocks4), dim3(256), 0, stream,
+      ccb_launch(gla_prepare_vec_kernel<__nv_bfloat16>, blocks4, dim3(256), 0, stream,
                  (const __nv_bfloat16*)proj, ld, oq, ok, ov, (const __nv_bfloat16*)a, lda, bias, qn, kn, vv, gg, rows, H,
                  dk, dv, q_mult, 1.0f / tau);
     return ccb_launch_status();

@@ -39,6 +39,13 @@ struct SsmChunkRows {
 };
 
 __device__ __forceinline__ float sigmoid_acc(float x) { return 1.f / (1.f + expf(-x)); }
+// x sigmoid(x) in steps of many rows: the accurate form in 32 bits; where inputs and results of the layer are bfloat16 anyway,
+// the fast exponential and division (a few units of the last place of a float), an eighth of the instructions.
+template <typename T> __device__ __forceinline__ float silu_of(float x) { return x * sigmoid_acc(x); }
+template <> __device__ __forceinline__ float silu_of<__nv_bfloat16>(float x) { return __fdividef(x, 1.f + __expf(-x)); }
+template <typename T> __device__ __forceinline__ float4 silu4_of(float4 x) {
+  return make_float4(silu_of<T>(x.x), silu_of<T>(x.y), silu_of<T>(x.z), silu_of<T>(x.w));
+}
 __device__ __forceinline__ float softplus_acc(float x) { return x > 20.f ? x : log1pf(expf(x)); }
 
 // proj [T, ld]: the convolved channels (x | B | C, `C` of them) start at column ox, dt at odt.
@@ -213,7 +220,7 @@ __global__ void ssm_prepare_vec_kernel(const T* __restrict__ proj, int ld, int o
 // The same for steps of many rows: a thread takes its four channels (or its head) through kSsmRun neighbouring rows.  The taps'
 // weights are loaded once for all of them, a row once for all the taps it meets, all loads are in flight together, and no
 // thread divides to find its place.  TAPS taps.  2,048 rows of 10,240 channels with four taps, 150 MB: 90 us a row a
-// thread, 60 us.
+// thread, 60 us with the accurate sigmoid, 46 so.
 constexpr int kSsmRun = 4;
 // from here on, rows times (groups of four channels and heads): before that a row a thread has more loads under way (10,240 channels
 // and 128 heads, with 20 us of launch, a row / four rows a thread: 128 rows 28.5 / 29.9 us, 256 34.5 / 34.6, 512 45 / 38)
@@ -282,8 +289,7 @@ ssm_prepare_run_kernel(const T* __restrict__ proj, int ld, int ox, int odt, cons
         acc.z = fmaf(cw[j].z, win[j].z, acc.z);
         acc.w = fmaf(cw[j].w, win[j].w, acc.w);
       }
-      v = make_float4(acc.x * sigmoid_acc(acc.x), acc.y * sigmoid_acc(acc.y), acc.z * sigmoid_acc(acc.z),
-                      acc.w * sigmoid_acc(acc.w));
+      v = silu4_of<T>(acc);
       if (shift_single && TAPS > 1 && slot >= 0 && s_single[r]) {   // (as in the kernel above)
         V* st = reinterpret_cast<V*>(state_rw + (size_t)slot * (TAPS - 1) * C + c);
         for (int k = 0; k + 1 < TAPS - 1; ++k) st[(size_t)k * C4] = st[(size_t)(k + 1) * C4];
@@ -353,10 +359,11 @@ ssm_gate_norm_kernel(T* __restrict__ y, const float* __restrict__ o, const float
 
 // The same, a warp a (token, slice) that holds it in registers, four neighbouring channels a lane at a time: slices of up to
 // 128 VPL channels (a multiple of 4), P, the columns and the row strides multiples of 4, rows on 16 (bfloat16: 8) bytes.
-// One pass over 201 MB for 2,048 tokens of 8,192 channels in 8 slices, no barrier: 97 us before, 66 now.
+// One pass over 201 MB for 2,048 tokens of 8,192 channels in 8 slices, no barrier: 97 us before, 66 with the accurate sigmoid and
+// all rows at once, 54 so.
 constexpr int kGateWarps = 8;
 template <typename T, int VPL>
-__global__ void __launch_bounds__(kGateWarps * 32)
+__global__ void __launch_bounds__(kGateWarps * 32, VPL == 8 ? 3 : 4)   // (loads under way count)
 ssm_gate_norm_vec_kernel(T* __restrict__ y, const float* __restrict__ o, const float* __restrict__ xs,
                          const T* __restrict__ proj, int ld, int oz, const float* __restrict__ Dskip,
                          const float* __restrict__ w, int P, int inner, int parts, float eps, int units) {
@@ -367,26 +374,34 @@ ssm_gate_norm_vec_kernel(T* __restrict__ y, const float* __restrict__ o, const f
   const float* orow = o + (size_t)t * inner + c0;
   const float* xrow = xs + (size_t)t * inner + c0;
   const T* zrow = proj + (size_t)t * ld + oz + c0;
-  float4 v[VPL], x[VPL], z[VPL];
+  float4 v[VPL];
+  typename In4<T>::Raw z[VPL];
 #pragma unroll
   for (int i = 0; i < VPL; ++i) {
     const int c = 4 * lane + 128 * i;
-    v[i] = x[i] = z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    z[i] = {};
     if (c < width) {
       v[i] = *reinterpret_cast<const float4*>(orow + c);
-      x[i] = *reinterpret_cast<const float4*>(xrow + c);
-      z[i] = In4<T>::load(zrow + c);
+      z[i] = *reinterpret_cast<const typename In4<T>::Raw*>(zrow + c);
     }
+  }
+#pragma unroll
+  for (int i = 0; i < VPL; ++i) {   // (x goes in as it comes: three rows at once would leave an SM half its warps)
+    const int c = 4 * lane + 128 * i;
+    if (c >= width) continue;
+    const float4 x = *reinterpret_cast<const float4*>(xrow + c);
+    const float d = Dskip[(c0 + c) / P];
+    v[i].x = fmaf(d, x.x, v[i].x);
+    v[i].y = fmaf(d, x.y, v[i].y);
+    v[i].z = fmaf(d, x.z, v[i].z);
+    v[i].w = fmaf(d, x.w, v[i].w);
   }
   float ss = 0.f;
 #pragma unroll
   for (int i = 0; i < VPL; ++i) {
-    const int c = 4 * lane + 128 * i;
-    const float d = c < width ? Dskip[(c0 + c) / P] : 0.f;
-    v[i].x = fmaf(d, x[i].x, v[i].x) * (z[i].x * sigmoid_acc(z[i].x));
-    v[i].y = fmaf(d, x[i].y, v[i].y) * (z[i].y * sigmoid_acc(z[i].y));
-    v[i].z = fmaf(d, x[i].z, v[i].z) * (z[i].z * sigmoid_acc(z[i].z));
-    v[i].w = fmaf(d, x[i].w, v[i].w) * (z[i].w * sigmoid_acc(z[i].w));
+    const float4 g = silu4_of<T>(In4<T>::value(z[i]));
+    v[i].x *= g.x; v[i].y *= g.y; v[i].z *= g.z; v[i].w *= g.w;
     ss += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
   }
   ss = warp_sum(ss);

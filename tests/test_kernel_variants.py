@@ -922,3 +922,21 @@ def test_latent_attention_of_single_tokens(H, R, r, page, window, splits):
     k.latent_attention_mma(qa, cache, sink, gate, out, dev(list(range(E + 1))), dev([n - 1 for n in ctx] + [0]),
                            dev(list(range(E - 1)) + [-1]), table.cuda(), 0, E, 1, page, window, scale, splits, acc, ml, status)
     assert int(status) == 4
+
+
+# rows x heads from which on a warp takes four heads: left-over heads, lanes without channels, a gate inside wider rows
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("silu", [False, True])
+@pytest.mark.parametrize("T,H,dv", [(2763, 3, 128), (8289, 1, 4), (830, 10, 100), (8287, 1, 64)])
+def test_gated_head_norm_of_many_rows(T, H, dv, silu, dtype):
+    """Against float64: the norm, a weight and the gate, rounded once."""
+    k, g = _k(), _gen(T + dv)
+    o, w = torch.randn((T, H, dv), generator=g, device="cuda"), torch.randn(dv, generator=g, device="cuda")
+    wide = 4 * torch.randn((T, H * dv + 8), generator=g, device="cuda").to(dtype)
+    gate, y = wide[:, 8:], torch.full((T, H * dv), float("nan"), dtype=dtype, device="cuda")
+    k.gated_head_rmsnorm(y, o, gate, w, H, dv, 1e-5, silu_gate=silu)
+    z = gate.double().view(T, H, dv)
+    x = o.double()
+    want = x / torch.sqrt(x.square().mean(-1, keepdim=True) + 1e-5) * w.double() * torch.sigmoid(z) * (z if silu else 1)
+    rel = (2.0 ** -8 if dtype == torch.bfloat16 else 0) + 2.0 ** -19   # (a sum of dv squares and some twenty operations; the rounding)
+    assert ((y.double().view(T, H, dv) - want).abs() <= rel * want.abs() + 1e-30).all()

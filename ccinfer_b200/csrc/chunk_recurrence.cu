@@ -49,6 +49,15 @@ constexpr int kRun = 16;           // tokens of a run
 constexpr float kLeastLog2 = -115.f;
 constexpr float kSteepLog2 = 55.f;   // (2^110 times 128 products stays in a float, also in places that nobody sees)
 
+// Gated linear attention's rows as the projections left them, in place of q, k, v and g: q times q_mult, k and v; the decay is
+// sigmoid(a + bias)^(1 / tau).
+struct RawRows {
+  const __nv_bfloat16 *q, *k, *v, *a;   // q, k [T, ld] with head h at column h DK, v [T, ld] at h dv, a [T, lda] at h DK
+  int ld, lda;
+  const float* bias;                    // [H DK] or null
+  float q_mult, inv_tau;
+};
+
 struct ChunkRows {
   const float *q, *k, *v, *g, *beta;   // q, k [T, G, DK]; v [T, H, dv]; g [T, H, DK], or [T, H] with one decay a head
   __nv_bfloat16 *qs, *ks, *w;          // [T, H, 2, DK]: a row's bfloat16 values, then what their rounding left
@@ -58,7 +67,15 @@ struct ChunkRows {
   float *state, *out;                  // [slots, H, dv, DK], [T, H, dv]
   const int *cu_q, *state_slot;
   int entry0, G, H, dv, n_slots;
+  RawRows raw;
 };
+
+__device__ __forceinline__ float4 four(const __nv_bfloat16* p) {
+  const uint2 r = *reinterpret_cast<const uint2*>(p);
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.x));
+  const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.y));
+  return make_float4(a.x, a.y, b.x, b.y);
+}
 
 __device__ __forceinline__ float ex2(float x) {
   float y;
@@ -132,7 +149,7 @@ __device__ __noinline__ RunSides separate(float x0, float x1, float x2, float x3
   return r;
 }
 
-template <int DK, bool DELTA, bool HEAD>
+template <int DK, bool DELTA, bool HEAD, bool RAW = false>
 __global__ void __launch_bounds__(kThreads, 2)
 chunk_prepare_kernel(const ChunkRows a) {
   ccb::pdl_begin();
@@ -157,7 +174,12 @@ chunk_prepare_kernel(const ChunkRows a) {
   for (int i = tid; i < kChunk * DK / 4; i += kThreads) {
     const int t = i / (DK / 4), c = 4 * (i % (DK / 4));
     float4 q = make_float4(0.f, 0.f, 0.f, 0.f), k = q;
-    if (t < cnt) {
+    if (RAW && t < cnt) {
+      const size_t row = (size_t)(r0 + t) * a.raw.ld + kvh * DK + c;
+      q = four(a.raw.q + row);
+      k = four(a.raw.k + row);
+      q.x *= a.raw.q_mult; q.y *= a.raw.q_mult; q.z *= a.raw.q_mult; q.w *= a.raw.q_mult;
+    } else if (t < cnt) {
       const size_t row = ((size_t)(r0 + t) * a.G + kvh) * DK + c;
       q = *reinterpret_cast<const float4*>(a.q + row);
       k = *reinterpret_cast<const float4*>(a.k + row);
@@ -199,15 +221,23 @@ chunk_prepare_kernel(const ChunkRows a) {
 #pragma unroll
     for (int i = 0; i < PT; ++i) {
       const int t = part * PT + i;
-      x[i] = t < cnt ? a.g[((size_t)(r0 + t) * a.H + h) * DK + d] : 1.f;
+      if (RAW) x[i] = t < cnt ? __bfloat162float(a.raw.a[(size_t)(r0 + t) * a.raw.lda + h * DK + d]) : 0.f;
+      else x[i] = t < cnt ? a.g[((size_t)(r0 + t) * a.H + h) * DK + d] : 1.f;
     }
+    const float bias = RAW && a.raw.bias != nullptr ? a.raw.bias[h * DK + d] : 0.f;
+    // (straight from the logistic's argument: a decay near one would lose its logarithm's places to its own rounding)
+    auto log_logistic = [&](float z) {
+      const float l = (fminf(z, 0.f) - log1pf(expf(-fabsf(z)))) * (a.raw.inv_tau * 1.44269504088896f);
+      return l < kLeastLog2 ? kLeastLog2 : l;
+    };
     int mine = 0;
 #pragma unroll
     for (int m = 0; m < PT / kRun; ++m) {
       float sum = 0.f, first_sum = 0.f, mid = 0.f;
 #pragma unroll
       for (int i = 0; i < kRun; ++i) {
-        sum += log_decay(x[m * kRun + i]);
+        if (RAW) sum += part * PT + m * kRun + i < cnt ? log_logistic(x[m * kRun + i] + bias) : 0.f;
+        else sum += log_decay(x[m * kRun + i]);
         c_s[at<DK>(part * PT + m * kRun + i, d)] = sum;
         if (i == 0) first_sum = sum;
         if (i == kRun / 2 - 1) mid = sum;
@@ -545,7 +575,7 @@ template <int DK, bool DELTA> struct WalkShape {
   static constexpr int kBytes = kElements * 2;
 };
 
-template <int DK, bool DELTA>
+template <int DK, bool DELTA, bool RAW = false>
 __global__ void __launch_bounds__(kThreads)
 chunk_walk_kernel(const ChunkRows a) {
   ccb::pdl_begin();
@@ -636,9 +666,12 @@ chunk_walk_kernel(const ChunkRows a) {
     for (int up = 0; up < 2; ++up) {
       const int t = wr * 16 + gid + 8 * up;
       const float* row = src + ((size_t)(r0 + ch * kChunk + t) * a.H + h) * a.dv + col0 + wc * 16 + 2 * tig;
+      const __nv_bfloat16* raw = a.raw.v + (size_t)(r0 + ch * kChunk + t) * a.raw.ld + h * a.dv + col0 + wc * 16 + 2 * tig;
 #pragma unroll
       for (int nb = 0; nb < 2; ++nb) {
-        const float2 x = t < left ? *reinterpret_cast<const float2*>(row + nb * 8) : make_float2(0.f, 0.f);
+        const float2 x = t >= left ? make_float2(0.f, 0.f)
+                         : RAW     ? __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(raw + nb * 8))
+                                   : *reinterpret_cast<const float2*>(row + nb * 8);
         u[nb][2 * up] = x.x;
         u[nb][2 * up + 1] = x.y;
         o[nb][2 * up] = o[nb][2 * up + 1] = 0.f;
@@ -762,10 +795,10 @@ chunk_walk_kernel(const ChunkRows a) {
   }
 }
 
-template <int DK, bool DELTA, bool HEAD>
+template <int DK, bool DELTA, bool HEAD, bool RAW = false>
 int launch_chunked(const ChunkRows& a, int n_entries, int max_tokens, cudaStream_t stream) {
-  auto prepare = chunk_prepare_kernel<DK, DELTA, HEAD>;
-  auto walk = chunk_walk_kernel<DK, DELTA>;
+  auto prepare = chunk_prepare_kernel<DK, DELTA, HEAD, RAW>;
+  auto walk = chunk_walk_kernel<DK, DELTA, RAW>;
   constexpr int prep_bytes = PrepShape<DK, DELTA, HEAD>::kBytes, walk_bytes = WalkShape<DK, DELTA>::kBytes;
   static_assert(walk_bytes <= 227 * 1024 && prep_bytes <= 227 * 1024, "shared memory of a block");
   static std::atomic<unsigned long long> prep_done{0}, walk_done{0};
@@ -801,11 +834,31 @@ CCB_API int ccb_chunk_recurrence(const float* q, const float* k, const float* v,
     return CCB_REFUSE_ARG;
   if (G != H && (qs == (const void*)q || ks == (const void*)k)) return CCB_REFUSE_ARG;
   const ChunkRows a{q, k, v, g, beta, (__nv_bfloat16*)qs, (__nv_bfloat16*)ks, (__nv_bfloat16*)w, u, (__nv_bfloat16*)p, keep,
-                    state, out, cu_q, state_slot, entry0, G, H, dv, n_slots};
+                    state, out, cu_q, state_slot, entry0, G, H, dv, n_slots, RawRows{}};
 #define CCB_CHUNK(DK, DELTA)                                                                \
   (head_decay ? launch_chunked<DK, DELTA, true>(a, n_entries, max_tokens, stream) \
               : launch_chunked<DK, DELTA, false>(a, n_entries, max_tokens, stream))
   if (dk == 128) return beta != nullptr ? CCB_CHUNK(128, true) : CCB_CHUNK(128, false);
   return beta != nullptr ? CCB_CHUNK(64, true) : CCB_CHUNK(64, false);
 #undef CCB_CHUNK
+}
+
+// The form without the delta rule and with one decay per channel, from the projections' bfloat16 rows (see RawRows): q, k and v
+// are the first columns of rows ld apart, on 8 bytes, a's rows lda apart.  Workspace as above.
+CCB_API int ccb_chunk_recurrence_raw(const void* q, const void* k, const void* v, int ld, const void* a_rows, int lda,
+                                     const float* bias, float q_mult, float tau, void* qs, void* ks, void* p, float* keep,
+                                     float* state, float* out, const int* cu_q, const int* state_slot, int entry0, int n_entries,
+                                     int max_tokens, int H, int dk, int dv, int n_slots, cudaStream_t stream) {
+  if (n_entries <= 0) return 0;
+  if (H <= 0 || (dk != 64 && dk != 128) || dv <= 0 || dv % kCols || entry0 < 0 || max_tokens <= 0 || H > 65535 ||
+      n_entries > 65535 || ld % 4 || !(tau > 0.f))
+    return CCB_REFUSE_SIZE;
+  const auto bits = [](const void* x) { return reinterpret_cast<uintptr_t>(x); };
+  if (((bits(qs) | bits(ks) | bits(p) | bits(out)) & 15) || ((bits(q) | bits(k) | bits(v)) & 7)) return CCB_REFUSE_ARG;
+  const RawRows raw{(const __nv_bfloat16*)q, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, (const __nv_bfloat16*)a_rows, ld, lda,
+                    bias, q_mult, 1.0f / tau};
+  const ChunkRows a{nullptr, nullptr, nullptr, nullptr, nullptr, (__nv_bfloat16*)qs, (__nv_bfloat16*)ks, nullptr, nullptr,
+                    (__nv_bfloat16*)p, keep, state, out, cu_q, state_slot, entry0, H, H, dv, n_slots, raw};
+  return dk == 128 ? launch_chunked<128, false, false, true>(a, n_entries, max_tokens, stream)
+                   : launch_chunked<64, false, false, true>(a, n_entries, max_tokens, stream);
 }

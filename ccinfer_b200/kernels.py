@@ -205,6 +205,8 @@ _SIGNATURES = {
                        + [c_int] * 7 + [c_float, c_float, c_int, c_int, c_void_p],
     "ccb_memory_chunks": [c_void_p] * 4 + [c_int, c_void_p, c_int] + [c_void_p] * 6 + [c_int] * 7 + [c_float, c_void_p],
     "ccb_chunk_recurrence": [c_void_p] * 15 + [c_int] * 9 + [c_void_p],
+    "ccb_chunk_recurrence_raw": [c_void_p] * 3 + [c_int, c_void_p, c_int, c_void_p, c_float, c_float] + [c_void_p] * 8 + [c_int] * 7
+                                + [c_void_p],
     "ccb_latent_rows": [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p] + [c_int] * 6
                        + [c_void_p, c_void_p],
     "ccb_latent_query_rows": [c_void_p, c_void_p, c_int, c_void_p, c_int, c_float, c_void_p] + [c_int] * 5 + [c_void_p],
@@ -702,6 +704,33 @@ def chunk_recurrence(scratch, qn, kn, vv, gg, bb, state, out, cu_q, state_slot, 
                                       out.data_ptr(), cu_q.data_ptr(), state_slot.data_ptr(), entry0, n_entries, max_tokens,
                                       G, H, dk, dv, state.shape[0], 1 if head else 0, _stream()), "chunk_recurrence")
     counters.own += 1   # two kernels
+
+
+def chunk_recurrence_raw(scratch, proj, offsets, a, bias, qs, ks, state, out, cu_q, state_slot, entry0: int, n_entries: int,
+                         max_tokens: int, H: int, dk: int, dv: int, q_mult: float, tau: float) -> None:
+    """``gla_prepare`` and ``chunk_recurrence`` (bb None) of the entries entry0 .. in one: the chunks read the projections'
+    bfloat16 rows themselves (``chunk_raw_fits``).  qs, ks: float workspaces [T, H, dk]."""
+    _cuda(qs, ks, state, out, cu_q, state_slot, bias)
+    T = out.shape[0]
+    assert proj.dtype == a.dtype == torch.bfloat16 and proj.stride(1) == a.stride(1) == 1 and a.shape == (T, H * dk)
+    assert out.shape == (T, H, dv) and state.shape[1:] == (H, dv, dk) and state.dtype == out.dtype == torch.float32
+    assert qs.shape[0] >= T and ks.shape[0] >= T and qs.dtype == ks.dtype == torch.float32 and qs[0].numel() == ks[0].numel() == H * dk
+    assert bias is None or (bias.dtype == torch.float32 and bias.numel() == H * dk)
+    p = scratch("chunk_p", "tokens", (H, 2, 64), torch.bfloat16)
+    keep = scratch("chunk_keep", "chunks", (H, dk), torch.float32)
+    assert p.shape[0] >= T and keep.shape[0] >= T // 64 + entry0 + n_entries
+    base = proj.data_ptr()
+    _check(lib().ccb_chunk_recurrence_raw(base + 2 * offsets[0], base + 2 * offsets[1], base + 2 * offsets[2], proj.stride(0),
+                                          a.data_ptr(), a.stride(0), _p(bias), float(q_mult), float(tau), qs.data_ptr(), ks.data_ptr(),
+                                          p.data_ptr(), keep.data_ptr(), state.data_ptr(), out.data_ptr(), cu_q.data_ptr(),
+                                          state_slot.data_ptr(), entry0, n_entries, max_tokens, H, dk, dv, state.shape[0],
+                                          _stream()), "chunk_recurrence_raw")
+    counters.own += 1   # two kernels
+
+
+def chunk_raw_fits(proj, offsets) -> bool:
+    """Whether the chunks can read these rows themselves: four neighbouring columns at once."""
+    return proj.stride(0) % 4 == 0 and all(o % 4 == 0 for o in offsets) and proj.data_ptr() % 8 == 0
 
 
 class HeadDelta:

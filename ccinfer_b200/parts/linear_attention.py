@@ -89,16 +89,24 @@ class GatedLinearAttention(Mixer):
         kn = rt.scratch.get("delta_k", (rt.max_tokens, H, dk), f32)[:T]
         vv = rt.scratch.get("delta_v", (rt.max_tokens, H, dv), f32)[:T]
         gg = rt.scratch.get("delta_g", (rt.max_tokens, H, dk), f32)[:T]
-        kernels.gla_prepare(proj, (self.oq, self.ok, self.ov), a, self.a2_bias, qn, kn, vv, gg, H, dk, dv,
-                            dk ** -0.5, self.tau)
+        offsets = (self.oq, self.ok, self.ov)
         o = rt.scratch.get("delta_o", (rt.max_tokens, H, dv), f32)[:T]
-        # (a step lists its single tokens first: they, and short portions, go token by token)
+        # (a step lists its single tokens first: they, and short portions, go token by token, from rows made for them; the chunks
+        # read the projections' rows themselves)
         chunks = kernels.chunk_recurrence_fits(rt.dtype, dk, dv, step.max_q_len, (T - step.n_single) * H, False)
         n1 = step.n_single if chunks else step.n_entries
+        raw = chunks and kernels.chunk_raw_fits(proj, offsets)
+        made = n1 if raw else T   # rows (single tokens: one each)
+        if made:
+            kernels.gla_prepare(proj[:made], offsets, a[:made], self.a2_bias, qn[:made], kn[:made], vv[:made], gg[:made], H, dk, dv,
+                                dk ** -0.5, self.tau)
         if n1:
             kernels.gated_linear_recurrence(qn, kn, vv, gg, state, o, step.cu_q, step.state_slot, n1, H, dk, dv,
                                             single=n1 == step.n_single, status=rt.status)
-        if step.n_entries > n1:
+        if step.n_entries > n1 and raw:
+            kernels.chunk_recurrence_raw(rt.chunk_scratch, proj, offsets, a, self.a2_bias, qn, kn, state, o, step.cu_q,
+                                         step.state_slot, n1, step.n_entries - n1, step.max_q_len, H, dk, dv, dk ** -0.5, self.tau)
+        elif step.n_entries > n1:
             kernels.chunk_recurrence(rt.chunk_scratch, qn, kn, vv, gg, None, state, o, step.cu_q, step.state_slot, n1,
                                      step.n_entries - n1, step.max_q_len, H, H, dk, dv)
         y = rt.scratch.get("delta_y", (rt.max_tokens, H * dv), rt.dtype)[:T]

@@ -940,3 +940,40 @@ def test_gated_head_norm_of_many_rows(T, H, dv, silu, dtype):
     want = x / torch.sqrt(x.square().mean(-1, keepdim=True) + 1e-5) * w.double() * torch.sigmoid(z) * (z if silu else 1)
     rel = (2.0 ** -8 if dtype == torch.bfloat16 else 0) + 2.0 ** -19   # (a sum of dv squares and some twenty operations; the rounding)
     assert ((y.double().view(T, H, dv) - want).abs() <= rel * want.abs() + 1e-30).all()
+
+
+# portions around the runs of 16 and chunks of 64, behind single tokens; rows and decays inside wider rows; with and without a bias
+@pytest.mark.parametrize("H,dk,dv,tau,bias", [(3, 128, 128, 16.0, True), (2, 64, 32, 1.0, False), (1, 128, 64, 0.5, True)])
+def test_gated_linear_chunks_from_the_projections_rows(H, dk, dv, tau, bias):
+    """Against float64 from the same bfloat16 rows: operands as two bfloat16 (2^-17 each), as the chunks from float rows."""
+    k, g = _k(), _gen(H + dk + dv)
+    lens, first = [1, 1, 2, 15, 17, 64, 65, 130], 2
+    T, oq, ok, ov = sum(lens), 4, 4 + H * dk, 8 + 2 * H * dk
+    proj = torch.randn((T, 12 + 2 * H * dk + H * dv), generator=g, device="cuda").to(torch.bfloat16)
+    a = (3 * torch.randn((T, H * dk + 1), generator=g, device="cuda")).to(torch.bfloat16)[:, 1:]
+    b = 2 + torch.randn(H * dk, generator=g, device="cuda") if bias else None
+    state = torch.randn((len(lens) + 1, H, dv, dk), generator=g, device="cuda")
+    slots = torch.randperm(len(lens) + 1, generator=torch.Generator().manual_seed(2)).tolist()[:len(lens)]
+    slots[4] = -1
+    cu = [0] + torch.tensor(lens).cumsum(0).tolist()
+
+    def dev(x):
+        return torch.tensor(x, dtype=torch.int32, device="cuda")
+
+    def scratch(key, per, shape, dtype):
+        return torch.full((T if per == "tokens" else T // 64 + len(lens),) + tuple(shape), float("nan"), dtype=dtype, device="cuda")
+
+    q, key = (proj[:, o:o + H * dk].double().view(T, H, dk) for o in (oq, ok))
+    v = proj[:, ov:ov + H * dv].double().view(T, H, dv)
+    decay = torch.sigmoid(a.double() + (b.double() if bias else 0)).view(T, H, dk) ** (1 / tau)
+    out, after = torch.full((T, H, dv), 7.0, device="cuda"), state.double()
+    want = out.double()
+    for e, slot in enumerate(slots):
+        if e >= first and slot >= 0:
+            s = slice(cu[e], cu[e + 1])
+            want[s], after[slot] = _recurrence64(0.3 * q[s], key[s], v[s], decay[s], None, state[slot].double())
+    work = [torch.full((T, H, dk), float("nan"), device="cuda") for _ in range(2)]
+    k.chunk_recurrence_raw(scratch, proj, (oq, ok, ov), a, b, *work, state, out, dev(cu), dev(slots), first, len(lens) - first,
+                           max(lens), H, dk, dv, 0.3, tau)
+    assert (out.double() - want).abs().max() <= 2.0 ** -14 * want.abs().max()
+    assert (state.double() - after).abs().max() <= 2.0 ** -14 * after.abs().max()

@@ -31,7 +31,7 @@
 //
 // Bound by: the walk by the chain of its products (one block of eight warps an SM, an instruction on 0.30 of the cycles),
 // the preparation by what it issues (0.42).  Measured on B200, 2,048 tokens of one request, 32 heads of 128 x 128 with a
-// decay per channel and the delta rule: 188 + 105 us (196 with the solve's operands split again by every 16 columns); token by
+// decay per channel and the delta rule: 190 + 105 us (196 with the solve's operands split again by every 16 columns); token by
 // token 959 us.  Outputs and memory are right to 5e-6 in the
 // 2-norm, token by token to 1e-7 to 4e-7; in a layer's results, whose rows are bfloat16 (3.7e-3), neither shows.
 #include "common.cuh"
@@ -50,12 +50,16 @@ constexpr float kLeastLog2 = -115.f;
 constexpr float kSteepLog2 = 55.f;   // (2^110 times 128 products stays in a float, also in places that nobody sees)
 
 // Gated linear attention's rows as the projections left them, in place of q, k, v and g: q times q_mult, k and v; the decay is
-// sigmoid(a + bias)^(1 / tau).
+// sigmoid(a + bias)^(1 / tau).  Measured on B200, 1,537 tokens of three requests, 16 heads of 128, a layer: 173 -> 162 us (the rows'
+// kernel of 18 us gone, preparation 33 -> 40, walk 40 -> 43).
+// The delta rule takes only its decays so, exp(-exp(A_log) softplus(a + bias)): at 2,048 tokens of 32 heads the rows' kernel 76 -> 60 us,
+// the preparation 190 -> 197, a layer 605 -> 596.  Its q, k and v too, convolved by the preparation: 270 without a rows' kernel, 617.
 struct RawRows {
   const __nv_bfloat16 *q, *k, *v, *a;   // q, k [T, ld] with head h at column h DK, v [T, ld] at h dv, a [T, lda] at h DK
   int ld, lda;
   const float* bias;                    // [H DK] or null
   float q_mult, inv_tau;
+  const float* A_log;                   // [H] (delta rule)
 };
 
 struct ChunkRows {
@@ -174,7 +178,7 @@ chunk_prepare_kernel(const ChunkRows a) {
   for (int i = tid; i < kChunk * DK / 4; i += kThreads) {
     const int t = i / (DK / 4), c = 4 * (i % (DK / 4));
     float4 q = make_float4(0.f, 0.f, 0.f, 0.f), k = q;
-    if (RAW && t < cnt) {
+    if (RAW && !DELTA && t < cnt) {
       const size_t row = (size_t)(r0 + t) * a.raw.ld + kvh * DK + c;
       q = four(a.raw.q + row);
       k = four(a.raw.k + row);
@@ -225,9 +229,12 @@ chunk_prepare_kernel(const ChunkRows a) {
       else x[i] = t < cnt ? a.g[((size_t)(r0 + t) * a.H + h) * DK + d] : 1.f;
     }
     const float bias = RAW && a.raw.bias != nullptr ? a.raw.bias[h * DK + d] : 0.f;
-    // (straight from the logistic's argument: a decay near one would lose its logarithm's places to its own rounding)
-    auto log_logistic = [&](float z) {
-      const float l = (fminf(z, 0.f) - log1pf(expf(-fabsf(z)))) * (a.raw.inv_tau * 1.44269504088896f);
+    // (straight from the projections' row: a decay near one would lose its logarithm's places to its own rounding)
+    const float rate = RAW && DELTA ? expf(a.raw.A_log[h]) : 0.f;
+    auto log_raw = [&](float z) {
+      float l;
+      if (DELTA) l = -rate * (z > 20.f ? z : log1pf(expf(z))) * 1.44269504088896f;
+      else l = (fminf(z, 0.f) - log1pf(expf(-fabsf(z)))) * (a.raw.inv_tau * 1.44269504088896f);
       return l < kLeastLog2 ? kLeastLog2 : l;
     };
     int mine = 0;
@@ -236,7 +243,7 @@ chunk_prepare_kernel(const ChunkRows a) {
       float sum = 0.f, first_sum = 0.f, mid = 0.f;
 #pragma unroll
       for (int i = 0; i < kRun; ++i) {
-        if (RAW) sum += part * PT + m * kRun + i < cnt ? log_logistic(x[m * kRun + i] + bias) : 0.f;
+        if (RAW) sum += part * PT + m * kRun + i < cnt ? log_raw(x[m * kRun + i] + bias) : 0.f;
         else sum += log_decay(x[m * kRun + i]);
         c_s[at<DK>(part * PT + m * kRun + i, d)] = sum;
         if (i == 0) first_sum = sum;
@@ -798,7 +805,7 @@ chunk_walk_kernel(const ChunkRows a) {
 template <int DK, bool DELTA, bool HEAD, bool RAW = false>
 int launch_chunked(const ChunkRows& a, int n_entries, int max_tokens, cudaStream_t stream) {
   auto prepare = chunk_prepare_kernel<DK, DELTA, HEAD, RAW>;
-  auto walk = chunk_walk_kernel<DK, DELTA, RAW>;
+  auto walk = chunk_walk_kernel<DK, DELTA, RAW && !DELTA>;
   constexpr int prep_bytes = PrepShape<DK, DELTA, HEAD>::kBytes, walk_bytes = WalkShape<DK, DELTA>::kBytes;
   static_assert(walk_bytes <= 227 * 1024 && prep_bytes <= 227 * 1024, "shared memory of a block");
   static std::atomic<unsigned long long> prep_done{0}, walk_done{0};
@@ -819,9 +826,10 @@ int launch_chunked(const ChunkRows& a, int n_entries, int max_tokens, cudaStream
 // or [T, H], beta float [T, H] (null: no delta rule).  Workspace: qs, ks and (delta rule) w [T, H, 2, dk] and p
 // [T, H, 2, 64] bfloat16, u float [T, H, dv] (delta rule), keep float [T / 64 + entries, H, dk].  qs, ks, w and u may be
 // the memory of q, k (where G = H), g (one decay per channel) and v: a block writes a row after it has read it, and
-// nobody else reads it.
-CCB_API int ccb_chunk_recurrence(const float* q, const float* k, const float* v, const float* g, const float* beta, void* qs,
-                                 void* ks, void* w, float* u, void* p, float* keep, float* state, float* out,
+// nobody else reads it.  With the delta rule the decays per channel may come as the projection's bfloat16 rows a_rows, lda apart
+// (see RawRows; g is not read then).
+CCB_API int ccb_chunk_recurrence(const float* q, const float* k, const float* v, const float* g, const float* beta,
+                                 const void* a_rows, int lda, const float* a_bias, const float* A_log, void* qs, void* ks, void* w, float* u, void* p, float* keep, float* state, float* out,
                                  const int* cu_q, const int* state_slot, int entry0, int n_entries, int max_tokens, int G, int H,
                                  int dk, int dv, int n_slots, int head_decay, cudaStream_t stream) {
   if (n_entries <= 0) return 0;
@@ -829,12 +837,17 @@ CCB_API int ccb_chunk_recurrence(const float* q, const float* k, const float* v,
       H > 65535 || n_entries > 65535)
     return CCB_REFUSE_SIZE;
   if (beta != nullptr && (w == nullptr || u == nullptr)) return CCB_REFUSE_ARG;
+  if (a_rows != nullptr && (beta == nullptr || head_decay || a_bias == nullptr || A_log == nullptr)) return CCB_REFUSE_ARG;
   const auto bits = [](const void* x) { return reinterpret_cast<uintptr_t>(x); };
   if ((bits(q) | bits(k) | bits(v) | bits(g) | bits(qs) | bits(ks) | bits(w) | bits(u) | bits(p) | bits(out)) & 15)
     return CCB_REFUSE_ARG;
   if (G != H && (qs == (const void*)q || ks == (const void*)k)) return CCB_REFUSE_ARG;
   const ChunkRows a{q, k, v, g, beta, (__nv_bfloat16*)qs, (__nv_bfloat16*)ks, (__nv_bfloat16*)w, u, (__nv_bfloat16*)p, keep,
-                    state, out, cu_q, state_slot, entry0, G, H, dv, n_slots, RawRows{}};
+                    state, out, cu_q, state_slot, entry0, G, H, dv, n_slots,
+                    RawRows{nullptr, nullptr, nullptr, (const __nv_bfloat16*)a_rows, 0, lda, a_bias, 0.f, 0.f, A_log}};
+  if (a_rows != nullptr)
+    return dk == 128 ? launch_chunked<128, true, false, true>(a, n_entries, max_tokens, stream)
+                     : launch_chunked<64, true, false, true>(a, n_entries, max_tokens, stream);
 #define CCB_CHUNK(DK, DELTA)                                                                \
   (head_decay ? launch_chunked<DK, DELTA, true>(a, n_entries, max_tokens, stream) \
               : launch_chunked<DK, DELTA, false>(a, n_entries, max_tokens, stream))
@@ -856,7 +869,7 @@ CCB_API int ccb_chunk_recurrence_raw(const void* q, const void* k, const void* v
   const auto bits = [](const void* x) { return reinterpret_cast<uintptr_t>(x); };
   if (((bits(qs) | bits(ks) | bits(p) | bits(out)) & 15) || ((bits(q) | bits(k) | bits(v)) & 7)) return CCB_REFUSE_ARG;
   const RawRows raw{(const __nv_bfloat16*)q, (const __nv_bfloat16*)k, (const __nv_bfloat16*)v, (const __nv_bfloat16*)a_rows, ld, lda,
-                    bias, q_mult, 1.0f / tau};
+                    bias, q_mult, 1.0f / tau, nullptr};
   const ChunkRows a{nullptr, nullptr, nullptr, nullptr, nullptr, (__nv_bfloat16*)qs, (__nv_bfloat16*)ks, nullptr, nullptr,
                     (__nv_bfloat16*)p, keep, state, out, cu_q, state_slot, entry0, H, H, dv, n_slots, raw};
   return dk == 128 ? launch_chunked<128, false, false, true>(a, n_entries, max_tokens, stream)

@@ -50,7 +50,7 @@ delta_prepare_kernel(const T* __restrict__ proj, int ld, int oq, int ok, int ov,
                      const int* __restrict__ entry_of_token, const int* __restrict__ cu_q,
                      const int* __restrict__ state_slot, float* __restrict__ qn, float* __restrict__ kn,
                      float* __restrict__ vv, float* __restrict__ gg, float* __restrict__ bb, int G, int H, int dk,
-                     int dv, float q_mult, float unit_eps) {
+                     int dv, float q_mult, float unit_eps, int g_rows) {
   ccb::pdl_begin();
   const int t = blockIdx.x;
   const int e = entry_of_token[t];
@@ -77,7 +77,7 @@ delta_prepare_kernel(const T* __restrict__ proj, int ld, int oq, int ok, int ov,
   };
 
   // units: G query heads, G key heads (unit vectors), H value heads, H decay rows
-  const int units = 2 * G + 2 * H;
+  const int units = 2 * G + (t < g_rows ? 2 : 1) * H;   // (no decays beyond g_rows)
   const int u = blockIdx.y * kPrepWarps + (threadIdx.x >> 5);   // a warp per unit
   if (u < units) {
     if (u < 2 * G) {
@@ -131,7 +131,7 @@ delta_prepare_vec_kernel(const T* __restrict__ proj, int ld, int oq, int ok, int
                          const int* __restrict__ entry_of_token, const int* __restrict__ cu_q,
                          const int* __restrict__ state_slot, float* __restrict__ qn, float* __restrict__ kn,
                          float* __restrict__ vv, float* __restrict__ gg, float* __restrict__ bb, int G, int H, int dk,
-                         int dv, float q_mult, float unit_eps) {
+                         int dv, float q_mult, float unit_eps, int g_rows) {
   ccb::pdl_begin();
   const int t = blockIdx.x;
   const int e = entry_of_token[t];
@@ -160,7 +160,7 @@ delta_prepare_vec_kernel(const T* __restrict__ proj, int ld, int oq, int ok, int
                        acc[3] * sigmoid_f(acc[3]));
   };
 
-  const int units = 2 * G + 2 * H;
+  const int units = 2 * G + (t < g_rows ? 2 : 1) * H;   // (no decays beyond g_rows)
   const int u = blockIdx.y * kPrepWarps + (threadIdx.x >> 5);
   if (u >= units) return;
   if (u < 2 * G) {
@@ -233,12 +233,12 @@ delta_prepare_run_kernel(const T* __restrict__ proj, int ld, int oq, int ok, int
                          const float* __restrict__ dt_bias, const int* __restrict__ entry_of_token,
                          const int* __restrict__ cu_q, const int* __restrict__ state_slot, float* __restrict__ qn,
                          float* __restrict__ kn, float* __restrict__ vv, float* __restrict__ gg, float* __restrict__ bb,
-                         int rows, int G, int H, int dk, int dv, float q_mult, float unit_eps) {
+                         int rows, int G, int H, int dk, int dv, float q_mult, float unit_eps, int g_rows) {
   using V = typename Raw4<T>::V;
   ccb::pdl_begin();
   const int t0 = blockIdx.x * kPrepRun, lane = threadIdx.x & 31;
   const int u = blockIdx.y * kPrepWarps + (threadIdx.x >> 5);
-  if (u >= 2 * G + 2 * H) return;
+  if (u >= 2 * G + 2 * H || (u >= 2 * G + H && t0 >= g_rows)) return;
   // what the rows' requests are: a lane a row, handed round below
   int m_slot = -1, m_lt = 0;
   if (lane < kPrepRun && t0 + lane < rows) {
@@ -263,7 +263,7 @@ delta_prepare_run_kernel(const T* __restrict__ proj, int ld, int oq, int ok, int
     const float4 b = load4(dt_bias + head * dk + i);
 #pragma unroll
     for (int r = 0; r < kPrepRun; ++r) {
-      if (t0 + r >= rows) break;
+      if (t0 + r >= g_rows) break;
       const int e = entry_of_token[t0 + r];
       if (e < 0 || state_slot[e] < 0) continue;
       const float4 x = Raw4<T>::value(raw[r]);
@@ -671,9 +671,10 @@ CCB_API int ccb_delta_prepare(const void* proj, int ld, int oq, int ok, int ov, 
                               const float* conv_w, int taps, const void* conv_state, const float* A_log,
                               const float* dt_bias, const int* entry_of_token, const int* cu_q,
                               const int* state_slot, float* qn, float* kn, float* vv, float* gg, float* bb, int T_,
-                              int G, int H, int dk, int dv, float q_mult, float unit_eps, int dtype,
+                              int G, int H, int dk, int dv, float q_mult, float unit_eps, int g_rows, int dtype,
                               cudaStream_t stream) {
   if (T_ <= 0) return 0;
+  g_rows = g_rows < T_ ? g_rows : T_;
   if (G <= 0 || H <= 0 || H % G || dk <= 0 || dv <= 0 || taps < 1) return CCB_REFUSE_SIZE;
   const dim3 grid(T_, (2 * G + 2 * H + kPrepWarps - 1) / kPrepWarps);
   const int esz = dtype == CCB_F32 ? 4 : 2;
@@ -692,7 +693,7 @@ CCB_API int ccb_delta_prepare(const void* proj, int ld, int oq, int ok, int ov, 
 #define CCB_RUN(TT, TAPS)                                                                                                  \
   ccb_launch(delta_prepare_run_kernel<TT, TAPS>, run_grid, dim3(kPrepWarps * 32), 0, stream, (const TT*)proj, ld, oq, ok, ov, \
              ob, (const TT*)a, lda, conv_w, (const TT*)conv_state, A_log, dt_bias, entry_of_token, cu_q, state_slot, qn, kn, \
-             vv, gg, bb, T_, G, H, dk, dv, q_mult, unit_eps)
+             vv, gg, bb, T_, G, H, dk, dv, q_mult, unit_eps, g_rows)
 #define CCB_RUN_TAPS(TT)             \
   do {                               \
     if (taps == 1) CCB_RUN(TT, 1);   \
@@ -709,24 +710,24 @@ CCB_API int ccb_delta_prepare(const void* proj, int ld, int oq, int ok, int ov, 
   if (vec && dtype == CCB_F32) {
     ccb_launch(delta_prepare_vec_kernel<float>, grid, dim3(kPrepWarps * 32), 0, stream, (const float*)proj, ld, oq, ok,
                ov, ob, (const float*)a, lda, conv_w, taps, (const float*)conv_state, A_log, dt_bias, entry_of_token,
-               cu_q, state_slot, qn, kn, vv, gg, bb, G, H, dk, dv, q_mult, unit_eps);
+               cu_q, state_slot, qn, kn, vv, gg, bb, G, H, dk, dv, q_mult, unit_eps, g_rows);
     return ccb_launch_status();
   }
   if (vec && dtype == CCB_BF16) {
     ccb_launch(delta_prepare_vec_kernel<__nv_bfloat16>, grid, dim3(kPrepWarps * 32), 0, stream,
                (const __nv_bfloat16*)proj, ld, oq, ok, ov, ob, (const __nv_bfloat16*)a, lda, conv_w, taps,
                (const __nv_bfloat16*)conv_state, A_log, dt_bias, entry_of_token, cu_q, state_slot, qn, kn, vv, gg, bb,
-               G, H, dk, dv, q_mult, unit_eps);
+               G, H, dk, dv, q_mult, unit_eps, g_rows);
     return ccb_launch_status();
   }
   if (dtype == CCB_F32)
     ccb_launch(delta_prepare_kernel<float>, grid, dim3(kPrepWarps * 32), 0, stream, (const float*)proj, ld, oq, ok, ov, ob,
                (const float*)a, lda, conv_w, taps, (const float*)conv_state, A_log, dt_bias, entry_of_token, cu_q,
-               state_slot, qn, kn, vv, gg, bb, G, H, dk, dv, q_mult, unit_eps);
+               state_slot, qn, kn, vv, gg, bb, G, H, dk, dv, q_mult, unit_eps, g_rows);
   else if (dtype == CCB_BF16)
     ccb_launch(delta_prepare_kernel<__nv_bfloat16>, grid, dim3(kPrepWarps * 32), 0, stream, (const __nv_bfloat16*)proj, ld,
                oq, ok, ov, ob, (const __nv_bfloat16*)a, lda, conv_w, taps, (const __nv_bfloat16*)conv_state, A_log,
-               dt_bias, entry_of_token, cu_q, state_slot, qn, kn, vv, gg, bb, G, H, dk, dv, q_mult, unit_eps);
+               dt_bias, entry_of_token, cu_q, state_slot, qn, kn, vv, gg, bb, G, H, dk, dv, q_mult, unit_eps, g_rows);
   else
     return CCB_REFUSE_DTYPE;
   return ccb_launch_status();

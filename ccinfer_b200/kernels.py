@@ -70,7 +70,7 @@ _SIGNATURES = {
     "ccb_gated_act": [c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_float, c_float, c_float, c_int, c_void_p],
     "ccb_delta_prepare": [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p,
                           c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                          c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_int, c_void_p],
+                          c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_int, c_int, c_void_p],
     "ccb_conv_state_update": [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int,
                               c_int, c_int, c_int, c_int, c_int, c_void_p],
     "ccb_delta_recurrence": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -204,7 +204,7 @@ _SIGNATURES = {
                        + [c_void_p] * 4 + [c_int] + [c_void_p] * 4 + [c_float, c_float, c_int, c_void_p]
                        + [c_int] * 7 + [c_float, c_float, c_int, c_int, c_void_p],
     "ccb_memory_chunks": [c_void_p] * 4 + [c_int, c_void_p, c_int] + [c_void_p] * 6 + [c_int] * 7 + [c_float, c_void_p],
-    "ccb_chunk_recurrence": [c_void_p] * 15 + [c_int] * 9 + [c_void_p],
+    "ccb_chunk_recurrence": [c_void_p] * 6 + [c_int] + [c_void_p] * 12 + [c_int] * 9 + [c_void_p],
     "ccb_chunk_recurrence_raw": [c_void_p] * 3 + [c_int, c_void_p, c_int, c_void_p, c_float, c_float] + [c_void_p] * 8 + [c_int] * 7
                                 + [c_void_p],
     "ccb_latent_rows": [c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p] + [c_int] * 6
@@ -575,11 +575,13 @@ def clamped_glu(act, gate_up, block: int, limit: float, alpha: float, up_shift: 
 
 
 def delta_prepare(proj, offsets, a, conv_w, taps: int, conv_state, A_log, dt_bias, entry_of_token, cu_q, state_slot,
-                  qn, kn, vv, gg, bb, G: int, H: int, dk: int, dv: int, q_mult: float, unit_eps: float) -> None:
+                  qn, kn, vv, gg, bb, G: int, H: int, dk: int, dv: int, q_mult: float, unit_eps: float,
+                  decays: int | None = None) -> None:
     """The inputs of the gated delta rule from the projections' rows: convolution + silu of q, k, v (with the
     request's convolution state before the portion), unit q and k per head (q times ``q_mult``),
     beta = sigmoid(b), decay = exp(-exp(A_log) softplus(a + dt_bias)); outputs float.  ``offsets`` = the first
-    columns of q, k, v, b in ``proj``; ``conv_w`` [taps, channels of q|k|v]."""
+    columns of q, k, v, b in ``proj``; ``conv_w`` [taps, channels of q|k|v].  Only the first ``decays`` rows of ``gg`` are made
+    (None: all)."""
     _cuda(conv_w, conv_state, A_log, dt_bias, entry_of_token, cu_q, state_slot, qn, kn, vv, gg, bb)
     T = qn.shape[0]
     assert proj.stride(1) == 1 and a.stride(1) == 1 and proj.dtype == a.dtype == conv_state.dtype
@@ -588,7 +590,7 @@ def delta_prepare(proj, offsets, a, conv_w, taps: int, conv_state, A_log, dt_bia
     _check(lib().ccb_delta_prepare(_p(proj), proj.stride(0), oq, ok, ov, ob, _p(a), a.stride(0), _p(conv_w), taps,
                                    _p(conv_state), _p(A_log), _p(dt_bias), _p(entry_of_token), _p(cu_q),
                                    _p(state_slot), _p(qn), _p(kn), _p(vv), _p(gg), _p(bb), T, G, H, dk, dv,
-                                   float(q_mult), float(unit_eps), _dt(proj), _stream()), "delta_prepare")
+                                   float(q_mult), float(unit_eps), T if decays is None else decays, _dt(proj), _stream()), "delta_prepare")
 
 
 def conv_state_update(proj, offsets, conv_state, taps: int, cu_q, state_slot, n_entries: int, G: int, H: int,
@@ -680,11 +682,12 @@ def chunk_recurrence_fits(dtype, dk: int, dv: int, longest: int, units: int, del
 
 
 def chunk_recurrence(scratch, qn, kn, vv, gg, bb, state, out, cu_q, state_slot, entry0: int, n_entries: int,
-                     max_tokens: int, G: int, H: int, dk: int, dv: int) -> None:
+                     max_tokens: int, G: int, H: int, dk: int, dv: int, decay_rows=None) -> None:
     """``delta_recurrence`` / ``delta_head_recurrence`` (gg [T, H]) / with bb None ``gated_linear_recurrence`` for the
     entries entry0 .. entry0 + n_entries - 1 in chunks on tensor cores.  The rows are consumed: what the chunks leave
     between the two kernels goes into the memory of qn, kn, vv and gg where sizes allow.  ``scratch(key, tokens_or_chunks,
-    shape, dtype)``: a workspace of shape [tokens or chunks, *shape]."""
+    shape, dtype)``: a workspace of shape [tokens or chunks, *shape].  ``decay_rows`` = (a, dt_bias, A_log) of ``delta_prepare``
+    (delta rule, one decay per channel, bfloat16): the chunks make the decays themselves and gg [T, H, dk] is a workspace."""
     _cuda(qn, kn, vv, gg, bb, state, out, cu_q, state_slot)
     f32, bf = torch.float32, torch.bfloat16
     assert qn.dtype == kn.dtype == vv.dtype == gg.dtype == state.dtype == out.dtype == f32
@@ -698,8 +701,14 @@ def chunk_recurrence(scratch, qn, kn, vv, gg, bb, state, out, cu_q, state_slot, 
     keep = scratch("chunk_keep", "chunks", (H, dk), f32)
     assert qs.shape[0] >= T and ks.shape[0] >= T and (w is None or w.shape[0] >= T) and p.shape[0] >= T
     assert keep.shape[0] >= T // 64 + entry0 + n_entries
+    a, a_bias, A_log = decay_rows or (None, None, None)
+    if a is not None:
+        _cuda(a_bias, A_log)
+        assert bb is not None and not head and a.is_cuda and a.dtype == bf and a.stride(1) == 1 and a.shape[0] == T and a.shape[1] >= H * dk
+        assert a_bias.dtype == A_log.dtype == f32 and a_bias.numel() == H * dk and A_log.numel() == H
     pv = vv.data_ptr()
-    _check(lib().ccb_chunk_recurrence(qn.data_ptr(), kn.data_ptr(), pv, gg.data_ptr(), _p(bb), qs.data_ptr(), ks.data_ptr(),
+    _check(lib().ccb_chunk_recurrence(qn.data_ptr(), kn.data_ptr(), pv, gg.data_ptr(), _p(bb), _p(a),
+                                      a.stride(0) if a is not None else 0, _p(a_bias), _p(A_log), qs.data_ptr(), ks.data_ptr(),
                                       _p(w), pv if bb is not None else 0, p.data_ptr(), keep.data_ptr(), state.data_ptr(),
                                       out.data_ptr(), cu_q.data_ptr(), state_slot.data_ptr(), entry0, n_entries, max_tokens,
                                       G, H, dk, dv, state.shape[0], 1 if head else 0, _stream()), "chunk_recurrence")

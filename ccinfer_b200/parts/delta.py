@@ -134,21 +134,21 @@ class ChannelGatedDelta(Mixer):
         bb = rt.scratch.get("delta_beta", (rt.max_tokens, H), f32)[:T]
         offsets = (self.oq, self.ok, self.ov, self.ob)
         S, conv = state["S"], state["conv"]
-        kernels.delta_prepare(proj, offsets, ag, self.conv_w, self.taps, conv, self.A_log, self.dt_bias,
-                              step.entry_of_token, step.cu_q, step.state_slot, qn, kn, vv, gg, bb, G, H, dk, dv,
-                              dk ** -0.5, UNIT_EPS)
-        kernels.conv_state_update(proj, offsets, conv, self.taps, step.cu_q, step.state_slot, step.n_entries,
-                                  G, H, dk, dv)
-        o = rt.scratch.get("delta_o", (rt.max_tokens, H, dv), f32)[:T]
         # (a step lists its single tokens first: they, and short portions, go token by token)
         chunks = kernels.chunk_recurrence_fits(rt.dtype, dk, dv, step.max_q_len, (T - step.n_single) * H, True)
         n1 = step.n_single if chunks else step.n_entries
+        kernels.delta_prepare(proj, offsets, ag, self.conv_w, self.taps, conv, self.A_log, self.dt_bias,
+                              step.entry_of_token, step.cu_q, step.state_slot, qn, kn, vv, gg, bb, G, H, dk, dv,
+                              dk ** -0.5, UNIT_EPS, decays=n1 if chunks else None)   # (chunks make theirs)
+        kernels.conv_state_update(proj, offsets, conv, self.taps, step.cu_q, step.state_slot, step.n_entries,
+                                  G, H, dk, dv)
+        o = rt.scratch.get("delta_o", (rt.max_tokens, H, dv), f32)[:T]
         if n1:
             kernels.delta_recurrence(qn, kn, vv, gg, bb, S, o, step.cu_q, step.state_slot, n1, G, H, dk, dv,
                                      single=n1 == step.n_single, status=rt.status)
         if step.n_entries > n1:
             kernels.chunk_recurrence(rt.chunk_scratch, qn, kn, vv, gg, bb, S, o, step.cu_q, step.state_slot, n1,
-                                     step.n_entries - n1, step.max_q_len, G, H, dk, dv)
+                                     step.n_entries - n1, step.max_q_len, G, H, dk, dv, decay_rows=(ag, self.dt_bias, self.A_log))
         y = rt.scratch.get("delta_y", (rt.max_tokens, self.v_width), rt.dtype)[:T]
         kernels.gated_head_rmsnorm(y, o, ag[:, self.oga:], self.norm_w, H, dv, self.eps)
         out = rt.scratch.get(self.out_key, (rt.max_tokens, self.hidden), rt.dtype)[:T]

@@ -977,3 +977,46 @@ def test_gated_linear_chunks_from_the_projections_rows(H, dk, dv, tau, bias):
                            max(lens), H, dk, dv, 0.3, tau)
     assert (out.double() - want).abs().max() <= 2.0 ** -14 * want.abs().max()
     assert (state.double() - after).abs().max() <= 2.0 ** -14 * after.abs().max()
+
+
+# slow decays, ordinary ones and such that keep nothing of a run; the rows' decays inside wider rows
+@pytest.mark.parametrize("shift", [-8.0, 0.0, 6.0])
+@pytest.mark.parametrize("H,G,dk,dv", [(2, 2, 128, 128), (4, 2, 64, 32)])
+def test_delta_chunks_that_make_their_decays(H, G, dk, dv, shift):
+    """Against float64 from the same bfloat16 rows, and that only the single tokens' decays are made beforehand."""
+    k, g = _k(), _gen(H + dk + dv + int(shift))
+    lens, first = [1, 1, 2, 15, 17, 64, 65, 130], 2
+    T = sum(lens)
+
+    def rnd(*shape):
+        return torch.randn(shape, generator=g, device="cuda")
+
+    def dev(x):
+        return torch.tensor(x, dtype=torch.int32, device="cuda")
+
+    def scratch(key, per, shape, dtype):
+        return torch.full((T if per == "tokens" else T // 64 + len(lens),) + tuple(shape), float("nan"), dtype=dtype, device="cuda")
+
+    cu, slots = [0] + torch.tensor(lens).cumsum(0).tolist(), list(range(len(lens)))[::-1]
+    slots[4] = -1
+    a, A_log, dt_bias = rnd(T, H * dk + 5).bfloat16()[:, 5:], rnd(H), rnd(H * dk) + shift
+    ob = 2 * G * dk + H * dv
+    proj, state = rnd(T, ob + H).bfloat16(), rnd(len(lens), H, dv, dk)
+    entry = dev([e for e, n in enumerate(lens) for _ in range(n)])
+    rows = [torch.full(s, float("nan"), device="cuda") for s in ((T, G, dk), (T, G, dk), (T, H, dv), (T, H, dk), (T, H))]
+    k.delta_prepare(proj, (0, G * dk, 2 * G * dk, ob), a, rnd(1, ob), 1, rnd(len(lens), 0, ob).bfloat16(), A_log, dt_bias, entry, dev(cu),
+                    dev(slots), *rows, G, H, dk, dv, dk ** -0.5, 1e-6, decays=first)
+    assert torch.isfinite(rows[3][:first]).all() and torch.isnan(rows[3][first:]).all()
+    q, kk, v, _, beta = (r.double() for r in rows)
+    decay = torch.exp(-torch.exp(A_log.double())[:, None] * torch.nn.functional.softplus(a.double() + dt_bias.double()).view(T, H, dk))
+    out, after = torch.full((T, H, dv), 7.0, device="cuda"), state.double()
+    want = out.double()
+    for e, slot in enumerate(slots):
+        if e >= first and slot >= 0:
+            s = slice(cu[e], cu[e + 1])
+            want[s], after[slot] = _recurrence64(q[s].repeat_interleave(H // G, 1), kk[s].repeat_interleave(H // G, 1), v[s], decay[s],
+                                                 beta[s], state[slot].double())
+    k.chunk_recurrence(scratch, *rows, state, out, dev(cu), dev(slots), first, len(lens) - first, max(lens), G, H, dk, dv,
+                       decay_rows=(a, dt_bias, A_log))
+    assert (out.double() - want).abs().max() <= 2.0 ** -14 * want.abs().max()
+    assert (state.double() - after).abs().max() <= 2.0 ** -14 * after.abs().max()

@@ -30,9 +30,9 @@
 // it belongs to, from its token on, is made NaN afterwards.
 //
 // Bound by: the walk by the chain of its products (one block of eight warps an SM, an instruction on 0.30 of the cycles),
-// the preparation by what it issues (0.42).  Measured on B200, 2,048 tokens of one request, 32 heads of 128 x 128 with a
-// decay per channel and the delta rule: 190 + 105 us (196 with the solve's operands split again by every 16 columns); token by
-// token 959 us.  Outputs and memory are right to 5e-6 in the
+// the preparation by what it issues (0.5).  Measured on B200, 2,048 tokens of one request, 32 heads of 128 x 128 with a
+// decay per channel and the delta rule: 163 + 105 us (with what it reads loaded as it is needed 199, with the solve's operands split
+// again by every 16 columns 8 more); token by token 959 us.  Outputs and memory are right to 5e-6 in the
 // 2-norm, token by token to 1e-7 to 4e-7; in a layer's results, whose rows are bfloat16 (3.7e-3), neither shows.
 #include "common.cuh"
 #include "mma_common.cuh"
@@ -53,7 +53,7 @@ constexpr float kSteepLog2 = 55.f;   // (2^110 times 128 products stays in a flo
 // sigmoid(a + bias)^(1 / tau).  Measured on B200, 1,537 tokens of three requests, 16 heads of 128, a layer: 173 -> 162 us (the rows'
 // kernel of 18 us gone, preparation 33 -> 40, walk 40 -> 43).
 // The delta rule takes only its decays so, exp(-exp(A_log) softplus(a + bias)): at 2,048 tokens of 32 heads the rows' kernel 76 -> 60 us,
-// the preparation 190 -> 197, a layer 605 -> 596.  Its q, k and v too, convolved by the preparation: 270 without a rows' kernel, 617.
+// the preparation 7 more, a layer 605 -> 596.  Its q, k and v too, convolved by the preparation: 270 without a rows' kernel, 617.
 struct RawRows {
   const __nv_bfloat16 *q, *k, *v, *a;   // q, k [T, ld] with head h at column h DK, v [T, ld] at h dv, a [T, lda] at h DK
   int ld, lda;
@@ -80,6 +80,11 @@ __device__ __forceinline__ float4 four(const __nv_bfloat16* p) {
   const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r.y));
   return make_float4(a.x, a.y, b.x, b.y);
 }
+
+__device__ __forceinline__ void copy16(float* smem, const float* gmem) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void copies_landed() { asm volatile("cp.async.wait_all;" ::: "memory"); }   // (this thread's)
 
 __device__ __forceinline__ float ex2(float x) {
   float y;
@@ -112,7 +117,7 @@ __device__ __forceinline__ int lat(int t, int s) { return t * kPitchL + (s ^ ((t
 template <int DK, bool DELTA, bool HEAD> struct PrepShape {
   static constexpr int kC = HEAD ? kChunk : kChunk * DK;   // sums of logarithms
   static constexpr int kFloats = 2 * kChunk * DK + kC + (DELTA ? kChunk * kPitchL : 0) + kChunk;   // (two blocks an SM)
-  static constexpr int kBytes = kFloats * 4 + 16;   // (two blocks an SM)
+  static constexpr int kBytes = kFloats * 4 + 48;
 };
 
 // 32 values a lane, one for each lane: the sum of value i over all lanes ends in lane i
@@ -165,7 +170,7 @@ chunk_prepare_kernel(const ChunkRows a) {
   float* l_s = c_s + Sh::kC;                 // [64][64]: diag(beta) M below the diagonal
   float* b_s = l_s + (DELTA ? kChunk * kPitchL : 0);
   int* next_item = reinterpret_cast<int*>(b_s + kChunk);
-  int* steep = next_item + 1;                // a bit for each run that takes every pair's decay by itself
+  int* steep = next_item + 1;                // [8 warps]: a bit for each run that takes every pair's decay by itself
 
   const int e = a.entry0 + blockIdx.z, h = blockIdx.y, chunk = blockIdx.x;
   const int first = a.cu_q[e], n = a.cu_q[e + 1] - first;
@@ -175,25 +180,27 @@ chunk_prepare_kernel(const ChunkRows a) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int kvh = h / (a.H / a.G);
 
+  // Float rows go straight to shared memory while the logarithms below are loaded and taken.  (Through registers, with a barrier
+  // before the logarithms: 174 us, 163 so; the logarithms' loads before the rows': 185.)
   for (int i = tid; i < kChunk * DK / 4; i += kThreads) {
     const int t = i / (DK / 4), c = 4 * (i % (DK / 4));
-    float4 q = make_float4(0.f, 0.f, 0.f, 0.f), k = q;
-    if (RAW && !DELTA && t < cnt) {
+    float* q_at = q_s + at<DK>(t, c);
+    float* k_at = k_s + at<DK>(t, c);
+    if (t >= cnt) {
+      *reinterpret_cast<float4*>(q_at) = *reinterpret_cast<float4*>(k_at) = make_float4(0.f, 0.f, 0.f, 0.f);
+    } else if (RAW && !DELTA) {
       const size_t row = (size_t)(r0 + t) * a.raw.ld + kvh * DK + c;
-      q = four(a.raw.q + row);
-      k = four(a.raw.k + row);
-      q.x *= a.raw.q_mult; q.y *= a.raw.q_mult; q.z *= a.raw.q_mult; q.w *= a.raw.q_mult;
-    } else if (t < cnt) {
+      const float4 q = four(a.raw.q + row);
+      *reinterpret_cast<float4*>(k_at) = four(a.raw.k + row);
+      *reinterpret_cast<float4*>(q_at) = make_float4(q.x * a.raw.q_mult, q.y * a.raw.q_mult, q.z * a.raw.q_mult, q.w * a.raw.q_mult);
+    } else {
       const size_t row = ((size_t)(r0 + t) * a.G + kvh) * DK + c;
-      q = *reinterpret_cast<const float4*>(a.q + row);
-      k = *reinterpret_cast<const float4*>(a.k + row);
+      copy16(q_at, a.q + row);
+      copy16(k_at, a.k + row);
     }
-    *reinterpret_cast<float4*>(q_s + at<DK>(t, c)) = q;
-    *reinterpret_cast<float4*>(k_s + at<DK>(t, c)) = k;
   }
   if (tid < kChunk) b_s[tid] = DELTA && tid < cnt ? a.beta[(size_t)(r0 + tid) * a.H + h] : 0.f;
-  if (tid == 0) *next_item = *steep = 0;
-  __syncthreads();
+  if (tid == 0) *next_item = 0;
   auto log_decay = [](float g) {
     const float x = log2f(g);
     return x < kLeastLog2 ? kLeastLog2 : x;
@@ -252,8 +259,9 @@ chunk_prepare_kernel(const ChunkRows a) {
       if (!(first_sum - mid <= kSteepLog2 && mid - sum <= kSteepLog2)) mine |= 1 << (part * (PT / kRun) + m);
     }
     mine = __reduce_or_sync(0xffffffffu, mine);
-    if (mine != 0 && lane == 0) atomicOr(steep, mine);
+    if (lane == 0) steep[warp] = mine;
   }
+  copies_landed();
   __syncthreads();
   auto in_run = [&](int t, int d) { return HEAD ? c_s[t] : c_s[at<DK>(t, d)]; };
   // the decay of whole runs lo .. hi - 1
@@ -269,7 +277,9 @@ chunk_prepare_kernel(const ChunkRows a) {
 
   // ---- blocks of 16 x 16 pairs, a warp each, to whoever is free: rows of run i, columns of run j
   const int gid = lane >> 2, tig = lane & 3;
-  const int steep_runs = HEAD ? 0 : *steep;
+  int steep_runs = 0;
+  if (!HEAD)
+    for (int w = 0; w < kThreads / 32; ++w) steep_runs |= steep[w];
   auto take = [&]() {
     int item = 0;
     if (lane == 0) item = atomicAdd(next_item, 1);
@@ -428,6 +438,14 @@ chunk_prepare_kernel(const ChunkRows a) {
   // ---- the triangular solve for X = [W | U]: with L the strictly lower blocks, X_i = (I + L_ii)^-1 (B_i - sum L_ij X_j)
   if constexpr (DELTA) {
     __syncthreads();
+    // The values go where the queries were while the diagonal's blocks are inverted (values of more channels: read one by one).
+    // Loaded where the solve needs them, each 16 x 16 block waited: 199 us, 174 so.
+    const bool values_in = a.dv <= DK;
+    if (values_in)
+      for (int x = tid; x < cnt * (a.dv / 4); x += kThreads) {
+        const int t = x / (a.dv / 4), c = 4 * (x - t * (a.dv / 4));
+        copy16(q_s + at<DK>(t, c), a.v + ((size_t)(r0 + t) * a.H + h) * a.dv + c);
+      }
     // (as operands, two neighbouring columns as their two bfloat16 in the place of two floats: every 16 columns of X read them)
     if (tid < kChunk) {   // a thread a column of an inverse, which takes its block's place
       const int run = tid / kRun, c = tid % kRun;
@@ -461,6 +479,7 @@ chunk_prepare_kernel(const ChunkRows a) {
         *reinterpret_cast<uint2*>(at) = both;
       }
     }
+    copies_landed();
     __syncthreads();
     const int runs = (cnt + kRun - 1) / kRun;
     // A warp 16 columns at a time: the transposed block [columns, tokens] is an accumulator, and split in two an A operand
@@ -483,7 +502,7 @@ chunk_prepare_kernel(const ChunkRows a) {
                 float b = 0.f;
                 if (t < cnt)
                   b = is_w ? k_s[at<DK>(t, col)] * ex2(before[up] + in_run(t, col))
-                           : a.v[((size_t)(r0 + t) * a.H + h) * a.dv + col - DK];
+                           : values_in ? q_s[at<DK>(t, col - DK)] : a.v[((size_t)(r0 + t) * a.H + h) * a.dv + col - DK];
                 x[nb][2 * up + y] = b * b_s[t];
               }
             if (is_w) before[up] += in_run(i * kRun + kRun - 1, col);

@@ -31,7 +31,7 @@
 //
 // Bound by: the walk by the chain of its products (one block of eight warps an SM, an instruction on 0.30 of the cycles),
 // the preparation by what it issues (0.5).  Measured on B200, 2,048 tokens of one request, 32 heads of 128 x 128 with a
-// decay per channel and the delta rule: 163 + 105 us (with what it reads loaded as it is needed 199, with the solve's operands split
+// decay per channel and the delta rule: 163 + 104 us (with what it reads loaded as it is needed 199, with the solve's operands split
 // again by every 16 columns 8 more); token by token 959 us.  Outputs and memory are right to 5e-6 in the
 // 2-norm, token by token to 1e-7 to 4e-7; in a layer's results, whose rows are bfloat16 (3.7e-3), neither shows.
 #include "common.cuh"
@@ -624,7 +624,9 @@ chunk_walk_kernel(const ChunkRows a) {
   if (slot < 0 || slot >= a.n_slots || n <= 0) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gid = lane >> 2, tig = lane & 3;
-  const int wr = warp & 3, wc = warp >> 2;   // 16 rows of the chunk, 16 columns of the slice
+  // 16 rows of the chunk, 16 columns of the slice.  Later rows meet more tokens, and the two warps of a scheduler share that (107 ->
+  // 103.5 us; without the delta rule, where the update of S is all that follows, 43.0 / 43.4)
+  const int wc = warp >> 2, wr = DELTA && wc == 1 ? 3 - (warp & 3) : warp & 3;
 
   // 64 rows of two halves of `COLS` elements each, a row (r0 + t, h), into two swizzled tiles
   auto issue = [&](__nv_bfloat16* dst, const __nv_bfloat16* src, int chunk, auto cols) {

@@ -25,7 +25,7 @@
 // groups of heads that share queries and keys.  The two halves of queries and keys fill an SM's shared memory, so one block
 // runs on it: of two teams of four warps, a slice of value columns each, that share the tiles of queries and keys and the
 // weighted scores (a team makes those of every second block of 16 keys and leaves them for the other).  2,048 tokens of two
-// requests, 128 heads of 64 x 128: 1,034 us token by token, 459 us in chunks by one team a block, 230 us by two.
+// requests, 128 heads of 64 x 128: 1,034 us token by token, 459 us in chunks by one team a block, 222 us by two.
 // Outputs and memory are right to 5e-6 in the 2-norm, token by token to 2e-7; in a layer's results, whose rows are bfloat16
 // (3.5e-3), neither shows.
 // A value that is no finite number must not reach the tokens before it, whose weight of it is a zero that would still
@@ -95,7 +95,10 @@ memory_chunks_kernel(const ChunkArgs a) {
   const int slot = a.state_slot[e];
   const int r0 = a.cu_q[e], n = a.cu_q[e + 1] - r0;
   if (slot < 0 || slot >= a.max_slots || n <= 0) return;
-  const int tid = threadIdx.x % kThreads, lane = tid & 31, warp = tid >> 5;   // in the team
+  const int tid = threadIdx.x % kThreads, lane = tid & 31;   // in the team
+  // Later rows of a chunk meet more keys: the second team's warps take theirs the other way round, so that each of an SM's four
+  // schedulers has as much to do (the sizes above: 232 -> 222 us)
+  const int warp = team == 0 ? tid >> 5 : 3 - (tid >> 5);
   const int gid = lane >> 2, tig = lane & 3;
   const int kvh = h / a.group;
   const int col0 = slice * BN;

@@ -31,7 +31,7 @@
 //
 // Bound by: the walk by the chain of its products (one block of eight warps an SM, an instruction on 0.30 of the cycles),
 // the preparation by what it issues (0.5).  Measured on B200, 2,048 tokens of one request, 32 heads of 128 x 128 with a
-// decay per channel and the delta rule: 163 + 104 us (with what it reads loaded as it is needed 199, with the solve's operands split
+// decay per channel and the delta rule: 163 + 95 us (with what it reads loaded as it is needed 199, with the solve's operands split
 // again by every 16 columns 8 more); token by token 959 us.  Outputs and memory are right to 5e-6 in the
 // 2-norm, token by token to 1e-7 to 4e-7; in a layer's results, whose rows are bfloat16 (3.7e-3), neither shows.
 #include "common.cuh"
@@ -718,7 +718,7 @@ chunk_walk_kernel(const ChunkRows a) {
     float d[2][4];   // W S0
 #pragma unroll
     for (int nb = 0; nb < 2; ++nb) d[nb][0] = d[nb][1] = d[nb][2] = d[nb][3] = 0.f;
-#pragma unroll 2
+#pragma unroll(DELTA ? DK / 16 : 2)   // (delta rule, two at a time: 103.5 us, all eight 95.4; without: 43.0 / 43.5)
     for (int ks = 0; ks < DK / 16; ++ks) {
       uint32_t bh[4], bl[4], xh[4], xl[4];
       ldmatrix_x4_trans(bh[0], bh[1], bh[2], bh[3], smem_u32(s_hi + (ks * 16 + trow) * kPitch + wc * 16 + tcol));

@@ -325,17 +325,22 @@ moe_grouped_tc_kernel(const __grid_constant__ TokenMaps tmX, const __grid_consta
         for (int x = 0; x < 2; ++x) {
           const size_t row = g0 + tok[x];
           const int left = n - tok[x];   // of the sixteen tokens
+          if (left <= 0) continue;   // (columns without tokens: the whole part of 8 tokens, two of 32 columns filled, 0.7 % slower than with
+                                     // two accumulators, so 0.9 % faster)
           if (MODE == 1) {
             float* dst = (float*)Cout + row * ldc + col;
 #pragma unroll
-            for (int j = 0; j < 16; ++j)
-              if (j < left && col < N) dst[(size_t)j * ldc] = __uint_as_float(v[16 * x + j]);
+            for (int j = 0; j < 16; ++j) {
+              if (j >= left) break;
+              if (col < N) dst[(size_t)j * ldc] = __uint_as_float(v[16 * x + j]);
+            }
           } else if (MODE == 0) {
             __nv_bfloat16* dst = (__nv_bfloat16*)Cout + row * ldc + col;
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
+              if (j >= left) break;
               const float w = __shfl_sync(0xffffffffu, my_w, 16 * x + j), a = fmaxf(__uint_as_float(v[16 * x + j]), 0.f);
-              if (j < left && col < N) dst[(size_t)j * ldc] = __float2bfloat16_rn(a * a * w);
+              if (col < N) dst[(size_t)j * ldc] = __float2bfloat16_rn(a * a * w);
             }
           } else {   // columns (2 f, 2 f + 1) are gate f and up f: the even lane takes token j, the odd one token j + 1
             const int odd = lane & 1;
@@ -350,6 +355,7 @@ moe_grouped_tc_kernel(const __grid_constant__ TokenMaps tmX, const __grid_consta
             };
 #pragma unroll
             for (int j = 0; j < 16; j += 2) {
+              if (j >= left) break;
               const float y = one(j);
               if (mine_col && j + odd < left) dst[(size_t)j * ldc] = __float2bfloat16_rn(y);
             }

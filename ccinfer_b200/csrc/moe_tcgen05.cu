@@ -36,6 +36,7 @@
 #include <cuda.h>
 #include <type_traits>
 
+#include "slot_ring.h"
 #include "tc_pair_common.cuh"
 #include "tma_host.h"
 
@@ -45,8 +46,6 @@ namespace {
 
 constexpr int kFeatures = 256;     // weight rows of a tile; each block loads 128 of them
 constexpr int kTokenStep = 32;     // what the number of a tile's tokens is rounded up to; each block loads half of them
-constexpr int kSlots = 16;         // of kTokenStep columns of tensor memory
-constexpr int kMostSlots = 8;      // of a product
 constexpr int kK = 64;
 constexpr int kWBytes = (kFeatures / 2) * kK * 2;   // 16 KB
 template <int CAP> struct Ring {
@@ -55,23 +54,6 @@ template <int CAP> struct Ring {
 };
 constexpr int kBoxes = 4;          // token copies come in boxes of 16, 32, 64 and 128 rows: at most three make up a block's half
 constexpr int kThreads = 352;     // warps: 0 weights, 1 products, 2 .. 9 epilogue, 10 tokens
-
-// Where a tile's slots begin: behind the ones before, but a tile of one product is not cut by the ring's end.
-__device__ __forceinline__ int tile_place(int at, int slots) { return slots <= kMostSlots && at + slots > kSlots ? 0 : at; }
-
-// The products of a tile of `slots` slots from slot `at` on: runs that neither pass the ring's end nor have more than 256
-// columns, of about the same size where a run is cut; at most three (slots of the first, second, third).
-struct TileParts {
-  int len[3];
-  __device__ __forceinline__ TileParts(int at, int slots) {
-    const int head = min(slots, kSlots - at), tail = slots - head;
-    const int h = head > kMostSlots ? (head + 1) / 2 : head, t = tail > kMostSlots ? (tail + 1) / 2 : tail;
-    len[0] = h;
-    len[1] = head > h ? head - h : t;
-    len[2] = head > h ? t : tail - t;
-  }
-  __device__ __forceinline__ int count() const { return 1 + (len[1] > 0) + (len[2] > 0); }
-};
 
 struct TokenMaps {
   CUtensorMap box[kBoxes];   // 16 << i rows
@@ -199,22 +181,21 @@ moe_grouped_tc_kernel(const __grid_constant__ TokenMaps tmX, const __grid_consta
     }
   } else if (warp == 1) {
     if (lane == 0 && leader) {  // ---- MMA issuer (the leader's): products of M = 256 over both blocks ----
-      int s = 0, ph = 0, local = 0, at = 0;
+      int s = 0, ph = 0, local = 0;
+      SlotRing ring;
       uint32_t used = 0;   // a bit a slot: how often it has been used, its last place
       bool alive = true;
       Item now = item(pair), next = now;
       for (int t = pair; now.n > 0 && alive; t += n_pairs, now = kAhead ? next : item(t), ++local) {
         if (kAhead) next = item(t + n_pairs);
         const int slots = columns(now.n) / kTokenStep;
-        at = tile_place(at, slots);
-        // Warps read tiles in order, and a tile's even and odd slots in order, so that where the last two slots have been read
-        // all have (a wait for each of ten slots would take longer than the products of a short tile leave).
-        for (int i = max(0, slots - 2); i < slots && alive; ++i) {
-          const int b = at + i < kSlots ? at + i : at + i - kSlots;
+        ring.enter(slots);
+        const int at = ring.at;
+        for (int i = ring.first_waited(slots); i < ring.end_waited(slots) && alive; ++i) {
+          const int b = (at + i) % kSlots;
           alive = mbar_wait_cluster(tempty0 + 8 * b, (used >> b & 1) ^ 1);
         }
-        const uint32_t taken = ((1u << slots) - 1) << at;
-        used ^= (taken | taken >> kSlots) & 0xffffu;
+        used ^= slot_bits(at, slots);
         if (!alive) {
           set_status(status, CCB_ST_WAIT_TIMEOUT);
           break;
@@ -252,13 +233,14 @@ moe_grouped_tc_kernel(const __grid_constant__ TokenMaps tmX, const __grid_consta
                 : count == 2 ? walk(std::integral_constant<int, 2>{})
                              : walk(std::integral_constant<int, 3>{});
         if (!alive) set_status(status, CCB_ST_WAIT_TIMEOUT);
-        at = (at + slots) % kSlots;
+        ring.leave(slots);
       }
     }
   } else {  // ---- epilogue: this block's 128 weight rows (lanes), all tokens of the tile (columns) ----
     // two warps a quarter of the lanes, which take a slot in turn
     const int q = warp & 3, turn = (warp - 2) >> 2;
-    int local = 0, at = 0;
+    int local = 0;
+    SlotRing ring;
     Item now = item(pair), next = now;
     for (int t = pair; now.n > 0; t += n_pairs, now = kAhead ? next : item(t), ++local) {
       if (kAhead) next = item(t + n_pairs);
@@ -269,7 +251,8 @@ moe_grouped_tc_kernel(const __grid_constant__ TokenMaps tmX, const __grid_consta
       }
       tc_fence_after();
       const int slots = columns(n) / kTokenStep, half = slots * (kTokenStep / 2);
-      at = tile_place(at, slots);
+      ring.enter(slots);
+      const int at = ring.at;
       const TileParts parts(at, slots);
       const size_t g0 = (size_t)now.r0;
       const int col = now.tf * kFeatures + (int)rank * (kFeatures / 2) + q * 32 + lane;   // this lane's column of the product
@@ -362,7 +345,7 @@ moe_grouped_tc_kernel(const __grid_constant__ TokenMaps tmX, const __grid_consta
           }
         }
       }
-      at = (at + slots) % kSlots;
+      ring.leave(slots);
     }
   }
   tc_fence_before();

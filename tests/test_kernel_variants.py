@@ -1020,3 +1020,55 @@ def test_delta_chunks_that_make_their_decays(H, G, dk, dv, shift):
                        decay_rows=(a, dt_bias, A_log))
     assert (out.double() - want).abs().max() <= 2.0 ** -14 * want.abs().max()
     assert (state.double() - after).abs().max() <= 2.0 ** -14 * after.abs().max()
+
+
+# walks in which a tile is cut by the ring's end or passes over slots (rows / 32 rounded up: 8 6 6 10, 9 8 3, 7 8 8 8, 5 5 5 5 5 6 ...),
+# by one pair of SMs in this order, and by all of them over many columns
+@pytest.mark.parametrize("mode", [0, 1, 2])
+@pytest.mark.parametrize("K", [64, 256, 2048])
+@pytest.mark.parametrize("N,sms", [(256, 2), (4096, None)])
+def test_grouped_products_of_long_walks(N, sms, K, mode, monkeypatch):
+    """Tensor memory taken in turn by tiles of mixed sizes, against float64 with the bounds of
+    test_grouped_products_of_experts: every walk goes round it many times (as tests/test_slot_ring.py follows)."""
+    k, g = _k(), _gen(N + K + mode)
+    slots = [8, 6, 6, 10, 9, 8, 3, 7, 8, 8, 8, 8, 6, 8, 8, 5, 5, 5, 5, 5, 6, 1, 10, 10, 10, 1, 1, 9, 9, 2, 4]
+    slots += torch.randint(1, 11, (29,), generator=torch.Generator().manual_seed(K)).tolist()
+    rows = [32 * s - (7 * i) % 32 for i, s in enumerate(slots)]
+    E, pairs = 16, sum(rows)
+    if sms is not None:
+        monkeypatch.setattr(k, "sm_count", lambda: sms)
+    else:
+        assert len(rows) * (N // 256) >= 12 * (k.sm_count() // 2)
+
+    def rnd(*shape):
+        return torch.randn(shape, generator=g, device="cuda")
+
+    def dev(x):
+        return torch.tensor(x, dtype=torch.int32, device="cuda")
+
+    r0 = [0] + torch.tensor(rows).cumsum(0).tolist()[:-1]
+    xs, row_w = rnd(pairs, K).to(torch.bfloat16), torch.rand(pairs, generator=g, device="cuda") + 0.5
+    w = (rnd(N, E * K) if mode == 1 else rnd(E * N, K)).mul(K ** -0.5).to(torch.bfloat16)
+    c = torch.full((pairs, N // 2 if mode == 2 else N), float("nan"), dtype=torch.float32 if mode == 1 else torch.bfloat16, device="cuda")
+    status = dev([0])
+    k.moe_grouped_tc(c, xs, w, row_w, dev([i % E for i in range(len(rows))] + [0]), dev(r0 + [0]), dev(rows + [0]), N, K,
+                     K if mode == 1 else N, mode, status=status, BM=320)
+    assert int(status.item()) == 0
+    for i, n in enumerate(rows):
+        e, at = i % E, slice(r0[i], r0[i] + n)
+        we = (w[:, e * K:(e + 1) * K] if mode == 1 else w[e * N:(e + 1) * N]).double()
+        a, got = xs[at].double(), c[at].double()
+        ref, size = a @ we.T, a.abs() @ we.abs().T
+        slack = K * 2.0 ** -24 * size
+        if mode == 1:
+            assert ((got - ref).abs() <= slack).all(), i
+            continue
+        rw = row_w[at].double()[:, None]
+        if mode == 0:
+            ref, slack = ref.clamp_min(0) ** 2 * rw, 2 * ref.abs() * slack * rw + slack ** 2 * rw
+        else:
+            gate, up = ref[:, ::2], ref[:, 1::2]
+            sg, su = slack[:, ::2], slack[:, 1::2]
+            ref = torch.nn.functional.silu(gate) * up * rw
+            slack = (1.1 * sg * up.abs() + gate.abs() * su + sg * su) * rw + 2.0 ** -20 * ref.abs()   # (silu's slope is below 1.1)
+        assert ((got - ref).abs() <= 2.0 ** -8 * ref.abs() + slack + 1e-30).all(), i

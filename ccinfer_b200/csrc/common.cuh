@@ -68,7 +68,8 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 // the stream still runs; `pdl_wait` blocks until the predecessor has completed and its writes are visible,
 // `pdl_trigger` lets the successor start early in turn.  Without the attribute both are no-ops.
 // Every kernel calls pdl_begin() (or the two halves, with read-only prefetching of weights in between)
-// before it touches memory that another kernel may have written.
+// before it touches memory that another kernel may have written.  The single tokens of delta_head.cu alone ask for their states
+// and the step's tables before, which the kernel directly ahead must not write.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Kernels without weights to prefetch: wait for the predecessor, then let the successor start (a product

@@ -74,7 +74,7 @@ __device__ __forceinline__ float4 silu4(const float4 x) { return make_float4(sil
 
 // Many single tokens: what state_stream.cuh needs of a head.  A warp each makes q, k and v, four channels a lane.
 template <typename T> struct HeadDeltaJob {
-  static constexpr bool DELTA = true, CHANNEL = false, NORM = true;
+  static constexpr bool DELTA = true, CHANNEL = false, NORM = true, AHEAD = true;
   const T* proj;
   T* ring;
   const float* w;
@@ -550,8 +550,8 @@ CCB_API int ccb_delta_head_step(const void* proj, int ld, const int* offsets, co
   if (vec && (long long)n_entries * H >= kStreamItems && state_stream_fits(dk, dv, state) && (dtype == CCB_F32 || dtype == CCB_BF16)) {
     const StateStream st{state, state_slot, cu_q, n_slots, n_entries, H, dk, dv, 0, status};
     if (dtype == CCB_F32)
-      return state_stream_launch(true, st, HeadDeltaJob<float>{(const float*)proj, (float*)ring, w, (float*)y, ldy, eps, a}, stream);
-    return state_stream_launch(true, st, HeadDeltaJob<__nv_bfloat16>{(const __nv_bfloat16*)proj, (__nv_bfloat16*)ring, w,
+      return state_stream_launch(st, HeadDeltaJob<float>{(const float*)proj, (float*)ring, w, (float*)y, ldy, eps, a}, stream);
+    return state_stream_launch(st, HeadDeltaJob<__nv_bfloat16>{(const __nv_bfloat16*)proj, (__nv_bfloat16*)ring, w,
                                                                      (__nv_bfloat16*)y, ldy, eps, a}, stream);
   }
   // else about 32 value channels a block, at most eight blocks a head

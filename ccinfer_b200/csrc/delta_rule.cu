@@ -533,7 +533,7 @@ delta_recurrence_kernel(const float* __restrict__ qn, const float* __restrict__ 
 
 // Many single tokens: what state_stream.cuh needs of a head, whose rows are there already.
 template <bool DELTA_, bool CHANNEL_> struct RowsJob {
-  static constexpr bool DELTA = DELTA_, CHANNEL = CHANNEL_, NORM = false;
+  static constexpr bool DELTA = DELTA_, CHANNEL = CHANNEL_, NORM = false, AHEAD = false;
   const float *q, *k, *v, *g, *beta;   // as in delta_recurrence_kernel
   float* out;
   int G, H, dk, dv;
@@ -781,7 +781,7 @@ static int pick_recurrence(const float* qn, const float* kn, const float* vv, co
   if (single_slots > 0 && entry0 == 0 && (long long)n_entries * H * dv >= kStreamColumns && state_stream_fits(dk, dv, state) &&
       ((bits(qn) | bits(kn) | bits(vv) | (HEAD ? 0 : bits(gg))) & 15) == 0) {
     const StateStream st{state, state_slot, cu_q, single_slots, n_entries, H, dk, dv, 0, status};
-    return state_stream_launch(true, st, RowsJob<DELTA, !HEAD>{qn, kn, vv, gg, bb, out, G, H, dk, dv, 0.f}, stream);
+    return state_stream_launch(st, RowsJob<DELTA, !HEAD>{qn, kn, vv, gg, bb, out, G, H, dk, dv, 0.f}, stream);
   }
   int R = 1;
   while (R * kLanes < dk) R *= 2;

@@ -56,7 +56,9 @@ __device__ __forceinline__ float stream_dot4(const float4 a, const float4 b) { r
 
 // Job: prepare(part, lane, t, e, h, slot, rows, wait): part 0, 1, 2 of a team's work for token row t (a warp each), which
 //      loads, calls wait() and, if that is true, writes to rows;
-//      DELTA, CHANNEL (a decay per key channel), NORM (o / rms(o) * w is what is stored);  store(t, h, c, value), eps.
+//      DELTA, CHANNEL (a decay per key channel), NORM (o / rms(o) * w is what is stored);  store(t, h, c, value), eps;
+//      AHEAD: the copies may begin while the kernel ahead in the stream still runs, which then must not write the states or
+//      the step's tables (that kernel is the projection of this one's rows; a second call on the same states would have to wait).
 // U: value channels of a warp, 8 or 16.
 template <class Job, int U>
 __global__ void __launch_bounds__(kStreamThreads, 1)
@@ -90,7 +92,7 @@ state_stream_kernel(const StateStream a, const Job job) {
 
   if (warp == 0) {
     if (lane == 0) {
-      // (the states and the step's tables were written before the kernel ahead of this one began)
+      if (!Job::AHEAD) pdl_wait();
       auto out = [&](int n) {   // the state of item n, once it has been computed
         const int s = n % a.stages;
         if (!mbar_wait(done0 + 8 * s, (n / a.stages) & 1)) {
@@ -234,7 +236,7 @@ static inline bool state_stream_fits(int dk, int dv, const void* state) {
 }
 
 template <class Job>
-static int state_stream_launch(bool early, StateStream a, const Job& job, cudaStream_t stream) {
+static int state_stream_launch(StateStream a, const Job& job, cudaStream_t stream) {
   const int bytes = a.dk * a.dv * 4;
   a.stages = kStreamBytes / bytes < kStreamStages ? kStreamBytes / bytes : kStreamStages;
   const long long items = (long long)a.n_entries * a.H;
@@ -245,7 +247,7 @@ static int state_stream_launch(bool early, StateStream a, const Job& job, cudaSt
   const auto kernel = wide ? state_stream_kernel<Job, 16> : state_stream_kernel<Job, 8>;
   const int rc = ccb_allow_smem(kernel, kStreamBytes, done[wide]);
   if (rc != 0) return rc;
-  ccb_launch_ex(early, kernel, dim3(grid), dim3(kStreamThreads), (size_t)a.stages * bytes, stream, a, job);
+  ccb_launch_ex(true, kernel, dim3(grid), dim3(kStreamThreads), (size_t)a.stages * bytes, stream, a, job);
   return ccb_launch_status();
 }
 

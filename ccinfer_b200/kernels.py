@@ -645,7 +645,8 @@ def delta_recurrence(qn, kn, vv, gg, bb, state, out, cu_q, state_slot, n_entries
                      dv: int, single: bool = False, status=None) -> None:
     """The gated delta rule over each request's tokens of the step, from and into ``state``
     [slots, H, dv, dk] (float); out float [T, H, dv].  ``single`` (here and in the recurrences below): every entry brings
-    one token, so that many of them may go through the stream of states (``csrc/state_stream.cuh``)."""
+    one token, so that many of them may go through the stream of states (``csrc/state_stream.cuh``; in order with whatever is ahead
+    in the stream, as every kernel but ``delta_head_step``)."""
     _cuda(qn, kn, vv, gg, bb, state, out, cu_q, state_slot)
     assert state.dtype == torch.float32 and state.shape[1:] == (H, dv, dk) and out.dtype == torch.float32
     _check(lib().ccb_delta_recurrence(_p(qn), _p(kn), _p(vv), _p(gg), _p(bb), _p(state), _p(out), _p(cu_q),
@@ -765,7 +766,8 @@ def delta_head_step(rule: HeadDelta, proj, ring, state, w, eps: float, positions
                     status=None) -> None:
     """A step's first ``n_entries`` entries, one token each, through the whole mixer between its projections: y [T, H dv]
     = o / rms(o) * w * silu(gate); the convolution's ``ring`` [slots, taps, channels] and ``state`` float [slots, H, dv, dk]
-    move on."""
+    move on.  Under programmatic launches ``state``, ``state_slot``, ``cu_q`` and ``positions`` are read while the kernel ahead in the
+    stream still runs: that one, ``proj``'s projection as a rule, must not write them (a second call on the same states, say)."""
     G, H, dk, dv = rule.sizes
     rule.check(proj, ring)
     _cuda(state, w, positions, cu_q, state_slot)

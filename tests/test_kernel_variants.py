@@ -1072,3 +1072,46 @@ def test_grouped_products_of_long_walks(N, sms, K, mode, monkeypatch):
             ref = torch.nn.functional.silu(gate) * up * rw
             slack = (1.1 * sg * up.abs() + gate.abs() * su + sg * su) * rw + 2.0 ** -20 * ref.abs()   # (silu's slope is below 1.1)
         assert ((got - ref).abs() <= 2.0 ** -8 * ref.abs() + slack + 1e-30).all(), i
+
+
+@pytest.mark.parametrize("pdl", [1, 2])
+@pytest.mark.parametrize("kind", ["delta", "linear", "state space"])
+@pytest.mark.parametrize("E,H,dk,dv", [(48, 16, 128, 128), (160, 2, 68, 64), (150, 1, 128, 128)])
+def test_tokens_in_a_row_on_the_same_states(kind, pdl, E, H, dk, dv):
+    """Calls directly behind one another, each with the states that the last one left, with early launches: against float64 as in
+    test_single_tokens_of_many_requests_stream_their_states, whose bound a token of each of four calls adds once."""
+    k, g = _k(), _gen(E + H + dk + dv + pdl)
+    n = 4
+
+    def rnd(*shape):
+        return torch.randn(shape, generator=g, device="cuda")
+
+    q, kk = (torch.nn.functional.normalize(rnd(n, E, H, dk), dim=-1) for _ in range(2))
+    v, beta = rnd(n, E, H, dv), torch.rand((n, E, H), generator=g, device="cuda")
+    decay = 0.5 + 0.5 * torch.rand((n, E, H) if kind == "state space" else (n, E, H, dk), generator=g, device="cuda")
+    state, out = rnd(E, H, dv, dk), torch.full((n, E, H, dv), float("nan"), device="cuda")
+    before = state.double()
+    args = (torch.arange(E + 1, dtype=torch.int32, device="cuda"), torch.arange(E, dtype=torch.int32, device="cuda").flip(0), E)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    was = k._pdl
+    k.set_pdl(pdl)
+    try:
+        for i in range(n):
+            if kind == "delta":
+                k.delta_recurrence(q[i], kk[i], v[i], decay[i], beta[i], state, out[i], *args, H, H, dk, dv, single=True, status=status)
+            elif kind == "linear":
+                k.gated_linear_recurrence(q[i], kk[i], v[i], decay[i], state, out[i], *args, H, dk, dv, single=True, status=status)
+            else:
+                k.ssm_recurrence(q[i], kk[i], v[i], decay[i], beta[i], state, out[i], *args, H, H, dk, dv, single=True, status=status)
+        torch.cuda.synchronize()
+    finally:
+        k.set_pdl(was or 0)
+    want, after = out.double(), before.clone()
+    for e in range(E):
+        put = v[:, e].double() * (beta[:, e, :, None].double() if kind == "state space" else 1)
+        want[:, e], after[E - 1 - e] = _recurrence64(
+            q[:, e].double(), kk[:, e].double(), put, (decay[:, e, :, None] if kind == "state space" else decay[:, e]).double(),
+            beta[:, e].double() if kind == "delta" else None, before[E - 1 - e])
+    assert int(status) == 0
+    assert (out.double() - want).abs().max() <= n * 2.0 ** -20 * want.abs().max()
+    assert (state.double() - after).abs().max() <= n * 2.0 ** -20 * after.abs().max()

@@ -28,8 +28,9 @@ namespace {
 
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + expf(-x)); }
 __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log1pf(expf(x)); }
-// The sigmoid in steps of many rows: the accurate form in 32 bits; where inputs and results of the layer are bfloat16 anyway,
-// the fast exponential and division (a few units of the last place of a float), an eighth of the instructions.
+// The gate's sigmoid in the norm of many rows: the accurate form in 32 bits; where the result is rounded to bfloat16, the fast
+// exponential and division (some units of the last place of a float), an eighth of the instructions.  Rows that stay float, as
+// those of the recurrences, have the accurate one.
 template <typename T> __device__ __forceinline__ float silu_of(float x) { return x * sigmoid_f(x); }
 template <> __device__ __forceinline__ float silu_of<__nv_bfloat16>(float x) { return __fdividef(x, 1.f + __expf(-x)); }
 template <typename T> __device__ __forceinline__ float sigmoid_of(float x) { return sigmoid_f(x); }
@@ -209,7 +210,8 @@ delta_prepare_vec_kernel(const T* __restrict__ proj, int ld, int oq, int ok, int
 
 // The same with four neighbouring rows a warp as well: the taps' weights are loaded once for all of them, a row once for all
 // the taps it meets, and all loads are in flight together.  dk, dv <= 128, TAPS taps.  A warp a row set what it issued by
-// its loads: 140 us for 2,048 tokens of 32 heads of 128 with four taps, 87 us with the accurate sigmoid, 77 so.
+// its loads: 140 us for 2,048 tokens of 32 heads of 128 with four taps, 87 us so (with the fast exponential
+// 77, but its rows go into a float memory).
 constexpr int kPrepRun = 4;
 
 template <typename T> struct Raw4;   // four neighbouring elements as they are stored
@@ -305,7 +307,8 @@ delta_prepare_run_kernel(const T* __restrict__ proj, int ld, int oq, int ok, int
       acc[2] += cw[j].z * win[j].z;
       acc[3] += cw[j].w * win[j].w;
     }
-    const float4 y = make_float4(silu_of<T>(acc[0]), silu_of<T>(acc[1]), silu_of<T>(acc[2]), silu_of<T>(acc[3]));
+    const float4 y = make_float4(acc[0] * sigmoid_f(acc[0]), acc[1] * sigmoid_f(acc[1]), acc[2] * sigmoid_f(acc[2]),
+                                 acc[3] * sigmoid_f(acc[3]));
     float f = 1.f;
     if (!is_v)   // (zeros beyond the head's channels)
       f = (is_q ? q_mult : 1.0f) / sqrtf(warp_sum((y.x * y.x + y.y * y.y) + (y.z * y.z + y.w * y.w)) + unit_eps);

@@ -39,8 +39,9 @@ struct SsmChunkRows {
 };
 
 __device__ __forceinline__ float sigmoid_acc(float x) { return 1.f / (1.f + expf(-x)); }
-// x sigmoid(x) in steps of many rows: the accurate form in 32 bits; where inputs and results of the layer are bfloat16 anyway,
-// the fast exponential and division (a few units of the last place of a float), an eighth of the instructions.
+// The gate in the norm of many rows: the accurate form in 32 bits; where the result is rounded to bfloat16, the fast exponential
+// and division (some units of the last place of a float), an eighth of the instructions.  Rows that stay float, as those of
+// the recurrence, have the accurate one.
 template <typename T> __device__ __forceinline__ float silu_of(float x) { return x * sigmoid_acc(x); }
 template <> __device__ __forceinline__ float silu_of<__nv_bfloat16>(float x) { return __fdividef(x, 1.f + __expf(-x)); }
 template <typename T> __device__ __forceinline__ float4 silu4_of(float4 x) {
@@ -220,7 +221,7 @@ __global__ void ssm_prepare_vec_kernel(const T* __restrict__ proj, int ld, int o
 // The same for steps of many rows: a thread takes its four channels (or its head) through kSsmRun neighbouring rows.  The taps'
 // weights are loaded once for all of them, a row once for all the taps it meets, all loads are in flight together, and no
 // thread divides to find its place.  TAPS taps.  2,048 rows of 10,240 channels with four taps, 150 MB: 90 us a row a
-// thread, 60 us with the accurate sigmoid, 46 so.
+// thread, 60 us so (with the fast exponential 46, but its rows go into a float memory).
 constexpr int kSsmRun = 4;
 // from here on, rows times (groups of four channels and heads): before that a row a thread has more loads under way (10,240 channels
 // and 128 heads, with 20 us of launch, a row / four rows a thread: 128 rows 28.5 / 29.9 us, 256 34.5 / 34.6, 512 45 / 38)
@@ -289,7 +290,8 @@ ssm_prepare_run_kernel(const T* __restrict__ proj, int ld, int ox, int odt, cons
         acc.z = fmaf(cw[j].z, win[j].z, acc.z);
         acc.w = fmaf(cw[j].w, win[j].w, acc.w);
       }
-      v = silu4_of<T>(acc);
+      v = make_float4(acc.x * sigmoid_acc(acc.x), acc.y * sigmoid_acc(acc.y), acc.z * sigmoid_acc(acc.z),
+                      acc.w * sigmoid_acc(acc.w));
       if (shift_single && TAPS > 1 && slot >= 0 && s_single[r]) {   // (as in the kernel above)
         V* st = reinterpret_cast<V*>(state_rw + (size_t)slot * (TAPS - 1) * C + c);
         for (int k = 0; k + 1 < TAPS - 1; ++k) st[(size_t)k * C4] = st[(size_t)(k + 1) * C4];

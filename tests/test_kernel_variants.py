@@ -1115,3 +1115,33 @@ def test_tokens_in_a_row_on_the_same_states(kind, pdl, E, H, dk, dv):
     assert int(status) == 0
     assert (out.double() - want).abs().max() <= n * 2.0 ** -20 * want.abs().max()
     assert (state.double() - after).abs().max() <= n * 2.0 ** -20 * after.abs().max()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("layer", ["delta", "state space"])
+def test_float_rows_of_many_tokens_have_float_activations(layer, dtype):
+    """x sigmoid(x) of an input that is exact (one tap of weight one), as rows that go into a float memory: an exponential right to
+    one unit of the last place, a sum, a division and a product right to half of one, so to 2.5 together; over inputs of both signs."""
+    k, g = _k(), _gen(5)
+    T, H, d = 16384, 4, 64
+
+    def dev(x):
+        return torch.tensor(x, dtype=torch.int32, device="cuda")
+
+    x = (60 * torch.rand((T, 3 * H * d + H), generator=g, device="cuda") - 30).to(dtype)
+    entry, cu, slots = torch.zeros(T, dtype=torch.int32, device="cuda"), dev([0, T]), dev([0])
+    heads = torch.zeros(H, device="cuda")
+    q, kk, v = (torch.full((T, H, d), float("nan"), device="cuda") for _ in range(3))
+    if layer == "delta":
+        gg, bb = torch.empty((T, H, d), device="cuda"), torch.empty((T, H), device="cuda")
+        k.delta_prepare(x, (0, H * d, 2 * H * d, 3 * H * d), x[:, :H * d], torch.ones((1, 3 * H * d), device="cuda"), 1,
+                        torch.zeros((1, 0, 3 * H * d), dtype=dtype, device="cuda"), heads, torch.zeros(H * d, device="cuda"), entry, cu, slots,
+                        q, kk, v, gg, bb, H, H, d, d, 1.0, 1e-6)
+        want = x[:, 2 * H * d:3 * H * d]
+    else:
+        dts, decay = (torch.empty((T, H), device="cuda") for _ in range(2))
+        k.ssm_prepare(x, 0, 3 * H * d, torch.ones((1, 3 * H * d), device="cuda"), torch.zeros(3 * H * d, device="cuda"), 1, None, heads, heads,
+                      entry, cu, slots, v, kk, q, dts, decay, H, d, H, d, shift_single=True, chunk=None)
+        want = x[:, :H * d]
+    want = torch.nn.functional.silu(want.double()).view(T, H, d)
+    assert ((v.double() - want).abs() <= 2.5 * 2.0 ** -23 * want.abs()).all()

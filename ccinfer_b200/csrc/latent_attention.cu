@@ -626,8 +626,14 @@ __device__ __forceinline__ float ex2(float x) {
 }
 
 // Pieces of a token's keys: no more than the launch has, of at least kSingleTiles tiles each (tokens of few keys are finished by
-// one block, and the merge passes them over; with four the pieces of 3,000 keys take 12.3 us in place of 8.8).
+// one block, and the merge passes them over; with four the pieces of 3,000 keys take 12.3 us in place of 8.8, with one the layer of
+// 4 requests of 1,500 to 3,000 keys 42.3 in place of 41.0).
 constexpr int kSingleTiles = 2;
+// Weights are rounded to bfloat16 beside the largest of those that they are taken relative to, which itself is exact.  In pieces of
+// so few tiles every tile takes its own (unless that is so far below the last one's that sums might leave a float's range, in
+// powers of two), for which its sums so far are scaled; relative to the larger of the two the error against 64 bits is a little larger than
+// with a piece for every tile (16 heads, 500 keys: 1.969e-3, 1.941e-3 so).
+constexpr float kSingleFall = 20.f;
 __device__ __forceinline__ int single_pieces(int p, int window, int num_splits) {
   const int n_tiles = p / kSingleKeys - max(0, p - window + 1) / kSingleKeys + 1;
   return min(num_splits, (n_tiles + kSingleTiles - 1) / kSingleTiles);
@@ -703,7 +709,7 @@ latent_single_kernel(const __grid_constant__ CUtensorMap tm_rows, const float* _
   }
   const int rt = warp / kSingleWarps, w = warp % kSingleWarps;
   const int h0 = (blockIdx.x * MTL + rt) * 16;
-  const float scale2 = scale * kLog2e;
+  const float scale2 = scale * kLog2e, fall = per <= kSingleTiles ? kSingleFall : 0.f;
   const bool ok[2] = {h0 + gid < H, h0 + gid + 8 < H};   // this lane's heads
   // the queries' coordinates of this warp, as the A operand
   const int n_pairs = R >> 4;
@@ -807,7 +813,7 @@ latent_single_kernel(const __grid_constant__ CUtensorMap tm_rows, const float* _
         }
       v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
       v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 2));
-      const float most = fmaxf(m[hh], v), mn = most == -CUDART_INF_F ? 0.f : most;   // (no key with a weight so far: all weights zero)
+      const float most = fmaxf(m[hh] - fall, v), mn = most == -CUDART_INF_F ? 0.f : most;   // (no key with a weight so far: all weights zero)
       corr[hh] = ex2(m[hh] - mn);
       m[hh] = most;
       float ps = 0.f;

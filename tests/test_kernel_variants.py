@@ -1145,3 +1145,40 @@ def test_float_rows_of_many_tokens_have_float_activations(layer, dtype):
         want = x[:, :H * d]
     want = torch.nn.functional.silu(want.double()).view(T, H, d)
     assert ((v.double() - want).abs() <= 2.5 * 2.0 ** -23 * want.abs()).all()
+
+
+@pytest.mark.parametrize("n", [41, 100, 500, 1700])
+def test_latent_pieces_of_single_tokens_round_beside_their_own_largest_weight(n):
+    """Where a launch has a piece for each tile of 32 keys, or for every second one, weights are rounded beside their piece's
+    largest, and the error against float64 is that of these roundings (and of the result's) made in float64: but for the few weights so near
+    the middle of two that a float sum's order decides."""
+    k, g = _k(), _gen(n)
+    E, H, R, W, page, splits = 8, 16, 512, 576, 16, 64
+    pages, scale = -(-n // page), 576 ** -0.5
+    cache = torch.randn((E * pages, page, W), generator=g, device="cuda").to(torch.bfloat16)
+    qa, sink = torch.randn((E, H, W), generator=g, device="cuda").to(torch.bfloat16).float(), torch.randn(H, generator=g, device="cuda")
+    out = torch.empty((E, H, R), dtype=torch.bfloat16, device="cuda")
+    acc, ml = (torch.empty(E * H * splits * m, device="cuda") for m in (R, 2))
+
+    def dev(x):
+        return torch.tensor(x, dtype=torch.int32, device="cuda")
+
+    status = dev([0])
+    k.latent_attention_mma(qa, cache, sink, None, out, dev(list(range(E + 1))), dev([n - 1] * E), dev(list(range(E))),
+                           torch.arange(E * pages, dtype=torch.int32, device="cuda").view(E, pages), 0, E, 1, page, 1 << 30, scale, splits, acc, ml,
+                           status)
+    rows = cache.view(E, pages * page, W)[:, :n].double()
+    s = torch.einsum("ehw,enw->ehn", qa.double(), rows) * scale
+    want = torch.einsum("ehn,enr->ehr", torch.softmax(torch.cat([s, sink.double()[None, :, None].expand(E, H, 1)], -1), -1)[..., :-1], rows[..., :R])
+    per = 32 * -(-(-(-n // 32)) // splits)
+    total, weight = torch.zeros_like(want), torch.exp(sink.double())[None, :, None].expand(E, H, 1)
+    for a in range(0, n, per):
+        top = s[..., a:a + per].amax(-1, keepdim=True)
+        if a == 0:
+            top = torch.maximum(top, sink.double()[None, :, None])   # (the first piece has the sink)
+        p = torch.exp(s[..., a:a + per] - top)
+        weight = weight + torch.exp(top) * p.sum(-1, keepdim=True)
+        total = total + torch.exp(top) * torch.einsum("ehn,enr->ehr", p.bfloat16().double(), rows[:, a:a + per, :R])
+    rounded = (total / weight).bfloat16().double()
+    assert int(status) == 0
+    assert (out.double() - want).norm() <= 1.004 * (rounded - want).norm()

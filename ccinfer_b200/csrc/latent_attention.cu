@@ -684,7 +684,7 @@ latent_single_kernel(const __grid_constant__ CUtensorMap tm_rows, const float* _
       int page = lp < bt_stride ? bt[lp] : -1;
       if (page < 0 || page >= num_pages) {
         if (j + box_rows > j_lo) set_status(status, CCB_ST_BAD_PAGE);   // (a page before the window may be gone)
-        else page = bt[p / page_size];
+        else page = p / page_size < bt_stride ? bt[p / page_size] : -1;
       }
       if (page < 0 || page >= num_pages) page = 0;
       return page * page_size + (j - lp * page_size);

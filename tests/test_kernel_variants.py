@@ -1182,3 +1182,28 @@ def test_latent_pieces_of_single_tokens_round_beside_their_own_largest_weight(n)
     rounded = (total / weight).bfloat16().double()
     assert int(status) == 0
     assert (out.double() - want).norm() <= 1.004 * (rounded - want).norm()
+
+
+def test_latent_position_beyond_the_table_of_pages():
+    """The last request's position lies past its table's columns, and its window begins inside of them: the status says so, no
+    page is looked up beyond the table, and the other requests have their results."""
+    k, g = _k(), _gen(3)
+    E, H, R, W, page, cols, window = 3, 16, 512, 576, 16, 8, 40
+    cache = torch.randn((E * cols, page, W), generator=g, device="cuda").to(torch.bfloat16)
+    qa, sink = torch.randn((E, H, W), generator=g, device="cuda").to(torch.bfloat16).float(), torch.randn(H, generator=g, device="cuda")
+
+    def dev(x):
+        return torch.tensor(x, dtype=torch.int32, device="cuda")
+
+    table = torch.arange(E * cols, dtype=torch.int32).view(E, cols)
+    table[:, :5] = -1   # (pages before the windows are gone)
+    status, outs = dev([0]), []
+    for last in (127, 160):   # (the last one's window: rows 88 to 127; 121 to 160, of which the table has 121 to 127)
+        if last == 160:
+            table[2, :7] = -1   # (so rows 96 to 111 of the walk's first tile lie before the window, and their page is gone)
+        out = torch.zeros((E, H, R), dtype=torch.bfloat16, device="cuda")
+        k.latent_attention_mma(qa, cache, sink, None, out, dev(list(range(E + 1))), dev([127, 120, last]), dev(list(range(E))), table.cuda(), 0, E,
+                               1, page, window, 0.05, status=status)
+        outs.append(out)
+        assert int(status) == (0 if last == 127 else 4)
+    assert torch.equal(outs[0][:2], outs[1][:2]) and torch.isfinite(outs[1].float()).all()

@@ -22,7 +22,7 @@
 // registers alone reach 65 TFLOP/s, with reads of shared memory beside them.  us, tiles of 32, 64 or 128 rows with 8 x 8 places
 // a thread, one block an SM / so: 17 x 16,384 x 2,048 77 / 60, 64 x 4,096 x 2,048 35 / 35, 100 x 16,384 x 2,048 267 / 187,
 // 210 x 2,048 x 8,192 307 / 174, 210 x 16,384 x 2,048 524 / 349 (40 TFLOP/s), 300 x 16,384 x 2,048 511 / 501, 2,048 x 4,096 x
-// 4,096 1,593 / 1,452 (47).  Sums of even and of odd k side by side (no element stored by itself, eight columns a thread) took
+// 4,096 1,593 / 1,389 (49).  Sums of even and of odd k side by side (no element stored by itself, eight columns a thread) took
 // 419 us for 210 x 16,384 x 2,048.
 #include "cluster_common.cuh"
 #include "mma_common.cuh"
@@ -398,10 +398,16 @@ template <class Sh> int tiles_go(const F32Product& p, int vec_a, int vec_w, bool
 }
 
 // The rows of a tile and whether a cluster shares it, by the cycles that the busiest SM would need: its blocks go round by
-// round, a k of a block costs an SM its multiply-adds or its reads and stores of shared memory, whichever is more, and a
-// round no less than one thread's chain of instructions; a block multiplies some 16 k more than it has, and not every SM can
-// be part of a cluster.  The constants are fitted to 66 shapes of 17 to 2,048 rows, each timed with every tile: what is
-// chosen takes 3 per cent longer than the best on average (5 and 9 of 66 more than that beyond 5 and 10 per cent).
+// round, a k of a block costs an SM its multiply-adds or its reads of shared memory, whichever is more, and stores beside them;
+// a round is no less than one thread's chain of instructions, under which only a tenth of what other blocks do hides; a block
+// multiplies some 10 k more than it has.  How many clusters of eight find room with so many blocks on an SM is kRoom (what
+// cudaOccupancyMaxActiveClusters says here: the 16th gives some SM a second block, and takes as long as 33).  The constants are
+// fitted to 390 shapes of 17 to 2,048 rows, each timed with every tile: what is chosen takes 1 per cent longer than the best on
+// average (32 and 8 of 390 more than 5 and 10).  With 136 SMs for clusters and one block's work hidden under another's chain, 37 of
+// 353 other shapes took more than 2 per cent longer than with tiles of 32, 64 and 128 rows alone, 29 more than 5; now 10 and 3 (us, such tiles /
+// then / now: 55 x 655 x 1,086 twice 15.6 / 23.0 / 15.4, 59 x 1,536 x 12,224 101 / 136 / 106, 285 x 365 x 12,978 119 / 159 / 134; all
+// 353 on average 1 / 0.70 / 0.67).
+constexpr int kRoom[] = {0, 15, 33, 48, 71, 86};
 struct TileChoice {
   int family, tm;   // family 0: 16 columns a thread, 4 x 1 warps; 1: 8, 2 x 2; 2: 8, 1 x 2
   bool cluster;
@@ -411,17 +417,20 @@ TileChoice choose_tiles(int M, int N, int K, int batch) {
   double least = 0;
   for (int family = 0; family < 3; ++family) {
     const int tn = family == 0 ? 16 : 8, wr = 4 >> family, warps = family == 2 ? 2 : 4, blocks = family == 0 ? 2 : family == 1 ? 3 : 5;
-    for (int tm = kTileMaxRows; tm >= kTileMinRows; --tm) {
+    for (int tm = kTileMaxRows; tm >= (family == 0 ? kTileMinRows + 1 : kTileMinRows); --tm) {   // (three rows of sixteen columns: never the best)
       const int rows = 4 * wr * tm;
-      const double adds = warps * tm * tn / 4., moves = warps * (0.8 * tm + tn) + (rows + kTileN) / 20.;
-      const double cost = adds > moves ? adds : moves, chain = 1.2 * tm * tn + 80;
+      const double adds = warps * tm * tn / 4., reads = 1.4 * warps * tn, cost = (adds > reads ? adds : reads) + 11, chain = 1.2 * tm * tn + 33;
+      const auto round = [&](int n) {   // of n blocks an SM
+        const double hidden = chain + .9 * (n - 1) * cost;
+        return n == 0 ? 0. : n * cost > hidden ? n * cost : hidden;
+      };
       const long long tiles = (long long)((N + kTileN - 1) / kTileN) * ((M + rows - 1) / rows) * batch;
-      for (int cluster = 0; cluster < 2; ++cluster) {
-        const long long units = cluster ? tiles * kSegments : tiles, sms = cluster ? 136 : 148;
-        const long long full = units / (sms * blocks), rest = (units % (sms * blocks) + sms - 1) / sms;
-        double cycles = full * (blocks * cost > chain ? blocks * cost : chain);
-        if (rest) cycles += rest * cost > chain ? rest * cost : chain;
-        cycles = cycles * ((cluster ? segment_of(K) : K) + 16) + (cluster ? 2000 : 0);
+      for (int cluster = 0; cluster < 2; ++cluster) {   // (units: blocks, or clusters of eight)
+        const int full = cluster ? kRoom[blocks] : 148 * blocks, left = (int)(tiles % full);
+        int rest = cluster ? 0 : (left + 147) / 148;
+        while (cluster && kRoom[rest] < left) ++rest;
+        const double k = (cluster ? segment_of(K) : K) + 10;
+        const double cycles = (tiles / full * round(blocks) + round(rest)) * k + (cluster ? 2400 : 0);
         if (least == 0 || cycles < least) least = cycles, best = {family, tm, cluster != 0};
       }
     }
@@ -430,7 +439,8 @@ TileChoice choose_tiles(int M, int N, int K, int batch) {
 }
 
 template <int TM> int tiles_of(const F32Product& p, int vec_a, int vec_w, const TileChoice& t, cudaStream_t stream) {
-  if (t.family == 0) return tiles_go<TileShape<TM, 16, 4, 1>>(p, vec_a, vec_w, t.cluster, stream);
+  if constexpr (TM > kTileMinRows)
+    if (t.family == 0) return tiles_go<TileShape<TM, 16, 4, 1>>(p, vec_a, vec_w, t.cluster, stream);
   if (t.family == 1) return tiles_go<TileShape<TM, 8, 2, 2>>(p, vec_a, vec_w, t.cluster, stream);
   return tiles_go<TileShape<TM, 8, 1, 2>>(p, vec_a, vec_w, t.cluster, stream);
 }

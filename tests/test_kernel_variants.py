@@ -68,6 +68,32 @@ def test_float_product_of_every_tile_height(M, N, K):
         assert torch.equal(c1, c[r:r + 16])
 
 
+# a shape for each height of a tile, columns a thread, warps and, in lines of their own, whole or shared by a cluster that the rule takes
+@pytest.mark.parametrize("M,N,K,batch", [
+    (2132, 421, 33, 1), (3337, 285, 33, 1), (3628, 803, 33, 1), (1732, 2005, 33, 1), (338, 9840, 35, 1),
+    (442, 144, 108, 1), (525, 150, 123, 1), (1514, 132, 197, 1), (1576, 153, 219, 1), (1793, 151, 207, 1),
+    (31, 138, 33, 1), (1878, 132, 33, 1), (2447, 134, 35, 1), (3083, 137, 35, 1), (3627, 134, 34, 1), (3311, 525, 34, 1),
+    (26, 131, 72, 1), (176, 132, 79, 1), (230, 136, 84, 1), (281, 138, 105, 1), (361, 132, 102, 1), (977, 133, 157, 1),
+    (57, 19213, 35, 1), (67, 29287, 33, 1), (82, 31452, 35, 1), (30, 61839, 34, 1),
+    (17, 145, 104, 8), (59, 996, 98, 1), (67, 978, 118, 1), (81, 2106, 187, 1), (193, 1225, 192, 1), (126, 2091, 216, 1)])
+def test_float_product_of_every_tile(M, N, K, batch):
+    """As above: a segment is 32 k or more, a chain of as many roundings, and eight sums are added."""
+    g = _gen(M + 7 * N + 13 * K)
+    a, w = torch.randn((batch, M, K), generator=g, device="cuda"), torch.randn((batch, N, K), generator=g, device="cuda")
+    c = torch.full((batch, M, N), float("nan"), device="cuda")
+    k = _k()
+    if batch > 1:
+        k.gemm_f32_batched(c, a, w)
+    else:
+        k.gemm_f32(c[0], a[0], w[0])
+    ref, size = a.double() @ w.double().mT, a.double().abs() @ w.double().abs().mT
+    assert ((c.double() - ref).abs() <= (-(-K // 256) * 32 + 8) * 2.0 ** -24 * size).all()
+    for r in range(0, M, 16):
+        c1 = torch.empty((min(16, M - r), N), device="cuda")
+        k.gemm_f32(c1, a[0, r:r + 16], w[0])
+        assert torch.equal(c1, c[0, r:r + 16])
+
+
 def _recurrence64(q, k, v, g, beta, S):
     """Token by token in float64: q, k [n, H, dk], v [n, H, dv], g [n, H, dk or 1], beta [n, H] or None, S [H, dv, dk]."""
     out = torch.empty_like(v)

@@ -848,12 +848,14 @@ CCB_API int ccb_ssm_recurrence(const float* qn, const float* kn, const float* vv
 }
 
 // rows x heads from which on a warp takes four; before, one head a warp has more loads under way (heads of 128, a head / four a
-// warp, us alone: 4,800 3.65 / 4.11, 9,600 5.05 / 4.68, 38,400 13.9 / 10.6, 65,536 22.3 / 15.8)
-constexpr int kNormRunUnits = 148 * 56;
+// warp, us alone: 4,800 3.65 / 4.11, 9,600 5.05 / 4.68, 38,400 13.9 / 10.6, 65,536 22.3 / 15.8; of 32 bits, with the accurate
+// sigmoid, 8,288 4.19 / 4.60, 9,600 4.91 / 5.29, 12,000 5.34 / 5.31, 14,000 5.89 / 5.33, 20,000 7.98 / 8.07, 32,000 11.5 / 9.8)
+constexpr int kNormRunUnits = 148 * 56, kNormRunUnitsF32 = 148 * 80;
 template <typename T, bool SILU>
 static void launch_head_norm(bool vec, dim3 grid, void* y, const float* o, const void* gate, int ldg, const float* w,
                              int rows, int H, int dv, float eps, cudaStream_t stream) {
-  if (vec && dv <= 128 && rows * H >= kNormRunUnits)
+  constexpr int least = sizeof(T) == 4 ? kNormRunUnitsF32 : kNormRunUnits;
+  if (vec && dv <= 128 && rows * H >= least)
     ccb_launch(gated_head_rmsnorm_run_kernel<T, SILU>, dim3((rows * H + 8 * kNormRun - 1) / (8 * kNormRun)), dim3(256), 0, stream,
                (T*)y, o, (const T*)gate, ldg, w, rows * H, H, dv, eps);
   else if (vec)

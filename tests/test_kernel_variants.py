@@ -953,7 +953,7 @@ def test_latent_attention_of_single_tokens(H, R, r, page, window, splits):
 # rows x heads from which on a warp takes four heads: left-over heads, lanes without channels, a gate inside wider rows
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("silu", [False, True])
-@pytest.mark.parametrize("T,H,dv", [(2763, 3, 128), (8289, 1, 4), (830, 10, 100), (8287, 1, 64)])
+@pytest.mark.parametrize("T,H,dv", [(2763, 3, 128), (8289, 1, 4), (830, 10, 100), (8287, 1, 64), (3947, 3, 128), (11841, 1, 4)])
 def test_gated_head_norm_of_many_rows(T, H, dv, silu, dtype):
     """Against float64: the norm, a weight and the gate, rounded once."""
     k, g = _k(), _gen(T + dv)

@@ -52,8 +52,8 @@ constexpr float kSteepLog2 = 55.f;   // (2^110 times 128 products stays in a flo
 // Gated linear attention's rows as the projections left them, in place of q, k, v and g: q times q_mult, k and v; the decay is
 // sigmoid(a + bias)^(1 / tau).  Measured on B200, 1,537 tokens of three requests, 16 heads of 128, a layer: 173 -> 162 us (the rows'
 // kernel of 18 us gone, preparation 33 -> 40, walk 40 -> 43).
-// The delta rule takes only its decays so, exp(-exp(A_log) softplus(a + bias)): at 2,048 tokens of 32 heads the rows' kernel 76 -> 60 us,
-// the preparation 7 more, a layer 605 -> 596.  Its q, k and v too, convolved by the preparation: 270 without a rows' kernel, 617.
+// The delta rule takes only its decays so, exp(-exp(A_log) softplus(a + bias)): at 2,048 tokens of 32 heads the rows' kernel 87 -> 72 us,
+// the preparation 7 more (a layer 605 -> 596, both with a faster activation in the rows' kernel).  Its q, k and v too, convolved by the preparation: 270 without a rows' kernel, 617.
 struct RawRows {
   const __nv_bfloat16 *q, *k, *v, *a;   // q, k [T, ld] with head h at column h DK, v [T, ld] at h dv, a [T, lda] at h DK
   int ld, lda;

@@ -57,7 +57,8 @@ __device__ __forceinline__ float decay_of(float z, float inv_tau) {
 }
 
 // A block a row, its threads the channels: with all rows' channels in one line, a thread's division of a 64-bit index to find its row
-// was much of what it did (1,537 tokens of 16 heads of 128: 20 us so, 18 now).
+// was much of what it did (1,537 rows of 16 heads of 128: 20 us so, 18 now; rows of that many are those of chunks that cannot read
+// the projections' rows themselves).
 template <typename T>
 __global__ void __launch_bounds__(256)
 gla_prepare_vec_kernel(const T* __restrict__ proj, int ld, int oq, int ok, int ov, const T* __restrict__ a, int lda,

@@ -7,7 +7,8 @@
 // weight rows and half of the tokens), one cluster per pair of SMs walks over (token tile, 256 weight rows), weight rows
 // fastest, so that the clusters running at one time share a few tokens in L2 and read every weight once.  The ring of
 // stages (64 k) runs on from tile to tile, and so does tensor memory: its 512 columns are a ring of sixteen slots of 32, a tile
-// takes as many as it has columns, and the next one's products begin as soon as the slots that it needs have been read.  (Two
+// takes as many as it has columns, and the next one's products begin as soon as the slots that it needs have been read
+// (`slot_ring.h`).  (Two
 // accumulators of 256 columns, both of which a tile of more tokens took, left its whole epilogue without products beside it.)
 // Weights and tokens have a producer warp
 // each: one thread for both set the pace (one instruction more in its loop, a copy to L2 ahead of the ring, made 64 tokens
@@ -29,9 +30,10 @@
 // Every wait on an mbarrier is bounded as in gemm_tcgen05.cu.
 // Bound by the stream of weights up to some 130 rows an expert (32 of 4096 x 3072, 4 chosen, 128 tokens: 2.4 GB in 414 us, 5.9
 // TB/s), by that and the products together at 2,048 tokens (0.62 TFLOP in 580 us).  The whole part, 8 / 2,048 tokens: tiles of
-// 128 x 256 on one SM and 16 rows on mma.sync 413 / 1,161 us; this with two accumulators and four epilogue warps 284 / 956, with
-// eight 280 / 770, with the ring of slots 280 / 665 (width 2,048, 2,048 tokens: 357 / 285).  A warp's signal that a slot has been
-// read does not wait for its stores (with a releasing one, 1,100 tokens of width 2,048 took 127 us in the first product, 109 so).
+// 128 x 256 on one SM and 16 rows on mma.sync 413 / 1,161 us; this with two accumulators and eight epilogue warps 281 / 898, with the
+// ring of slots 279 / 779 (width 2,048: 125 / 377 and 121 / 318; 128 to 1,100 tokens the same within 2 per cent).  A warp's signal that
+// a slot has been read does not wait for its stores: what it orders is a read of tensor memory, which tcgen05.wait::ld and the fence
+// have ended (with a releasing one, 1,100 tokens of width 2,048 took 127 us in the first product, 109 so).
 #include "cluster_common.cuh"
 #include <cuda.h>
 #include <type_traits>
@@ -308,8 +310,7 @@ moe_grouped_tc_kernel(const __grid_constant__ TokenMaps tmX, const __grid_consta
         for (int x = 0; x < 2; ++x) {
           const size_t row = g0 + tok[x];
           const int left = n - tok[x];   // of the sixteen tokens
-          if (left <= 0) continue;   // (columns without tokens: the whole part of 8 tokens, two of 32 columns filled, 0.7 % slower than with
-                                     // two accumulators, so 0.9 % faster)
+          if (left <= 0) continue;   // (columns without tokens, of which a step of few has most)
           if (MODE == 1) {
             float* dst = (float*)Cout + row * ldc + col;
 #pragma unroll

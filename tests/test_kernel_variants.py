@@ -21,7 +21,7 @@ def _rel(got, ref):
     return float((got - ref).abs().max() / ref.abs().max().clamp_min(1e-30))
 
 
-# rows kernel: 1, 2, 3, 5, 9, 16 rows; tiles of 32, 64, 128 rows; with and without a cluster (K below and from 512); rows
+# rows kernel: 1, 2, 3, 5, 9, 16 rows; tiles from 17 rows on; K of less than a segment, of whole segments and with a remainder; rows
 # that start on no 16 bytes; more tiles than two rounds
 @pytest.mark.parametrize("M,N,K,pad,batch", [
     (1, 1, 1, 0, 1), (2, 15, 31, 0, 1), (3, 17, 256, 0, 2), (4, 33, 260, 1, 1), (5, 64, 2048, 0, 1), (8, 300, 1001, 3, 1),
@@ -50,7 +50,7 @@ def test_float_product_of_every_shape_is_one_order_of_sums(M, N, K, pad, batch):
         assert torch.equal(c1, c[0, M - n:])
 
 
-# every height of a tile, whole and with rows left over, whole tiles and shared ones
+# numbers of rows between those of the tiles' heights, at a few, some and many columns (every tile: the test below)
 @pytest.mark.parametrize("M", [20, 21, 23, 29, 31, 41, 47, 50, 57, 63, 77, 79, 90, 96, 101, 107, 112, 125, 140, 175, 223])
 @pytest.mark.parametrize("N,K", [(200, 1030), (3001, 96), (640, 2048)])
 def test_float_product_of_every_tile_height(M, N, K):
